@@ -486,7 +486,8 @@ int astro_thermal_node_load_drdd(astro_ctx *ctx, int32_t dvar, double time, doub
  * (Working/AStrO_solvers.f90:10-126), all panels in one persistent launch: a blocked band LDL^T
  * in FP64 with one thread-block cluster per panel, panels ordered along their longest extent.
  * The FP64 stiffness must be assembled (astro_el_soln_load) and the constraints scaled
- * (astro_scale_mpc).  cluster_size: CTAs per panel (1, 2, 4 or 8; 0 = 8). */
+ * (astro_scale_mpc).  cluster_size: CTAs per panel (1, 2, 4 or 8; 0 = chosen
+ * for the batch: 8, or 16 for a few wide panels factored with FP64 updates). */
 typedef struct astro_panels_info {
     int32_t num_panels;
     int32_t max_bandwidth;   /* largest lower bandwidth in DOF */

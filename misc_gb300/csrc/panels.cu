@@ -10,9 +10,9 @@
 //             lower bandwidth is about dpn * (short side + 2) DOF);
 //   storage   per panel the lower band in 32 x 32 FP64 tiles, column-major within a tile: tile
 //             (J, d) holds block row J + d of block column J, d = 0 .. bt (bt = ceil(bw / 32));
-//   factor    right-looking blocked LDL^T, one thread-block cluster per panel: every CTA of the
-//             cluster factors the diagonal tile in shared memory, the CTAs split the panel rows
-//             below it (L = A L_JJ^-T D^-1) and then the band's trailing tile updates
+//   factor    right-looking blocked LDL^T, one thread-block cluster per panel: the diagonal tile is
+//             factored in shared memory, the CTAs of the cluster split the panel rows below it
+//             (L = A L_JJ^-T D^-1) and then the band's trailing tile updates
 //             (A_IK -= L_IJ D_J L_KJ^T), with a cluster barrier after each of the two phases.
 //             Panels are assigned to clusters by longest-processing-time first on the host, so a
 //             cluster never waits on another (no spin-waits, no inter-cluster dependencies);
@@ -77,6 +77,7 @@ struct SolveItem {
 struct PanelPlan {
     int np = 0;
     int cs = 0, workers = 0;
+    int csAsked = 0;  // the cluster size the plan was asked for (0: plan_build's choice)
     int factored = 0, kVersion = -1, penVersion = -1;
     int maxBw = 0;
     long long bandDoubles = 0, xRows = 0;
@@ -251,26 +252,24 @@ __device__ void split_tile(const double *T, const double (*sL)[TB + 1], int v, u
     }
 }
 
-// Blocked band LDL^T, one cluster per panel (the cluster's panels listed in sched).  MODE 0: the
-// trailing updates in FP64; MODE 1 and 2: the tensor-core emulation described at the top of the
-// file, MODE 1 on mma.sync (16 x 8 blocks per warp), MODE 2 on tcgen05 (128 x 32 per MMA, the
-// accumulators in tensor memory), with the slices of each worker (cluster) in
-// slices + worker * sliceStride and their scales in sexp + worker * expStride.  Both emulations
-// sum every level exactly and combine the levels in the same order: identical results.
+// Blocked band LDL^T, one cluster per panel (the cluster's panels listed in sched), the trailing
+// updates by the tensor-core emulation described at the top of the file: MODE 1 on mma.sync
+// (16 x 8 blocks per warp), MODE 2 on tcgen05 (128 x 32 per MMA, the accumulators in tensor
+// memory), with the slices of each worker (cluster) in slices + worker * sliceStride and their
+// scales in sexp + worker * expStride.  Both emulations sum every level exactly and combine the
+// levels in the same order: identical results.  The FP64 updates are k_band_ldl64.
 template <int MODE>
 __global__ void __launch_bounds__(kThreads, MODE == 2 ? 1 : 2) k_band_ldl(const PanelMeta *__restrict__ meta, const int *__restrict__ sched,
                                                        const int *__restrict__ schedPtr, double *band, int *status,
                                                        uint16_t *slices, int *sexp, long long sliceStride,
                                                        int expStride) {
-    constexpr bool TC = MODE == 1 || MODE == 2;
     cg::cluster_group cl = cg::this_cluster();
     const int crank = (int)cl.block_rank(), cs = (int)cl.num_blocks();
     const int worker = blockIdx.x / cs;
-    uint16_t *wsl = TC ? slices + (size_t)worker * sliceStride : nullptr;
-    int *wex = TC ? sexp + (size_t)worker * expStride : nullptr;
+    uint16_t *wsl = slices + (size_t)worker * sliceStride;
+    int *wex = sexp + (size_t)worker * expStride;
     __shared__ double sL[TB][TB + 1];  // diagonal tile: L below the diagonal, D on it
     __shared__ double sDi[TB];         // D^-1
-    __shared__ double sA[TB][TB + 1], sB[TB][TB + 1];
     const int t = threadIdx.x;
     // MODE 2: tensor memory, the completion barrier of the MMAs and the operand staging
     extern __shared__ __align__(1024) uint16_t tcSmem[];
@@ -337,178 +336,117 @@ __global__ void __launch_bounds__(kThreads, MODE == 2 ? 1 : 2) k_band_ldl(const 
             if (crank == 0)
                 for (int e = t; e < TT; e += kThreads) __stcg(Td + e, sL[e % TB][e / TB]);
             const int nt = M.bt * (M.bt + 1) / 2;
-            if constexpr (TC) {
-                // B2. slices of the tiles below the diagonal (versions L D_J and L), one warp each
-                const int lane = t & 31, wg = crank * kGroups + (t >> 5);
-                for (int uu = wg; uu < 2 * M.bt; uu += cs * kGroups) {
-                    const int d = 1 + uu / 2, v = uu % 2;
-                    if (J + d >= M.nbc) continue;
-                    split_tile(band + tile_off(M, J, d), sL, v, wsl + (size_t)uu * kSlices * TT, wex + uu * TB, lane);
-                }
-                __threadfence();
-                cl.sync();
-                if constexpr (MODE == 2) {
-                    // C. trailing update on tcgen05: items (group gi of block rows d0 .. d0+3, block
-                    // column e <= d0 + 3), round-robin over the cluster; a CTA keeps its A operand
-                    // while consecutive items share the group
-                    uint16_t *sAop = tcSmem, *sBop = tcSmem + kSlices * kTcSliceA;
-                    const int ng = (M.bt + 3) / 4;
-                    int nItems = 0;
-                    for (int gi = 0; gi < ng; ++gi) nItems += min(4 * gi + 4, M.bt);
-                    int curG = -1, gi = 0, gBase = 0;  // item index of group gi's first item
-                    const int w = t >> 5;
-                    for (int u = crank; u < nItems; u += cs) {
-                        while (u >= gBase + min(4 * gi + 4, M.bt)) {
-                            gBase += min(4 * gi + 4, M.bt);
-                            ++gi;
+            // B2. slices of the tiles below the diagonal (versions L D_J and L), one warp each
+            const int lane = t & 31, wg = crank * kGroups + (t >> 5);
+            for (int uu = wg; uu < 2 * M.bt; uu += cs * kGroups) {
+                const int d = 1 + uu / 2, v = uu % 2;
+                if (J + d >= M.nbc) continue;
+                split_tile(band + tile_off(M, J, d), sL, v, wsl + (size_t)uu * kSlices * TT, wex + uu * TB, lane);
+            }
+            __threadfence();
+            cl.sync();
+            if constexpr (MODE == 2) {
+                // C. trailing update on tcgen05: items (group gi of block rows d0 .. d0+3, block
+                // column e <= d0 + 3), round-robin over the cluster; a CTA keeps its A operand
+                // while consecutive items share the group
+                uint16_t *sAop = tcSmem, *sBop = tcSmem + kSlices * kTcSliceA;
+                const int ng = (M.bt + 3) / 4;
+                int nItems = 0;
+                for (int gi = 0; gi < ng; ++gi) nItems += min(4 * gi + 4, M.bt);
+                int curG = -1, gi = 0, gBase = 0;  // item index of group gi's first item
+                const int w = t >> 5;
+                for (int u = crank; u < nItems; u += cs) {
+                    while (u >= gBase + min(4 * gi + 4, M.bt)) {
+                        gBase += min(4 * gi + 4, M.bt);
+                        ++gi;
+                    }
+                    const int d0 = 1 + 4 * gi, e = 1 + (u - gBase);
+                    if (J + e >= M.nbc || tcFailed) continue;
+                    if (gi != curG) {
+                        for (int b = 0; b < 4; ++b) {
+                            const int d = d0 + b;
+                            const bool ok = d <= M.bt && J + d < M.nbc;
+                            tc_stage(ok ? wsl + (size_t)(2 * (d - 1)) * kSlices * TT : nullptr, sAop, kTcSliceA,
+                                     b * TB, t);
                         }
-                        const int d0 = 1 + 4 * gi, e = 1 + (u - gBase);
-                        if (J + e >= M.nbc || tcFailed) continue;
-                        if (gi != curG) {
-                            for (int b = 0; b < 4; ++b) {
-                                const int d = d0 + b;
-                                const bool ok = d <= M.bt && J + d < M.nbc;
-                                tc_stage(ok ? wsl + (size_t)(2 * (d - 1)) * kSlices * TT : nullptr, sAop, kTcSliceA,
-                                         b * TB, t);
-                            }
-                            curG = gi;
-                        }
-                        tc_stage(wsl + (size_t)(2 * (e - 1) + 1) * kSlices * TT, sBop, kTcSliceB, 0, t);
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                        __syncthreads();
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        if (t == 0) {
-                            const uint32_t aBase = smem_addr(sAop), bBase = smem_addr(sBop);
+                        curG = gi;
+                    }
+                    tc_stage(wsl + (size_t)(2 * (e - 1) + 1) * kSlices * TT, sBop, kTcSliceB, 0, t);
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncthreads();
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (t == 0) {
+                        const uint32_t aBase = smem_addr(sAop), bBase = smem_addr(sBop);
 #pragma unroll 1
-                            for (int li = 0; li < kLevels; ++li) {  // level l = li + 2 = p + q
-                                uint32_t acc = 0;
+                        for (int li = 0; li < kLevels; ++li) {  // level l = li + 2 = p + q
+                            uint32_t acc = 0;
 #pragma unroll 1
-                                for (int p = 1; p <= kSlices; ++p) {
-                                    const int q = li + 2 - p;
-                                    if (q < 1 || q > kSlices) continue;
+                            for (int p = 1; p <= kSlices; ++p) {
+                                const int q = li + 2 - p;
+                                if (q < 1 || q > kSlices) continue;
 #pragma unroll
-                                    for (int kk = 0; kk < 2; ++kk) {
-                                        tc_mma(tcBase + li * TB, tc_desc(aBase + (p - 1) * kTcSliceA * 2 + kk * 256),
-                                               tc_desc(bBase + (q - 1) * kTcSliceB * 2 + kk * 256), acc);
-                                        acc = 1;
-                                    }
+                                for (int kk = 0; kk < 2; ++kk) {
+                                    tc_mma(tcBase + li * TB, tc_desc(aBase + (p - 1) * kTcSliceA * 2 + kk * 256),
+                                           tc_desc(bBase + (q - 1) * kTcSliceB * 2 + kk * 256), acc);
+                                    acc = 1;
                                 }
                             }
-                            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                             smem_addr(&tcBar))
-                                         : "memory");
                         }
-                        uint32_t done = 0;
-                        for (int it = 0; it < kTcWaitLimit && !done; ++it)
-                            asm volatile(
-                                "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                                " selp.u32 %0, 1, 0, p;\n}"
-                                : "=r"(done)
-                                : "r"(smem_addr(&tcBar)), "r"(tcPhase)
-                                : "memory");
-                        tcPhase ^= 1u;
-                        if (!done) {
-                            tcFailed = true;
-                            atomicCAS(status, 0, -1);
-                        }
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        // epilogue: warp w reads lanes 32 (w % 4) .. of block row d0 + w % 4 and
-                        // columns 16 (w / 4) ..; the levels combined in FP64 as in MODE 1
-                        const int d = d0 + (w & 3), c0 = 16 * (w >> 2);
-                        if (done && d <= M.bt && J + d < M.nbc && d >= e) {
-                            double sum[16];
+                        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                                         smem_addr(&tcBar))
+                                     : "memory");
+                    }
+                    uint32_t done = 0;
+                    for (int it = 0; it < kTcWaitLimit && !done; ++it)
+                        asm volatile(
+                            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                            " selp.u32 %0, 1, 0, p;\n}"
+                            : "=r"(done)
+                            : "r"(smem_addr(&tcBar)), "r"(tcPhase)
+                            : "memory");
+                    tcPhase ^= 1u;
+                    if (!done) {
+                        tcFailed = true;
+                        atomicCAS(status, 0, -1);
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    // epilogue: warp w reads lanes 32 (w % 4) .. of block row d0 + w % 4 and
+                    // columns 16 (w / 4) ..; the levels combined in FP64 as in MODE 1
+                    const int d = d0 + (w & 3), c0 = 16 * (w >> 2);
+                    if (done && d <= M.bt && J + d < M.nbc && d >= e) {
+                        double sum[16];
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) sum[j] = 0.0;
-                            double sc = 1.0 / 65536.0;  // 2^(-8 l), l = 2 ..
+                        for (int j = 0; j < 16; ++j) sum[j] = 0.0;
+                        double sc = 1.0 / 65536.0;  // 2^(-8 l), l = 2 ..
 #pragma unroll 1
-                            for (int li = 0; li < kLevels; ++li) {
-                                float v[16];
-                                tc_ld16(tcBase + ((uint32_t)(32 * (w & 3)) << 16) + li * TB + c0, v);
-#pragma unroll
-                                for (int j = 0; j < 16; ++j) sum[j] += (double)v[j] * sc;
-                                sc *= 1.0 / 256.0;
-                            }
-                            double *Tt = band + tile_off(M, J + e, d - e);
-                            const int rr = lane;
-                            const int ea = __ldcg(wex + 2 * (d - 1) * TB + rr);
-                            const int *EB = wex + (2 * (e - 1) + 1) * TB;
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                double *pt = Tt + (c0 + j) * TB + rr;
-                                __stcg(pt, __ldcg(pt) - ldexp(sum[j], ea + __ldcg(EB + c0 + j)));
-                            }
-                        }
-                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                        __syncthreads();
-                    }
-                    __threadfence();
-                    cl.sync();
-                    continue;
-                }
-                // C. trailing update, tensor cores: warp w computes the 16 x 8 block (mi, ni) of the
-                // 32 x 32 tile, every level l of the slice products in its own FP32 accumulator
-                const int w = t >> 5, g = lane >> 2, tg = lane & 3, mi = w >> 2, ni = w & 3;
-                for (int u = crank; u < nt; u += cs) {
-                    int d = 1, rem = u;
-                    while (rem >= d) {
-                        rem -= d;
-                        ++d;
-                    }
-                    const int e = 1 + rem;
-                    if (J + d >= M.nbc) continue;
-                    const uint16_t *SA = wsl + (size_t)(2 * (d - 1)) * kSlices * TT;
-                    const uint16_t *SB = wsl + (size_t)(2 * (e - 1) + 1) * kSlices * TT;
-                    unsigned a[kSlices][2][4], b[kSlices][2][2];
-                    const int ra = (16 * mi + g) * TB, rb = (8 * ni + g) * TB;
-#pragma unroll
-                    for (int p = 0; p < kSlices; ++p)
-#pragma unroll
-                        for (int ks = 0; ks < 2; ++ks) {
-                            const uint16_t *pa = SA + (size_t)p * TT + 16 * ks + 2 * tg;
-                            const uint16_t *pb = SB + (size_t)p * TT + 16 * ks + 2 * tg;
-                            a[p][ks][0] = ld_pair(pa + ra);
-                            a[p][ks][1] = ld_pair(pa + ra + 8 * TB);
-                            a[p][ks][2] = ld_pair(pa + ra + 8);
-                            a[p][ks][3] = ld_pair(pa + ra + 8 * TB + 8);
-                            b[p][ks][0] = ld_pair(pb + rb);
-                            b[p][ks][1] = ld_pair(pb + rb + 8);
-                        }
-                    float acc[kLevels][4];
-#pragma unroll
-                    for (int li = 0; li < kLevels; ++li)
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) acc[li][i] = 0.f;
-#pragma unroll
-                    for (int li = 0; li < kLevels; ++li) {  // level l = li + 2 = p + q
-#pragma unroll
-                        for (int p = 1; p <= kSlices; ++p) {
-                            const int q = li + 2 - p;
-                            if (q < 1 || q > kSlices) continue;
-#pragma unroll
-                            for (int ks = 0; ks < 2; ++ks) mma_bf16(acc[li], a[p - 1][ks], b[q - 1][ks]);
-                        }
-                    }
-                    double *Tt = band + tile_off(M, J + e, d - e);
-                    const int *EA = wex + 2 * (d - 1) * TB, *EB = wex + (2 * (e - 1) + 1) * TB;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int rr = 16 * mi + g + (i >> 1) * 8, cc = 8 * ni + 2 * tg + (i & 1);
-                        double sum = 0.0, sc = 1.0 / 65536.0;  // 2^(-8 l), l = 2 ..
-#pragma unroll
                         for (int li = 0; li < kLevels; ++li) {
-                            sum += (double)acc[li][i] * sc;
+                            float v[16];
+                            tc_ld16(tcBase + ((uint32_t)(32 * (w & 3)) << 16) + li * TB + c0, v);
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) sum[j] += (double)v[j] * sc;
                             sc *= 1.0 / 256.0;
                         }
-                        double *pt = Tt + cc * TB + rr;
-                        __stcg(pt, __ldcg(pt) - ldexp(sum, __ldcg(EA + rr) + __ldcg(EB + cc)));
+                        double *Tt = band + tile_off(M, J + e, d - e);
+                        const int rr = lane;
+                        const int ea = __ldcg(wex + 2 * (d - 1) * TB + rr);
+                        const int *EB = wex + (2 * (e - 1) + 1) * TB;
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            double *pt = Tt + (c0 + j) * TB + rr;
+                            __stcg(pt, __ldcg(pt) - ldexp(sum[j], ea + __ldcg(EB + c0 + j)));
+                        }
                     }
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncthreads();
                 }
                 __threadfence();
                 cl.sync();
                 continue;
             }
-            // C. trailing update of the band: tile (J+e, d-e) -= L_{J+d,J} D_J L_{J+e,J}^T, 1 <= e <= d
+            // C. trailing update, tensor cores: warp w computes the 16 x 8 block (mi, ni) of the
+            // 32 x 32 tile, every level l of the slice products in its own FP32 accumulator
+            const int w = t >> 5, g = lane >> 2, tg = lane & 3, mi = w >> 2, ni = w & 3;
             for (int u = crank; u < nt; u += cs) {
                 int d = 1, rem = u;
                 while (rem >= d) {
@@ -517,27 +455,51 @@ __global__ void __launch_bounds__(kThreads, MODE == 2 ? 1 : 2) k_band_ldl(const 
                 }
                 const int e = 1 + rem;
                 if (J + d >= M.nbc) continue;
-                const double *Ld = band + tile_off(M, J, d), *Le = band + tile_off(M, J, e);
-                __syncthreads();
-                for (int x = t; x < TT; x += kThreads) {
-                    const int r = x % TB, c = x / TB;
-                    sA[r][c] = __ldcg(Ld + x) * sL[c][c];
-                    sB[r][c] = __ldcg(Le + x);
-                }
-                __syncthreads();
-                const int r = t % TB, c0 = (t / TB) * 4;
-                double acc[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 8
-                for (int k = 0; k < TB; ++k) {
-                    const double a = sA[r][k];
+                const uint16_t *SA = wsl + (size_t)(2 * (d - 1)) * kSlices * TT;
+                const uint16_t *SB = wsl + (size_t)(2 * (e - 1) + 1) * kSlices * TT;
+                unsigned a[kSlices][2][4], b[kSlices][2][2];
+                const int ra = (16 * mi + g) * TB, rb = (8 * ni + g) * TB;
 #pragma unroll
-                    for (int cc = 0; cc < 4; ++cc) acc[cc] += a * sB[c0 + cc][k];
+                for (int p = 0; p < kSlices; ++p)
+#pragma unroll
+                    for (int ks = 0; ks < 2; ++ks) {
+                        const uint16_t *pa = SA + (size_t)p * TT + 16 * ks + 2 * tg;
+                        const uint16_t *pb = SB + (size_t)p * TT + 16 * ks + 2 * tg;
+                        a[p][ks][0] = ld_pair(pa + ra);
+                        a[p][ks][1] = ld_pair(pa + ra + 8 * TB);
+                        a[p][ks][2] = ld_pair(pa + ra + 8);
+                        a[p][ks][3] = ld_pair(pa + ra + 8 * TB + 8);
+                        b[p][ks][0] = ld_pair(pb + rb);
+                        b[p][ks][1] = ld_pair(pb + rb + 8);
+                    }
+                float acc[kLevels][4];
+#pragma unroll
+                for (int li = 0; li < kLevels; ++li)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) acc[li][i] = 0.f;
+#pragma unroll
+                for (int li = 0; li < kLevels; ++li) {  // level l = li + 2 = p + q
+#pragma unroll
+                    for (int p = 1; p <= kSlices; ++p) {
+                        const int q = li + 2 - p;
+                        if (q < 1 || q > kSlices) continue;
+#pragma unroll
+                        for (int ks = 0; ks < 2; ++ks) mma_bf16(acc[li], a[p - 1][ks], b[q - 1][ks]);
+                    }
                 }
                 double *Tt = band + tile_off(M, J + e, d - e);
+                const int *EA = wex + 2 * (d - 1) * TB, *EB = wex + (2 * (e - 1) + 1) * TB;
 #pragma unroll
-                for (int cc = 0; cc < 4; ++cc) {
-                    double *pt = Tt + (c0 + cc) * TB + r;
-                    __stcg(pt, __ldcg(pt) - acc[cc]);
+                for (int i = 0; i < 4; ++i) {
+                    const int rr = 16 * mi + g + (i >> 1) * 8, cc = 8 * ni + 2 * tg + (i & 1);
+                    double sum = 0.0, sc = 1.0 / 65536.0;  // 2^(-8 l), l = 2 ..
+#pragma unroll
+                    for (int li = 0; li < kLevels; ++li) {
+                        sum += (double)acc[li][i] * sc;
+                        sc *= 1.0 / 256.0;
+                    }
+                    double *pt = Tt + cc * TB + rr;
+                    __stcg(pt, __ldcg(pt) - ldexp(sum, __ldcg(EA + rr) + __ldcg(EB + cc)));
                 }
             }
             __threadfence();
@@ -549,6 +511,259 @@ __global__ void __launch_bounds__(kThreads, MODE == 2 ? 1 : 2) k_band_ldl(const 
         __syncthreads();
         if (t < 32)
             asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tcBase), "r"(kTcCols));
+    }
+}
+
+// 1 / d by one third-order (Halley) step on the hardware's approximate reciprocal: with
+// y (1 - e) d = 1, y (1 + e + e^2) leaves a relative error of e^3 (below 2^-57 for the 20 bits of
+// the approximation), then one rounding.  Subnormal and huge arguments, for which the approximation
+// flushes or overflows, take the division.
+__device__ __forceinline__ double recip64(double d) {
+    const unsigned ex = ((unsigned)__double2hiint(d) >> 20) & 0x7ffu;
+    if (ex < 4u || ex > 2040u) return 1.0 / d;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double e = fma(-d, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+
+// LDL^T of the lower triangle of a 32 x 32 tile in shared memory (L below the diagonal, D on it),
+// the whole CTA.  GB300's FP64 pipe takes one warp instruction per 19 clocks from an SM and one
+// per 64 from a warp (measured), so the chain is kept to one warp and short: it factors four
+// columns at a time in registers (lane = row), the next four columns are brought up to date by
+// four warps, and the remaining columns by warps 1 .. 7 while warp 0 factors on.
+__device__ void tile_ldl(double (*S)[TB + 1], double (*sU)[4][TB], int t) {
+    const int lane = t & 31, w = t >> 5;
+    for (int b = 0; b < 8; ++b) {
+        const int c0 = 4 * b;
+        double(*U)[TB] = sU[b & 1];
+        if (w == 0) {
+            double v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[k] = S[lane][c0 + k];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const double inv = recip64(__shfl_sync(0xffffffffu, v[k], c0 + k));
+                const double l = v[k] * inv;
+#pragma unroll
+                for (int m = k + 1; m < 4; ++m) v[m] = fma(-l, __shfl_sync(0xffffffffu, v[k], c0 + m), v[m]);
+                U[k][lane] = v[k];
+                if (lane > c0 + k) S[lane][c0 + k] = l;
+                if (lane == c0 + k) S[lane][c0 + k] = v[k];
+            }
+        }
+        __syncthreads();
+        if (b == 7) break;
+        auto update = [&](int j) {
+            double s = S[lane][j];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) s = fma(-S[lane][c0 + k], U[k][j], s);
+            if (lane >= j) S[lane][j] = s;
+        };
+        if (w < 4) update(c0 + 4 + w);
+        __syncthreads();
+        if (w > 0)
+            for (int j = c0 + 7 + w; j < TB; j += kGroups - 1) update(j);
+    }
+}
+
+// Rows of a 32 x 32 tile in shared memory (A[row][column]) times L^-T (sL: unit lower L), the whole
+// CTA, the columns in fours as in tile_ldl.
+__device__ void tile_rows(double (*A)[TB + 1], const double (*sL)[TB + 1], int t) {
+    const int lane = t & 31, w = t >> 5;
+    for (int b = 0; b < 8; ++b) {
+        const int c0 = 4 * b;
+        if (w == 0) {
+            double v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                v[k] = A[lane][c0 + k];
+#pragma unroll
+                for (int m = 0; m < k; ++m) v[k] = fma(-v[m], sL[c0 + k][c0 + m], v[k]);
+                A[lane][c0 + k] = v[k];
+            }
+        }
+        __syncthreads();
+        if (b == 7) break;
+        auto update = [&](int j) {
+            double s = A[lane][j];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) s = fma(-A[lane][c0 + k], sL[j][c0 + k], s);
+            A[lane][j] = s;
+        };
+        if (w < 4) update(c0 + 4 + w);
+        __syncthreads();
+        if (w > 0)
+            for (int j = c0 + 7 + w; j < TB; j += kGroups - 1) update(j);
+    }
+}
+
+// Blocked band LDL^T in FP64, one cluster per panel (the cluster's panels listed in sched).  Per
+// block column J:
+//   rows      the tiles below the diagonal, L_IJ = A_IJ L_JJ^-T D_J^-1, dealt to the CTAs; a CTA with
+//             one or two takes each with all its warps (tile_rows), with more a warp per tile (one
+//             row per thread): the FP64 pipe is then full from the tiles alone;
+//   update    tiles (J+e, d-e) -= L_{J+d,J} D_J L_{J+e,J}^T, 1 <= e <= d.  CTA 0 takes the next
+//             diagonal tile first and factors it in shared memory (tile_ldl) while the others go on
+//             with the rest, so the chain of the pivots is off the critical path; it joins again
+//             two rounds later (the factorisation takes about as long as a tile update).  Every
+//             thread loads the next item's operands during the current one.
+// One cluster barrier after each.  Bound: the FP64 pipe in the updates (9.5 us a tile and SM), and
+// for a narrow band the chain rows -> first update -> diagonal tile.  32 panels of 8 .. 36 elements a
+// side: 12.5 ms, against 26.1 ms with every CTA factoring the diagonal tile for itself (a division
+// per thread and pivot) and the rows below on consecutive threads of the first CTA; the 64 x 64
+// plate's two halves at 8 CTAs: 50.8 against 70.8 ms.
+__global__ void __launch_bounds__(kThreads, 2) k_band_ldl64(const PanelMeta *__restrict__ meta,
+                                                         const int *__restrict__ sched,
+                                                         const int *__restrict__ schedPtr, double *band,
+                                                         int *status) {
+    cg::cluster_group cl = cg::this_cluster();
+    const int crank = (int)cl.block_rank(), cs = (int)cl.num_blocks();
+    const int worker = blockIdx.x / cs;
+    __shared__ double sL[TB][TB + 1];  // the block column's diagonal tile: L below the diagonal, D on it
+    __shared__ double sN[TB][TB + 1];  // CTA 0: the next one
+    __shared__ double sA[TB][TB + 1], sB[TB][TB + 1];
+    __shared__ double sU[2][4][TB];
+    __shared__ double sDi[TB];  // D^-1
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    for (int q = schedPtr[worker]; q < schedPtr[worker + 1]; ++q) {
+        const int p = sched[q];
+        const PanelMeta M = meta[p];
+        // CTA 0: the factored diagonal tile of block column J from sN, to memory and the pivot test
+        auto diag_out = [&](int J) {
+            tile_ldl(sN, sU, t);
+            double *Td = band + tile_off(M, J, 0);
+            for (int e = t; e < TT; e += kThreads) __stcg(Td + e, sN[e % TB][e / TB]);
+            if (t < TB && J * TB + t < M.n) {
+                const double dk = sN[t][t];
+                if (!(dk != 0.0 && isfinite(dk))) atomicCAS(status, 0, p + 1);
+            }
+        };
+        if (crank == 0) {
+            const double *Td = band + tile_off(M, 0, 0);
+            for (int e = t; e < TT; e += kThreads) sN[e % TB][e / TB] = __ldcg(Td + e);
+            __syncthreads();
+            if (M.nfac > 0) diag_out(0);
+        }
+        cl.sync();
+        for (int J = 0; J < M.nfac; ++J) {
+            const int nd = min(M.bt, M.nbc - 1 - J);  // tiles below the diagonal
+            {
+                const double *Td = band + tile_off(M, J, 0);
+                for (int e = t; e < TT; e += kThreads) sL[e % TB][e / TB] = __ldcg(Td + e);
+                __syncthreads();
+                if (t < TB) sDi[t] = 1.0 / sL[t][t];
+                __syncthreads();
+            }
+            // the rows below
+            if ((nd + cs - 1) / cs <= 2) {
+                for (int d = 1 + crank; d <= nd; d += cs) {
+                    double *T = band + tile_off(M, J, d);
+                    for (int e = t; e < TT; e += kThreads) sA[e % TB][e / TB] = __ldcg(T + e);
+                    __syncthreads();
+                    tile_rows(sA, sL, t);
+                    for (int e = t; e < TT; e += kThreads) __stcg(T + e, sA[e % TB][e / TB] * sDi[e / TB]);
+                    __syncthreads();
+                }
+            } else {
+                for (int d = 1 + crank + cs * w; d <= nd; d += cs * kGroups) {
+                    double *T = band + tile_off(M, J, d);
+                    double v[TB];
+#pragma unroll
+                    for (int c = 0; c < TB; ++c) v[c] = __ldcg(T + c * TB + lane);
+#pragma unroll
+                    for (int k = 1; k < TB; ++k) {
+                        double s = v[k];
+#pragma unroll
+                        for (int m = 0; m < k; ++m) s -= v[m] * sL[k][m];
+                        v[k] = s;
+                    }
+#pragma unroll
+                    for (int c = 0; c < TB; ++c) __stcg(T + c * TB + lane, v[c] * sDi[c]);
+                }
+            }
+            cl.sync();
+            // the update: item i = d (d - 1) / 2 + e - 1 of nt; item 0 (the next diagonal tile) and the
+            // round after it belong to CTA 0, the others are dealt round-robin
+            const int nt = nd * (nd + 1) / 2;
+            auto item = [&](int round) {
+                if (round == 0) return crank;
+                if (round == 1) return crank == 0 ? -1 : cs - 1 + crank;
+                return 2 * cs - 1 + (round - 2) * cs + crank;
+            };
+            auto tiles = [&](int i, int &d, int &e) {
+                d = 1;
+                while (i >= d) {
+                    i -= d;
+                    ++d;
+                }
+                e = 1 + i;
+            };
+            double pa[4], pb[4];
+            auto fetch = [&](int i) {
+                int d, e;
+                tiles(i, d, e);
+                const double *Ld = band + tile_off(M, J, d), *Le = band + tile_off(M, J, e);
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    pa[x] = __ldcg(Ld + t + x * kThreads);
+                    pb[x] = __ldcg(Le + t + x * kThreads);
+                }
+            };
+            int i = item(0);
+            if (i < nt) fetch(i);
+            for (int round = 0; i < nt; ++round) {
+                if (i >= 0) {
+                    __syncthreads();
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        const int c = w + x * kGroups;
+                        sA[lane][c] = pa[x] * sL[c][c];
+                        sB[lane][c] = pb[x];
+                    }
+                    __syncthreads();
+                }
+                const int nxt = item(round + 1);
+                if (nxt >= 0 && nxt < nt) fetch(nxt);
+                if (i >= 0) {
+                    int d, e;
+                    tiles(i, d, e);
+                    double *Tt = band + tile_off(M, J + e, d - e) + 4 * w * TB + lane;
+                    double o[4], acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+                    for (int cc = 0; cc < 4; ++cc) o[cc] = __ldcg(Tt + cc * TB);
+#pragma unroll 8
+                    for (int k = 0; k < TB; ++k) {
+                        const double a = sA[lane][k];
+#pragma unroll
+                        for (int cc = 0; cc < 4; ++cc) acc[cc] += a * sB[4 * w + cc][k];
+                    }
+                    if (i > 0) {
+#pragma unroll
+                        for (int cc = 0; cc < 4; ++cc) __stcg(Tt + cc * TB, o[cc] - acc[cc]);
+                    } else {
+#pragma unroll
+                        for (int cc = 0; cc < 4; ++cc) sN[lane][4 * w + cc] = o[cc] - acc[cc];
+                        __syncthreads();
+                        if (J + 1 < M.nfac) {
+                            diag_out(J + 1);
+                        } else {
+#pragma unroll
+                            for (int cc = 0; cc < 4; ++cc) __stcg(Tt + cc * TB, o[cc] - acc[cc]);
+                        }
+                    }
+                }
+                i = nxt;
+            }
+            if (nd == 0 && crank == 0 && J + 1 < M.nfac) {  // a band of one tile: nothing couples to the next
+                const double *Td = band + tile_off(M, J + 1, 0);
+                __syncthreads();
+                for (int e = t; e < TT; e += kThreads) sN[e % TB][e / TB] = __ldcg(Td + e);
+                __syncthreads();
+                diag_out(J + 1);
+            }
+            cl.sync();
+        }
     }
 }
 
@@ -1466,6 +1681,17 @@ int plan_build(astro_ctx *ctx, PanelPlan &L, int cs) {
     }
     L.bandDoubles = band;
     L.xRows = xr;
+    L.maxBt = 0;
+    for (const PanelMeta &M : L.meta) L.maxBt = std::max(L.maxBt, M.bt);
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    L.csAsked = cs;
+    if (cs == 0)
+        // 16 CTAs a panel (the largest cluster of the hardware) for the FP64 factorisation of few
+        // panels, when the GPU holds them all at a CTA per SM and a block column has more tile
+        // updates than 8 CTAs: the updates are bound by the FP64 pipes of the panel's own SMs.
+        // 64 x 64 plate in two halves, bandwidth 401: 50.8 ms with 8, 26.5 ms with 16.
+        cs = ctx->bandFp64Update == 1 && 16 * std::max(np, 2) <= sms && L.maxBt >= 4 ? 16 : 8;
     // clusters: as many as fit at once, panels by longest processing time first
     L.cs = cs;
     int maxClusters = 0;
@@ -1485,16 +1711,13 @@ int plan_build(astro_ctx *ctx, PanelPlan &L, int cs) {
         // surplus clusters wait for the resident ones (and at most two CTAs per SM hold tensor
         // memory: the allocation never waits)
         cudaFuncSetAttribute(k_band_ldl<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
-        if (cudaOccupancyMaxActiveClusters(&maxClusters, k_band_ldl<1>, &cfg) != cudaSuccess) {
+        cudaFuncSetAttribute(k_band_ldl64, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (cudaOccupancyMaxActiveClusters(&maxClusters, k_band_ldl64, &cfg) != cudaSuccess) {
             cudaGetLastError();
             maxClusters = 0;
         }
     }
-    if (maxClusters < 1) {
-        int sms = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-        maxClusters = std::max(1, sms / cs);
-    }
+    if (maxClusters < 1) maxClusters = std::max(1, sms / cs);
     L.workers = std::max(1, std::min(np, maxClusters));
     std::vector<int> order(np);
     std::iota(order.begin(), order.end(), 0);
@@ -1513,8 +1736,6 @@ int plan_build(astro_ctx *ctx, PanelPlan &L, int cs) {
         L.schedPtr.push_back((int)L.sched.size());
     }
     // slice scratch of the tensor-core trailing update, one block column's tiles per worker
-    L.maxBt = 0;
-    for (const PanelMeta &M : L.meta) L.maxBt = std::max(L.maxBt, M.bt);
     L.sliceStride = 2LL * std::max(L.maxBt, 1) * kSlices * TT;
     L.expStride = 2 * std::max(L.maxBt, 1) * TB;
     int rc;
@@ -1567,14 +1788,15 @@ void panels_release(astro_ctx *ctx) {
 // (the twisted many-column solve).
 int panels_factor_impl(astro_ctx *ctx, int32_t cluster_size, astro_panels_info *info, int factor) {
     if (!ctx) return ASTRO_ERR_ARG;
-    if (cluster_size == 0) cluster_size = ctx->tunePanelCluster ? ctx->tunePanelCluster : 8;  // autotuned or 8
-    if (cluster_size != 1 && cluster_size != 2 && cluster_size != 4 && cluster_size != 8)
+    if (cluster_size == 0) cluster_size = ctx->tunePanelCluster;  // autotuned, or 0: plan_build's choice
+    if (cluster_size != 0 && cluster_size != 1 && cluster_size != 2 && cluster_size != 4 && cluster_size != 8)
         return set_err(ctx, ASTRO_ERR_ARG, "panels: cluster_size must be 1, 2, 4 or 8");
     if (!ctx->haveK64) return set_err(ctx, ASTRO_ERR_STATE, "panels: FP64 stiffness not assembled");
     if (ctx->P.mpcDim > 0 && !ctx->mpcScaled)
         return set_err(ctx, ASTRO_ERR_STATE, "panels: constraints not scaled (astro_scale_mpc)");
     PanelPlan *L = static_cast<PanelPlan *>(ctx->panels);
-    if (L && L->cs != cluster_size) {
+    // (16 CTAs are for the FP64 updates: the other variants' clusters are of the portable sizes)
+    if (L && ((L->csAsked != cluster_size && L->cs != cluster_size) || (L->cs == 16 && ctx->bandFp64Update != 1))) {
         panels_release(ctx);
         L = nullptr;
     }
@@ -1631,10 +1853,9 @@ int panels_factor_impl(astro_ctx *ctx, int32_t cluster_size, astro_panels_info *
     cfg.attrs = at;
     cfg.numAttrs = 1;
     if (ctx->bandFp64Update == 1) {
-        CK(cudaLaunchKernelEx(&cfg, k_band_ldl<0>, (const PanelMeta *)dptr<PanelMeta>(L->d_meta),
+        CK(cudaLaunchKernelEx(&cfg, k_band_ldl64, (const PanelMeta *)dptr<PanelMeta>(L->d_meta),
                               (const int *)dptr<int>(L->d_sched), (const int *)dptr<int>(L->d_schedPtr),
-                              dptr<double>(L->d_band), dptr<int>(L->d_status), (uint16_t *)nullptr, (int *)nullptr,
-                              0LL, 0));
+                              dptr<double>(L->d_band), dptr<int>(L->d_status)));
     } else if (ctx->bandFp64Update == 3) {
         // the band in double-float for the factorisation, FP64 again after it
         const long long nb = L->bandDoubles;
@@ -1801,7 +2022,7 @@ extern "C" int astro_panels_solve_batched(astro_ctx *ctx, int32_t num_rhs, const
     PanelPlan *L = static_cast<PanelPlan *>(ctx->panels);
     int rc;
     if (!L || !L->factored || L->kVersion != ctx->k64Version || L->penVersion != ctx->penVersion)
-        if ((rc = astro_panels_factor(ctx, L ? L->cs : 0, info))) return rc;
+        if ((rc = astro_panels_factor(ctx, L ? L->csAsked : 0, info))) return rc;
     return astro_panels_solve(ctx, num_rhs, rhs, x, info);
 }
 
@@ -1942,8 +2163,7 @@ static int twist_prepare(astro_ctx *ctx, PanelPlan *L, int ncols) {
         at[0].val.clusterDim.z = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, k_band_ldl<0>, dm, schedBase, schedP, db,
-                                  dptr<int>(L->d_twStatus), (uint16_t *)nullptr, (int *)nullptr, 0LL, 0);
+        return cudaLaunchKernelEx(&cfg, k_band_ldl64, dm, schedBase, schedP, db, dptr<int>(L->d_twStatus));
     };
     CK(factor(2, dptr<int>(L->d_twSched), dptr<int>(L->d_twSchedPtr)));
     k_tw_window<<<wg, 256, 0, s>>>(G, w, dm, db, dptr<double>(L->d_twAw), 1);

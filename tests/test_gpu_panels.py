@@ -93,6 +93,26 @@ def test_panels_on_a_brick_block():
     _check(A, x, b, spla.spsolve(A, b))
 
 
+@pytest.mark.parametrize("dims,cs", [((9, 1, 1), 0), ((7, 2, 2), 8), ((8, 5, 5), 0), ((8, 5, 5), 1), ((5, 8, 7), 4),
+                                     ((6, 10, 9), 0), ((6, 10, 9), 2)])
+def test_fp64_factor_tile_counts(dims, cs):
+    """The FP64 factorisation where its work split changes: one tile below the diagonal, fewer tiles
+    than CTAs, two and more tiles per CTA (the rows below by the whole CTA or a warp each), and the
+    cluster size chosen for the batch (16 CTAs for one wide panel)."""
+    nx, ny, nz = dims
+    m = M.hex_block(nx, ny, nz, lx=nx * 0.25, ly=ny * 0.25, lz=nz * 0.25, seed=nx)
+    g, o = AstroGPU(m), Oracle(m)
+    g.getElasticSolnLoad(1, export=False)
+    g.scaleElasticMPC()
+    A = o.static_system()[0].tocsc()
+    info = g.panels_factor(cs)
+    assert info.cluster_size == (cs or (16 if info.max_bandwidth > 96 else 8))
+    B = np.random.default_rng(2).standard_normal((g.n, 3))
+    X, _ = g.panels_solve(B)
+    R = spla.splu(A).solve(B)
+    assert np.all(np.linalg.norm(X - R, axis=0) <= 1e-10 * np.linalg.norm(R, axis=0))
+
+
 def test_panel_sensitivity_pipeline(batch):
     """Pressure load per panel, the complex-step sensitivity right-hand sides at the solved state
     (against the oracle) and the batched solves of all of them."""
