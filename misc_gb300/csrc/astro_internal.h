@@ -137,7 +137,7 @@ struct astro_ctx {
     // exported CSR values and column numbers
     DevBuf d_ioRef, d_ioInt, d_exMat, d_exCols;
     HostStage *stage = nullptr;
-    DevBuf d_sky[5];  // grow-only scratch of the host-buffer skyline entry points
+    DevBuf d_sky[9];  // grow-only scratch of the skyline entry points
     // scratch
     DevBuf d_scratch;
     DevBuf d_status;  // int status words written by kernels

@@ -47,28 +47,19 @@
 #include <vector>
 
 #include "astro_internal.h"
+#include "band_tiles.cuh"
 #include "dfloat.cuh"
 
 namespace cg = cooperative_groups;
+using namespace astro_band;
 
 namespace {
 
-constexpr int TB = 32;  // tile edge
-constexpr int TT = TB * TB;
 constexpr int kThreads = 256;
 constexpr int kGroups = kThreads / TB;  // warps per CTA
 constexpr int kSolveCols = 8;           // right-hand sides per solve CTA
 constexpr int kSlices = 7;              // 8-bit slices per FP64 value in the emulated tile update
 constexpr int kLevels = kSlices;        // levels l = p + q = 2 .. kSlices + 1 of the slice products
-
-struct PanelMeta {
-    long long band;   // first double of the panel's tiles
-    long long xUnit;  // rows of the padded right-hand-side layout before this panel (times nrhs)
-    int n;            // DOF
-    int nbc;          // block columns, ceil(n / 32)
-    int bt;           // tiles below the diagonal tile in a block column
-    int nfac;         // block columns the factorisation eliminates (nbc; fewer for a partial factor)
-};
 
 struct SolveItem {
     int panel, col0, ncol, pad;
@@ -107,10 +98,6 @@ struct PanelPlan {
     DevBuf d_twMeta, d_twBand, d_twAw, d_twSched, d_twSchedPtr, d_twStatus, d_twLf, d_twLb, d_twWf, d_twWb, d_twDinv,
         d_twItems, d_twX;
 };
-
-__device__ __forceinline__ size_t tile_off(const PanelMeta &M, int J, int d) {
-    return (size_t)M.band + ((size_t)J * (M.bt + 1) + d) * TT;
-}
 
 // lower-band entries of the BSR stiffness (dpn x dpn row-major blocks) into the tiles
 __global__ void k_band_fill(int nb, int dpn, const int *__restrict__ bRow, const int *__restrict__ bCol,
@@ -766,6 +753,28 @@ __global__ void __launch_bounds__(kThreads, 2) k_band_ldl64(const PanelMeta *__r
         }
     }
 }
+
+}  // namespace
+
+cudaError_t band_ldl64(const PanelMeta *meta, const int *sched, const int *schedPtr, int workers, int cs, double *band,
+                       int *status, cudaStream_t s) {
+    cudaError_t e = cudaFuncSetAttribute(k_band_ldl64, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(workers * cs);
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cs;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_band_ldl64, meta, sched, schedPtr, band, status);
+}
+
+namespace {
 
 // ---- the band LDL^T carried in double-float (ASTRO_OPT_BAND_FP64_UPDATE = 3) ---------------
 //
@@ -1853,9 +1862,8 @@ int panels_factor_impl(astro_ctx *ctx, int32_t cluster_size, astro_panels_info *
     cfg.attrs = at;
     cfg.numAttrs = 1;
     if (ctx->bandFp64Update == 1) {
-        CK(cudaLaunchKernelEx(&cfg, k_band_ldl64, (const PanelMeta *)dptr<PanelMeta>(L->d_meta),
-                              (const int *)dptr<int>(L->d_sched), (const int *)dptr<int>(L->d_schedPtr),
-                              dptr<double>(L->d_band), dptr<int>(L->d_status)));
+        CK(band_ldl64(dptr<PanelMeta>(L->d_meta), dptr<int>(L->d_sched), dptr<int>(L->d_schedPtr), L->workers, L->cs,
+                      dptr<double>(L->d_band), dptr<int>(L->d_status), s));
     } else if (ctx->bandFp64Update == 3) {
         // the band in double-float for the factorisation, FP64 again after it
         const long long nb = L->bandDoubles;
@@ -2152,18 +2160,7 @@ static int twist_prepare(astro_ctx *ctx, PanelPlan *L, int ncols) {
     if ((rc = cuda_check(ctx, cudaGetLastError(), "twisted band fill"))) return rc;
     // the partial factorisations of T and B (one cluster each), the window matrix, its factor
     auto factor = [&](int workers, const int *schedBase, const int *schedP) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(workers * L->cs);
-        cfg.blockDim = dim3(kThreads);
-        cfg.stream = s;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = L->cs;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, k_band_ldl64, dm, schedBase, schedP, db, dptr<int>(L->d_twStatus));
+        return band_ldl64(dm, schedBase, schedP, workers, L->cs, db, dptr<int>(L->d_twStatus), s);
     };
     CK(factor(2, dptr<int>(L->d_twSched), dptr<int>(L->d_twSchedPtr)));
     k_tw_window<<<wg, 256, 0, s>>>(G, w, dm, db, dptr<double>(L->d_twAw), 1);

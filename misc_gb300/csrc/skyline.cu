@@ -3,9 +3,10 @@
 //   getSparseLDLFact   (Working/AStrO_solvers.f90:10-78)        row-skyline LDL^T, no pivoting
 //   solveSparseLDLFact (:83-126)                                forward by rows, backward by columns
 //   gMRes              (:128-297) with rFactorMat/solveRFactor (:299-404)
-// The skyline recurrences are sequential along the profile, so the factor and the solves run in
-// one CTA that sweeps the rows with block-wide reductions; gMRes runs as one persistent CTA
-// (sparse products, preconditioner solves, modified Gram-Schmidt, Givens QR of the Hessenberg
+// The factor and the solves run in 32 x 32 band tiles, the parts of the profile that no row crosses
+// side by side (the section on band tiles below).  gMRes, the allocation-free solve and profiles
+// that band tiles do not suit use the reference's row sweeps in one CTA with block-wide
+// reductions; gMRes runs as one persistent CTA (sparse products, preconditioner solves, modified Gram-Schmidt, Givens QR of the Hessenberg
 // matrix) so that nothing returns to the host inside the iteration.  Every loop is bounded by the
 // reference's own limits (maxIt/numVecs + 1 restarts), so the kernels always terminate.  These
 // are the parity path for the reference's algorithm on the small and mid-size models it is used
@@ -14,6 +15,9 @@
 #include <cmath>
 
 #include "astro_internal.h"
+#include "band_tiles.cuh"
+
+using namespace astro_band;
 
 namespace {
 
@@ -123,6 +127,189 @@ __global__ void __launch_bounds__(kT) k_ldl_fact(double *A, const int *R, int n,
 __global__ void __launch_bounds__(kT) k_ldl_solve(double *soln, const double *rhs, const double *L, const int *R, int n,
                                                   int maxBW, double *z) {
     ldl_solve(soln, rhs, L, R, n, maxBW, z);
+}
+
+// ---- the factor and the solves in band tiles ----------------------------------------------------
+// A row of the sweeps above waits for the one before it (2 us a row and sweep on one CTA).  The
+// profile of a component-major DOF numbering falls into blocks that no row crosses (one per
+// component), and inside a block the rows of 32 share their columns: so the profile is split into
+// panels at the rows it does not cross, each panel is laid out in 32 x 32 band tiles, and the panels
+// run side by side: the factor by the FP64 band LDL^T of the panels (band_ldl64), the solves by one
+// CTA per panel.  What lies outside the profile is zero in the tiles and stays zero.  Factor and solve
+// through the host-buffer entry points: 2,214 rows of at most 11 entries 8.2 -> 0.58 ms, 6,750 rows
+// of 101 55.0 -> 3.4 ms.
+constexpr int kSkyThreads = 256;
+
+struct SkyPanels {
+    const PanelMeta *meta;
+    const int *row0;  // first row (0-based) of each panel, np + 1 entries
+    const int *R;     // row ranges of the profile
+    int np;
+};
+
+// The panel of tile number t, counted over all panels; J and d of the tile.
+__device__ __forceinline__ int sky_tile(const SkyPanels &S, long long t, int &J, int &d) {
+    int p = 0;
+    for (; p + 1 < S.np; ++p) {
+        const long long c = (long long)S.meta[p].nbc * (S.meta[p].bt + 1);
+        if (t < c) break;
+        t -= c;
+    }
+    J = (int)(t / (S.meta[p].bt + 1));
+    d = (int)(t % (S.meta[p].bt + 1));
+    return p;
+}
+
+// Profile -> tiles, a CTA per tile, the rows read along the columns: the lower triangle column-major
+// in colMajor and, for the backward sweep, row-major in rowMajor (may be null).  Padding rows get a
+// unit diagonal.
+__global__ void __launch_bounds__(kSkyThreads) k_sky_tiles(SkyPanels S, const double *__restrict__ A,
+                                                          double *__restrict__ colMajor, double *__restrict__ rowMajor) {
+    __shared__ double T[TB][TB + 1];
+    int J, d;
+    const int p = sky_tile(S, blockIdx.x, J, d);
+    const PanelMeta M = S.meta[p];
+    if (J + d >= M.nbc) return;
+    const int t = threadIdx.x, lane = t % TB, w = t / TB;
+    for (int r = w; r < TB; r += kSkyThreads / TB) {
+        const int i = (J + d) * TB + r, j = J * TB + lane;
+        double v = 0.0;
+        if (i < M.n) {
+            const int row = S.row0[p] + i, end = S.R[row + 1], len = end - S.R[row] - 1;
+            if (j <= i && j >= i - len) v = A[end - 1 - (i - j)];
+        } else if (i == j) {
+            v = 1.0;
+        }
+        T[r][lane] = v;
+        if (rowMajor) rowMajor[tile_off(M, J, d) + r * TB + lane] = v;
+    }
+    __syncthreads();
+    for (int c = w; c < TB; c += kSkyThreads / TB) colMajor[tile_off(M, J, d) + c * TB + lane] = T[lane][c];
+}
+
+// Tiles (column-major) -> profile; bad[0] = the first row (1-based) with a zero or non-finite pivot
+// (the pivots before it do not depend on it).
+__global__ void __launch_bounds__(kSkyThreads) k_sky_untile(SkyPanels S, const double *__restrict__ tiles,
+                                                           double *__restrict__ A, int *bad) {
+    __shared__ double T[TB][TB + 1];
+    int J, d;
+    const int p = sky_tile(S, blockIdx.x, J, d);
+    const PanelMeta M = S.meta[p];
+    if (J + d >= M.nbc) return;
+    const int t = threadIdx.x, lane = t % TB, w = t / TB;
+    for (int c = w; c < TB; c += kSkyThreads / TB) T[lane][c] = tiles[tile_off(M, J, d) + c * TB + lane];
+    __syncthreads();
+    for (int r = w; r < TB; r += kSkyThreads / TB) {
+        const int i = (J + d) * TB + r, j = J * TB + lane;
+        if (i >= M.n) continue;
+        const int row = S.row0[p] + i, end = S.R[row + 1], len = end - S.R[row] - 1;
+        if (j > i || j < i - len) continue;
+        const double v = T[r][lane];
+        A[end - 1 - (i - j)] = v;
+        if (i == j && !(v != 0.0 && isfinite(v))) atomicMin(bad, row + 1);
+    }
+}
+
+// One sweep of a panel's block rows: y_I = L_II^-1 (b_I - sum_d L_{I,I-d} y_{I-d}) forward, the
+// transposed backward (tiles then row-major, so that lanes are consecutive in both).  Warp 0 runs
+// the 32-step substitution of a block row with shuffles; meanwhile the other warps sum the next
+// row's products with the rows solved before the current one (d >= 2) and bring its diagonal tile
+// and its d = 1 tile into shared memory, so between two substitutions there is only the 32 x 32
+// product with the row just solved (four warps).  Bound: that chain (a shuffle and an FP64
+// multiply-add of 64 clocks per step of the substitution).
+constexpr int kSkyWarps = kSkyThreads / TB;
+struct SkySmem {
+    double diag[2][TT], next[2][TT];  // a block row's diagonal and d = 1 tiles
+    double part[kSkyWarps][TB];       // partial sums over d >= 2
+    double sum[2][TB];                // their sum
+    double near[4][TB];               // partial products with the row just solved
+};
+
+template <bool FWD>
+__device__ void sky_sweep(const PanelMeta &M, const double *__restrict__ tiles, double *v, double *ring, int nring,
+                          SkySmem &S) {
+    const int t = threadIdx.x, lane = t % TB, w = t / TB;
+    auto stage = [&](int s) {  // warps 1 ..: what block row s needs besides the row just before it
+        const int I = FWD ? s : M.nbc - 1 - s;
+        const double *D = tiles + tile_off(M, I, 0);
+        for (int e = t - TB; e < TT; e += kSkyThreads - TB) S.diag[s & 1][e] = __ldg(D + e);
+        if (s > 0 && M.bt > 0) {
+            const double *T1 = tiles + tile_off(M, FWD ? I - 1 : I, 1);
+            for (int e = t - TB; e < TT; e += kSkyThreads - TB) S.next[s & 1][e] = __ldg(T1 + e);
+        }
+        const int dmax = min(M.bt, s);
+        double acc = 0.0;
+        for (int q = w - 1; q < 4 * (dmax - 1); q += kSkyWarps - 1) {  // quarters of tiles
+            const int d = 2 + q / 4, k0 = 8 * (q % 4);
+            const double *T = tiles + tile_off(M, FWD ? I - d : I, d);
+            const double *y = ring + (size_t)((s - d) % nring) * TB;
+#pragma unroll
+            for (int k = k0; k < k0 + 8; ++k) acc += __ldg(T + k * TB + lane) * y[k];
+        }
+        S.part[w][lane] = acc;
+        asm volatile("bar.sync 1, %0;" ::"n"(kSkyThreads - TB) : "memory");  // warps 1 .. only
+        if (w == 1) {
+            double a = 0.0;
+#pragma unroll
+            for (int g = 1; g < kSkyWarps; ++g) a += S.part[g][lane];
+            S.sum[s & 1][lane] = a;
+        }
+    };
+    if (w > 0) stage(0);
+    double b = w == 0 ? v[(size_t)(FWD ? 0 : M.nbc - 1) * TB + lane] : 0.0;
+    for (int s = 0; s < M.nbc; ++s) {
+        __syncthreads();
+        const bool near = s > 0 && M.bt > 0;
+        if (near && w >= 1 && w <= 4) {
+            const double *y = ring + (size_t)((s - 1) % nring) * TB, *T1 = S.next[s & 1];
+            double acc = 0.0;
+#pragma unroll
+            for (int k = 8 * (w - 1); k < 8 * w; ++k) acc += T1[k * TB + lane] * y[k];
+            S.near[w - 1][lane] = acc;
+        }
+        __syncthreads();
+        if (w == 0) {
+            const int I = FWD ? s : M.nbc - 1 - s;
+            double x = b - S.sum[s & 1][lane];
+            if (s + 1 < M.nbc) b = v[(size_t)(FWD ? I + 1 : I - 1) * TB + lane];
+            if (near) x -= (S.near[0][lane] + S.near[1][lane]) + (S.near[2][lane] + S.near[3][lane]);
+            const double *D = S.diag[s & 1];
+#pragma unroll 8
+            for (int q = 0; q < TB - 1; ++q) {
+                const int k = FWD ? q : TB - 1 - q;
+                const double xk = __shfl_sync(0xffffffffu, x, k);
+                if (FWD ? lane > k : lane < k) x = fma(-D[k * TB + lane], xk, x);
+            }
+            ring[(size_t)(s % nring) * TB + lane] = x;
+            v[(size_t)I * TB + lane] = x;
+        } else if (s + 1 < M.nbc) {
+            stage(s + 1);
+        }
+    }
+    __syncthreads();
+}
+
+// L D L^T soln = rhs, one CTA per panel: forward, division by D, backward.  v: the panels' padded
+// rows (scratch); zout: the forward result, as solveSparseLDLFact leaves it in its scratch vector.
+__global__ void __launch_bounds__(kSkyThreads) k_sky_solve(SkyPanels P, const double *__restrict__ tilesF,
+                                                          const double *__restrict__ tilesB,
+                                                          const double *__restrict__ rhs, double *v_, double *zout,
+                                                          double *soln, int nring) {
+    __shared__ SkySmem S;
+    extern __shared__ double ring[];
+    const PanelMeta M = P.meta[blockIdx.x];
+    const int row0 = P.row0[blockIdx.x];
+    double *v = v_ + M.xUnit;
+    for (int i = threadIdx.x; i < M.nbc * TB; i += kSkyThreads) v[i] = i < M.n ? rhs[row0 + i] : 0.0;
+    __syncthreads();
+    sky_sweep<true>(M, tilesF, v, ring, nring, S);
+    for (int i = threadIdx.x; i < M.nbc * TB; i += kSkyThreads) {
+        if (i < M.n) zout[row0 + i] = v[i];
+        v[i] /= tilesF[tile_off(M, i / TB, 0) + (i % TB) * (TB + 1)];
+    }
+    __syncthreads();
+    sky_sweep<false>(M, tilesB, v, ring, nring, S);
+    for (int i = threadIdx.x; i < M.n; i += kSkyThreads) soln[row0 + i] = v[i];
 }
 
 struct RefGmresArgs {
@@ -345,22 +532,107 @@ static int sky_scratch(astro_ctx *ctx, DevBuf &b, size_t bytes) {
 // cost: one warp up to 32, then multiples of 32 up to 512.
 static int sky_threads(int maxBW) { return std::min(kT, std::max(32, (maxBW + 31) / 32 * 32)); }
 
-static int ldl_fact_dev(astro_ctx *ctx, double *d_A, const int *d_R, const int *h_R, int n) {
-    const int maxBW = skyline_maxbw(h_R, n);
-    DevBuf &diag = ctx->d_sky[3], &dl = ctx->d_sky[4];
+// The panels of a profile, with their tables packed as they lie on the device.
+struct SkyPlan {
+    std::vector<PanelMeta> meta;
+    std::vector<int> ints;  // row0 (np + 1), then sched (np) and schedPtr (np + 1): a cluster per panel
+    long long tiles = 0, rows = 0;  // of all panels
+    int maxBt = 0;
+};
+constexpr size_t kSkyRingMax = 128 * 1024;  // shared memory for the solve's ring of solved rows
+
+// Splits the profile at the rows that no later row reaches across (panels of at least 64 rows and
+// n / 128, so that a profile of many tiny blocks does not become as many padded tiles).  False where
+// band tiles do not suit the profile: the band of its longest row is so much larger than the profile
+// itself (over 8 times, and over 256 MB) or so wide that the row sweeps of one CTA are the better way.
+static bool sky_plan(const int *R, int n, SkyPlan &L) {
+    std::vector<int> reach(n + 1);  // first column of any row >= i
+    reach[n] = n;
+    for (int i = n - 1; i >= 0; --i) reach[i] = std::min(reach[i + 1], i - (R[i + 1] - R[i] - 1));
+    const int minRows = std::max(64, n / 128);
+    std::vector<int> row0(1, 0);
+    int len = 0;
+    long long band = 0;
+    for (int i = 0; i < n; ++i) {
+        len = std::max(len, R[i + 1] - R[i] - 1);
+        const int first = row0.back();
+        if (i + 1 < n && (reach[i + 1] < i + 1 || i + 1 - first < minRows)) continue;
+        PanelMeta M{};
+        M.n = i + 1 - first;
+        M.nbc = M.nfac = (M.n + TB - 1) / TB;
+        M.bt = std::min((len + TB - 1) / TB, M.nbc - 1);
+        M.band = band;
+        M.xUnit = L.rows;
+        band += (long long)M.nbc * (M.bt + 1) * TT;
+        L.rows += (long long)M.nbc * TB;
+        L.maxBt = std::max(L.maxBt, M.bt);
+        L.meta.push_back(M);
+        row0.push_back(i + 1);
+        len = 0;
+    }
+    L.tiles = band / TT;
+    if (sizeof(double) * (size_t)(L.maxBt + 2) * TB > kSkyRingMax || L.tiles > 0x7fffffffLL) return false;
+    if (band > (256LL << 20) / 8 && band > 8LL * R[n]) return false;
+    const int np = (int)L.meta.size();
+    L.ints = row0;
+    for (int p = 0; p < np; ++p) L.ints.push_back(p);
+    for (int p = 0; p <= np; ++p) L.ints.push_back(p);
+    return true;
+}
+
+// The plan's tables to the device (d_sky[5]) and the tile buffers (d_sky[6], and d_sky[7] for the
+// solves' row-major copy); the profile's row ranges are d_R.
+static int sky_upload(astro_ctx *ctx, const SkyPlan &L, const int *d_R, bool both, SkyPanels &S) {
+    DevBuf &tab = ctx->d_sky[5];
+    const size_t nb = sizeof(PanelMeta) * L.meta.size(), bytes = nb + sizeof(int) * L.ints.size();
+    const size_t tb = sizeof(double) * (size_t)L.tiles * TT;
     int rc;
-    if ((rc = sky_scratch(ctx, diag, sizeof(double) * (size_t)(n + 1))) ||
-        (rc = sky_scratch(ctx, dl, sizeof(double) * (size_t)(maxBW + 2))))
+    if ((rc = sky_scratch(ctx, tab, bytes)) || (rc = sky_scratch(ctx, ctx->d_sky[6], tb)) ||
+        (both && (rc = sky_scratch(ctx, ctx->d_sky[7], tb))))
         return rc;
+    CK(cudaMemcpyAsync(tab.p, L.meta.data(), nb, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(static_cast<char *>(tab.p) + nb, L.ints.data(), sizeof(int) * L.ints.size(),
+                       cudaMemcpyHostToDevice, ctx->stream));
+    S.meta = dptr<PanelMeta>(tab);
+    S.row0 = reinterpret_cast<const int *>(static_cast<char *>(tab.p) + nb);
+    S.R = d_R;
+    S.np = (int)L.meta.size();
+    return ASTRO_OK;
+}
+
+static int ldl_fact_dev(astro_ctx *ctx, double *d_A, const int *d_R, const int *h_R, int n) {
     int *st = dptr<int>(ctx->d_status);
-    CK(cudaMemsetAsync(st, 0, sizeof(int), ctx->stream));
-    k_ldl_fact<<<1, sky_threads(maxBW), 0, ctx->stream>>>(d_A, d_R, n, maxBW, dptr<double>(diag), dptr<double>(dl),
-                                                         st);
+    constexpr int kNone = 0x7f7f7f7f;
+    int rc, hs = 0;
+    SkyPlan L;
+    if (sky_plan(h_R, n, L)) {
+        SkyPanels S;
+        if ((rc = sky_upload(ctx, L, d_R, false, S))) return rc;
+        CK(cudaMemsetAsync(st, 0x7f, sizeof(int), ctx->stream));
+        CK(cudaMemsetAsync(st + 1, 0, sizeof(int), ctx->stream));
+        // as many CTAs a panel as its update has tiles, and as the GPU holds for all panels
+        int sms = 0, cs = 1;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+        while (cs < 16 && cs < L.maxBt * (L.maxBt + 1) / 2 && 2 * cs * S.np <= sms) cs *= 2;
+        double *tiles = dptr<double>(ctx->d_sky[6]);
+        k_sky_tiles<<<(unsigned)L.tiles, kSkyThreads, 0, ctx->stream>>>(S, d_A, tiles, nullptr);
+        const int *sched = S.row0 + S.np + 1;
+        CK(band_ldl64(S.meta, sched, sched + S.np, S.np, cs, tiles, st + 1, ctx->stream));
+        k_sky_untile<<<(unsigned)L.tiles, kSkyThreads, 0, ctx->stream>>>(S, tiles, d_A, st);
+    } else {
+        const int maxBW = skyline_maxbw(h_R, n);
+        DevBuf &diag = ctx->d_sky[3], &dl = ctx->d_sky[4];
+        if ((rc = sky_scratch(ctx, diag, sizeof(double) * (size_t)(n + 1))) ||
+            (rc = sky_scratch(ctx, dl, sizeof(double) * (size_t)(maxBW + 2))))
+            return rc;
+        CK(cudaMemsetAsync(st, 0, sizeof(int), ctx->stream));
+        k_ldl_fact<<<1, sky_threads(maxBW), 0, ctx->stream>>>(d_A, d_R, n, maxBW, dptr<double>(diag),
+                                                             dptr<double>(dl), st);
+    }
     CK(cudaGetLastError());
-    int hs = 0;
     CK(cudaMemcpyAsync(&hs, st, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    if (hs) return set_err(ctx, ASTRO_ERR_PIVOT, "zero or non-finite pivot in row " + std::to_string(hs));
+    if (hs && hs != kNone) return set_err(ctx, ASTRO_ERR_PIVOT, "zero or non-finite pivot in row " + std::to_string(hs));
     return ASTRO_OK;
 }
 
@@ -405,9 +677,24 @@ extern "C" int astro_ldl_solve(astro_ctx *ctx, double *soln, const double *rhs, 
     CK(cudaMemcpyAsync(dL.p, l_mat, sizeof(double) * (size_t)l_size, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(dR.p, l_range, sizeof(int) * (size_t)(l_dim + 1), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(db.p, rhs, sizeof(double) * (size_t)l_dim, cudaMemcpyHostToDevice, ctx->stream));
-    k_ldl_solve<<<1, sky_threads(maxBW), 0, ctx->stream>>>(dptr<double>(dx), dptr<double>(db), dptr<double>(dL),
-                                                          dptr<int>(dR), l_dim, maxBW, dptr<double>(dz));
-    CK(cudaGetLastError());
+    SkyPlan P;
+    if (sky_plan(l_range, l_dim, P)) {
+        SkyPanels S;
+        if ((rc = sky_upload(ctx, P, dptr<int>(dR), true, S)) ||
+            (rc = sky_scratch(ctx, ctx->d_sky[8], sizeof(double) * (size_t)P.rows)))
+            return rc;
+        double *tf = dptr<double>(ctx->d_sky[6]), *tb = dptr<double>(ctx->d_sky[7]);
+        k_sky_tiles<<<(unsigned)P.tiles, kSkyThreads, 0, ctx->stream>>>(S, dptr<double>(dL), tf, tb);
+        const int nring = P.maxBt + 2;
+        const size_t smem = sizeof(double) * (size_t)nring * TB;
+        CK(cudaFuncSetAttribute(k_sky_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSkyRingMax));
+        k_sky_solve<<<(unsigned)S.np, kSkyThreads, smem, ctx->stream>>>(S, tf, tb, dptr<double>(db),
+                                                                       dptr<double>(ctx->d_sky[8]),
+                                                                       dptr<double>(dz), dptr<double>(dx), nring);
+    } else {
+        k_ldl_solve<<<1, sky_threads(maxBW), 0, ctx->stream>>>(dptr<double>(dx), dptr<double>(db), dptr<double>(dL),
+                                                              dptr<int>(dR), l_dim, maxBW, dptr<double>(dz));
+    }
     CK(cudaMemcpyAsync(soln, dx.p, sizeof(double) * (size_t)l_dim, cudaMemcpyDeviceToHost, ctx->stream));
     if (z_vec) CK(cudaMemcpyAsync(z_vec, dz.p, sizeof(double) * (size_t)l_dim, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));

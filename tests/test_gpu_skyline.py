@@ -108,3 +108,64 @@ def test_zero_pivot_reports_error():
     with pytest.raises(AstroError) as e:
         g.getSparseLDLFact(lt, o.lt_range)
     assert e.value.code == 4
+
+
+def _profile(lens, seed, zero_row=None):
+    """A diagonally dominant row skyline with off-diagonal row lengths lens (clipped to the row
+    number); zero_row (0-based) gets a zero diagonal and no off-diagonal entries of its own."""
+    rng = np.random.default_rng(seed)
+    n = len(lens)
+    lens = np.minimum(lens, np.arange(n))
+    if zero_row is not None:
+        lens[zero_row] = 0
+    r = np.concatenate([[0], np.cumsum(lens + 1)]).astype(np.int32)
+    a = rng.uniform(-1.0, 1.0, r[-1])
+    off = np.zeros(n)
+    for i in range(n):
+        row = a[r[i]:r[i + 1] - 1]
+        off[i] += np.abs(row).sum()
+        off[i - lens[i]:i] += np.abs(row)
+    a[r[1:] - 1] = 1.0 + off
+    if zero_row is not None:
+        a[r[zero_row + 1] - 1] = 0.0
+    return a, r
+
+
+PROFILES = {
+    "one_row": np.zeros(1, int),
+    "diagonal": np.zeros(300, int),
+    "tile_less_one": np.full(31, 30),
+    "one_tile": np.full(32, 31),
+    "tile_plus_one": np.full(33, 32),
+    "band_31": np.full(200, 31),
+    "band_32": np.full(200, 32),
+    "band_33": np.full(131, 33),
+    "ragged": np.random.default_rng(0).integers(0, 140, 500),
+    "blocks": np.concatenate([np.minimum(np.arange(k), w) for k, w in ((70, 9), (64, 63), (90, 40), (5, 4), (200, 100))]),
+    "wide": np.full(900, 470),
+    "arrow": np.concatenate([np.full(11999, 2), [11999]]),  # kept on the row sweeps: one row spans the profile
+}
+
+
+@pytest.mark.parametrize("name", list(PROFILES))
+def test_factor_and_solve_over_profiles(system, name):
+    """Panels, tiles and the chain of block rows where they change: row lengths around the tile
+    edge, rows that no later row reaches across, and a profile that band tiles do not suit."""
+    if system["name"] != "hex":
+        pytest.skip("one context is enough")
+    o, g = system["o"], system["g"]
+    a, r = _profile(PROFILES[name], 3)
+    fac, fo = g.getSparseLDLFact(a, r), o.ldl_fact(a, r)
+    assert _nrel(fac, fo) < 1e-10
+    rhs = np.random.default_rng(4).standard_normal(len(r) - 1)
+    assert _nrel(g.solveSparseLDLFact(rhs, fo, r), o.ldl_solve(fo, r, rhs)) < 1e-10
+
+
+@pytest.mark.parametrize("row", [0, 33, 150])
+def test_first_zero_pivot_is_reported(system, row):
+    if system["name"] != "hex":
+        pytest.skip("one context is enough")
+    a, r = _profile(PROFILES["blocks"].copy(), 5, zero_row=row)
+    with pytest.raises(AstroError) as e:
+        system["g"].getSparseLDLFact(a, r)
+    assert e.value.code == 4 and str(e.value).endswith(f"row {row + 1}")
