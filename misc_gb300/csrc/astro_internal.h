@@ -265,6 +265,9 @@ int solid_drdd_batch(astro_ctx *ctx, int d0, int nd, double h, const ElemDevStat
 int solid_orient_prepare(astro_ctx *ctx);
 int shell4_drdd(astro_ctx *ctx, int dvar, double h, const ElemDevState &s, double *d_acc,
                 double *d_intAcc);                                                              // elem_shell4.cu
+int shell4_drdd_condensed(astro_ctx *ctx, int num, const int *dvars, double h, const ElemDevState &s,
+                          double *d_out);                                                       // elem_shell4.cu
+int scale_neg(astro_ctx *ctx, long long n, double s, double *d_x);  // x = s (-x) (ctx.cu)
 void krylov_release(astro_ctx *ctx);
 // per-step device histories of the time loop (reference numbering; any may be null)
 struct NewmarkHist {

@@ -786,9 +786,14 @@ void dvar_elements_by_colour(const astro_ctx *ctx, int dvar, std::vector<int> &l
     }
 }
 
-__global__ void k_scale_neg(int n, const double *x, double s, double *y) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) y[i] = s * -x[i];
+__global__ void k_scale_neg(long long n, double s, double *x) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i < n) x[i] = s * -x[i];
+}
+
+int scale_neg(astro_ctx *ctx, long long n, double s, double *d_x) {
+    if (n > 0) k_scale_neg<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(n, s, d_x);
+    return cuda_check(ctx, cudaGetLastError(), "scale");
 }
 
 // getdRelasticdD, element part (Working/AStrO_commandFunctions.f90:1172-1250).  The elements that
@@ -828,9 +833,8 @@ static int drdd_device(astro_ctx *ctx, int dvar, double h, DrddState &D, double 
     }
     if (rc) return rc;
     const double hInv = 1.0 / h;
-    k_scale_neg<<<(n + 255) / 256, 256, 0, ctx->stream>>>(n, d_acc, hInv, d_acc);
-    if (ni > 0 && d_iacc) k_scale_neg<<<(ni + 255) / 256, 256, 0, ctx->stream>>>(ni, d_iacc, hInv, d_iacc);
-    return cuda_check(ctx, cudaGetLastError(), "drdd");
+    if ((rc = scale_neg(ctx, n, hInv, d_acc))) return rc;
+    return d_iacc ? scale_neg(ctx, ni, hInv, d_iacc) : ASTRO_OK;
 }
 
 extern "C" int astro_drdd_complex(astro_ctx *ctx, int32_t dvar, double h, const astro_state *state, double *drudd,
@@ -890,11 +894,19 @@ extern "C" int astro_drdd_complex_condensed(astro_ctx *ctx, int32_t num, const i
             dev_free(out);
         }
     } T;
-    if ((rc = dev_alloc(ctx, T.acc, sizeof(double) * n)) ||
+    const bool all = ctx->hasShell != 0;  // shells: all variables at once
+    if ((rc = dev_alloc(ctx, T.acc, sizeof(double) * (size_t)n * (all ? num : 1))) ||
         (rc = dev_alloc(ctx, T.out, sizeof(double) * (size_t)n * num)))
         return rc;
-    if (ni > 0 && (rc = dev_alloc(ctx, T.iacc, sizeof(double) * ni))) return rc;
-    for (int k = 0; k < num; ++k) {
+    if (all) {
+        if ((rc = shell4_drdd_condensed(ctx, num, dvars, h, D.ds, dptr<double>(T.acc)))) return rc;
+        for (int k = 0; k < num; ++k)
+            if ((rc = int_to_ref_vec(ctx, dptr<double>(T.acc) + (size_t)k * n, dptr<double>(T.out) + (size_t)k * n, n)))
+                return rc;
+    } else if (ni > 0 && (rc = dev_alloc(ctx, T.iacc, sizeof(double) * ni))) {
+        return rc;
+    }
+    for (int k = 0; k < num && !all; ++k) {
         if ((rc = drdd_device(ctx, dvars[k], h, D, dptr<double>(T.acc), ni > 0 ? dptr<double>(T.iacc) : nullptr)))
             return rc;
         if (condense && (rc = elem_update_external_rhs(ctx, dptr<double>(T.iacc), dptr<double>(T.acc)))) return rc;

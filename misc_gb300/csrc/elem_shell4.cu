@@ -18,8 +18,9 @@
 // stale column offset there; its evident intent is kept).
 //
 // Mapping: the evaluation is a pipeline of one-thread-per-item kernels (elem_shell4_pipe.cuh)
-// over per-element global scratch, run one element colour at a time; elements of a colour share
-// no node, so their 6x6 block updates never collide (no atomics, deterministic).
+// over per-element global scratch; the element stages take the elements of all colours at once, the
+// updates of shared entries one colour at a time: elements of a colour share no node, so their 6x6
+// block updates never collide (no atomics, deterministic).
 #include <algorithm>
 #include <functional>
 
@@ -96,30 +97,36 @@ int shell_sections_prepare(astro_ctx *ctx, const astro_model *m) {
     return cuda_check(ctx, e, "shell properties");
 }
 
-// The five pipeline kernels over the elements of each colour in turn: colour c covers
-// els[ptr[c] .. ptr[c+1]) (device list).
+// The pipeline over a colour-grouped element list: colour c covers els[ptr[c] .. ptr[c+1]) (device
+// list).  The list is taken in chunks whose scratch (22.6 KB an element) stays below 0.75 GB; a chunk
+// may cover several colours and a colour several chunks, the updates keep the order of the list.
+// byItem (complex step): element k of the list has its own properties, props[k], and with slot adds to
+// load vector slot[k] (of lengths n and intVecSize).
+constexpr int kShellChunk = 32768;
+
 static int shell_pipeline(astro_ctx *ctx, const ElemDevState &st, const int *d_els, const std::vector<int> &ptr,
                           const ShellProps *props, double gpc, double *d_loadInt, double *d_intLoad, int buildMat,
-                          double *d_K, double *d_intMat, double *d_ke, double *d_ru, bool sync = true) {
-    int maxc = 0;
-    for (size_t c = 0; c + 1 < ptr.size(); ++c) maxc = std::max(maxc, ptr[c + 1] - ptr[c]);
-    if (!maxc) return ASTRO_OK;
+                          double *d_K, double *d_intMat, double *d_ke, double *d_ru, bool sync = true,
+                          bool byItem = false, const int *slot = nullptr) {
+    const int first = ptr.front(), last = ptr.back();
+    if (first == last) return ASTRO_OK;
     // per-element scratch of the pipeline, kept in the context (grown on demand)
     DevBuf &fr = ctx->d_shFr, &gp = ctx->d_shGp, &de = ctx->d_shDe, &kf = ctx->d_shKf;
     int rc;
-    if (maxc > ctx->shScratchEls) {
-        if ((rc = dev_alloc(ctx, fr, sizeof(ShellFrame) * (size_t)maxc))) return rc;
-        if ((rc = dev_alloc(ctx, gp, sizeof(ShellGP) * 4 * (size_t)maxc))) return rc;
-        if ((rc = dev_alloc(ctx, de, sizeof(double) * 4 * 32 * 9 * (size_t)maxc))) return rc;
-        if ((rc = dev_alloc(ctx, kf, sizeof(double) * 32 * 33 * (size_t)maxc))) return rc;
-        ctx->shScratchEls = maxc;
+    const int cap = std::min(kShellChunk, last - first);
+    if (cap > ctx->shScratchEls) {
+        ctx->shScratchEls = 0;
+        if ((rc = dev_alloc(ctx, fr, sizeof(ShellFrame) * (size_t)cap))) return rc;
+        if ((rc = dev_alloc(ctx, gp, sizeof(ShellGP) * 4 * (size_t)cap))) return rc;
+        if ((rc = dev_alloc(ctx, de, sizeof(double) * 4 * 32 * 9 * (size_t)cap))) return rc;
+        if ((rc = dev_alloc(ctx, kf, sizeof(double) * 32 * 33 * (size_t)cap))) return rc;
+        ctx->shScratchEls = cap;
     }
     ShellPipe A = {};
     A.nodes = dptr<double>(ctx->d_nodes);
     A.elist = dptr<int>(ctx->d_elist);
     A.rank = dptr<int>(ctx->d_rank);
     A.elBlk = dptr<int>(ctx->d_elBlk);
-    A.props = props;
     A.disp = st.disp;
     A.pdisp = st.pdisp;
     A.pvel = st.pvel;
@@ -149,10 +156,15 @@ static int shell_pipeline(astro_ctx *ctx, const ElemDevState &st, const int *d_e
     A.scratchEls = ctx->shScratchEls;
     A.status = ASTRO_CHECKED ? dptr<int>(ctx->d_guard) : nullptr;
     cudaStream_t s = ctx->stream;
-    for (size_t col = 0; col + 1 < ptr.size(); ++col) {
-        const int cnt = ptr[col + 1] - ptr[col];
-        if (!cnt) continue;
-        A.els = d_els + ptr[col];
+    A.propsByItem = byItem;
+    A.loadLen = (size_t)ctx->P.n;
+    A.intLoadLen = (size_t)ctx->P.intVecSize;
+    size_t col = 0;
+    for (int c0 = first; c0 < last; c0 += cap) {
+        const int c1 = std::min(last, c0 + cap), cnt = c1 - c0;
+        A.els = d_els + c0;
+        A.props = props + (byItem ? c0 : 0);
+        A.slot = slot ? slot + c0 : nullptr;
         A.count = cnt;
         k_shell_frame<<<(cnt + 63) / 64, 64, 0, s>>>(A);
         k_shell_frame_rot<<<(10 * cnt + 63) / 64, 64, 0, s>>>(A);
@@ -160,12 +172,22 @@ static int shell_pipeline(astro_ctx *ctx, const ElemDevState &st, const int *d_e
         if (A.dynamic) k_shell_inam<<<(4 * cnt + 127) / 128, 128, 0, s>>>(A);
         k_shell_gauss<<<(4 * cnt + 127) / 128, 128, 0, s>>>(A);
         k_shell_dedu<<<(128 * cnt + 127) / 128, 128, 0, s>>>(A);
-        k_shell_kcol<<<(32 * cnt + 127) / 128, 128, 0, s>>>(A);
+        k_shell_kcol<<<(32 * cnt + kKcolThreads - 1) / kKcolThreads, kKcolThreads, 0, s>>>(A);
         if (A.buildMat) {
             k_shell_cond_lu<<<(cnt + 63) / 64, 64, 0, s>>>(A);
             k_shell_cond_col<<<(24 * cnt + 127) / 128, 128, 0, s>>>(A);
         }
-        k_shell_scatter<<<(32 * cnt + 127) / 128, 128, 0, s>>>(A);
+        // the colours of the chunk
+        while (col + 2 < ptr.size() && ptr[col + 1] <= c0) ++col;
+        for (size_t c = col; c + 1 < ptr.size() && ptr[c] < c1; ++c) {
+            const int b0 = std::max(ptr[c], c0), b1 = std::min(ptr[c + 1], c1);
+            if (b0 >= b1) continue;
+            A.q0 = b0 - c0;
+            A.count = b1 - b0;
+            if (A.buildMat && A.K)
+                k_shell_addk<<<(unsigned)((576LL * A.count + 255) / 256), 256, 0, s>>>(A);
+            k_shell_scatter<<<(32 * A.count + 127) / 128, 128, 0, s>>>(A);
+        }
     }
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess && (sync || ASTRO_CHECKED)) e = cudaStreamSynchronize(s);
@@ -189,25 +211,38 @@ int launch_shell4_assemble(astro_ctx *ctx, const ElemDevState &st, double *d_loa
                           toK ? dptr<double>(ctx->d_intMat) : nullptr, d_ke, d_ru, sync);
 }
 
-// Complex-step properties of the listed elements: orientation (real part), imaginary parts of
-// ABD and of the section mass, written over a copy of the per-element properties.
-__global__ void k_shell_props_im(int count, const int *els, const double *nodes, const int *elist, const int *esec,
-                                 const double *secOrient, const int *layRange, const LayerDev *lay, const double *zoff,
-                                 const int *e2dR, const int *e2d, const double *e2c, const int *dcat, const int *dlay,
-                                 const int *dcomp, const double *dval, int dvar, double h, ShellProps *out) {
+// Complex-step properties of the listed elements, one entry per listed element: orientation (real
+// part), imaginary parts of ABD and of the section mass, for design variable dvar or, with slot,
+// dvars[slot[q]].
+__global__ void k_shell_props_im(int count, const int *els, const int *slot, const int *dvars, const double *nodes,
+                                 const int *elist, const int *esec, const double *secOrient, const int *layRange,
+                                 const LayerDev *lay, const double *zoff, const int *e2dR, const int *e2d,
+                                 const double *e2c, const int *dcat, const int *dlay, const int *dcomp,
+                                 const double *dval, int dvar, double h, ShellProps *out) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= count) return;
     const int e = els[q];
     cplx o[3][3], ABD[9][9], M[6][6];
     shell_props<cplx>(nodes, elist + 8 * (size_t)e, secOrient, esec[e], layRange, lay, zoff, e2dR, e2d, e2c, dcat, dlay,
-                      dcomp, dval, e, dvar, h, o, ABD, M);
-    ShellProps &P = out[e];
+                      dcomp, dval, e, slot ? dvars[slot[q]] : dvar, h, o, ABD, M);
+    ShellProps &P = out[q];
     for (int i = 0; i < 3; ++i)
         for (int j = 0; j < 3; ++j) P.orient[3 * i + j] = o[i][j].re;
     for (int i = 0; i < 9; ++i)
         for (int j = 0; j < 9; ++j) P.ABD[9 * i + j] = ABD[i][j].im;
     for (int i = 0; i < 6; ++i)
         for (int j = 0; j < 6; ++j) P.M[6 * i + j] = M[i][j].im;
+}
+
+static int shell_props_im(astro_ctx *ctx, int cnt, const int *d_list, const int *d_slot, const int *d_dvars, int dvar,
+                          double h, ShellProps *out) {
+    k_shell_props_im<<<(cnt + 63) / 64, 64, 0, ctx->stream>>>(
+        cnt, d_list, d_slot, d_dvars, dptr<double>(ctx->d_nodes), dptr<int>(ctx->d_elist), dptr<int>(ctx->d_esec),
+        dptr<double>(ctx->d_secOrient), dptr<int>(ctx->d_shLayRange), dptr<LayerDev>(ctx->d_shLay),
+        dptr<double>(ctx->d_shZoff), dptr<int>(ctx->d_e2dR), dptr<int>(ctx->d_e2d), dptr<double>(ctx->d_e2c),
+        dptr<int>(ctx->d_dCat), dptr<int>(ctx->d_dLayer), dptr<int>(ctx->d_dComp), dptr<double>(ctx->d_dVal), dvar, h,
+        out);
+    return cuda_check(ctx, cudaGetLastError(), "shell complex-step properties");
 }
 
 // Complex step of the pipeline's residual over a colour-grouped element list (colour c covering
@@ -218,29 +253,17 @@ int shell4_drdd_list(astro_ctx *ctx, int dvar, double h, const ElemDevState &st,
                      const std::function<int(const int *, int)> &hook) {
     const int cnt = (int)list.size();
     if (!cnt) return ASTRO_OK;
-    const int E = ctx->P.E;
     DevBuf dl, props;
     int rc;
     if ((rc = upload(ctx, dl, list.data(), sizeof(int) * cnt))) return rc;
-    if ((rc = dev_alloc(ctx, props, sizeof(ShellProps) * (size_t)E))) {
+    if ((rc = dev_alloc(ctx, props, sizeof(ShellProps) * (size_t)cnt))) {
         dev_free(dl);
         return rc;
     }
-    cudaError_t e = cudaMemcpyAsync(props.p, ctx->d_secABD.p, sizeof(ShellProps) * (size_t)E, cudaMemcpyDeviceToDevice,
-                                    ctx->stream);
-    if (e == cudaSuccess) {
-        k_shell_props_im<<<(cnt + 63) / 64, 64, 0, ctx->stream>>>(
-            cnt, dptr<int>(dl), dptr<double>(ctx->d_nodes), dptr<int>(ctx->d_elist), dptr<int>(ctx->d_esec),
-            dptr<double>(ctx->d_secOrient), dptr<int>(ctx->d_shLayRange), dptr<LayerDev>(ctx->d_shLay),
-            dptr<double>(ctx->d_shZoff), dptr<int>(ctx->d_e2dR), dptr<int>(ctx->d_e2d), dptr<double>(ctx->d_e2c),
-            dptr<int>(ctx->d_dCat), dptr<int>(ctx->d_dLayer), dptr<int>(ctx->d_dComp), dptr<double>(ctx->d_dVal), dvar, h,
-            dptr<ShellProps>(props));
-        e = cudaGetLastError();
-    }
-    rc = cuda_check(ctx, e, "shell complex-step properties");
+    rc = shell_props_im(ctx, cnt, dptr<int>(dl), nullptr, nullptr, dvar, h, dptr<ShellProps>(props));
     if (!rc && !hook)
         rc = shell_pipeline(ctx, st, dptr<int>(dl), ptr, dptr<ShellProps>(props), kShellRt3c, d_acc, d_intAcc, 0, nullptr,
-                            nullptr, nullptr, nullptr);
+                            nullptr, nullptr, nullptr, true, true);
     for (size_t c = 0; !rc && hook && c + 1 < ptr.size(); ++c) {
         const int n = ptr[c + 1] - ptr[c];
         if (!n) continue;
@@ -248,19 +271,25 @@ int shell4_drdd_list(astro_ctx *ctx, int dvar, double h, const ElemDevState &st,
         const std::vector<int> one = {ptr[c], ptr[c + 1]};
         if (!rc)
             rc = shell_pipeline(ctx, st, dptr<int>(dl), one, dptr<ShellProps>(props), kShellRt3c, d_acc, d_intAcc, 0,
-                                nullptr, nullptr, nullptr, nullptr);
+                                nullptr, nullptr, nullptr, nullptr, true, true);
     }
     dev_free(dl);
     dev_free(props);
     return rc;
 }
 
-int shell4_drdd(astro_ctx *ctx, int dvar, double h, const ElemDevState &st, double *d_acc, double *d_intAcc) {
+static int shell_dvar_check(astro_ctx *ctx, int dvar) {
     const int cat = ctx->dCat[dvar - 1];
     if (cat == ASTRO_DCAT_ORIENTATION || cat == ASTRO_DCAT_NODE_COORD)
         return set_err(ctx, ASTRO_ERR_UNSUPPORTED,
                        "complex step of shell orientation or node-coordinate design variables (they enter the shell "
                        "kinematics, which run in real arithmetic) is not provided");
+    return ASTRO_OK;
+}
+
+int shell4_drdd(astro_ctx *ctx, int dvar, double h, const ElemDevState &st, double *d_acc, double *d_intAcc) {
+    int rc = shell_dvar_check(ctx, dvar);
+    if (rc) return rc;
     std::vector<int> list, ptr;
     dvar_elements_by_colour(ctx, dvar, list, ptr);
     return shell4_drdd_list(ctx, dvar, h, st, list, ptr, d_acc, d_intAcc, nullptr);
@@ -275,10 +304,15 @@ int shell4_drdd(astro_ctx *ctx, int dvar, double h, const ElemDevState &st, doub
 // updates of a launch never collide).
 __global__ void k_shell_ext_rhs(int count, const int *__restrict__ els, const int *__restrict__ elist,
                                 const int *__restrict__ rank, const double *__restrict__ intMat,
-                                const double *__restrict__ intVec, double *__restrict__ extInt) {
+                                const double *__restrict__ intVec, double *__restrict__ extInt,
+                                const int *__restrict__ slot = nullptr, size_t intLen = 0, size_t extLen = 0) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= count) return;
     const int e = els[q];
+    if (slot) {  // vector slot[q] of several
+        intVec += slot[q] * intLen;
+        extInt += slot[q] * extLen;
+    }
     const double *M = intMat + 256 * (size_t)e;
     double L[8][8], b[8], x[8];
     for (int r = 0; r < 8; ++r)
@@ -325,6 +359,87 @@ int shell4_update_external_rhs(astro_ctx *ctx, const double *d_intVec, double *d
             dptr<double>(ctx->d_intMat), d_intVec, d_extInt);
     }
     return cuda_check(ctx, cudaGetLastError(), "shell external rhs");
+}
+
+// The complex-step derivatives of design variables dvars[0 .. num-1], condensed to the nodal DOF, into
+// d_out (num x n): all (element, variable) items of a colour together, so that small groups of elements
+// fill the GPU and the stages run once (32 panels, 8 thickness groups of 1,768 elements: @DRDD@).
+// The variables are taken in groups whose items' properties (1 KB each) stay below a GB or so.
+int shell4_drdd_condensed(astro_ctx *ctx, int num, const int *dvars, double h, const ElemDevState &st, double *d_out) {
+    const AstroPrep &P = ctx->P;
+    const size_t n = (size_t)P.n, ni = (size_t)P.intVecSize;
+    int rc;
+    std::vector<long long> count(ctx->numDvars + 1, 0);
+    for (int e = 0; e < P.E; ++e)
+        for (int q = ctx->e2dRange[e]; q < ctx->e2dRange[e + 1]; ++q) ++count[ctx->e2d[q]];
+    for (int k = 0; k < num; ++k)
+        if ((rc = shell_dvar_check(ctx, dvars[k]))) return rc;
+    const long long limit = std::max<long long>(P.E, 1 << 20);
+    struct Tmp {
+        DevBuf iacc, list, slot, dv, props;
+        ~Tmp() {
+            DevBuf *b[] = {&iacc, &list, &slot, &dv, &props};
+            for (DevBuf *x : b) dev_free(*x);
+        }
+    } T;
+    for (int k0 = 0; k0 < num;) {
+        int k1 = k0;
+        long long items = 0;
+        std::vector<std::vector<int>> slots(ctx->numDvars + 1);  // of each variable in this group
+        while (k1 < num && (k1 == k0 || items + count[dvars[k1]] <= limit)) {
+            items += count[dvars[k1]];
+            slots[dvars[k1]].push_back(k1 - k0);
+            ++k1;
+        }
+        const int g = k1 - k0;
+        std::vector<int> list, slot, ptr(1, 0);
+        for (int col = 0; col < P.ncolors; ++col) {
+            for (int c = P.colorPtr[col]; c < P.colorPtr[col + 1]; ++c) {
+                const int e = P.colorEls[c];
+                for (int q = ctx->e2dRange[e]; q < ctx->e2dRange[e + 1]; ++q) {
+                    bool seen = false;  // a variable with several terms on the element is one item
+                    for (int p = ctx->e2dRange[e]; p < q; ++p) seen = seen || ctx->e2d[p] == ctx->e2d[q];
+                    if (seen) continue;
+                    for (int sl : slots[ctx->e2d[q]]) {
+                        list.push_back(e);
+                        slot.push_back(sl);
+                    }
+                }
+            }
+            ptr.push_back((int)list.size());
+        }
+        double *acc = d_out + (size_t)k0 * n;
+        CK(cudaMemsetAsync(acc, 0, sizeof(double) * n * g, ctx->stream));
+        if (!list.empty()) {
+            const int cnt = (int)list.size();
+            if ((rc = upload(ctx, T.list, list.data(), sizeof(int) * cnt)) ||
+                (rc = upload(ctx, T.slot, slot.data(), sizeof(int) * cnt)) ||
+                (rc = upload(ctx, T.dv, dvars + k0, sizeof(int) * g)) ||
+                (rc = dev_alloc(ctx, T.props, sizeof(ShellProps) * (size_t)cnt)) ||
+                (rc = dev_alloc(ctx, T.iacc, sizeof(double) * ni * g)))
+                return rc;
+            CK(cudaMemsetAsync(T.iacc.p, 0, sizeof(double) * ni * g, ctx->stream));
+            double *iacc = dptr<double>(T.iacc);
+            if ((rc = shell_props_im(ctx, cnt, dptr<int>(T.list), dptr<int>(T.slot), dptr<int>(T.dv), 0, h,
+                                     dptr<ShellProps>(T.props))) ||
+                (rc = shell_pipeline(ctx, st, dptr<int>(T.list), ptr, dptr<ShellProps>(T.props), kShellRt3c, acc, iacc, 0,
+                                     nullptr, nullptr, nullptr, nullptr, false, true, dptr<int>(T.slot))) ||
+                (rc = scale_neg(ctx, (long long)n * g, 1.0 / h, acc)) ||
+                (rc = scale_neg(ctx, (long long)ni * g, 1.0 / h, iacc)))
+                return rc;
+            // only the listed elements have an internal part
+            for (int col = 0; col < P.ncolors; ++col) {
+                const int c = ptr[col + 1] - ptr[col];
+                if (c)
+                    k_shell_ext_rhs<<<(c + 127) / 128, 128, 0, ctx->stream>>>(
+                        c, dptr<int>(T.list) + ptr[col], dptr<int>(ctx->d_elist), dptr<int>(ctx->d_rank),
+                        dptr<double>(ctx->d_intMat), iacc, acc, dptr<int>(T.slot) + ptr[col], ni, n);
+            }
+            if ((rc = cuda_check(ctx, cudaGetLastError(), "shell design derivatives"))) return rc;
+        }
+        k0 = k1;
+    }
+    return ASTRO_OK;
 }
 
 int shell4_update_internal_soln(astro_ctx *ctx, const double *d_extInt, double *d_intSoln, const double *d_intRhs) {

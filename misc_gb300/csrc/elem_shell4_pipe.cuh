@@ -1,6 +1,8 @@
 // shell4 element evaluation as a pipeline of one-thread-per-item kernels over per-element global
-// scratch (device code; the algorithm is described in elem_shell4.cu).  For one colour's
-// elements at a time:
+// scratch (device code; the algorithm is described in elem_shell4.cu).  The element stages run over
+// the elements of all colours at once, only what adds into shared entries colour by colour: most
+// stages are a short chain of FP64 per item, so their time is that of the chain until the GPU is
+// full (1,552 elements a colour: 20-30 us a stage and colour).
 //   frame    thread per element:            state gather; then thread per (element, rotation):
 //                                            the instantaneous frame and its first and second
 //                                            rotation derivatives (ten rotations); then thread
@@ -11,9 +13,9 @@
 //   kcol     thread per (element, column j): column j of K (material + stress part) and Ru_j,
 //                                            plus the Newmark mass column
 //   cond     thread per element:             8x8 internal LU; then thread per (element,
-//                                            column): condensation, outputs and the colour-ordered
-//                                            block-CSR update (with a matrix only)
-//   scatter  thread per (element, DOF):      residual into the load vectors
+//                                            column): condensation and outputs (with a matrix only)
+//   addk     thread per (element, entry):    block-CSR update, colour by colour
+//   scatter  thread per (element, DOF):      residual into the load vectors, colour by colour
 #pragma once
 #include "bounds.cuh"
 #include "shell_props.cuh"
@@ -47,6 +49,7 @@ struct ShellPipe {
     const int *elist, *rank, *els, *elBlk;
     int count;
     const ShellProps *props;
+    int propsByItem;  // props holds one entry per listed element (complex step), else per element
     const double *disp, *pdisp, *pvel, *pacc, *idisp;
     int dynamic;
     double beta, gamma, delT;
@@ -58,11 +61,18 @@ struct ShellPipe {
     double *dedU;    // count*4*32*9
     double *Kf;      // count*32*33: column j = 33 values (K(0..31, j), Ru_j)
     double *K, *load, *intLoad, *intMat, *keOut, *ruOut;
+    const int *slot;            // per listed element the load vector it adds to (null: the first)
+    size_t loadLen, intLoadLen;  // distance of two load vectors
+    int q0;                     // first element of the colour in the chunk (addk, scatter)
     // sizes the index guards of the checked build test against (bounds.cuh): nodes, elements,
     // block-CSR blocks, elements the scratch above holds; status receives the failing guard's site
     int nNodes, nEls, nBlocks, scratchEls;
     int *status;
 };
+
+__device__ __forceinline__ const ShellProps &item_props(const ShellPipe &A, int q, int e) {
+    return A.props[A.propsByItem ? q : e];
+}
 
 // The frame stage in three parts: the gather (per element), the ten frame rotations (per
 // element and rotation: the instantaneous frame and its first and second derivatives, the costly
@@ -73,7 +83,7 @@ __device__ void pipe_frame_gather(const ShellPipe &A, int q) {
     ASTRO_GUARD(A.status, 102, ASTRO_IN(e, A.nEls));
     const int *el = A.elist + 8 * (size_t)e;
     for (int a = 0; a < 4; ++a) ASTRO_GUARD(A.status, 103, ASTRO_IN(el[a] - 1, A.nNodes));
-    const ShellProps &P = A.props[e];
+    const ShellProps &P = item_props(A, q, e);
     ShellFrame &F = A.fr[q];
     double orient[3][3];
     for (int i = 0; i < 9; ++i) orient[i / 3][i % 3] = P.orient[i];
@@ -106,7 +116,7 @@ __device__ void pipe_frame_rot(const ShellPipe &A, int q, int v) {
     ASTRO_GUARD(A.status, 111, ASTRO_IN(q, A.scratchEls) && ASTRO_IN(v, 10));
     const int e = A.els[q];
     ASTRO_GUARD(A.status, 112, ASTRO_IN(e, A.nEls));
-    const ShellProps &P = A.props[e];
+    const ShellProps &P = item_props(A, q, e);
     ShellFrame &F = A.fr[q];
     double orient[3][3];
     for (int i = 0; i < 9; ++i) orient[i / 3][i % 3] = P.orient[i];
@@ -138,7 +148,7 @@ __device__ void pipe_frame_rest(const ShellPipe &A, int q) {
     const int e = A.els[q];
     ASTRO_GUARD(A.status, 122, ASTRO_IN(e, A.nEls));
     const int *el = A.elist + 8 * (size_t)e;
-    const ShellProps &P = A.props[e];
+    const ShellProps &P = item_props(A, q, e);
     ShellFrame &F = A.fr[q];
     double orient[3][3];
     for (int i = 0; i < 9; ++i) orient[i / 3][i % 3] = P.orient[i];
@@ -206,7 +216,7 @@ __device__ void pipe_gauss(const ShellPipe &A, int q, int g) {
     ASTRO_GUARD(A.status, 131, ASTRO_IN(q, A.scratchEls) && ASTRO_IN(g, 4) && ASTRO_IN(A.els[q], A.nEls));
     const ShellFrame &F = A.fr[q];
     ShellGP &G = A.gp[4 * (size_t)q + g];
-    const ShellProps &P = A.props[A.els[q]];
+    const ShellProps &P = item_props(A, q, A.els[q]);
     const double r3 = A.gpc;
     const double s1 = (g & 1) ? r3 : -r3, s2 = (g & 2) ? r3 : -r3;
     double N[11], d0[11], d1[11];
@@ -324,40 +334,91 @@ __device__ void def_first(const ShellFrame &F, const ShellGP &G, int i, int quir
     shell_def(ux, rx, pr, d);
 }
 
-// second derivative of the deformation vector with respect to DOF i and j (0-based)
-__device__ void def_second(const ShellFrame &F, const ShellGP &G, int i, int j, double d[9]) {
-    int vi, ni, vj, nj;
-    dof_of(i, vi, ni);
-    dof_of(j, vj, nj);
-    int var1, nd1, var2, nd2;
-    if (vi < vj) {
-        var1 = vi; nd1 = ni; var2 = vj; nd2 = nj;
-    } else {
-        var1 = vj; nd1 = nj; var2 = vi; nd2 = ni;
-    }
-    double ux[3][3] = {}, rx[3][3] = {}, pr[3] = {0.0, 0.0, 0.0};
-    if (var1 < 4 && var2 >= 4) {
-        const int v2 = var2 - 3;
-        for (int a = 0; a < 3; ++a)
-            for (int b = 0; b < 3; ++b) ux[a][b] = 0.25 * F.io[v2][3 * a + var1 - 1] * G.Nx[nd1 - 1][b];
-    } else if (var1 >= 4 && var2 >= 4) {
-        const int blk = 4 * (var1 - 3) + (var2 - 3);
-        for (int a = 0; a < 3; ++a) {
-            double tr[4];
-            for (int n = 0; n < 4; ++n) {
-                double s = 0.0;
-                for (int k = 0; k < 3; ++k) s += F.io[blk][3 * a + k] * (F.u[k][n] + F.X[n][k]);
-                tr[n] = 0.0625 * s;
-            }
-            for (int b = 0; b < 3; ++b) ux[a][b] = tr[0] * G.Nx[0][b] + tr[1] * G.Nx[1][b] + tr[2] * G.Nx[2][b] + tr[3] * G.Nx[3][b];
+// The stress part of K, sum_g w detJ F . d2 def/du_i du_j, needs no second derivatives per (i, j):
+// they are nonzero only with a rotation among i, j, and linear in the shape functions, so the points
+// enter through T[n][a] = sum_g w detJ Fu_a . Nx_n and Q[n][a] = sum_g w detJ (Fp_a N_n + Fr_a . Nx_n)
+// (Fu, Fr, Fp: the section force as the factors of the displacement gradient, the rotation gradient
+// and the rotation in the deformation vector):
+//   translation v of node n, rotation r (any node):  1/4 sum_a dR_r(a, v) T[n][a]
+//   rotations r of node m, s of node n:              G[r][s] + [m = n] sum_a dr_rs(a) Q[n][a],
+//                      G[r][s] = 1/16 sum_n sum_a (d2R_rs (u + X)_n)(a) T[n][a].
+// (6,208 elements at a displaced state: kcol 4.49 ms with the second derivatives evaluated for every
+// point and pair, @KCOL@ ms so.)
+struct ShellStress {
+    double T[10][3], Q[4][3], G[3][3];
+};
+
+// One warp per element (lane j); returns false when no point carries a section force.
+__device__ bool stress_tables(const ShellPipe &A, const ShellFrame &F, int q, int j, ShellStress &S) {
+    bool stressed = false;
+    const int n = j / 3, a = j % 3;
+    double T = 0.0, Q = 0.0;
+    for (int g = 0; g < 4; ++g) {
+        const ShellGP &G = A.gp[4 * (size_t)q + g];
+        const double *f = G.F;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) stressed = stressed || f[k] != 0.0;
+        if (n >= 10) continue;
+        const double u0 = a == 0 ? f[0] : (a == 1 ? f[2] - f[8] : f[6]);
+        const double u1 = a == 0 ? f[2] + f[8] : (a == 1 ? f[1] : f[7]);
+        T += G.wdet * (u0 * G.Nx[n][0] + u1 * G.Nx[n][1]);
+        if (n < 4) {
+            const double p = a == 0 ? -f[7] : (a == 1 ? f[6] : 2.0 * f[8]);
+            const double r0 = a == 0 ? -f[5] : (a == 1 ? f[3] : 0.0);
+            const double r1 = a == 0 ? -f[4] : (a == 1 ? f[5] : 0.0);
+            Q += G.wdet * (p * G.Nv[n] + r0 * G.Nx[n][0] + r1 * G.Nx[n][1]);
         }
-        if (nd1 == nd2)
-            for (int a = 0; a < 3; ++a) {
-                pr[a] = F.dr[blk][a] * G.Nv[nd1 - 1];
-                for (int b = 0; b < 3; ++b) rx[a][b] = F.dr[blk][a] * G.Nx[nd1 - 1][b];
-            }
     }
-    shell_def(ux, rx, pr, d);
+    if (!stressed) return false;
+    if (n < 10) S.T[n][a] = T;
+    if (n < 4) S.Q[n][a] = Q;
+    __syncwarp();
+    if (j < 9) {
+        const double *io = F.io[4 * (n + 1) + a + 1];
+        double g = 0.0;
+        for (int m = 0; m < 4; ++m)
+            for (int b = 0; b < 3; ++b) {
+                double tr = 0.0;
+                for (int k = 0; k < 3; ++k) tr += io[3 * b + k] * (F.u[k][m] + F.X[m][k]);
+                g += tr * S.T[m][b];
+            }
+        S.G[n][a] = 0.0625 * g;
+    }
+    __syncwarp();
+    return true;
+}
+
+// Adds column j of the stress part to Kc.
+__device__ void stress_column(const ShellFrame &F, const ShellStress &S, int j, double Kc[32]) {
+    int vj, nj;
+    dof_of(j, vj, nj);
+    if (vj < 4) {
+        // the rotations of every node alike
+#pragma unroll
+        for (int r = 1; r <= 3; ++r) {
+            double s = 0.0;
+            for (int a = 0; a < 3; ++a) s += F.io[r][3 * a + vj - 1] * S.T[nj - 1][a];
+#pragma unroll
+            for (int m = 0; m < 4; ++m) Kc[4 * (2 + r) + m] += 0.25 * s;
+        }
+        return;
+    }
+    const int r = vj - 3;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+        int vi, ni;
+        dof_of(i, vi, ni);
+        double s = 0.0;
+        if (vi < 4) {
+            for (int a = 0; a < 3; ++a) s += F.io[r][3 * a + vi - 1] * S.T[ni - 1][a];
+            s *= 0.25;
+        } else {
+            s = S.G[r - 1][vi - 4];
+            if (ni == nj)
+                for (int a = 0; a < 3; ++a) s += F.dr[4 * r + vi - 3][a] * S.Q[nj - 1][a];
+        }
+        Kc[i] += s;
+    }
 }
 
 __device__ void pipe_dedu(const ShellPipe &A, int q, int g, int i) {
@@ -400,7 +461,7 @@ __device__ __forceinline__ double mass_weight(const ShellGP &G, int var, int nd,
 
 __device__ void pipe_inam(const ShellPipe &A, int q, int n) {
     ASTRO_GUARD(A.status, 151, ASTRO_IN(q, A.scratchEls) && ASTRO_IN(n, 4) && ASTRO_IN(A.els[q], A.nEls));
-    const ShellProps &P = A.props[A.els[q]];
+    const ShellProps &P = item_props(A, q, A.els[q]);
     ShellFrame &F = A.fr[q];
     double ina[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     for (int var = 1; var <= 6; ++var) {
@@ -425,9 +486,9 @@ __device__ void pipe_inam(const ShellPipe &A, int q, int n) {
     }
 }
 
-__device__ void pipe_kcol(const ShellPipe &A, int q, int j) {
+__device__ void pipe_kcol(const ShellPipe &A, int q, int j, ShellStress &S) {
     ASTRO_GUARD(A.status, 161, ASTRO_IN(q, A.scratchEls) && ASTRO_IN(j, 32) && ASTRO_IN(A.els[q], A.nEls));
-    const ShellProps &P = A.props[A.els[q]];
+    const ShellProps &P = item_props(A, q, A.els[q]);
     const ShellFrame &F = A.fr[q];
     double *out = A.Kf + ((size_t)q * 32 + j) * 33;
     double Kc[32];
@@ -437,11 +498,8 @@ __device__ void pipe_kcol(const ShellPipe &A, int q, int j) {
         const ShellGP &G = A.gp[4 * (size_t)q + g];
         const double *dj = A.dedU + (((size_t)q * 4 + g) * 32 + j) * 9;
         const double wd = G.wdet;
-        bool stressed = false;
-        for (int a = 0; a < 9; ++a) {
-            if (!A.massOnly) ru += G.F[a] * (wd * dj[a]);
-            if (G.F[a] != 0.0) stressed = true;
-        }
+        if (!A.massOnly)
+            for (int a = 0; a < 9; ++a) ru += G.F[a] * (wd * dj[a]);
         if (!A.buildMat) continue;
         double c[9];
         for (int a = 0; a < 9; ++a) {
@@ -455,16 +513,8 @@ __device__ void pipe_kcol(const ShellPipe &A, int q, int j) {
             for (int a = 0; a < 9; ++a) s += di[a] * c[a];
             Kc[i] += s;
         }
-        if (stressed) {
-            for (int i = 0; i < 32; ++i) {
-                double d2[9];
-                def_second(F, G, i < j ? i : j, i < j ? j : i, d2);
-                double s = 0.0;
-                for (int a = 0; a < 9; ++a) s += G.F[a] * (wd * d2[a]);
-                Kc[i] += s;
-            }
-        }
     }
+    if (A.buildMat && stress_tables(A, F, q, j, S)) stress_column(F, S, j, Kc);
     if (A.dynamic && j < 24) {
         const double c1 = 0.5 / A.beta, c2 = 2.0 / (A.delT * A.delT);
         const double(*inam)[4] = F.inam;
@@ -556,17 +606,20 @@ __device__ void pipe_cond_col(const ShellPipe &A, int q, int j) {
         double *dst = A.intMat + 256 * (size_t)e;
         for (int k = 0; k < 8; ++k) dst[8 * j + k] = Kq[33 * j + 24 + k];
     }
-    const int cvar = j / 4, bn = j % 4;
-    for (int i = 0; i < 24; ++i) {
-        const double v = Kq[33 * j + i];
-        if (A.K) {
-            const int rvar = i / 4, a = i % 4;
-            const int blk = A.elBlk[16 * (size_t)e + 4 * a + bn];
-            ASTRO_GUARD(A.status, 183, ASTRO_IN(blk, A.nBlocks));
-            A.K[36 * (size_t)blk + 6 * rvar + cvar] += v;
-        }
-        if (A.keOut) A.keOut[576 * (size_t)e + 24 * (size_t)j + i] = v;
-    }
+    if (A.keOut)
+        for (int i = 0; i < 24; ++i) A.keOut[576 * (size_t)e + 24 * (size_t)j + i] = Kq[33 * j + i];
+}
+
+// one entry of the condensed matrix into the block-CSR matrix: t = 36 * (node pair) + entry, so that
+// consecutive threads write consecutive entries of a block
+__device__ void pipe_addk(const ShellPipe &A, int q, int t) {
+    ASTRO_GUARD(A.status, 183, ASTRO_IN(q, A.scratchEls));
+    const int e = A.els[q];
+    ASTRO_GUARD(A.status, 184, ASTRO_IN(e, A.nEls));
+    const int pair = t / 36, ent = t % 36, a = pair / 4, bn = pair % 4, rvar = ent / 6, cvar = ent % 6;
+    const int blk = A.elBlk[16 * (size_t)e + pair];
+    ASTRO_GUARD(A.status, 185, ASTRO_IN(blk, A.nBlocks));
+    A.K[36 * (size_t)blk + ent] += A.Kf[(size_t)q * 32 * 33 + 33 * (4 * cvar + bn) + 4 * rvar + a];
 }
 
 __global__ void k_shell_cond_lu(ShellPipe A) {
@@ -576,6 +629,11 @@ __global__ void k_shell_cond_lu(ShellPipe A) {
 __global__ void k_shell_cond_col(ShellPipe A) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < 24 * A.count) pipe_cond_col(A, t / 24, t % 24);
+}
+
+__global__ void k_shell_addk(ShellPipe A) {
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (t < 576LL * A.count) pipe_addk(A, A.q0 + (int)(t / 576), (int)(t % 576));
 }
 
 __global__ void k_shell_frame(ShellPipe A) {
@@ -594,25 +652,26 @@ __global__ void k_shell_inam(ShellPipe A) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < 4 * A.count) pipe_inam(A, t / 4, t % 4);
 }
-// residual scatter without a matrix: one thread per (element, DOF) (a colour's elements share no
+// residual scatter: one thread per (element, DOF) (a colour's elements share no
 // node, an element's DOF are distinct entries)
 __global__ void k_shell_scatter(ShellPipe A) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= 32 * A.count) return;
-    const int q = t / 32, i = t % 32;
+    const int q = A.q0 + t / 32, i = t % 32;
     ASTRO_GUARD(A.status, 191, ASTRO_IN(q, A.scratchEls));
     const int e = A.els[q];
     ASTRO_GUARD(A.status, 192, ASTRO_IN(e, A.nEls));
     const double ru = A.Kf[(size_t)q * 32 * 33 + 33 * i + 32];
+    const size_t slot = A.slot ? A.slot[q] : 0;
     if (i < 24) {
         const int var = i / 4, a = i % 4;
         ASTRO_GUARD(A.status, 193, ASTRO_IN(A.elist[8 * (size_t)e + a] - 1, A.nNodes));
         const int r = A.rank[A.elist[8 * (size_t)e + a] - 1] - 1;
         ASTRO_GUARD(A.status, 194, ASTRO_IN(r, A.nNodes));
-        if (A.load) A.load[6 * (size_t)r + var] -= ru;
+        if (A.load) A.load[slot * A.loadLen + 6 * (size_t)r + var] -= ru;
         if (A.ruOut) A.ruOut[24 * (size_t)e + i] = ru;
     } else if (A.intLoad) {
-        A.intLoad[8 * (size_t)e + i - 24] -= ru;
+        A.intLoad[slot * A.intLoadLen + 8 * (size_t)e + i - 24] -= ru;
     }
 }
 __global__ void k_shell_gauss(ShellPipe A) {
@@ -623,9 +682,11 @@ __global__ void k_shell_dedu(ShellPipe A) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < 128 * A.count) pipe_dedu(A, t / 128, (t / 32) % 4, t % 32);
 }
-__global__ void k_shell_kcol(ShellPipe A) {
+constexpr int kKcolThreads = 128;  // four elements, a warp each
+__global__ void __launch_bounds__(kKcolThreads) k_shell_kcol(ShellPipe A) {
+    __shared__ ShellStress S[kKcolThreads / 32];
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < 32 * A.count) pipe_kcol(A, t / 32, t % 32);
+    if (t < 32 * A.count) pipe_kcol(A, t / 32, t % 32, S[threadIdx.x / 32]);
 }
 
 }  // namespace

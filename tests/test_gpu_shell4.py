@@ -129,3 +129,41 @@ def test_internal_dof_recovery(plate):
     s_g0 = g.updateInternalSoln(ext, i0)
     s_o0 = o.update_internal_soln(ext, i0, None, imat)
     assert np.linalg.norm(s_g0 - s_o0) <= 1e-11 * np.linalg.norm(s_o0)
+
+
+def test_assembly_over_pipeline_chunks():
+    """A mesh of more elements than one chunk of the pipeline's scratch holds (32,768), at a displaced
+    state: loads and matrix against the oracle."""
+    m = M.plate_shell(nx=221, ny=149, lx=22.1, ly=14.9)
+    g, o = AstroGPU(m), Oracle(m)
+    rng = np.random.default_rng(6)
+    st = M.make_state(o.n, disp=1e-4 * rng.standard_normal(o.n),
+                      internal_disp=1e-5 * rng.standard_normal(o.int_vec_size))
+    load, iload, mat, cols, _ = g.getElasticSolnLoad(1, state=st)
+    oload, oiload, omat, ocols, _ = o.el_soln_load(1, state=st)
+    assert np.array_equal(cols, ocols)
+    assert np.linalg.norm(mat - omat) <= 1e-11 * np.linalg.norm(omat)
+    assert np.linalg.norm(load - oload) <= 1e-11 * np.linalg.norm(oload)
+    assert np.linalg.norm(iload - oiload[:o.int_vec_size]) <= 1e-11 * np.linalg.norm(oiload[:o.int_vec_size])
+
+
+def test_condensed_derivatives_of_several_variables():
+    """All (element, variable) items together against one variable at a time: variables that share
+    elements, listed twice and in any order, give the same bits."""
+    m = M.plate_shell(nx=9, ny=5, lx=3.0, ly=2.0)
+    E = m.num_els
+    # variable 1 on every element, 2 and 3 on halves, two terms of variable 3 on the second half
+    terms = [[1, 2] if e < E // 2 else [3, 1, 3] for e in range(E)]
+    m.el_to_d_range = np.concatenate([[0], np.cumsum([len(t) for t in terms])]).astype(np.int32)
+    m.el_to_d = np.concatenate(terms).astype(np.int32)
+    m.el_to_coef = np.linspace(0.5, 1.5, len(m.el_to_d))
+    m.d_category = np.array([M.DCAT_LAYUP_THICKNESS, M.DCAT_LAYUP_ANGLE, M.DCAT_LAYUP_ZOFFSET], np.int32)
+    m.d_component, m.d_layer, m.d_value = np.ones(3, np.int32), np.ones(3, np.int32), np.zeros(3)
+    g = AstroGPU(m)
+    rng = np.random.default_rng(2)
+    st = M.make_state(g.n, disp=1e-3 * rng.standard_normal(g.n))
+    g.getElasticSolnLoad(1, state=st, export=False)
+    D = g.drdd_condensed([3, 1, 2, 1], state=st)
+    for k, d in enumerate([3, 1, 2, 1]):
+        r, ir = g.getdRelasticdD(d, state=st)
+        assert np.any(r) and np.array_equal(D[:, k], g.updateExternalRHS(r, ir)), d
