@@ -18,6 +18,8 @@ struct PanelMeta {
     int nbc;          // block columns, ceil(n / 32)
     int bt;           // tiles below the diagonal tile in a block column
     int nfac;         // block columns the factorisation eliminates (nbc; fewer for a partial factor)
+    int bw;           // entries (i, j) with i - j > bw are zero
+    int pad;
 };
 
 __device__ __forceinline__ size_t tile_off(const PanelMeta &M, int J, int d) {

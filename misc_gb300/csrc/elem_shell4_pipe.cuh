@@ -343,7 +343,7 @@ __device__ void def_first(const ShellFrame &F, const ShellGP &G, int i, int quir
 //   rotations r of node m, s of node n:              G[r][s] + [m = n] sum_a dr_rs(a) Q[n][a],
 //                      G[r][s] = 1/16 sum_n sum_a (d2R_rs (u + X)_n)(a) T[n][a].
 // (6,208 elements at a displaced state: kcol 4.49 ms with the second derivatives evaluated for every
-// point and pair, @KCOL@ ms so.)
+// point and pair, 0.80 ms so.)
 struct ShellStress {
     double T[10][3], Q[4][3], G[3][3];
 };

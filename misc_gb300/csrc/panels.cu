@@ -518,8 +518,9 @@ __device__ __forceinline__ double recip64(double d) {
 // the whole CTA.  GB300's FP64 pipe takes one warp instruction per 19 clocks from an SM and one
 // per 64 from a warp (measured), so the chain is kept to one warp and short: it factors four
 // columns at a time in registers (lane = row), the next four columns are brought up to date by
-// four warps, and the remaining columns by warps 1 .. 7 while warp 0 factors on.
-__device__ void tile_ldl(double (*S)[TB + 1], double (*sU)[4][TB], int t) {
+// four warps, and the remaining columns within the bandwidth by warps 1 .. 7 while warp 0 factors on
+// (20.7 k clocks for a full tile).
+__device__ void tile_ldl(double (*S)[TB + 1], double (*sU)[4][TB], int t, int bw) {
     const int lane = t & 31, w = t >> 5;
     for (int b = 0; b < 8; ++b) {
         const int c0 = 4 * b;
@@ -550,15 +551,16 @@ __device__ void tile_ldl(double (*S)[TB + 1], double (*sU)[4][TB], int t) {
         if (w < 4) update(c0 + 4 + w);
         __syncthreads();
         if (w > 0)
-            for (int j = c0 + 7 + w; j < TB; j += kGroups - 1) update(j);
+            for (int j = c0 + 7 + w; j < min(TB, c0 + 4 + bw); j += kGroups - 1) update(j);
     }
 }
 
 // Rows of a 32 x 32 tile in shared memory (A[row][column]) times L^-T (sL: unit lower L), the whole
-// CTA, the columns in fours as in tile_ldl.
-__device__ void tile_rows(double (*A)[TB + 1], const double (*sL)[TB + 1], int t) {
+// CTA, the columns in fours as in tile_ldl, from column cBegin (a multiple of four) on: the columns
+// before it are zero.
+__device__ void tile_rows(double (*A)[TB + 1], const double (*sL)[TB + 1], int t, int cBegin) {
     const int lane = t & 31, w = t >> 5;
-    for (int b = 0; b < 8; ++b) {
+    for (int b = cBegin / 4; b < 8; ++b) {
         const int c0 = 4 * b;
         if (w == 0) {
             double v[4];
@@ -590,14 +592,14 @@ __device__ void tile_rows(double (*A)[TB + 1], const double (*sL)[TB + 1], int t
 //   rows      the tiles below the diagonal, L_IJ = A_IJ L_JJ^-T D_J^-1, dealt to the CTAs; a CTA with
 //             one or two takes each with all its warps (tile_rows), with more a warp per tile (one
 //             row per thread): the FP64 pipe is then full from the tiles alone;
-//   update    tiles (J+e, d-e) -= L_{J+d,J} D_J L_{J+e,J}^T, 1 <= e <= d.  CTA 0 takes the next
+//   update    tiles (J+e, d-e) -= L_{J+d,J} D_J L_{J+e,J}^T, 1 <= e <= d (d = e: the lower half).  CTA 0 takes the next
 //             diagonal tile first and factors it in shared memory (tile_ldl) while the others go on
 //             with the rest, so the chain of the pivots is off the critical path; it joins again
 //             two rounds later (the factorisation takes about as long as a tile update).  Every
 //             thread loads the next item's operands during the current one.
 // One cluster barrier after each.  Bound: the FP64 pipe in the updates (9.5 us a tile and SM), and
 // for a narrow band the chain rows -> first update -> diagonal tile.  32 panels of 8 .. 36 elements a
-// side: 12.5 ms, against 26.1 ms with every CTA factoring the diagonal tile for itself (a division
+// side: 12.1 ms, against 26.1 ms with every CTA factoring the diagonal tile for itself (a division
 // per thread and pivot) and the rows below on consecutive threads of the first CTA; the 64 x 64
 // plate's two halves at 8 CTAs: 50.8 against 70.8 ms.
 __global__ void __launch_bounds__(kThreads, 2) k_band_ldl64(const PanelMeta *__restrict__ meta,
@@ -613,12 +615,24 @@ __global__ void __launch_bounds__(kThreads, 2) k_band_ldl64(const PanelMeta *__r
     __shared__ double sU[2][4][TB];
     __shared__ double sDi[TB];  // D^-1
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    // the thread's entries (row tr, column tc) of a lower triangle packed by rows: t, t + 256 and, for
+    // the first 16 threads, t + 512
+    int tr[3], tc[3];
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+        int e = x < 2 || t < 16 ? t + x * kThreads : 0, r = 0;
+        while (e > r) e -= ++r;
+        tr[x] = r;
+        tc[x] = e;
+    }
     for (int q = schedPtr[worker]; q < schedPtr[worker + 1]; ++q) {
         const int p = sched[q];
         const PanelMeta M = meta[p];
+        // leading columns of a tile d below the diagonal that lie outside the band, in fours
+        auto zero_cols = [&](int d) { return max(0, d * TB - M.bw) & ~3; };
         // CTA 0: the factored diagonal tile of block column J from sN, to memory and the pivot test
         auto diag_out = [&](int J) {
-            tile_ldl(sN, sU, t);
+            tile_ldl(sN, sU, t, M.bw);
             double *Td = band + tile_off(M, J, 0);
             for (int e = t; e < TT; e += kThreads) __stcg(Td + e, sN[e % TB][e / TB]);
             if (t < TB && J * TB + t < M.n) {
@@ -648,7 +662,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_band_ldl64(const PanelMeta *__r
                     double *T = band + tile_off(M, J, d);
                     for (int e = t; e < TT; e += kThreads) sA[e % TB][e / TB] = __ldcg(T + e);
                     __syncthreads();
-                    tile_rows(sA, sL, t);
+                    tile_rows(sA, sL, t, zero_cols(d));
                     for (int e = t; e < TT; e += kThreads) __stcg(T + e, sA[e % TB][e / TB] * sDi[e / TB]);
                     __syncthreads();
                 }
@@ -715,29 +729,43 @@ __global__ void __launch_bounds__(kThreads, 2) k_band_ldl64(const PanelMeta *__r
                 if (i >= 0) {
                     int d, e;
                     tiles(i, d, e);
-                    double *Tt = band + tile_off(M, J + e, d - e) + 4 * w * TB + lane;
-                    double o[4], acc[4] = {0.0, 0.0, 0.0, 0.0};
+                    if (d == e) {
+                        // a diagonal tile: its 528 lower entries, two or three to a thread
+                        double *Tt = band + tile_off(M, J + e, 0);
+                        double o[3], acc[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-                    for (int cc = 0; cc < 4; ++cc) o[cc] = __ldcg(Tt + cc * TB);
-#pragma unroll 8
-                    for (int k = 0; k < TB; ++k) {
-                        const double a = sA[lane][k];
+                        for (int x = 0; x < 3; ++x)
+                            if (x < 2 || t < 16) o[x] = __ldcg(Tt + tc[x] * TB + tr[x]);
+#pragma unroll 4
+                        for (int k = zero_cols(d); k < TB; ++k) {
 #pragma unroll
-                        for (int cc = 0; cc < 4; ++cc) acc[cc] += a * sB[4 * w + cc][k];
-                    }
-                    if (i > 0) {
+                            for (int x = 0; x < 2; ++x) acc[x] += sA[tr[x]][k] * sB[tc[x]][k];
+                            if (w == 0) acc[2] += sA[tr[2]][k] * sB[tc[2]][k];
+                        }
+                        const bool next = i == 0 && J + 1 < M.nfac;  // factored here and now
+#pragma unroll
+                        for (int x = 0; x < 3; ++x) {
+                            if (x == 2 && t >= 16) continue;
+                            if (next) sN[tr[x]][tc[x]] = o[x] - acc[x];
+                            else __stcg(Tt + tc[x] * TB + tr[x], o[x] - acc[x]);
+                        }
+                        if (next) {
+                            __syncthreads();
+                            diag_out(J + 1);
+                        }
+                    } else {
+                        double *Tt = band + tile_off(M, J + e, d - e) + 4 * w * TB + lane;
+                        double o[4], acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+                        for (int cc = 0; cc < 4; ++cc) o[cc] = __ldcg(Tt + cc * TB);
+#pragma unroll 4
+                        for (int k = zero_cols(d); k < TB; ++k) {
+                            const double a = sA[lane][k];
+#pragma unroll
+                            for (int cc = 0; cc < 4; ++cc) acc[cc] += a * sB[4 * w + cc][k];
+                        }
 #pragma unroll
                         for (int cc = 0; cc < 4; ++cc) __stcg(Tt + cc * TB, o[cc] - acc[cc]);
-                    } else {
-#pragma unroll
-                        for (int cc = 0; cc < 4; ++cc) sN[lane][4 * w + cc] = o[cc] - acc[cc];
-                        __syncthreads();
-                        if (J + 1 < M.nfac) {
-                            diag_out(J + 1);
-                        } else {
-#pragma unroll
-                            for (int cc = 0; cc < 4; ++cc) __stcg(Tt + cc * TB, o[cc] - acc[cc]);
-                        }
                     }
                 }
                 i = nxt;
@@ -1064,72 +1092,114 @@ __global__ void __launch_bounds__(kThreads) k_band_solve(const PanelMeta *__rest
 // rows; the forward sweep leaves y in X as (hi, lo) float pairs, which the backward sweep
 // overwrites with the FP64 value of the solution.  Items have 1 .. kSolveCols columns (a
 // template instantiation each).
+// Each row waits for the one before it, so everything a row needs besides the solved rows is under
+// way one row ahead: every warp's first tile in registers, W in shared memory (cp.async, two
+// buffers), the row's right-hand side in registers; a warp's further tiles are loaded whole.
+__device__ __forceinline__ void cp_async16(void *smem, const void *g) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(g));
+}
+
 template <int NC>
 __device__ __forceinline__ void band_solve_df_item(const PanelMeta &M, const float2 *__restrict__ Lf,
                                                    const float2 *__restrict__ Lb, const float2 *__restrict__ Wfp,
                                                    const float2 *__restrict__ Wbp, const float2 *__restrict__ Dinv,
-                                                   double *Xp, int ring, float2 *sRing, float2 *sP, float2 *sV) {
+                                                   double *Xp, int ring, int cols, float2 *sRing, float2 *sP,
+                                                   float2 *sV, float2 *sW) {
     const int npad = M.nbc * TB;
     float2 *Yp = reinterpret_cast<float2 *>(Xp);
     const int t = threadIdx.x, r = t % TB, g = t / TB;
     for (int sweep = 0; sweep < 2; ++sweep) {
         const bool fwd = sweep == 0;
         const float2 *Lt = fwd ? Lf : Lb;
+        // partial products: forward sum_d L_{I,I-d} y_{I-d}; backward sum_d L_{I+d,I}^T x_{I+d}
+        auto row = [&](int s) { return fwd ? s : M.nbc - 1 - s; };
+        auto tile = [&](int s, int d) { return Lt + tile_off(M, fwd ? s - d : row(s), d) + r; };
+        auto fetch_w = [&](int s) {
+            const float4 *W = reinterpret_cast<const float4 *>((fwd ? Wfp : Wbp) + (size_t)row(s) * TT);
+            float4 *d = reinterpret_cast<float4 *>(sW + (size_t)(s & 1) * TT);
+            for (int e = t; e < TT / 2; e += kThreads) cp_async16(d + e, W + e);
+        };
+        float2 tp[TB];  // the warp's first tile (d = 1 + g) of the coming row
+        double bx = 0.0;  // the coming row's right-hand side: forward b, backward y as a float pair
+        float2 bd = make_float2(0.f, 0.f);
+        auto fetch = [&](int s) {
+            if (1 + g <= min(M.bt, s)) {
+                const float2 *T = tile(s, 1 + g);
+#pragma unroll
+                for (int k = 0; k < TB; ++k) tp[k] = __ldg(T + k * TB);
+            }
+            if (g < NC) {
+                bx = Xp[(size_t)g * npad + (size_t)row(s) * TB + r];
+                if (!fwd) bd = __ldg(Dinv + M.xUnit + (size_t)row(s) * TB + r);
+            }
+        };
+        fetch_w(0);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        fetch(0);
         for (int s = 0; s < M.nbc; ++s) {
-            const int I = fwd ? s : M.nbc - 1 - s;
-            // partial products: forward sum_d L_{I,I-d} y_{I-d}; backward sum_d L_{I+d,I}^T x_{I+d}
+            const int I = row(s);
             DF acc[NC];
 #pragma unroll
             for (int c = 0; c < NC; ++c) acc[c] = DF{0.f, 0.f};
-            const int dmax = min(M.bt, fwd ? I : M.nbc - 1 - I);
+            const int dmax = min(M.bt, s);
             for (int d = 1 + g; d <= dmax; d += kGroups) {
-                const int J = fwd ? I - d : I + d;
-                const float2 *T = Lt + tile_off(M, fwd ? J : I, d);
-                const float2 *y = sRing + (size_t)(J % ring) * kSolveCols * TB;
-#pragma unroll 4
+                if (d > 1 + g) {
+                    const float2 *T = tile(s, d);
+#pragma unroll
+                    for (int k = 0; k < TB; ++k) tp[k] = __ldg(T + k * TB);
+                }
+                const float2 *y = sRing + (size_t)((fwd ? I - d : I + d) % ring) * cols * TB;
+#pragma unroll
                 for (int k = 0; k < TB; ++k) {
-                    const float2 l = __ldg(T + k * TB + r);
 #pragma unroll
                     for (int c = 0; c < NC; ++c) {
                         const float2 v = y[c * TB + k];
-                        df_acc(acc[c], l.x, l.y, v.x, v.y);
+                        df_acc(acc[c], tp[k].x, tp[k].y, v.x, v.y);
                     }
                 }
             }
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
                 const DF a = df_norm(acc[c]);
-                sP[(g * kSolveCols + c) * TB + r] = make_float2(a.hi, a.lo);
+                sP[(g * cols + c) * TB + r] = make_float2(a.hi, a.lo);
             }
+            const double b = bx;
+            const float2 di = bd;
+            if (s + 1 < M.nbc) {
+                fetch_w(s + 1);
+                fetch(s + 1);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            asm volatile("cp.async.wait_group 1;" ::: "memory");  // W of this row is there
             __syncthreads();
             if (g < NC) {
                 const int c = g;
                 const size_t xi = (size_t)c * npad + (size_t)I * TB + r;
                 DF v;
                 if (fwd) {
-                    v = df_from_double(Xp[xi]);
+                    v = df_from_double(b);
                 } else {
-                    const float2 yv = Yp[xi], di = __ldg(Dinv + M.xUnit + (size_t)I * TB + r);
+                    const float2 yv = make_float2(__int_as_float(__double2loint(b)), __int_as_float(__double2hiint(b)));
                     v = df_mul(DF{yv.x, yv.y}, DF{di.x, di.y});
                 }
                 for (int q = 0; q < kGroups; ++q) {
-                    const float2 p = sP[(q * kSolveCols + c) * TB + r];
+                    const float2 p = sP[(q * cols + c) * TB + r];
                     v = df_sub(v, DF{p.x, p.y});
                 }
                 sV[c * TB + r] = make_float2(v.hi, v.lo);
                 __syncwarp();
                 // forward y = W v (W[r][k] at Wf[k TB + r]); backward x = W^T v (W[k][r] at Wb[k TB + r])
-                const float2 *W = (fwd ? Wfp : Wbp) + (size_t)I * TT;
+                const float2 *W = sW + (size_t)(s & 1) * TT;
                 DF o = {0.f, 0.f}, o2 = {0.f, 0.f};
 #pragma unroll 4
                 for (int k = 0; k < TB; k += 2) {
-                    const float2 w0 = __ldg(W + k * TB + r), w1 = __ldg(W + (k + 1) * TB + r);
+                    const float2 w0 = W[k * TB + r], w1 = W[(k + 1) * TB + r];
                     const float2 v0 = sV[c * TB + k], v1 = sV[c * TB + k + 1];
                     df_acc(o, w0.x, w0.y, v0.x, v0.y);
                     df_acc(o2, w1.x, w1.y, v1.x, v1.y);
                 }
                 o = df_add(df_norm(o), df_norm(o2));
-                sRing[((size_t)(I % ring) * kSolveCols + c) * TB + r] = make_float2(o.hi, o.lo);
+                sRing[((size_t)(I % ring) * cols + c) * TB + r] = make_float2(o.hi, o.lo);
                 if (fwd)
                     Yp[xi] = make_float2(o.hi, o.lo);
                 else
@@ -1137,21 +1207,23 @@ __device__ __forceinline__ void band_solve_df_item(const PanelMeta &M, const flo
             }
             __syncthreads();
         }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
 }
 
-__global__ void __launch_bounds__(kThreads) k_band_solve_df(const PanelMeta *__restrict__ meta,
+__global__ void __launch_bounds__(kThreads, 2) k_band_solve_df(const PanelMeta *__restrict__ meta,
                                                             const SolveItem *__restrict__ items,
                                                             const float2 *__restrict__ Lf,
                                                             const float2 *__restrict__ Lb,
                                                             const float2 *__restrict__ Wf,
                                                             const float2 *__restrict__ Wb,
                                                             const float2 *__restrict__ Dinv, double *X, int nrhs,
-                                                            int ring) {
-    extern __shared__ float2 sdf[];
-    float2 *sRing = sdf;                                // [ring][kSolveCols][TB]
-    float2 *sP = sRing + (size_t)ring * kSolveCols * TB;  // [kGroups][kSolveCols][TB]
-    float2 *sV = sP + kGroups * kSolveCols * TB;        // [kSolveCols][TB]
+                                                            int ring, int cols) {
+    extern __shared__ __align__(16) float2 sdf[];
+    float2 *sW = sdf;                                   // [2][TT]
+    float2 *sRing = sW + 2 * TT;                        // [ring][cols][TB], cols: the widest item's
+    float2 *sP = sRing + (size_t)ring * cols * TB;      // [kGroups][cols][TB]
+    float2 *sV = sP + (size_t)kGroups * cols * TB;      // [cols][TB]
     const SolveItem it = items[blockIdx.x];
     const PanelMeta M = meta[it.panel];
     double *Xp = X + (size_t)M.xUnit * nrhs + (size_t)it.col0 * (M.nbc * TB);
@@ -1159,14 +1231,14 @@ __global__ void __launch_bounds__(kThreads) k_band_solve_df(const PanelMeta *__r
     // the work of a group is in proportion to its columns: the item's column count picks the
     // instantiation
     switch (it.ncol) {
-    case 1: band_solve_df_item<1>(M, Lf, Lb, Wfp, Wbp, Dinv, Xp, ring, sRing, sP, sV); break;
-    case 2: band_solve_df_item<2>(M, Lf, Lb, Wfp, Wbp, Dinv, Xp, ring, sRing, sP, sV); break;
-    case 3: band_solve_df_item<3>(M, Lf, Lb, Wfp, Wbp, Dinv, Xp, ring, sRing, sP, sV); break;
-    case 4: band_solve_df_item<4>(M, Lf, Lb, Wfp, Wbp, Dinv, Xp, ring, sRing, sP, sV); break;
-    case 5: band_solve_df_item<5>(M, Lf, Lb, Wfp, Wbp, Dinv, Xp, ring, sRing, sP, sV); break;
-    case 6: band_solve_df_item<6>(M, Lf, Lb, Wfp, Wbp, Dinv, Xp, ring, sRing, sP, sV); break;
-    case 7: band_solve_df_item<7>(M, Lf, Lb, Wfp, Wbp, Dinv, Xp, ring, sRing, sP, sV); break;
-    default: band_solve_df_item<kSolveCols>(M, Lf, Lb, Wfp, Wbp, Dinv, Xp, ring, sRing, sP, sV); break;
+    case 1: band_solve_df_item<1>(M, Lf, Lb, Wfp, Wbp, Dinv, Xp, ring, cols, sRing, sP, sV, sW); break;
+    case 2: band_solve_df_item<2>(M, Lf, Lb, Wfp, Wbp, Dinv, Xp, ring, cols, sRing, sP, sV, sW); break;
+    case 3: band_solve_df_item<3>(M, Lf, Lb, Wfp, Wbp, Dinv, Xp, ring, cols, sRing, sP, sV, sW); break;
+    case 4: band_solve_df_item<4>(M, Lf, Lb, Wfp, Wbp, Dinv, Xp, ring, cols, sRing, sP, sV, sW); break;
+    case 5: band_solve_df_item<5>(M, Lf, Lb, Wfp, Wbp, Dinv, Xp, ring, cols, sRing, sP, sV, sW); break;
+    case 6: band_solve_df_item<6>(M, Lf, Lb, Wfp, Wbp, Dinv, Xp, ring, cols, sRing, sP, sV, sW); break;
+    case 7: band_solve_df_item<7>(M, Lf, Lb, Wfp, Wbp, Dinv, Xp, ring, cols, sRing, sP, sV, sW); break;
+    default: band_solve_df_item<kSolveCols>(M, Lf, Lb, Wfp, Wbp, Dinv, Xp, ring, cols, sRing, sP, sV, sW); break;
     }
 }
 
@@ -1681,6 +1753,7 @@ int plan_build(astro_ctx *ctx, PanelPlan &L, int cs) {
         const int bw = bwn[p] * dpn + dpn - 1;
         L.maxBw = std::max(L.maxBw, bw);
         M.bt = (bw + TB - 1) / TB;
+        M.bw = bw;
         M.band = band;
         M.xUnit = xr;
         M.nfac = M.nbc;
@@ -1941,8 +2014,23 @@ static int panels_solve_dev(astro_ctx *ctx, PanelPlan *L, int nrhs, double *d_ve
     const unsigned mg = (unsigned)((mv + 255) / 256);
     k_panel_move<<<mg, 256, 0, s>>>(P.n, P.dpn, nrhs, d_vec, dptr<int>(L->d_panelOf), dptr<int>(L->d_pos),
                                     dptr<PanelMeta>(L->d_meta), dptr<double>(X), 1);
-    // one item per (panel, group of right-hand sides), the largest panels first
-    const int groups = (nrhs + kSolveCols - 1) / kSolveCols;
+    // one item per (panel, group of right-hand sides), the largest panels first.  Groups of up to 8
+    // columns share the loads of the tiles; few panels get smaller groups, until there is an item for
+    // every SM: an item's time is in proportion to its panel's block rows and, beyond the chain of a
+    // row, to its columns (32 panels of 8 .. 36 elements a side: 8 columns 7.4 -> 1.2 ms, a single one 3.6 -> 0.9 ms
+    // from the loads a row ahead alone).
+    int sms = 0, smemMax = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    cudaDeviceGetAttribute(&smemMax, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
+    const int ring = L->maxBt + 1;
+    int groups = (nrhs + kSolveCols - 1) / kSolveCols;
+    if (ctx->panelsSolve != 1) groups = std::min(nrhs, std::max(groups, (sms + L->np - 1) / L->np));
+    auto dfSmem = [&](int g) {
+        const size_t cols = (nrhs + g - 1) / g;
+        return sizeof(float2) * (2 * TT + cols * TB * ((size_t)ring + kGroups + 1));
+    };
+    // a wide band's ring of solved rows leaves room for fewer columns
+    while (ctx->panelsSolve != 1 && groups < nrhs && dfSmem(groups) > (size_t)smemMax) ++groups;
     std::vector<int> order(L->np);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
@@ -1966,12 +2054,12 @@ static int panels_solve_dev(astro_ctx *ctx, PanelPlan *L, int nrhs, double *d_ve
             dptr<PanelMeta>(L->d_meta), dptr<SolveItem>(dItems), dptr<double>(L->d_band), dptr<double>(X), nrhs);
     } else {
         if ((rc = panels_df_copies(ctx, L))) return rc;
-        const int ring = L->maxBt + 1;
-        const size_t smem = sizeof(float2) * kSolveCols * TB * ((size_t)ring + kGroups + 1);
+        const size_t smem = dfSmem(groups);
         CK(cudaFuncSetAttribute(k_band_solve_df, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         k_band_solve_df<<<(unsigned)items.size(), kThreads, smem, s>>>(
             dptr<PanelMeta>(L->d_meta), dptr<SolveItem>(dItems), dptr<float2>(L->d_Lf), dptr<float2>(L->d_Lb),
-            dptr<float2>(L->d_Wf), dptr<float2>(L->d_Wb), dptr<float2>(L->d_Dinv), dptr<double>(X), nrhs, ring);
+            dptr<float2>(L->d_Wf), dptr<float2>(L->d_Wb), dptr<float2>(L->d_Dinv), dptr<double>(X), nrhs, ring,
+            (nrhs + groups - 1) / groups);
     }
     k_panel_move<<<mg, 256, 0, s>>>(P.n, P.dpn, nrhs, d_vec, dptr<int>(L->d_panelOf), dptr<int>(L->d_pos),
                                     dptr<PanelMeta>(L->d_meta), dptr<double>(X), 0);
@@ -2108,6 +2196,7 @@ static int twist_prepare(astro_ctx *ctx, PanelPlan *L, int ncols) {
     std::vector<PanelMeta> mt(3);
     long long band = 0, rows = 0;
     auto put = [&](PanelMeta &M, int n, int nb, int b, int nfac) {
+        M.bw = std::min(M0.bw, nb * TB);
         M.n = n;
         M.nbc = nb;
         M.bt = b;

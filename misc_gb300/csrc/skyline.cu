@@ -136,8 +136,8 @@ __global__ void __launch_bounds__(kT) k_ldl_solve(double *soln, const double *rh
 // panels at the rows it does not cross, each panel is laid out in 32 x 32 band tiles, and the panels
 // run side by side: the factor by the FP64 band LDL^T of the panels (band_ldl64), the solves by one
 // CTA per panel.  What lies outside the profile is zero in the tiles and stays zero.  Factor and solve
-// through the host-buffer entry points: 2,214 rows of at most 11 entries 8.2 -> 0.58 ms, 6,750 rows
-// of 101 55.0 -> 3.4 ms.
+// through the host-buffer entry points: 2,214 rows of at most 11 entries 8.2 -> 0.45 ms, 6,750 rows
+// of 101 55.0 -> 2.9 ms (factor 0.23 and 1.94 ms, solve 0.08 and 0.52 ms on the GPU).
 constexpr int kSkyThreads = 256;
 
 struct SkyPanels {
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(kSkyThreads) k_sky_untile(SkyPanels S, const d
 // product with the row just solved (four warps).  Bound: that chain (a shuffle and an FP64
 // multiply-add of 64 clocks per step of the substitution).
 constexpr int kSkyWarps = kSkyThreads / TB;
-struct SkySmem {
+struct __align__(16) SkySmem {
     double diag[2][TT], next[2][TT];  // a block row's diagonal and d = 1 tiles
     double part[kSkyWarps][TB];       // partial sums over d >= 2
     double sum[2][TB];                // their sum
@@ -231,11 +231,17 @@ __device__ void sky_sweep(const PanelMeta &M, const double *__restrict__ tiles, 
     const int t = threadIdx.x, lane = t % TB, w = t / TB;
     auto stage = [&](int s) {  // warps 1 ..: what block row s needs besides the row just before it
         const int I = FWD ? s : M.nbc - 1 - s;
-        const double *D = tiles + tile_off(M, I, 0);
-        for (int e = t - TB; e < TT; e += kSkyThreads - TB) S.diag[s & 1][e] = __ldg(D + e);
-        if (s > 0 && M.bt > 0) {
-            const double *T1 = tiles + tile_off(M, FWD ? I - 1 : I, 1);
-            for (int e = t - TB; e < TT; e += kSkyThreads - TB) S.next[s & 1][e] = __ldg(T1 + e);
+        // all loads of the two tiles in flight together (three pairs of entries a thread each)
+        constexpr int kN = (TT / 2 + kSkyThreads - TB - 1) / (kSkyThreads - TB);
+        const double2 *D = reinterpret_cast<const double2 *>(tiles + tile_off(M, I, 0));
+        const bool near = s > 0 && M.bt > 0;
+        const double2 *T1 = near ? reinterpret_cast<const double2 *>(tiles + tile_off(M, FWD ? I - 1 : I, 1)) : D;
+        double2 rd[kN], rn[kN];
+#pragma unroll
+        for (int x = 0; x < kN; ++x) {
+            const int e = min(t - TB + x * (kSkyThreads - TB), TT / 2 - 1);
+            rd[x] = __ldg(D + e);
+            rn[x] = __ldg(T1 + e);
         }
         const int dmax = min(M.bt, s);
         double acc = 0.0;
@@ -243,8 +249,19 @@ __device__ void sky_sweep(const PanelMeta &M, const double *__restrict__ tiles, 
             const int d = 2 + q / 4, k0 = 8 * (q % 4);
             const double *T = tiles + tile_off(M, FWD ? I - d : I, d);
             const double *y = ring + (size_t)((s - d) % nring) * TB;
+            double l[8];
 #pragma unroll
-            for (int k = k0; k < k0 + 8; ++k) acc += __ldg(T + k * TB + lane) * y[k];
+            for (int k = 0; k < 8; ++k) l[k] = __ldg(T + (k0 + k) * TB + lane);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc += l[k] * y[k0 + k];
+        }
+#pragma unroll
+        for (int x = 0; x < kN; ++x) {
+            const int e = t - TB + x * (kSkyThreads - TB);
+            if (e < TT / 2) {
+                reinterpret_cast<double2 *>(S.diag[s & 1])[e] = rd[x];
+                reinterpret_cast<double2 *>(S.next[s & 1])[e] = rn[x];
+            }
         }
         S.part[w][lane] = acc;
         asm volatile("bar.sync 1, %0;" ::"n"(kSkyThreads - TB) : "memory");  // warps 1 .. only
@@ -561,6 +578,7 @@ static bool sky_plan(const int *R, int n, SkyPlan &L) {
         M.n = i + 1 - first;
         M.nbc = M.nfac = (M.n + TB - 1) / TB;
         M.bt = std::min((len + TB - 1) / TB, M.nbc - 1);
+        M.bw = len;
         M.band = band;
         M.xUnit = L.rows;
         band += (long long)M.nbc * (M.bt + 1) * TT;

@@ -113,6 +113,21 @@ def test_fp64_factor_tile_counts(dims, cs):
     assert np.all(np.linalg.norm(X - R, axis=0) <= 1e-10 * np.linalg.norm(R, axis=0))
 
 
+@pytest.mark.parametrize("count,nrhs", [(153, 8), (153, 7), (77, 11), (51, 16), (31, 3), (2, 9)])
+def test_solve_column_groups(count, nrhs):
+    """The columns per solve item (8 down to 1 as the batch gets smaller) in the default solve."""
+    m = M.panel_batch(num_panels=count, seed0=11, n_range=(2, 4), t_range=(0.1, 0.2), n_dvars=0)
+    g, o = AstroGPU(m), Oracle(m)
+    g.getElasticSolnLoad(1, export=False)
+    g.scaleElasticMPC()
+    A = o.static_system()[0].tocsc()
+    g.panels_factor()
+    B = np.random.default_rng(3).standard_normal((g.n, nrhs))
+    X, _ = g.panels_solve(B)
+    R = spla.splu(A).solve(B)
+    assert np.all(np.linalg.norm(X - R, axis=0) <= 1e-10 * np.linalg.norm(R, axis=0))
+
+
 def test_panel_sensitivity_pipeline(batch):
     """Pressure load per panel, the complex-step sensitivity right-hand sides at the solved state
     (against the oracle) and the batched solves of all of them."""
