@@ -16,6 +16,7 @@
 
 #include <cstdint>
 #include <functional>
+#include <map>
 #include <string>
 #include <vector>
 
@@ -23,9 +24,15 @@
 
 #define ASTRO_MAX_COLORS 64
 
+struct astro_ctx;
+
+// A device buffer of `bytes` bytes (dev_alloc, dev_free); `cap` is what was allocated for it and
+// `own` the context whose pool it returns to.
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
+    size_t cap = 0;
+    astro_ctx *own = nullptr;
 };
 
 template <class T> static inline T *dptr(DevBuf &b) { return reinterpret_cast<T *>(b.p); }
@@ -65,6 +72,9 @@ struct HostStage;  // hostcopy.cu: page-locked staging of large pageable copies
 
 struct astro_ctx {
     std::string err;
+    // freed device buffers kept for the next dev_alloc of about their size, by capacity (dev_free)
+    std::multimap<size_t, void *> pool;
+    size_t poolBytes = 0;
     // workspaces of the static solvers (FP64, mixed, learned), kept with their restart-cycle graphs
     // across solves; owned by the Krylov unit (krylov_release)
     void *solveWork[3] = {nullptr, nullptr, nullptr};
