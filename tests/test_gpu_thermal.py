@@ -114,3 +114,55 @@ def test_thermal_errors():
     with pytest.raises(AstroError) as e:
         g.thermal_solve(np.ones(m.num_nodes))
     assert e.value.code == 8
+
+
+@pytest.mark.parametrize("dims", [(1, 1, 1), (5, 5, 5), (16, 4, 2), (43, 3, 1)])
+@pytest.mark.parametrize("dynamic", [0, 1])
+def test_brick_matrix_load_and_solve_over_sizes(dims, dynamic):
+    """The factorised brick kernel, the constraint load and the conjugate gradients where a CTA or a
+    tile of rows is not full: one element, a remainder, exactly one CTA, one element over; constraints
+    that share nodes; heat generation on a list with repeats."""
+    nx, ny, nz = dims
+    m = M.hex_block(nx, ny, nz, lx=nx * 0.3, ly=ny * 0.2, lz=nz * 0.25, seed=nx, jitter=0.2)
+    rng = np.random.default_rng(nx)
+    nm = len(m.material_density)
+    k = rng.uniform(20.0, 60.0, nm)
+    cond = np.concatenate([k[:, None] * [1.0, 0.8, 1.2], k[:, None] * rng.uniform(-0.2, 0.2, (nm, 3))], axis=1)
+    sh = rng.uniform(300.0, 500.0, nm)
+    N = m.num_nodes
+    mpc = (np.array([0, 1, 3, 5]), np.array([1, 2, 1, N, 2]), np.array([1.0, 1.0, -0.5, 2.0, 1.0]),
+           np.array([10.0, 3.0, 20.0]))
+    g, o = AstroGPU(m), Oracle(m)
+    g.thermal_setup(thermal_props(cond, sh, mpc))
+    t, tp, td = rng.uniform(10.0, 30.0, (3, N))
+    els = rng.integers(1, m.num_els + 1, 7)
+    st = thermal_state(t, tp, td, dynamic, 0.5, 0.1)
+    load, mat, cols = g.getThermalSolnLoad(1, st, g.thermal_heat_gen(5.0, els))
+    lo, mo, co, row = o.thermal_soln_load(cond, sh, 1, t, tp, td, dynamic, 0.5, 0.1, load=o.thermal_heat_gen(5.0, els))
+    assert np.array_equal(cols, co) and np.abs(mat - mo).max() <= 1e-12 * np.abs(mo).max()
+    assert np.linalg.norm(load - lo) <= 1e-12 * np.linalg.norm(lo)
+    mm, mr = g.scaleThermalMPC()
+    rank = g.current_rank - 1
+    C = np.zeros((3, N))
+    for r in range(3):
+        for q in range(mpc[0][r], mpc[0][r + 1]):
+            C[r, rank[mpc[1][q] - 1]] += mm[q]
+    f = g.getThermalConstraintLoad(t, load.copy())
+    fo = load + C.T @ (mr - C @ t)
+    assert np.linalg.norm(f - fo) <= 1e-12 * np.linalg.norm(fo)
+    # the solve with two fixed nodes (a diagonal penalty): direct solve of the symmetrically scaled system
+    mpc = (np.array([0, 1, 2]), np.array([1, N]), np.ones(2), np.zeros(2))
+    g.thermal_setup(thermal_props(cond, sh, mpc))
+    _, mat, cols = g.getThermalSolnLoad(1, st)
+    mm, _ = g.scaleThermalMPC()
+    K = np.zeros((N, N))
+    for r in range(N):
+        for q in range(row[r], row[r + 1]):
+            K[r, cols[q] - 1] += mat[q]
+    for q in range(2):
+        K[rank[mpc[1][q] - 1], rank[mpc[1][q] - 1]] += mm[q] ** 2
+    d = 1.0 / np.sqrt(np.diag(K))
+    b = rng.standard_normal(N)
+    x, stats = g.thermal_solve(b, rtol=1e-13)
+    xd = d * np.linalg.solve(d[:, None] * K * d, d * b)
+    assert stats.status == 0 and np.linalg.norm(x - xd) <= 1e-9 * np.linalg.norm(xd)
