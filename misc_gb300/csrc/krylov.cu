@@ -9,12 +9,14 @@
 //     per-block-row list and is added by the same thread;
 //   * preconditioner: Jacobi on the right (A D^-1 y = b, x = D^-1 y), so the Arnoldi residual
 //     estimate is the residual of the unpreconditioned system;
-//   * orthogonalisation: classical Gram-Schmidt with one re-orthogonalisation (CGS2).  The Krylov
+//   * orthogonalisation: classical Gram-Schmidt with a re-orthogonalisation where the first pass removed
+//     more than half of the vector (CGS2).  The Krylov
 //     basis is stored vector-major (V[k*ld + i]); the dot products stage a chunk of w in shared
 //     memory and let each warp stream whole basis vectors over that chunk, the updates run one
 //     thread per row; both work in the precision of the basis.  Dot products are reduced
-//     deterministically (per-CTA partials in FP64, then one reduction CTA).  Givens rotations
-//     and the stopping test run on the device; one Arnoldi step is 7 launches and a restart
+//     deterministically (per-CTA partials in FP64, added by the last CTA to arrive).  Givens rotations
+//     and the stopping test run on the device; one Arnoldi step is 4 launches (SpMV, dots, update,
+//     second update) and a restart
 //     cycle is captured once as a CUDA graph and replayed, the host reading one status word per
 //     cycle;
 //   * precision: the plain solver runs in FP64 throughout (the comparator).  The mixed solver
@@ -52,7 +54,8 @@ __device__ __forceinline__ void loop_cond_set(const LoopCond &lc, unsigned v) {
 template <class TV, int ROWS>
 __device__ __forceinline__ void chunk_dots(const TV *__restrict__ V, size_t ld, const TV *sw, int row0, int cnt, int j,
                                            double *part, int nCh, bool self) {
-    static_assert(ROWS % 256 == 0, "tile rows: a multiple of 32 lanes x 8 loads");
+    constexpr int B = ROWS / 32 < 8 ? ROWS / 32 : 8;  // loads in flight
+    static_assert(ROWS % (32 * B) == 0, "tile rows: a multiple of 32 lanes x B loads");
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nv = j + 1 + (self ? 1 : 0);
     for (int kk = wid; kk < nv; kk += kGsWarps) {
@@ -61,12 +64,12 @@ __device__ __forceinline__ void chunk_dots(const TV *__restrict__ V, size_t ld, 
         TV s = TV(0);
         if (cnt == ROWS) {
 #pragma unroll
-            for (int u0 = 0; u0 < ROWS / 32; u0 += 8) {
-                TV v[8];
+            for (int u0 = 0; u0 < ROWS / 32; u0 += B) {
+                TV v[B];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) v[u] = vk[lane + 32 * (u0 + u)];
+                for (int u = 0; u < B; ++u) v[u] = vk[lane + 32 * (u0 + u)];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) s = fma(v[u], sw[lane + 32 * (u0 + u)], s);
+                for (int u = 0; u < B; ++u) s = fma(v[u], sw[lane + 32 * (u0 + u)], s);
             }
         } else {
             for (int t = lane; t < cnt; t += 32) s = fma(vk[t], sw[t], s);
@@ -117,33 +120,65 @@ __device__ __forceinline__ void reduce_h(GmresCtl *ctl, const double *part, int 
     if (mode != 0) return;
     if (lane == 0) shh[wid] = hh;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int q = 0; q < kGsWarps; ++q) t += shh[q];
+    if (wid != 0) return;
+    static_assert(kGsWarps == 32, "one lane per warp");
+    const double t = warp_sum(shh[lane]);
+    if (lane == 0) {
         ctl->reorth = (sww - t < 0.5 * sww) ? 1 : 0;
         ctl->reorths += ctl->reorth;
     }
 }
 
-// Norm of w from the CTA partials, Hessenberg subdiagonal, Givens rotation, residual estimate
-// and stopping test (thread 0 of the last CTA).
+// The earlier rotations of the cycle applied to column j of H (one warp): the sequential part is the
+// carried entry alone, a_{k+1} = c_k H_{k+1} - s_k a_k; the rotated entries c_k a_k + s_k H_{k+1}
+// follow in all lanes at once.  Runs beside the vector update of the step (a lane's FP64 operation
+// takes 64 clocks, so 25 rotations of four in the step control were 3 us of every step).
+__device__ void rotate_column(GmresCtl *ctl) {
+    const int lane = threadIdx.x & 31;
+    const int j = ctl->j;
+    double *Hc = ctl->H + (size_t)j * (kMaxM + 1);
+    double cs[2], sn[2], h[2], ak[2] = {0.0, 0.0};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int k = lane + 32 * u;
+        cs[u] = k < j ? ctl->cs[k] : 0.0;
+        sn[u] = k < j ? ctl->sn[k] : 0.0;
+        h[u] = k < j ? Hc[k + 1] : 0.0;
+    }
+    double a = Hc[0];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+        for (int k = 0; k < 32 && k + 32 * u < j; ++k) {
+            if (lane == k) ak[u] = a;
+            const double c = __shfl_sync(0xffffffffu, cs[u], k), s = __shfl_sync(0xffffffffu, sn[u], k),
+                         hn = __shfl_sync(0xffffffffu, h[u], k);
+            a = -s * a + c * hn;
+        }
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+        if (lane + 32 * u < j) Hc[lane + 32 * u] = cs[u] * ak[u] + sn[u] * h[u];
+    if (lane == 0) ctl->hrot = a;
+    __threadfence();
+}
+
+// Norm of w from the CTA partials, Hessenberg subdiagonal, the step's Givens rotation, residual
+// estimate and stopping test (warp 0 of the last CTA; rotate_column has run).
 __device__ void step_control(GmresCtl *ctl, const double *part, int nCh, int m) {
     const int lane = threadIdx.x & 31;
     if (threadIdx.x >= 32) return;
     double s = 0.0;
-    for (int q = lane; q < nCh; q += 32) s += __ldcg(part + q);
+    for (int q0 = lane; q0 < nCh; q0 += 256) {
+        double v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = q0 + 32 * u < nCh ? __ldcg(part + q0 + 32 * u) : 0.0;
+        s += ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+    }
     s = warp_sum(s);
     if (lane != 0) return;
     const int j = ctl->j;
     const double nrm = sqrt(s);
     double *Hc = ctl->H + (size_t)j * (kMaxM + 1);
-    Hc[j + 1] = nrm;
-    for (int k = 0; k < j; ++k) {
-        const double a = Hc[k], b = Hc[k + 1];
-        Hc[k] = ctl->cs[k] * a + ctl->sn[k] * b;
-        Hc[k + 1] = -ctl->sn[k] * a + ctl->cs[k] * b;
-    }
-    const double a = Hc[j], b = Hc[j + 1];
+    const double a = __ldcg(&ctl->hrot), b = nrm;
     const double rr = hypot(a, b);
     double c = 1.0, sn = 0.0;
     if (rr > 0.0) {
@@ -177,25 +212,25 @@ __device__ void step_control(GmresCtl *ctl, const double *part, int nCh, int m) 
 // v_j = wprev * inv (written to V[j]); w = A D^-1 v_j = inv * A zprev with zprev = D^-1 wprev.
 // Warp-per-slot-group mapping (kRowThreads warps per 32 block rows, partials met in shared
 // memory); the products accumulate in the precision of the basis.
-template <class TM, class TV, int DPN>
+template <class TM, class TV, int DPN, int RT>
 __global__ void __launch_bounds__(kThreads) k_spmv_step(Op<TM> op, TV *__restrict__ V, size_t ld, const TV *__restrict__ wprev,
                                                         const TV *__restrict__ zprev, TV *__restrict__ w,
                                                         const GmresCtl *__restrict__ ctl) {
     if (ctl->done) return;
-    const CtaRow c = cta_row(op.N);  // (the FP64 branch keeps the CTA's 64 rows, lane-grouped)
+    const CtaRow c = cta_row(op.N);
     const int j = ctl->j;
     const TV inv = (TV)ctl->inv;
     TV y[DPN] = {};
     if constexpr (sizeof(TM) == 8) {
-        // FP64 comparator: kRowThreads adjacent lanes per block row, partials combined by shuffles
-        // (the FP64 products bound this kernel, not its loads); same grid, rows renumbered
-        const int r = blockIdx.x * kCtaRows + (int)threadIdx.x / kRowThreads, sub = threadIdx.x % kRowThreads;
+        // FP64 comparator: RT adjacent lanes per block row, partials combined by shuffles (the FP64
+        // products bound this kernel, not its loads)
+        const int r = blockIdx.x * (kThreads / RT) + (int)threadIdx.x / RT, sub = threadIdx.x % RT;
         const int rr = r < op.N ? r : op.N - 1;
-        ell_row_part<TV, TM, TV, DPN>(op, rr, sub, zprev, y);
+        ell_row_part<TV, TM, TV, DPN, RT>(op, rr, sub, zprev, y);
         if (r >= op.N) return;
 #pragma unroll
         for (int q = 0; q < DPN; ++q) {
-            if (q % kRowThreads != sub) continue;
+            if (q % RT != sub) continue;
             const size_t i = (size_t)r * DPN + q;
             V[(size_t)j * ld + i] = wprev[i] * inv;
             w[i] = y[q] * inv;
@@ -400,17 +435,17 @@ __global__ void k_add(int n, TV *__restrict__ x, const TV *__restrict__ d) {
 
 // First Gram-Schmidt pass: partial dots of w with V[0..j] and with itself over this CTA's rows;
 // the last CTA reduces them into h1 and decides whether a second pass is needed.
-template <class TV>
+template <class TV, int ROWS>
 __global__ void __launch_bounds__(kGsThreads, 2) k_dots(int n, const TV *__restrict__ V, size_t ld, const TV *__restrict__ w,
                                                         GmresCtl *__restrict__ ctl, double *part, int nCh) {
     if (ctl->done) return;
-    __shared__ TV sw[kChunk];
-    const int row0 = blockIdx.x * kChunk;
-    const int cnt = min(kChunk, n - row0);
+    __shared__ TV sw[ROWS];
+    const int row0 = blockIdx.x * ROWS;
+    const int cnt = min(ROWS, n - row0);
     const int j = ctl->j;
     for (int t = threadIdx.x; t < cnt; t += kGsThreads) sw[t] = w[row0 + t];
     __syncthreads();
-    chunk_dots<TV, kChunk>(V, ld, sw, row0, cnt, j, part, nCh, true);
+    chunk_dots<TV, ROWS>(V, ld, sw, row0, cnt, j, part, nCh, true);
     if (last_to_arrive(&ctl->arrive[0])) reduce_h(ctl, part, nCh, j, 0);
 }
 
@@ -420,13 +455,12 @@ __global__ void __launch_bounds__(kGsThreads, 2) k_dots(int n, const TV *__restr
 // (pass 1), the step finishes here: the partial ||w||^2, the Jacobi-scaled copy z = D^-1 w read
 // by the next SpMV, and the step control in the last CTA.  The second update returns at once
 // when no second pass was requested.
-template <class TV>
+template <class TV, int ROWS>
 __global__ void __launch_bounds__(kGsThreads, 2) k_update(int n, const TV *__restrict__ V, size_t ld, TV *__restrict__ w,
                                                           GmresCtl *__restrict__ ctl, double *__restrict__ partDots,
                                                           double *__restrict__ partNorm, int nCh, int pass,
                                                           const TV *__restrict__ dinv, TV *__restrict__ z, int m,
                                                           LoopCond lc) {
-    constexpr int ROWS = kChunk;
     if (ctl->done) return;
     const bool second = ctl->reorth != 0;
     if (pass == 1 && !second) return;
@@ -438,6 +472,9 @@ __global__ void __launch_bounds__(kGsThreads, 2) k_update(int n, const TV *__res
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (int k = threadIdx.x; k <= j; k += kGsThreads) sh[k] = (TV)ctl->h1[k];
     __syncthreads();
+    // the column is complete: its earlier rotations, beside the update (the last warp: idle in CTAs of
+    // fewer rows than threads)
+    if (finish && blockIdx.x == 0 && wid == kGsWarps - 1) rotate_column(ctl);
     const int row0 = blockIdx.x * ROWS;
     const int cnt = min(ROWS, n - row0);
     TV nrm = TV(0);
@@ -466,14 +503,15 @@ __global__ void __launch_bounds__(kGsThreads, 2) k_update(int n, const TV *__res
         chunk_dots<TV, ROWS>(V, ld, sw, row0, cnt, j, partDots, nCh, false);
         if (last_to_arrive(&ctl->arrive[1])) reduce_h(ctl, partDots, nCh, j, 1);
     } else {
-        nrm = warp_sum(nrm);
+        if (wid * 32 < ROWS) nrm = warp_sum(nrm);
         if (lane == 0) sred[wid] = (double)nrm;
         __syncthreads();
-        if (threadIdx.x == 0) {
-            double s = 0.0;
-            for (int q = 0; q < kGsWarps; ++q) s += sred[q];
-            partNorm[blockIdx.x] = s;
-            __threadfence();
+        if (wid == 0) {
+            const double s = warp_sum(sred[lane]);
+            if (lane == 0) {
+                partNorm[blockIdx.x] = s;
+                __threadfence();
+            }
         }
         if (last_to_arrive(&ctl->arrive[2])) {
             step_control(ctl, partNorm, nCh, m);
@@ -498,14 +536,33 @@ __device__ __forceinline__ double lane_sum(const double *part, int nparts, size_
     return s;
 }
 
-// Least squares H y = g (upper triangular j x j), one thread.
+// Least squares H y = g (upper triangular j x j), one warp: lane = row (two rows a lane), the columns from
+// the last; a quotient by the reciprocal with one correction, so that the chain per column is four
+// multiply-adds instead of a division (one thread: 128 us a cycle of 50 steps).
 __global__ void k_lsq(GmresCtl *ctl) {
-    const int j = ctl->j;
-    for (int i = j - 1; i >= 0; --i) {
-        double s = ctl->g[i];
-        for (int k = i + 1; k < j; ++k) s -= ctl->H[(size_t)k * (kMaxM + 1) + i] * ctl->y[k];
-        ctl->y[i] = s / ctl->H[(size_t)i * (kMaxM + 1) + i];
+    static_assert(kMaxM <= 64, "two rows a lane");
+    const int j = ctl->j, lane = threadIdx.x;
+    double g[2], d[2], r[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int i = lane + 32 * u;
+        g[u] = i < j ? ctl->g[i] : 0.0;
+        d[u] = i < j ? ctl->H[(size_t)i * (kMaxM + 1) + i] : 1.0;
+        r[u] = 1.0 / d[u];
     }
+#pragma unroll
+    for (int v = 1; v >= 0; --v)
+        for (int k = min(31, j - 1 - 32 * v); k >= 0; --k) {
+            const int col = 32 * v + k;
+            double h[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) h[u] = lane + 32 * u < col ? ctl->H[(size_t)col * (kMaxM + 1) + lane + 32 * u] : 0.0;
+            const double q0 = g[v] * r[v], y = __shfl_sync(0xffffffffu, fma(fma(-d[v], q0, g[v]), r[v], q0), k);
+            if (lane == k) ctl->y[col] = y;
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                if (u <= v) g[u] = fma(-h[u], y, g[u]);
+        }
 }
 
 // x += D^-1 V[0..j-1] y, or with out the preconditioner input out = D^-1 V[0..j-1] y (the
@@ -535,49 +592,60 @@ __global__ void __launch_bounds__(kThreads) k_xupdate(int n, const TV *__restric
 }
 
 // r = b - A x with the products accumulated in FP64, partial ||r||^2 and ||b||^2 per CTA; with
-// z also the Jacobi-scaled copy z = D^-1 r.  One thread per block row.
-template <class TM, class TX, class TR, int DPN>
+// z also the Jacobi-scaled copy z = D^-1 r.  RT lanes per block row (res_lanes): the FP64 pipe bounds the
+// products (81 .. 243 multiply-adds a row), so the rows have to reach all SMs with four warps or more,
+// and the lanes' sums add to its work (one thread a row took 70 us on every model up to 70,000 rows).
+template <class TM, class TX, class TR, int DPN, int RT>
 __global__ void __launch_bounds__(kThreads) k_residual(Op<TM> op, const TX *__restrict__ x, const double *__restrict__ b,
                                                        TR *__restrict__ r, double *part, const TR *__restrict__ dinv = nullptr,
                                                        TR *__restrict__ z = nullptr) {
-    __shared__ double sp[kWarps][2];
+    __shared__ double sp[2][kWarps][32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int row = blockIdx.x * kThreads + threadIdx.x;
+    const int row = blockIdx.x * (kThreads / RT) + threadIdx.x / RT, sub = threadIdx.x % RT;
     double rr = 0.0, bb = 0.0;
-    if (row < op.N) {
-        double y[DPN];
-        if (x) {
-            ell_row<double, TM, TX, DPN>(op, row, x, y);
-        } else {
+    double y[DPN];
+    if (x) {
+        ell_row_part<double, TM, TX, DPN, RT>(op, min(row, op.N - 1), sub, x, y);
+    } else {
 #pragma unroll
-            for (int q = 0; q < DPN; ++q) y[q] = 0.0;
-        }
+        for (int q = 0; q < DPN; ++q) y[q] = 0.0;
+    }
+    if (row < op.N) {
 #pragma unroll
         for (int q = 0; q < DPN; ++q) {
+            if (q % RT != sub) continue;
             const size_t i = (size_t)row * DPN + q;
-            const double v = b[i] - y[q];
+            const double bv = b[i], v = bv - y[q];
             const TR rv = (TR)v;
             r[i] = rv;
             if (z) z[i] = dinv[i] * rv;
             rr += v * v;
-            bb += b[i] * b[i];
+            bb += bv * bv;
         }
     }
-    rr = warp_sum(rr);
-    bb = warp_sum(bb);
-    if (lane == 0) {
-        sp[wid][0] = rr;
-        sp[wid][1] = bb;
-    }
+    sp[0][wid][lane] = rr;
+    sp[1][wid][lane] = bb;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double a = 0.0, c = 0.0;
-        for (int q = 0; q < kWarps; ++q) {
-            a += sp[q][0];
-            c += sp[q][1];
-        }
-        part[2 * blockIdx.x] = a;
-        part[2 * blockIdx.x + 1] = c;
+    if (wid < 2) {  // across the warps first: five additions of a shuffle tree once, not per warp
+        double a = 0.0;
+#pragma unroll
+        for (int q = 0; q < kWarps; ++q) a += sp[wid][q][lane];
+        a = warp_sum(a);
+        if (lane == 0) part[2 * blockIdx.x + wid] = a;
+    }
+}
+
+// Lanes per row of k_residual: enough that four warps of rows reach every SM (152).
+static int res_lanes(int N) { return N < 9728 ? 8 : (N < 38912 ? 2 : 1); }
+static int res_ctas(int N) { return (N + kThreads / res_lanes(N) - 1) / (kThreads / res_lanes(N)); }
+template <class TM, class TX, class TR, int DPN>
+static void launch_residual(const Op<TM> &op, const TX *x, const double *b, TR *r, double *part, const TR *dinv, TR *z,
+                            cudaStream_t s) {
+    const int g = res_ctas(op.N);
+    switch (res_lanes(op.N)) {
+    case 8: k_residual<TM, TX, TR, DPN, 8><<<g, kThreads, 0, s>>>(op, x, b, r, part, dinv, z); break;
+    case 2: k_residual<TM, TX, TR, DPN, 2><<<g, kThreads, 0, s>>>(op, x, b, r, part, dinv, z); break;
+    default: k_residual<TM, TX, TR, DPN, 1><<<g, kThreads, 0, s>>>(op, x, b, r, part, dinv, z); break;
     }
 }
 
@@ -684,10 +752,11 @@ struct GmresWork {
     // restart cycle captured as a graph, reused while the matrix and vectors stay the same
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    const void *gK = nullptr, *gx = nullptr, *gb = nullptr;
+    const void *gK = nullptr, *gx = nullptr, *gb = nullptr, *gPen = nullptr;
     PolyHost gPoly;  // the hop parameters the graph was captured with
     int n = 0, m = 0;
     size_t ld = 0;
+    int rows = 1024;  // vector rows per CTA of the Gram-Schmidt passes
     int nChunks = 0, nRowCtas = 0;
     std::vector<double> hp;
 };
@@ -792,6 +861,29 @@ static TV *enqueue_poly(astro_ctx *ctx, GmresWork &W, TV *y0, int always, cudaSt
     return z;
 }
 
+// Vector rows per CTA of the Gram-Schmidt passes: the fewest of 128 .. 1024 with at most two CTAs per SM
+// (152 SMs): below that the FP64 pipes of the SMs that have a CTA bound the passes, above it only the
+// number of partials grows.  14,112 rows in FP64: a step took 75 us with 1024 rows a CTA, 41 us with
+// these (the SpMV's eight lanes a row included).
+static int gs_rows(int n) {
+    int rows = 128;
+    while (rows < 1024 && (n + rows - 1) / rows > 304) rows *= 2;
+    return rows;
+}
+
+template <class TV, int ROWS>
+static void enqueue_gs(GmresWork &W, TV *wnew, TV *znew, const TV *dinv, int m, LoopCond lc, cudaStream_t s) {
+    GmresCtl *ctl = dptr<GmresCtl>(W.ctl);
+    const TV *V = dptr<TV>(W.V);
+    double *part = dptr<double>(W.part);
+    double *partB = part + (size_t)(kMaxM + 1) * W.nChunks;
+    double *partN = partB + (size_t)(kMaxM + 1) * W.nChunks;  // per-CTA ||w||^2 of the step's last update
+    k_dots<TV, ROWS><<<W.nChunks, kGsThreads, 0, s>>>(W.n, V, W.ld, wnew, ctl, part, W.nChunks);
+    for (int pass = 0; pass < 2; ++pass)
+        k_update<TV, ROWS><<<W.nChunks, kGsThreads, 0, s>>>(W.n, V, W.ld, wnew, ctl, partB, partN, W.nChunks, pass, dinv,
+                                                            znew, m, lc);
+}
+
 // Enqueues Arnoldi steps first..first+nsteps-1 on s (the w/z buffers alternate with the step's
 // parity); with lc.use each step's control sets the condition lc (of the next IF node).
 template <class TM, class TV, int DPN>
@@ -800,20 +892,27 @@ static void enqueue_cycle(astro_ctx *ctx, GmresWork &W, const Op<TM> &op, int m,
     TV *V = dptr<TV>(W.V), *wa = dptr<TV>(W.w0), *wb = dptr<TV>(W.w1);
     TV *za = dptr<TV>(W.z0), *zb = dptr<TV>(W.z1);
     GmresCtl *ctl = dptr<GmresCtl>(W.ctl);
-    double *part = dptr<double>(W.part);
     const TV *dinv = W.y0s<TV>();
-    const int n = W.n;
-    double *partB = part + (size_t)(kMaxM + 1) * W.nChunks;
-    double *partN = partB + (size_t)(kMaxM + 1) * W.nChunks;  // per-CTA ||w||^2 of the step's last update
-    const unsigned spmvGrid = (unsigned)((ctx->P.N + kCtaRows - 1) / kCtaRows);
+    // FP64: eight lanes a row while four leave SMs without a CTA
+    const int N = ctx->P.N;
+    const bool wide = sizeof(TM) == 8 && (N + kCtaRows - 1) / kCtaRows < 304;
+    const unsigned spmvGrid = (unsigned)(wide ? (N + kThreads / 8 - 1) / (kThreads / 8) : (N + kCtaRows - 1) / kCtaRows);
     for (int step = first; step < first + nsteps; ++step) {
         TV *wprev = (step % 2 == 0) ? wa : wb, *zprev = (step % 2 == 0) ? za : zb;
         TV *wnew = (step % 2 == 0) ? wb : wa, *znew = (step % 2 == 0) ? zb : za;
         const TV *zin = W.poly ? enqueue_poly<TM, TV, DPN>(ctx, W, zprev, 0, s) : zprev;
-        k_spmv_step<TM, TV, DPN><<<spmvGrid, kThreads, 0, s>>>(op, V, W.ld, wprev, zin, wnew, ctl);
-        k_dots<TV><<<W.nChunks, kGsThreads, 0, s>>>(n, V, W.ld, wnew, ctl, part, W.nChunks);
-        k_update<TV><<<W.nChunks, kGsThreads, 0, s>>>(n, V, W.ld, wnew, ctl, partB, partN, W.nChunks, 0, dinv, znew, m, lc);
-        k_update<TV><<<W.nChunks, kGsThreads, 0, s>>>(n, V, W.ld, wnew, ctl, partB, partN, W.nChunks, 1, dinv, znew, m, lc);
+        if (wide) {
+            if constexpr (sizeof(TM) == 8)
+                k_spmv_step<TM, TV, DPN, 8><<<spmvGrid, kThreads, 0, s>>>(op, V, W.ld, wprev, zin, wnew, ctl);
+        } else {
+            k_spmv_step<TM, TV, DPN, kRowThreads><<<spmvGrid, kThreads, 0, s>>>(op, V, W.ld, wprev, zin, wnew, ctl);
+        }
+        switch (W.rows) {
+        case 128: enqueue_gs<TV, 128>(W, wnew, znew, dinv, m, lc, s); break;
+        case 256: enqueue_gs<TV, 256>(W, wnew, znew, dinv, m, lc, s); break;
+        case 512: enqueue_gs<TV, 512>(W, wnew, znew, dinv, m, lc, s); break;
+        default: enqueue_gs<TV, 1024>(W, wnew, znew, dinv, m, lc, s); break;
+        }
     }
 }
 
@@ -841,7 +940,8 @@ static int gmres_solve(astro_ctx *ctx, GmresWork &W, const TM *K, TV *x, const d
     CK(cudaMemcpyAsync(W.tgt.p, &tgtAbs, sizeof(double), cudaMemcpyHostToDevice, s));
     const bool samePoly = W.poly ? (W.gPoly.deg == W.poly->deg && std::memcmp(&W.gPoly, W.poly, sizeof(PolyHost)) == 0)
                                  : W.gPoly.deg == 0;
-    if (!(W.exec && W.gK == K && W.gx == x && W.gb == b && samePoly)) {
+    // (the penalty lists are uploaded anew with every constraint scaling: their place is part of the key)
+    if (!(W.exec && W.gK == K && W.gx == x && W.gb == b && W.gPen == op.penVal && samePoly)) {
         if (W.exec) cudaGraphExecDestroy(W.exec);
         if (W.graph) cudaGraphDestroy(W.graph);
         W.exec = nullptr;
@@ -853,8 +953,7 @@ static int gmres_solve(astro_ctx *ctx, GmresWork &W, const TM *K, TV *x, const d
         bool cond = W.condOk;
         for (int attempt = 0; attempt < 2 && !W.graph; ++attempt) {
             CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-            k_residual<TM, TV, TV, DPN><<<W.nRowCtas, kThreads, 0, s>>>(op, x, b, dptr<TV>(W.w0), part, W.y0s<TV>(),
-                                                                         dptr<TV>(W.z0));
+            launch_residual<TM, TV, TV, DPN>(op, x, b, dptr<TV>(W.w0), part, W.y0s<TV>(), dptr<TV>(W.z0), s);
             // one handle per IF node (a handle belongs to one node): the cycle start sets the first,
             // the steps behind node i set the handle of node i + 1; every handle starts each
             // launch at 0, so the nodes after a skipped one are skipped too
@@ -902,7 +1001,7 @@ static int gmres_solve(astro_ctx *ctx, GmresWork &W, const TM *K, TV *x, const d
             } else {
                 enqueue_cycle<TM, TV, DPN>(ctx, W, op, m, 0, m, s, none);
             }
-            k_lsq<<<1, 1, 0, s>>>(ctl);
+            k_lsq<<<1, 32, 0, s>>>(ctl);
             if (W.poly) {
                 TV *y0 = dptr<TV>(W.z0);
                 k_xupdate<TV, TV><<<4 * 152, kThreads, 0, s>>>(W.n, dptr<TV>(W.V), W.ld, W.y0s<TV>(), ctl, x, y0);
@@ -938,6 +1037,7 @@ static int gmres_solve(astro_ctx *ctx, GmresWork &W, const TM *K, TV *x, const d
         W.gK = K;
         W.gx = x;
         W.gb = b;
+        W.gPen = op.penVal;
     }
     cudaGraphExec_t exec = W.exec;
     int status = ASTRO_OK;
@@ -967,8 +1067,9 @@ static int work_alloc(astro_ctx *ctx, GmresWork &W, int m, int tv) {
     W.n = n;
     W.m = m;
     W.ld = ((size_t)n + 31) / 32 * 32;
-    W.nChunks = (n + kChunk - 1) / kChunk;
-    W.nRowCtas = (ctx->P.N + kThreads - 1) / kThreads;
+    W.rows = gs_rows(n);
+    W.nChunks = (n + W.rows - 1) / W.rows;
+    W.nRowCtas = res_ctas(ctx->P.N);
     const size_t nparts = std::max((size_t)3 * W.nChunks * (kMaxM + 1), (size_t)2 * W.nRowCtas);
     int rc;
     if ((rc = dev_alloc(ctx, W.V, W.ld * (m + 1) * tv))) return rc;
@@ -1033,7 +1134,8 @@ void krylov_release(astro_ctx *ctx) {
     }
 }
 
-// r = b - A x with A from K64 (kind 64) or K32 (kind 32); returns ||r||/||b|| (||r|| if b = 0).
+// r = b - A x with A from K64 (kind 64) or K32 (kind 32); *rel = ||r||/||b|| (||r|| if b = 0), waited for
+// unless rel is null.
 template <int DPN>
 static int true_residual(astro_ctx *ctx, GmresWork &W, int kind, const double *x, const double *b, double *rel,
                          double *r_out, double *rnorm = nullptr, double *bnorm = nullptr) {
@@ -1044,14 +1146,15 @@ static int true_residual(astro_ctx *ctx, GmresWork &W, int kind, const double *x
         const double *Kp = ell_of<double>(ctx, &prc);
         if (prc) return prc;
         Op<double> op = make_op<double>(ctx, Kp);
-        k_residual<double, double, double, DPN><<<W.nRowCtas, kThreads, 0, s>>>(op, x, b, r_out, part);
+        launch_residual<double, double, double, DPN>(op, x, b, r_out, part, nullptr, nullptr, s);
     } else {
         const float *Kp = ell_of<float>(ctx, &prc);
         if (prc) return prc;
         Op<float> op = make_op<float>(ctx, Kp);
-        k_residual<float, double, double, DPN><<<W.nRowCtas, kThreads, 0, s>>>(op, x, b, r_out, part);
+        launch_residual<float, double, double, DPN>(op, x, b, r_out, part, nullptr, nullptr, s);
     }
-    int rc = ASTRO_OK;
+    int rc = cuda_check(ctx, cudaGetLastError(), "residual");
+    if (rc || !rel) return rc;
     const double a = sum_parts(ctx, W, 0, &rc);
     if (rc) return rc;
     double c = 0.0;
@@ -1497,15 +1600,14 @@ int krylov_power_lambda(astro_ctx *ctx, int kind, double *lam) {
 int krylov_apply(astro_ctx *ctx, int kind, const double *d_x, double *d_y) {
     GmresWork W;
     W.n = ctx->P.n;
-    W.nRowCtas = (ctx->P.N + kThreads - 1) / kThreads;
+    W.nRowCtas = res_ctas(ctx->P.N);
     int rc = dev_alloc(ctx, W.part, sizeof(double) * 2 * W.nRowCtas);
     if (rc) return rc;
     DevBuf zb;
     if ((rc = dev_alloc(ctx, zb, sizeof(double) * ctx->P.n))) return rc;
     CK(cudaMemsetAsync(zb.p, 0, sizeof(double) * ctx->P.n, ctx->stream));
-    double rel;
-    if (ctx->P.dpn == 3) rc = true_residual<3>(ctx, W, kind, d_x, dptr<double>(zb), &rel, d_y);
-    else rc = true_residual<6>(ctx, W, kind, d_x, dptr<double>(zb), &rel, d_y);
+    if (ctx->P.dpn == 3) rc = true_residual<3>(ctx, W, kind, d_x, dptr<double>(zb), nullptr, d_y);
+    else rc = true_residual<6>(ctx, W, kind, d_x, dptr<double>(zb), nullptr, d_y);
     dev_free(zb);
     dev_free(W.part);
     return rc;
@@ -1516,12 +1618,11 @@ int krylov_apply(astro_ctx *ctx, int kind, const double *d_x, double *d_y) {
 int krylov_residual64(astro_ctx *ctx, const double *d_x, const double *d_b, double *d_r) {
     GmresWork W;
     W.n = ctx->P.n;
-    W.nRowCtas = (ctx->P.N + kThreads - 1) / kThreads;
+    W.nRowCtas = res_ctas(ctx->P.N);
     int rc = dev_alloc(ctx, W.part, sizeof(double) * 2 * W.nRowCtas);
     if (rc) return rc;
-    double rel;
-    if (ctx->P.dpn == 3) rc = true_residual<3>(ctx, W, 64, d_x, d_b, &rel, d_r);
-    else rc = true_residual<6>(ctx, W, 64, d_x, d_b, &rel, d_r);
+    if (ctx->P.dpn == 3) rc = true_residual<3>(ctx, W, 64, d_x, d_b, nullptr, d_r);
+    else rc = true_residual<6>(ctx, W, 64, d_x, d_b, nullptr, d_r);
     dev_free(W.part);
     return rc;
 }

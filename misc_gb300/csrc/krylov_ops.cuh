@@ -12,7 +12,6 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kGsThreads = 1024;  // threads per CTA of the Gram-Schmidt passes
 constexpr int kGsWarps = kGsThreads / 32;
-constexpr int kChunk = 1024;      // vector rows per CTA in the Gram-Schmidt passes (one per thread)
 constexpr int kRowThreads = 4;    // threads per block row in the SpMV
 
 struct GmresCtl {
@@ -22,6 +21,7 @@ struct GmresCtl {
     double y[kMaxM];
     double inv;      // 1 / ||w|| of the last step (scales w into the next basis vector)
     double target;   // absolute residual target
+    double hrot;     // the last entry of the column of H, rotated by the earlier rotations
     double resest;   // |g[j]| after the last step
     int j;           // completed Arnoldi steps in this cycle
     int done;        // converged / broke down / cycle full: later steps are no-ops
@@ -90,35 +90,51 @@ __device__ __forceinline__ void ell_row(const Op<TM> &op, int r, const TX *__res
     }
 }
 
-// Partial (A x)_r over the slots s = sub, sub + kRowThreads, ... of block row r; the products
-// accumulate in TA.  The kRowThreads threads of a row are adjacent lanes and combine their
-// partials with xor-shuffles (result in all of them); thread sub == 0 adds the penalty.
-template <class TA, class TM, class TX, int DPN>
+// (A x)_r by RT adjacent lanes: the slots s = sub, sub + RT, ... each, the partials combined with
+// xor-shuffles (result in all of them); the products accumulate in TA, thread sub == 0 adds the penalty.
+template <class TA, class TM, class TX, int DPN, int RT>
 __device__ __forceinline__ void ell_row_part(const Op<TM> &op, int r, int sub, const TX *__restrict__ x, TA y[DPN]) {
+    // U slots at a time, every load of them in flight before the first product (one slot at a time waits
+    // for its column, then for x: two trips to L2 a slot)
+    constexpr int U = DPN == 3 ? 4 : 2;
 #pragma unroll
     for (int i = 0; i < DPN; ++i) y[i] = TA(0);
     const size_t ld = (size_t)op.ld;
-    for (int s = sub; s < op.S; s += kRowThreads) {
-        const int c = __ldg(op.col + (size_t)s * ld + r);
-        TA xv[DPN];
+    const int p0 = sub == 0 && op.penPtr ? __ldg(op.penPtr + r) : 0, p1 = sub == 0 && op.penPtr ? __ldg(op.penPtr + r + 1) : 0;
+    for (int s0 = sub; s0 < op.S; s0 += U * RT) {
+        int c[U];
+        TM k[U][DPN * DPN];
 #pragma unroll
-        for (int jj = 0; jj < DPN; ++jj) xv[jj] = (TA)x[(size_t)c * DPN + jj];
-        const TM *kp = op.K + (size_t)s * DPN * DPN * ld + r;
+        for (int u = 0; u < U; ++u) {
+            const bool has = s0 + u * RT < op.S;
+            const int s = has ? s0 + u * RT : s0;
+            c[u] = __ldg(op.col + (size_t)s * ld + r);
+            const TM *kp = op.K + (size_t)s * DPN * DPN * ld + r;
 #pragma unroll
-        for (int i = 0; i < DPN; ++i)
+            for (int q = 0; q < DPN * DPN; ++q) k[u][q] = has ? __ldg(kp + (size_t)q * ld) : TM(0);
+        }
+        TX xv[U][DPN];
 #pragma unroll
-            for (int jj = 0; jj < DPN; ++jj) y[i] += (TA)__ldg(kp + (size_t)(i * DPN + jj) * ld) * xv[jj];
-    }
-    if (sub == 0 && op.penPtr) {
-        for (int t = op.penPtr[r]; t < op.penPtr[r + 1]; ++t) {
-            const TA p = (TA)(op.penVal[t] * (double)x[op.penCol[t]]);
-            const int i = op.penRow[t];
+        for (int u = 0; u < U; ++u)
 #pragma unroll
-            for (int q = 0; q < DPN; ++q) y[q] += (q == i) ? p : TA(0);
+            for (int jj = 0; jj < DPN; ++jj) xv[u][jj] = x[(size_t)c[u] * DPN + jj];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (s0 + u * RT >= op.S) break;
+#pragma unroll
+            for (int i = 0; i < DPN; ++i)
+#pragma unroll
+                for (int jj = 0; jj < DPN; ++jj) y[i] += (TA)k[u][i * DPN + jj] * (TA)xv[u][jj];
         }
     }
+    for (int t = p0; t < p1; ++t) {
+        const TA p = (TA)(op.penVal[t] * (double)x[op.penCol[t]]);
+        const int i = op.penRow[t];
 #pragma unroll
-    for (int m = 1; m < kRowThreads; m <<= 1)
+        for (int q = 0; q < DPN; ++q) y[q] += (q == i) ? p : TA(0);
+    }
+#pragma unroll
+    for (int m = 1; m < RT; m <<= 1)
 #pragma unroll
         for (int i = 0; i < DPN; ++i) y[i] += __shfl_xor_sync(0xffffffffu, y[i], m);
 }
