@@ -592,61 +592,48 @@ __global__ void __launch_bounds__(kThreads) k_xupdate(int n, const TV *__restric
 }
 
 // r = b - A x with the products accumulated in FP64, partial ||r||^2 and ||b||^2 per CTA; with
-// z also the Jacobi-scaled copy z = D^-1 r.  RT lanes per block row (res_lanes): the FP64 pipe bounds the
-// products (81 .. 243 multiply-adds a row), so the rows have to reach all SMs with four warps or more,
-// and the lanes' sums add to its work (one thread a row took 70 us on every model up to 70,000 rows).
-template <class TM, class TX, class TR, int DPN, int RT>
-__global__ void __launch_bounds__(kThreads) k_residual(Op<TM> op, const TX *__restrict__ x, const double *__restrict__ b,
-                                                       TR *__restrict__ r, double *part, const TR *__restrict__ dinv = nullptr,
-                                                       TR *__restrict__ z = nullptr) {
-    __shared__ double sp[2][kWarps][32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int row = blockIdx.x * (kThreads / RT) + threadIdx.x / RT, sub = threadIdx.x % RT;
+// z also the Jacobi-scaled copy z = D^-1 r.  A thread takes one component of a block row (a warp 32
+// rows), 32 rows a CTA while there are few (res_rows): the FP64 pipe bounds the products (81 .. 243
+// multiply-adds a row), so the rows have to reach all SMs.  30,625 rows of 27 blocks of 3: 26 us (one thread
+// a row 70 us); the sum over a row keeps its order, slots ascending.
+template <class TM, class TX, class TR, int DPN>
+__global__ void __launch_bounds__(kResidT) k_residual(Op<TM> op, const TX *__restrict__ x, const double *__restrict__ b,
+                                                      TR *__restrict__ r, double *part, const TR *__restrict__ dinv = nullptr,
+                                                      TR *__restrict__ z = nullptr) {
+    __shared__ double sp[2][kResidT / 32][32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x / 32;
+    const int q = wid % DPN, row = (blockIdx.x * (nw / DPN) + wid / DPN) * 32 + lane;
     double rr = 0.0, bb = 0.0;
-    double y[DPN];
-    if (x) {
-        ell_row_part<double, TM, TX, DPN, RT>(op, min(row, op.N - 1), sub, x, y);
-    } else {
-#pragma unroll
-        for (int q = 0; q < DPN; ++q) y[q] = 0.0;
-    }
     if (row < op.N) {
-#pragma unroll
-        for (int q = 0; q < DPN; ++q) {
-            if (q % RT != sub) continue;
-            const size_t i = (size_t)row * DPN + q;
-            const double bv = b[i], v = bv - y[q];
-            const TR rv = (TR)v;
-            r[i] = rv;
-            if (z) z[i] = dinv[i] * rv;
-            rr += v * v;
-            bb += bv * bv;
-        }
+        const size_t i = (size_t)row * DPN + q;
+        double y = 0.0;
+        if (x) y = ell_row_comp<double, TM, TX, DPN>(op, row, q, x);
+        const double bv = b[i], v = bv - y;
+        const TR rv = (TR)v;
+        r[i] = rv;
+        if (z) z[i] = dinv[i] * rv;
+        rr = v * v;
+        bb = bv * bv;
     }
     sp[0][wid][lane] = rr;
     sp[1][wid][lane] = bb;
     __syncthreads();
     if (wid < 2) {  // across the warps first: five additions of a shuffle tree once, not per warp
         double a = 0.0;
-#pragma unroll
-        for (int q = 0; q < kWarps; ++q) a += sp[wid][q][lane];
+        for (int u = 0; u < nw; ++u) a += sp[wid][u][lane];
         a = warp_sum(a);
         if (lane == 0) part[2 * blockIdx.x + wid] = a;
     }
 }
 
-// Lanes per row of k_residual: enough that four warps of rows reach every SM (152).
-static int res_lanes(int N) { return N < 9728 ? 8 : (N < 38912 ? 2 : 1); }
-static int res_ctas(int N) { return (N + kThreads / res_lanes(N) - 1) / (kThreads / res_lanes(N)); }
+// Rows per CTA of k_residual: 32 while that gives every SM (152) no more than eight CTAs, else 128 (fewer
+// partial sums for the one warp that adds them).
+static int res_rows(int N) { return N <= 32 * 152 * 8 ? 32 : 128; }
+static int res_ctas(int N) { return (N + res_rows(N) - 1) / res_rows(N); }
 template <class TM, class TX, class TR, int DPN>
 static void launch_residual(const Op<TM> &op, const TX *x, const double *b, TR *r, double *part, const TR *dinv, TR *z,
                             cudaStream_t s) {
-    const int g = res_ctas(op.N);
-    switch (res_lanes(op.N)) {
-    case 8: k_residual<TM, TX, TR, DPN, 8><<<g, kThreads, 0, s>>>(op, x, b, r, part, dinv, z); break;
-    case 2: k_residual<TM, TX, TR, DPN, 2><<<g, kThreads, 0, s>>>(op, x, b, r, part, dinv, z); break;
-    default: k_residual<TM, TX, TR, DPN, 1><<<g, kThreads, 0, s>>>(op, x, b, r, part, dinv, z); break;
-    }
+    k_residual<TM, TX, TR, DPN><<<res_ctas(op.N), res_rows(op.N) * DPN, 0, s>>>(op, x, b, r, part, dinv, z);
 }
 
 // Start of a cycle: beta = ||r||, inv = 1/beta, g = [beta, 0...], j = 0.

@@ -13,6 +13,7 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kGsThreads = 1024;  // threads per CTA of the Gram-Schmidt passes
 constexpr int kGsWarps = kGsThreads / 32;
 constexpr int kRowThreads = 4;    // threads per block row in the SpMV
+constexpr int kResidT = 768;      // most threads of a residual's CTA
 
 struct GmresCtl {
     double H[(kMaxM + 1) * kMaxM];  // column-major (m+1) x m, Givens-rotated in place
@@ -88,6 +89,42 @@ __device__ __forceinline__ void ell_row(const Op<TM> &op, int r, const TX *__res
             for (int q = 0; q < DPN; ++q) y[q] += (q == i) ? p : TA(0);
         }
     }
+}
+
+// Component i of (A x)_r, one thread, slots in order: the products accumulate in TA.  U slots at a time,
+// every load of them in flight before the first product.
+template <class TA, class TM, class TX, int DPN>
+__device__ __forceinline__ TA ell_row_comp(const Op<TM> &op, int r, int i, const TX *__restrict__ x) {
+    constexpr int U = DPN == 3 ? 4 : 2;
+    const size_t ld = (size_t)op.ld;
+    const int p0 = op.penPtr ? __ldg(op.penPtr + r) : 0, p1 = op.penPtr ? __ldg(op.penPtr + r + 1) : 0;
+    TA y = TA(0);
+    for (int s0 = 0; s0 < op.S; s0 += U) {
+        int c[U];
+        TM k[U][DPN];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int s = s0 + u < op.S ? s0 + u : s0;
+            c[u] = __ldg(op.col + (size_t)s * ld + r);
+            const TM *kp = op.K + ((size_t)s * DPN + i) * DPN * ld + r;
+#pragma unroll
+            for (int jj = 0; jj < DPN; ++jj) k[u][jj] = __ldg(kp + (size_t)jj * ld);
+        }
+        TX xv[U][DPN];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int jj = 0; jj < DPN; ++jj) xv[u][jj] = x[(size_t)c[u] * DPN + jj];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (s0 + u >= op.S) break;
+#pragma unroll
+            for (int jj = 0; jj < DPN; ++jj) y += (TA)k[u][jj] * (TA)xv[u][jj];
+        }
+    }
+    for (int t = p0; t < p1; ++t)
+        if (op.penRow[t] == i) y += (TA)(op.penVal[t] * (double)x[op.penCol[t]]);
+    return y;
 }
 
 // (A x)_r by RT adjacent lanes: the slots s = sub, sub + RT, ... each, the partials combined with

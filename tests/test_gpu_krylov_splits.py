@@ -1,4 +1,4 @@
-"""The splits of the block-ELL solver by model size: lanes a row in the products, vector rows a CTA in the
+"""The splits of the block-ELL solver by model size: rows a CTA in the products, vector rows a CTA in the
 Gram-Schmidt passes.  The residual's products (all sizes of its split, remainders included) against a sparse
 product on the host; solves at each split converge and their reported residual is that of the host product."""
 import numpy as np
@@ -19,7 +19,7 @@ def _system(m):
     return g, (o.csr_scipy(mat, cols) + C.T @ C).tocsr()
 
 
-# nodes: 60 and 1,331 (8 lanes), 9,702 | 10,143 (8 | 2 lanes), 38,874 | 39,204 (2 | 1 lanes)
+# nodes: 60 and 1,331, remainders of 32 rows; 38,874 | 39,204 (32 | 128 rows a CTA)
 @pytest.mark.parametrize("dims", [(4, 3, 2), (10, 10, 10), (20, 20, 21), (20, 20, 22), (30, 32, 37), (32, 32, 35)])
 def test_products_match_host(dims):
     g, A = _system(M.hex_block(*dims, jitter=0.1, seed=3))
