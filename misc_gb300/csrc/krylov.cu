@@ -30,6 +30,7 @@
 
 #include "astro_internal.h"
 #include "krylov_ops.cuh"
+#include "krylov_resident.cuh"
 
 using namespace astro_kry;
 
@@ -734,6 +735,13 @@ struct GmresWork {
     cudaAccessPolicyWindow apw = {};
     bool apwOn = false;
     const PolyHost *poly = nullptr;
+    // restart cycle as one resident launch (krylov_resident.cuh): on when the operator fits the SMs
+    struct {
+        bool on = false;
+        int R = 0, G = 0, H = 0, vShared = 0;
+        size_t smem = 0;
+    } res;
+    DevBuf polyW, penLoc;  // its hop weights and the penalty entries' places in the halos
     // vector that scales a residual into the preconditioner's input: D^-1 (Jacobi) or S (poly)
     template <class TV> const TV *y0s() { return poly ? dptr<TV>(dsqT) : dptr<TV>(dinvT); }
     // restart cycle captured as a graph, reused while the matrix and vectors stay the same
@@ -747,6 +755,12 @@ struct GmresWork {
     int nChunks = 0, nRowCtas = 0;
     std::vector<double> hp;
 };
+
+static int device_sms(const astro_ctx *ctx) {
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    return std::max(1, sms);
+}
 
 // Version of the matrix the FP32 solver copy comes from: the FP32 assembly when there is one,
 // else the FP64 matrix converted (the shell path has no FP32 element kernels).
@@ -914,6 +928,95 @@ static double sum_parts(astro_ctx *ctx, GmresWork &W, int which, int *rc) {
     return s;
 }
 
+// Rows and shared memory of the resident cycle, or off when a CTA's part does not fit.  A CTA per SM, but
+// no fewer than sqrt(N / 10) rows: every CTA adds the partial sums of all of them, which in FP64 costs
+// it a tenth of a row's products per CTA.  The halo of the rows is counted on the device (the penalty
+// entries, which it includes, may have changed since the last solve).
+template <class TM, class TV, int DPN, bool POLY>
+static int resident_plan(astro_ctx *ctx, GmresWork &W, const Op<TM> &op, int m) {
+    W.res.on = false;
+    const int N = op.N, sms = device_sms(ctx);
+    int coop = 0, maxSm = 0, per = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device);
+    cudaDeviceGetAttribute(&maxSm, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
+    const int R = std::max((N + sms - 1) / sms, (int)std::ceil(std::sqrt(N / 10.0))), G = (N + R - 1) / R;
+    if (!coop || (POLY && R > kResMaxRows)) return ASTRO_OK;
+    const void *f = (const void *)k_gmres_resident<TM, TV, DPN, POLY>;
+    cudaFuncAttributes fa;
+    CK(cudaFuncGetAttributes(&fa, f));
+    const size_t room = (size_t)maxSm - fa.sharedSizeBytes;
+    auto need = [&](int H, int vShared) { return res_layout<TM, TV, DPN>(N, op.S, R, H, m, POLY, vShared).total; };
+    if (need(R, 0) > room) return ASTRO_OK;
+    int H = 0, rc;
+    if (!W.penLoc.p && (rc = dev_alloc(ctx, W.penLoc, sizeof(int) * std::max(1, ctx->penRows)))) return rc;
+    if (W.penLoc.bytes < sizeof(int) * (size_t)ctx->penRows) {
+        dev_free(W.penLoc);
+        if ((rc = dev_alloc(ctx, W.penLoc, sizeof(int) * (size_t)ctx->penRows))) return rc;
+    }
+    int *d_H = reinterpret_cast<int *>(W.tgt.p);
+    CK(cudaMemsetAsync(d_H, 0, sizeof(int), ctx->stream));
+    k_res_halo<TM><<<G, kThreads, (size_t)(N + 31) / 32 * 4, ctx->stream>>>(op, R, d_H);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(&H, d_H, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (H > 65535) return ASTRO_OK;  // 16-bit places
+    int vs = 1;
+    if (need(H, vs) > room && need(H, vs = 0) > room) return ASTRO_OK;
+    W.res.smem = need(H, vs);
+    // (the whole room whatever this solve needs: the attribute is shared by all solves on the device)
+    CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, kResT, W.res.smem) != cudaSuccess || per < 1) {
+        cudaGetLastError();
+        return ASTRO_OK;
+    }
+    W.res.R = R;
+    W.res.G = G;
+    W.res.H = H;
+    W.res.vShared = vs;
+    W.res.on = true;
+    return ASTRO_OK;
+}
+
+// Enqueues one resident cycle.
+template <class TM, class TV, int DPN, bool POLY>
+static cudaError_t resident_cycle(GmresWork &W, const Op<TM> &op, TV *x, const double *b, int m, cudaStream_t s) {
+    GmresCtl *ctl = dptr<GmresCtl>(W.ctl);
+    ResArgs<TM, TV> A{};
+    A.op = op;
+    if constexpr (POLY) {
+        A.hop = W.hop;
+        A.deg = W.poly->deg;
+        A.theta = W.poly->theta;
+        A.delta = W.poly->delta;
+        A.W = dptr<float>(W.polyW);
+        A.amod = W.poly->amod;
+    }
+    A.y0s = W.y0s<TV>();
+    A.x = x;
+    A.b = b;
+    A.V = dptr<TV>(W.V);
+    A.ld = W.ld;
+    A.z[0] = dptr<TV>(W.z0);
+    A.z[1] = dptr<TV>(W.z1);
+    A.ctl = ctl;
+    A.target = dptr<double>(W.tgt);
+    A.part = dptr<double>(W.part);
+    A.bar = &ctl->bar;
+    A.penLoc = dptr<int>(W.penLoc);
+    A.m = m;
+    A.n = W.n;
+    A.N = op.N;
+    A.R = W.res.R;
+    A.G = W.res.G;
+    A.H = W.res.H;
+    A.vShared = W.res.vShared;
+    const void *f = (const void *)k_gmres_resident<TM, TV, DPN, POLY>;
+    cudaError_t e = cudaMemsetAsync(&ctl->stuck, 0, 2 * sizeof(int), s);  // stuck and bar
+    void *args[] = {&A};
+    if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(f, dim3(W.res.G), dim3(kResT), args, W.res.smem, s);
+    return e;
+}
+
 // Restarted Jacobi-GMRES(m) on A x = b in precision TV with matrix values TM.  x (TV) in/out
 // on the device, b (double) on the device.
 template <class TM, class TV, int DPN>
@@ -925,10 +1028,12 @@ static int gmres_solve(astro_ctx *ctx, GmresWork &W, const TM *K, TV *x, const d
     double *part = dptr<double>(W.part);
     // the absolute target is read by the graph from device memory
     CK(cudaMemcpyAsync(W.tgt.p, &tgtAbs, sizeof(double), cudaMemcpyHostToDevice, s));
+    if (W.res.on && W.poly)
+        CK(cudaMemcpyAsync(W.polyW.p, W.poly->W, sizeof(W.poly->W), cudaMemcpyHostToDevice, s));
     const bool samePoly = W.poly ? (W.gPoly.deg == W.poly->deg && std::memcmp(&W.gPoly, W.poly, sizeof(PolyHost)) == 0)
                                  : W.gPoly.deg == 0;
     // (the penalty lists are uploaded anew with every constraint scaling: their place is part of the key)
-    if (!(W.exec && W.gK == K && W.gx == x && W.gb == b && W.gPen == op.penVal && samePoly)) {
+    if (!W.res.on && !(W.exec && W.gK == K && W.gx == x && W.gb == b && W.gPen == op.penVal && samePoly)) {
         if (W.exec) cudaGraphExecDestroy(W.exec);
         if (W.graph) cudaGraphDestroy(W.graph);
         W.exec = nullptr;
@@ -1030,12 +1135,15 @@ static int gmres_solve(astro_ctx *ctx, GmresWork &W, const TM *K, TV *x, const d
     int status = ASTRO_OK;
     struct {
         double resest;
-        int j, done, breakdown, nonfinite;
+        int j, done, breakdown, nonfinite, stuck;
     } hc;
     for (int cyc = 0; cyc < maxCycles; ++cyc) {
-        CK(cudaGraphLaunch(exec, s));
+        if (!W.res.on) CK(cudaGraphLaunch(exec, s));
+        else if (!W.poly) CK((resident_cycle<TM, TV, DPN, false>(W, op, x, b, m, s)));
+        else if constexpr (sizeof(TV) == 4) CK((resident_cycle<TM, TV, DPN, true>(W, op, x, b, m, s)));
         CK(cudaMemcpyAsync(&hc, &ctl->resest, sizeof(hc), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
+        if (hc.stuck) return set_err(ctx, ASTRO_ERR_CUDA, "a wait of the solver's cycle was given up");
         *iters += hc.j;
         *cycles += 1;
         *finalRes = hc.resest;
@@ -1057,7 +1165,8 @@ static int work_alloc(astro_ctx *ctx, GmresWork &W, int m, int tv) {
     W.rows = gs_rows(n);
     W.nChunks = (n + W.rows - 1) / W.rows;
     W.nRowCtas = res_ctas(ctx->P.N);
-    const size_t nparts = std::max((size_t)3 * W.nChunks * (kMaxM + 1), (size_t)2 * W.nRowCtas);
+    const size_t nparts = std::max({(size_t)3 * W.nChunks * (kMaxM + 1), (size_t)2 * W.nRowCtas,
+                                    (size_t)3 * (kMaxM + 2) * std::min(ctx->P.N, device_sms(ctx))});
     int rc;
     if ((rc = dev_alloc(ctx, W.V, W.ld * (m + 1) * tv))) return rc;
     if ((rc = dev_alloc(ctx, W.w0, (size_t)n * tv))) return rc;
@@ -1086,7 +1195,7 @@ static void work_free(GmresWork &W) {
     DevBuf *b[] = {&W.V,    &W.w0,   &W.w1,    &W.z0, &W.z1,  &W.part, &W.ctl, &W.dinv,
                    &W.dinvT, &W.rres, &W.xs,  &W.tgt, &W.yB0, &W.yB1,  &W.zacc, &W.pw,
                    &W.Kh,    &W.Kr,   &W.penS, &W.dsqT, &W.x64, &W.b64, &W.nfF, &W.nfL,
-                   &W.nfPd,  &W.nfPart, &W.mlpPrm, &W.amod};
+                   &W.nfPd,  &W.nfPart, &W.mlpPrm, &W.amod, &W.polyW, &W.penLoc};
     for (auto *x : b) dev_free(*x);
 }
 
@@ -1275,6 +1384,7 @@ static int solve_static_dev(astro_ctx *ctx, const double *d_b, double *d_x, cons
         const double *bb = dptr<double>(W.b64);
         CK(cudaMemcpyAsync(W.x64.p, d_x, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
         CK(cudaMemcpyAsync(W.b64.p, d_b, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
+        if ((rc = resident_plan<double, double, DPN, false>(ctx, W, make_op<double>(ctx, K64p), m))) return rc;
         rc = true_residual<DPN>(ctx, W, 64, nullptr, bb, &rel, r, &rn, &bn);
         const double tgt = o->rtol * bn;
         while (rc == ASTRO_OK) {
@@ -1367,9 +1477,15 @@ static int solve_static_dev(astro_ctx *ctx, const double *d_b, double *d_x, cons
                 ph.amod = dptr<float>(W.amod);
             }
             W.poly = &ph;
-            persistSet = persist_begin(ctx, W, &persistPrev);
+            if ((!W.polyW.p && (rc = dev_alloc(ctx, W.polyW, sizeof(ph.W)))) ||
+                (rc = resident_plan<float, float, DPN, true>(ctx, W, make_op<float>(ctx, K32p), m)))
+                return rc;
+            // (the resident cycle keeps the operator in shared memory)
+            if (!W.res.on) persistSet = persist_begin(ctx, W, &persistPrev);
+            else W.apwOn = false;
             if (W.apwOn) ph.apwKey = (double)W.apw.hitRatio * 1e12 + (double)W.apw.num_bytes;
         }
+        else if ((rc = resident_plan<float, float, DPN, false>(ctx, W, make_op<float>(ctx, K32p), m))) return rc;
         float *d32 = dptr<float>(W.xs);
         const double inner = o->inner_rtol > 0 ? o->inner_rtol : 1e-4;
         // the outer residual is formed with the FP64 matrix when it is resident (the system the

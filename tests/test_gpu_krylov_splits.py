@@ -53,3 +53,44 @@ def test_solves_converge_at_each_split(dims, method):
     r = np.linalg.norm(b - A @ u) / np.linalg.norm(b)
     noise = 81 * 1.1e-16 * np.linalg.norm(abs(A) @ abs(u)) / np.linalg.norm(b)
     assert abs(r - st.rel_residual) <= 2.0 * noise + 1e-3 * st.rel_residual, (r, st.rel_residual, noise)
+
+
+# the resident cycle: fewer rows than SMs, a last CTA with fewer rows, several row groups
+@pytest.mark.parametrize("dims", [(2, 1, 1), (7, 6, 5), (10, 10, 10), (16, 15, 14)])
+@pytest.mark.parametrize("restart", [7, 64])
+@pytest.mark.parametrize("method", [SOLVER_GMRES_JACOBI_FP64, SOLVER_FGMRES_MIXED, SOLVER_FGMRES_LEARNED])
+def test_resident_cycle_solves(dims, restart, method):
+    m = M.hex_block(*dims, lx=0.1 * dims[0], ly=0.1 * dims[1], lz=0.1 * dims[2], jitter=0.1, seed=4)
+    g, A = _system(m)
+    b = g.static_rhs()
+    u, st = g.solve_static(b, method=method, rtol=1e-8, restart=restart)
+    assert st.status == 0 and st.rel_residual <= 1e-8
+    r = np.linalg.norm(b - A @ u) / np.linalg.norm(b)
+    noise = 81 * 1.1e-16 * np.linalg.norm(abs(A) @ abs(u)) / np.linalg.norm(b)
+    assert abs(r - st.rel_residual) <= 2.0 * noise + 1e-3 * st.rel_residual, (r, st.rel_residual, noise)
+
+
+# one FP64 cycle of k steps against the least residual over the host's Krylov space (6 DOF and 3; the
+# thin plate's space of 64 steps moves by 1e-6 under roundings of its products alone)
+@pytest.mark.parametrize("shells, k", [(True, 1), (True, 2), (True, 33), (False, 1), (False, 2), (False, 33), (False, 64)])
+def test_resident_cycle_takes_the_least_residual(shells, k):
+    if shells:
+        m = M.plate_shell(nx=9, ny=7, lx=0.9, ly=0.7, t=0.05, E=7.0e10, nu=0.33, rho=2700.0, pressure=1.0e3)
+    else:
+        m = M.hex_block(7, 6, 5, jitter=0.1, seed=4)
+    g, A = _system(m)
+    b = g.static_rhs()
+    _, st = g.solve_static(b, method=SOLVER_GMRES_JACOBI_FP64, rtol=1e-14, restart=k, max_iters=k, allow_maxit=True)
+    AD = A.multiply(1.0 / A.diagonal()[None, :]).tocsr()
+    Q = np.zeros((len(b), k + 1))
+    Q[:, 0] = b / np.linalg.norm(b)
+    for j in range(k):
+        w = AD @ Q[:, j]
+        for _ in range(2):
+            w -= Q[:, : j + 1] @ (Q[:, : j + 1].T @ w)
+        Q[:, j + 1] = w / np.linalg.norm(w)
+    B = AD @ Q[:, :k]
+    y = np.linalg.lstsq(B, b, rcond=None)[0]
+    least = np.linalg.norm(b - B @ y) / np.linalg.norm(b)
+    # rounding moves the space by eps x the condition of its images (6e4 for the plate's 33), and more per step
+    assert abs(st.rel_residual - least) <= 1e-6 * max(least, 1e-2), (st.rel_residual, least)
