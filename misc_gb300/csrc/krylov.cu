@@ -738,10 +738,10 @@ struct GmresWork {
     // restart cycle as one resident launch (krylov_resident.cuh): on when the operator fits the SMs
     struct {
         bool on = false;
-        int R = 0, G = 0, H = 0, vShared = 0;
+        int R = 0, G = 0, H = 0, P = 0, vShared = 0;
         size_t smem = 0;
     } res;
-    DevBuf polyW, penLoc;  // its hop weights and the penalty entries' places in the halos
+    DevBuf polyW, resWords;  // its hop weights and exchanged words
     // vector that scales a residual into the preconditioner's input: D^-1 (Jacobi) or S (poly)
     template <class TV> const TV *y0s() { return poly ? dptr<TV>(dsqT) : dptr<TV>(dinvT); }
     // restart cycle captured as a graph, reused while the matrix and vectors stay the same
@@ -933,36 +933,35 @@ static double sum_parts(astro_ctx *ctx, GmresWork &W, int which, int *rc) {
 // it a tenth of a row's products per CTA.  The halo of the rows is counted on the device (the penalty
 // entries, which it includes, may have changed since the last solve).
 template <class TM, class TV, int DPN, bool POLY>
-static int resident_plan(astro_ctx *ctx, GmresWork &W, const Op<TM> &op, int m) {
+static int resident_plan(astro_ctx *ctx, GmresWork &W, const Op<TM> &op, int m, int deg) {
     W.res.on = false;
     const int N = op.N, sms = device_sms(ctx);
     int coop = 0, maxSm = 0, per = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device);
     cudaDeviceGetAttribute(&maxSm, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
-    const int R = std::max((N + sms - 1) / sms, (int)std::ceil(std::sqrt(N / 10.0))), G = (N + R - 1) / R;
+    const int R = std::max((N + std::min(sms, kResMaxCtas) - 1) / std::min(sms, kResMaxCtas), (int)std::ceil(std::sqrt(N / 10.0))), G = (N + R - 1) / R;
     if (!coop || (POLY && R > kResMaxRows)) return ASTRO_OK;
     const void *f = (const void *)k_gmres_resident<TM, TV, DPN, POLY>;
     cudaFuncAttributes fa;
     CK(cudaFuncGetAttributes(&fa, f));
     const size_t room = (size_t)maxSm - fa.sharedSizeBytes;
-    auto need = [&](int H, int vShared) { return res_layout<TM, TV, DPN>(N, op.S, R, H, m, POLY, vShared).total; };
-    if (need(R, 0) > room) return ASTRO_OK;
-    int H = 0, rc;
-    if (!W.penLoc.p && (rc = dev_alloc(ctx, W.penLoc, sizeof(int) * std::max(1, ctx->penRows)))) return rc;
-    if (W.penLoc.bytes < sizeof(int) * (size_t)ctx->penRows) {
-        dev_free(W.penLoc);
-        if ((rc = dev_alloc(ctx, W.penLoc, sizeof(int) * (size_t)ctx->penRows))) return rc;
-    }
-    int *d_H = reinterpret_cast<int *>(W.tgt.p);
-    CK(cudaMemsetAsync(d_H, 0, sizeof(int), ctx->stream));
-    k_res_halo<TM><<<G, kThreads, (size_t)(N + 31) / 32 * 4, ctx->stream>>>(op, R, d_H);
+    auto need = [&](int H, int P, int vShared) { return res_layout<TM, TV, DPN>(N, op.S, R, H, P, m, deg, vShared).total; };
+    if (need(R, 0, 0) > room) return ASTRO_OK;
+    int HP[2] = {0, 0}, rc;
+    if (!W.resWords.p && (rc = dev_alloc(ctx, W.resWords, sizeof(ulonglong2) * res_words<TV, DPN>(N, G)))) return rc;
+    int *d_HP = reinterpret_cast<int *>(W.tgt.p);
+    static_assert(sizeof(HP) <= sizeof(double), "counted in the target's place");
+    CK(cudaMemsetAsync(d_HP, 0, sizeof(HP), ctx->stream));
+    CK(cudaFuncSetAttribute(k_res_halo<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
+    k_res_halo<TM><<<G, kThreads, (size_t)(N + 3) / 4 * 4, ctx->stream>>>(op, R, d_HP);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(&H, d_H, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaMemcpyAsync(HP, d_HP, sizeof(HP), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    const int H = HP[0], P = HP[1];
     if (H > 65535) return ASTRO_OK;  // 16-bit places
     int vs = 1;
-    if (need(H, vs) > room && need(H, vs = 0) > room) return ASTRO_OK;
-    W.res.smem = need(H, vs);
+    if (need(H, P, vs) > room && need(H, P, vs = 0) > room) return ASTRO_OK;
+    W.res.smem = need(H, P, vs);
     // (the whole room whatever this solve needs: the attribute is shared by all solves on the device)
     CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, kResT, W.res.smem) != cudaSuccess || per < 1) {
@@ -972,6 +971,7 @@ static int resident_plan(astro_ctx *ctx, GmresWork &W, const Op<TM> &op, int m) 
     W.res.R = R;
     W.res.G = G;
     W.res.H = H;
+    W.res.P = P;
     W.res.vShared = vs;
     W.res.on = true;
     return ASTRO_OK;
@@ -996,22 +996,18 @@ static cudaError_t resident_cycle(GmresWork &W, const Op<TM> &op, TV *x, const d
     A.b = b;
     A.V = dptr<TV>(W.V);
     A.ld = W.ld;
-    A.z[0] = dptr<TV>(W.z0);
-    A.z[1] = dptr<TV>(W.z1);
+    A.words = dptr<ulonglong2>(W.resWords);
     A.ctl = ctl;
     A.target = dptr<double>(W.tgt);
-    A.part = dptr<double>(W.part);
-    A.bar = &ctl->bar;
-    A.penLoc = dptr<int>(W.penLoc);
     A.m = m;
-    A.n = W.n;
     A.N = op.N;
     A.R = W.res.R;
     A.G = W.res.G;
     A.H = W.res.H;
+    A.P = W.res.P;
     A.vShared = W.res.vShared;
     const void *f = (const void *)k_gmres_resident<TM, TV, DPN, POLY>;
-    cudaError_t e = cudaMemsetAsync(&ctl->stuck, 0, 2 * sizeof(int), s);  // stuck and bar
+    cudaError_t e = cudaMemsetAsync(W.resWords.p, 0, W.resWords.bytes, s);
     void *args[] = {&A};
     if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(f, dim3(W.res.G), dim3(kResT), args, W.res.smem, s);
     return e;
@@ -1143,7 +1139,10 @@ static int gmres_solve(astro_ctx *ctx, GmresWork &W, const TM *K, TV *x, const d
         else if constexpr (sizeof(TV) == 4) CK((resident_cycle<TM, TV, DPN, true>(W, op, x, b, m, s)));
         CK(cudaMemcpyAsync(&hc, &ctl->resest, sizeof(hc), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
-        if (hc.stuck) return set_err(ctx, ASTRO_ERR_CUDA, "a wait of the solver's cycle was given up");
+        if (hc.stuck) {
+            CK(cudaMemsetAsync(&ctl->stuck, 0, sizeof(int), s));
+            return set_err(ctx, ASTRO_ERR_CUDA, "a wait of the solver's cycle was given up");
+        }
         *iters += hc.j;
         *cycles += 1;
         *finalRes = hc.resest;
@@ -1165,8 +1164,7 @@ static int work_alloc(astro_ctx *ctx, GmresWork &W, int m, int tv) {
     W.rows = gs_rows(n);
     W.nChunks = (n + W.rows - 1) / W.rows;
     W.nRowCtas = res_ctas(ctx->P.N);
-    const size_t nparts = std::max({(size_t)3 * W.nChunks * (kMaxM + 1), (size_t)2 * W.nRowCtas,
-                                    (size_t)3 * (kMaxM + 2) * std::min(ctx->P.N, device_sms(ctx))});
+    const size_t nparts = std::max((size_t)3 * W.nChunks * (kMaxM + 1), (size_t)2 * W.nRowCtas);
     int rc;
     if ((rc = dev_alloc(ctx, W.V, W.ld * (m + 1) * tv))) return rc;
     if ((rc = dev_alloc(ctx, W.w0, (size_t)n * tv))) return rc;
@@ -1195,7 +1193,7 @@ static void work_free(GmresWork &W) {
     DevBuf *b[] = {&W.V,    &W.w0,   &W.w1,    &W.z0, &W.z1,  &W.part, &W.ctl, &W.dinv,
                    &W.dinvT, &W.rres, &W.xs,  &W.tgt, &W.yB0, &W.yB1,  &W.zacc, &W.pw,
                    &W.Kh,    &W.Kr,   &W.penS, &W.dsqT, &W.x64, &W.b64, &W.nfF, &W.nfL,
-                   &W.nfPd,  &W.nfPart, &W.mlpPrm, &W.amod, &W.polyW, &W.penLoc};
+                   &W.nfPd,  &W.nfPart, &W.mlpPrm, &W.amod, &W.polyW, &W.resWords};
     for (auto *x : b) dev_free(*x);
 }
 
@@ -1384,7 +1382,7 @@ static int solve_static_dev(astro_ctx *ctx, const double *d_b, double *d_x, cons
         const double *bb = dptr<double>(W.b64);
         CK(cudaMemcpyAsync(W.x64.p, d_x, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
         CK(cudaMemcpyAsync(W.b64.p, d_b, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
-        if ((rc = resident_plan<double, double, DPN, false>(ctx, W, make_op<double>(ctx, K64p), m))) return rc;
+        if ((rc = resident_plan<double, double, DPN, false>(ctx, W, make_op<double>(ctx, K64p), m, 0))) return rc;
         rc = true_residual<DPN>(ctx, W, 64, nullptr, bb, &rel, r, &rn, &bn);
         const double tgt = o->rtol * bn;
         while (rc == ASTRO_OK) {
@@ -1478,14 +1476,14 @@ static int solve_static_dev(astro_ctx *ctx, const double *d_b, double *d_x, cons
             }
             W.poly = &ph;
             if ((!W.polyW.p && (rc = dev_alloc(ctx, W.polyW, sizeof(ph.W)))) ||
-                (rc = resident_plan<float, float, DPN, true>(ctx, W, make_op<float>(ctx, K32p), m)))
+                (rc = resident_plan<float, float, DPN, true>(ctx, W, make_op<float>(ctx, K32p), m, ph.deg)))
                 return rc;
             // (the resident cycle keeps the operator in shared memory)
             if (!W.res.on) persistSet = persist_begin(ctx, W, &persistPrev);
             else W.apwOn = false;
             if (W.apwOn) ph.apwKey = (double)W.apw.hitRatio * 1e12 + (double)W.apw.num_bytes;
         }
-        else if ((rc = resident_plan<float, float, DPN, false>(ctx, W, make_op<float>(ctx, K32p), m))) return rc;
+        else if ((rc = resident_plan<float, float, DPN, false>(ctx, W, make_op<float>(ctx, K32p), m, 0))) return rc;
         float *d32 = dptr<float>(W.xs);
         const double inner = o->inner_rtol > 0 ? o->inner_rtol : 1e-4;
         // the outer residual is formed with the FP64 matrix when it is resident (the system the

@@ -29,7 +29,6 @@ struct GmresCtl {
     int breakdown;
     int nonfinite;
     int stuck;       // a wait of the resident cycle was given up
-    unsigned bar;    // its grid barrier
     unsigned arrive[3];  // CTAs finished in the current dots / update / update-and-norm launch
     int reorth;          // this step's first pass lost more than half of ||w||^2: run the second
     int reorths;         // second passes run in this cycle
