@@ -3,7 +3,7 @@
 // c_getElRu (Working/AStrO_c_elementEqns.f90, the complex twin of r_getElRu's solid branch).
 //
 // Every element that depends on the design variable d (through elToD, or through ndToD for node
-// coordinates) is evaluated in complex FP64 with d + i h, one thread per element:
+// coordinates) is evaluated in complex FP64 with d + i h, eight lanes per element, one a Gauss point:
 //   * node coordinates r_getNodeCoord (designProp :945-968): the real offsets of all nodeCoord
 //     variables are already in the context's node list; d's own nodes get + i h coef;
 //   * orientation r_getOrientation (:187-221): the section orientation rotated (r_rotateAlpha) by
@@ -13,8 +13,11 @@
 //     (r_getMaterialDensity, :82-103);
 //   * the residual of r_getElRuk's solid branch (Green-Lagrange strain over all shape functions,
 //     bubbles included for brickIM) and, for a Newmark state, r_getElRum's solid inertia.
-// d_acc -= Im(Ru) at the nodal DOF (internal layout) and d_intAcc -= Im(Ru) at the brickIM
-// internal DOF, colour by colour (a colour's elements share no node: no atomics).  The complex
+// The elements of all colours are evaluated at once, then Im(Ru) is subtracted from d_acc at the nodal
+// DOF (internal layout) and from d_intAcc at the brickIM internal DOF, colour by colour (a colour's
+// elements share no node: no atomics).  The FP64 pipe bounds the evaluation, once enough warps are there
+// to fill it: 7,680 elements in eight colours, a thread an element, put 64 threads on 15 SMs at a time
+// (8 x 1,100 us; now 1,200 us in all, and 8 x 3 us).  The complex
 // path's Gauss points are the single-precision 1/sqrt(3) of the reference's c_ constants.
 #include "astro_internal.h"
 #include "shell_math.cuh"
@@ -22,8 +25,9 @@
 namespace {
 
 struct SolidCsArgs {
-    const int *els;  // listed elements (0-based) of this colour
+    const int *els;  // listed elements (0-based)
     int count;
+    double *ru;      // their Im(Ru): 33 values each, shape function by shape function
     const int *etype, *elist, *rank, *esec;
     const double *nodes;      // (N,3), real design values applied
     const double *secOrig;    // (S,9) column-major section orientation as given
@@ -45,7 +49,8 @@ struct SolidCsArgs {
     double *acc, *intAcc;
 };
 
-template <class T> __device__ void material_c_cs(const T ep[9], T C[6][6]) {
+// Column col of C = S^-1 (col >= 6: none).
+template <class T> __device__ void material_c_cs(const T ep[9], int col, T x[6]) {
     T S[6][6];
     for (int i = 0; i < 6; ++i)
         for (int j = 0; j < 6; ++j) S[i][j] = T(0.0);
@@ -62,22 +67,22 @@ template <class T> __device__ void material_c_cs(const T ep[9], T C[6][6]) {
         for (int j = 0; j < i; ++j) S[i][j] = S[j][i];
     // C = S^-1 by the reference's unpivoted LU (r_GetInvLU), column by column
     a_lu<T, 6>(&S[0][0], 6);
-    for (int col = 0; col < 6; ++col) {
-        T b[6], x[6];
-        for (int i = 0; i < 6; ++i) b[i] = (i == col) ? T(1.0) : T(0.0);
-        // a_lu_solve handles n <= 9
-        a_lu_solve<T, 6>(&S[0][0], b, x, 6);
-        for (int i = 0; i < 6; ++i) C[i][col] = x[i];
-    }
+    T b[6];
+    for (int i = 0; i < 6; ++i) b[i] = (i == col) ? T(1.0) : T(0.0);
+    // a_lu_solve handles n <= 9
+    a_lu_solve<T, 6>(&S[0][0], b, x, 6);
 }
 
-__global__ void k_solid_cstep(SolidCsArgs A) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= A.count) return;
+constexpr int kCsItems = 16;  // elements of a CTA, eight lanes each
+
+__global__ void __launch_bounds__(8 * kCsItems) k_solid_cstep(SolidCsArgs A) {
+    __shared__ cplx sC[kCsItems][6][6];
+    __shared__ double sRu[kCsItems][8][33];
+    const int loc = threadIdx.x / 8, gp = threadIdx.x % 8;
+    const int it = blockIdx.x * kCsItems + loc;
+    const int q = min(it, A.count - 1);  // (the lanes past the end work on the last element, for the barriers)
     const int e = A.els[q];
     const int dvar = A.dvars ? A.dvars[q] : A.dvar;
-    double *acc = A.dvars ? A.acc + (size_t)(dvar - A.dvarBase) * A.accStride : A.acc;
-    double *intAcc = A.intAcc && A.dvars ? A.intAcc + (size_t)(dvar - A.dvarBase) * A.intAccStride : A.intAcc;
     const int et = A.etype[e];
     const int nsf = (et == 81) ? 11 : 8;  // shape functions: nodes (+ bubbles)
     const cplx ih(0.0, A.h);
@@ -111,8 +116,15 @@ __global__ void k_solid_cstep(SolidCsArgs A) {
         for (int i = 0; i < 3; ++i) gr[i] = al[0][i] * locRot[0] + al[1][i] * locRot[1] + al[2][i] * locRot[2];
         a_rotate<cplx>(orient, al, gr, 0, 0);
     }
-    cplx C[6][6];
-    material_c_cs<cplx>(ep, C);
+    // (the factors in every lane, a column of the inverse each)
+    {
+        cplx x[6];
+        material_c_cs<cplx>(ep, gp, x);
+        if (gp < 6)
+            for (int i = 0; i < 6; ++i) sC[loc][i][gp] = x[i];
+    }
+    __syncwarp();
+    const cplx(*C)[6] = sC[loc];
     // node coordinates (+ i h on d's nodeCoord nodes), local frame; displacement and acceleration
     cplx X[8][3];
     double U[11][3], Ac[11][3];
@@ -148,10 +160,7 @@ __global__ void k_solid_cstep(SolidCsArgs A) {
                                ? c1 * (c2 * (U[8 + j][v] - (A.st.pidisp ? A.st.pidisp[ioff + 3 * v + j] : 0.0)))
                                : 0.0;
         }
-    cplx ru[11][3];
-    for (int a = 0; a < 11; ++a)
-        for (int v = 0; v < 3; ++v) ru[a][v] = cplx(0.0);
-    for (int gp = 0; gp < 8; ++gp) {
+    {
         const double s1 = (gp & 1) ? A.gpc : -A.gpc, s2 = (gp & 2) ? A.gpc : -A.gpc, s3 = (gp & 4) ? A.gpc : -A.gpc;
         double N[11], Ns[11][3];
         for (int a = 0; a < 8; ++a) {
@@ -229,18 +238,36 @@ __global__ void k_solid_cstep(SolidCsArgs A) {
                 const cplx P0 = g0 * Gm[0][v], P1 = g1 * Gm[1][v], P2 = g2 * Gm[2][v];
                 const cplx P3 = g1 * Gm[0][v] + g0 * Gm[1][v], P4 = g2 * Gm[0][v] + g0 * Gm[2][v],
                            P5 = g2 * Gm[1][v] + g1 * Gm[2][v];
-                ru[a][v] += P0 * sw[0] + P1 * sw[1] + P2 * sw[2] + P3 * sw[3] + P4 * sw[4] + P5 * sw[5];
-                if (dyn && a < 8) ru[a][v] += (rho * det) * (ag[v] * N[a]);
+                cplx r = P0 * sw[0] + P1 * sw[1] + P2 * sw[2] + P3 * sw[3] + P4 * sw[4] + P5 * sw[5];
+                if (dyn && a < 8) r += (rho * det) * (ag[v] * N[a]);
+                sRu[loc][gp][3 * a + v] = r.im;
             }
         }
     }
-    for (int a = 0; a < 8; ++a) {
+    __syncwarp();
+    // summed over the points in order
+    if (it < A.count)
+        for (int k = gp; k < 3 * nsf; k += 8) {
+            double r = 0.0;
+            for (int g = 0; g < 8; ++g) r += sRu[loc][g][k];
+            A.ru[33 * (size_t)it + k] = r;
+        }
+}
+
+// Subtracts the Im(Ru) of one colour's elements, a thread per element and shape function.
+__global__ void k_solid_cs_add(SolidCsArgs A) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, q = t / 11, a = t % 11;
+    if (q >= A.count) return;
+    const int e = A.els[q], et = A.etype[e];
+    const double *ru = A.ru + 33 * (size_t)q + 3 * a;
+    if (a < 8) {
+        double *acc = A.dvars ? A.acc + (size_t)(A.dvars[q] - A.dvarBase) * A.accStride : A.acc;
         const int r = A.rank[A.elist[8 * (size_t)e + a] - 1] - 1;
-        for (int v = 0; v < 3; ++v) acc[3 * (size_t)r + v] -= ru[a][v].im;
+        for (int v = 0; v < 3; ++v) acc[3 * (size_t)r + v] -= ru[v];
+    } else if (et == 81 && A.intAcc) {
+        double *intAcc = A.dvars ? A.intAcc + (size_t)(A.dvars[q] - A.dvarBase) * A.intAccStride : A.intAcc;
+        for (int v = 0; v < 3; ++v) intAcc[A.intVecOff[e] + 3 * v + a - 8] -= ru[v];
     }
-    if (et == 81 && intAcc)
-        for (int j = 0; j < 3; ++j)
-            for (int v = 0; v < 3; ++v) intAcc[ioff + 3 * v + j] -= ru[8 + j][v].im;
 }
 
 }  // namespace
@@ -304,6 +331,35 @@ static SolidCsArgs solid_cs_args(astro_ctx *ctx, int dvar, double h, const ElemD
     return A;
 }
 
+// The listed elements (colour by colour: colour c's from start[c]), at most kCsChunk at once.
+static int solid_cs_run(astro_ctx *ctx, const SolidCsArgs &B, const std::vector<int> &start) {
+    constexpr int kCsChunk = 1 << 17;  // 35 MB of residuals
+    const int total = start.back();
+    DevBuf ru;
+    int rc;
+    if ((rc = dev_alloc(ctx, ru, sizeof(double) * 33 * (size_t)std::min(total, kCsChunk)))) return rc;
+    for (int k0 = 0; k0 < total; k0 += kCsChunk) {
+        const int k1 = std::min(total, k0 + kCsChunk);
+        auto part = [&](int lo, int hi) {
+            SolidCsArgs A = B;
+            A.els = B.els + lo;
+            A.dvars = B.dvars ? B.dvars + lo : nullptr;
+            A.count = hi - lo;
+            A.ru = dptr<double>(ru) + 33 * (size_t)(lo - k0);
+            return A;
+        };
+        k_solid_cstep<<<(k1 - k0 + kCsItems - 1) / kCsItems, 8 * kCsItems, 0, ctx->stream>>>(part(k0, k1));
+        for (size_t col = 0; col + 1 < start.size(); ++col) {
+            const int lo = std::max(start[col], k0), hi = std::min(start[col + 1], k1);
+            if (lo < hi) k_solid_cs_add<<<(11 * (hi - lo) + 127) / 128, 128, 0, ctx->stream>>>(part(lo, hi));
+        }
+    }
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    dev_free(ru);
+    return cuda_check(ctx, e, "solid complex-step kernel");
+}
+
 int solid_drdd(astro_ctx *ctx, int dvar, double h, const ElemDevState &s, double *d_acc, double *d_intAcc) {
     std::vector<int> list, ptr;
     solid_dvar_elements(ctx, dvar, list, ptr);
@@ -312,23 +368,15 @@ int solid_drdd(astro_ctx *ctx, int dvar, double h, const ElemDevState &s, double
     int rc;
     if ((rc = upload(ctx, dl, list.data(), sizeof(int) * list.size()))) return rc;
     SolidCsArgs A = solid_cs_args(ctx, dvar, h, s, d_acc, d_intAcc);
-    for (size_t col = 0; col + 1 < ptr.size(); ++col) {
-        const int cnt = ptr[col + 1] - ptr[col];
-        if (!cnt) continue;
-        A.els = dptr<int>(dl) + ptr[col];
-        A.count = cnt;
-        k_solid_cstep<<<(cnt + 63) / 64, 64, 0, ctx->stream>>>(A);
-    }
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    A.els = dptr<int>(dl);
+    rc = solid_cs_run(ctx, A, ptr);
     dev_free(dl);
-    return cuda_check(ctx, e, "solid complex-step kernel");
+    return rc;
 }
 
-// Design variables d0 .. d0+nd-1 at once: one launch per colour over the (element, variable) pairs
-// of that colour, variable d accumulating at d_acc + (d-d0) n (and d_intAcc + (d-d0) ni).  Each
+// Design variables d0 .. d0+nd-1 at once over the (element, variable) pairs, variable d accumulating at d_acc + (d-d0) n (and d_intAcc + (d-d0) ni).  Each
 // variable's accumulator receives its elements' terms in the same colour order as solid_drdd,
-// so the results are the same; the launches are nd times wider.
+// so the results are the same.
 int solid_drdd_batch(astro_ctx *ctx, int d0, int nd, double h, const ElemDevState &s, double *d_acc,
                      double *d_intAcc) {
     const int ncol = ctx->P.ncolors;
@@ -358,19 +406,12 @@ int solid_drdd_batch(astro_ctx *ctx, int d0, int nd, double h, const ElemDevStat
     A.dvarBase = d0;
     A.accStride = ctx->P.n;
     A.intAccStride = ctx->P.intVecSize;
-    for (int col = 0; col < ncol; ++col) {
-        const int cnt = start[col + 1] - start[col];
-        if (!cnt) continue;
-        A.els = dptr<int>(dl) + start[col];
-        A.dvars = dptr<int>(dd) + start[col];
-        A.count = cnt;
-        k_solid_cstep<<<(cnt + 63) / 64, 64, 0, ctx->stream>>>(A);
-    }
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    A.els = dptr<int>(dl);
+    A.dvars = dptr<int>(dd);
+    rc = solid_cs_run(ctx, A, start);
     dev_free(dl);
     dev_free(dd);
-    return cuda_check(ctx, e, "solid complex-step kernel (batched)");
+    return rc;
 }
 
 namespace {
