@@ -249,6 +249,12 @@ int surface_load_dev(astro_ctx *ctx, int nf, const int *d_faceEl, const int *d_f
 // into d_ke (E x 24 x 24) instead; d_ru receives the element residuals (E x 24).
 int solid_soln_load(astro_ctx *ctx, int build, const ElemDevState &s, double *d_loadInt, double *d_intLoad,
                     double *d_ke, double *d_ru);                                                   // elem_hex8.cu
+// Small solid meshes: all colours' elements at once, blocks and residuals by way of scratch.
+constexpr int kHexAtOnce = 4096;  // elements (19 MB of blocks)
+bool hex_at_once(int elements, size_t colours);
+int hex_at_once_alloc(astro_ctx *ctx, int elements, bool blk, bool ru, DevBuf &dBlk, DevBuf &dRu);
+void hex_at_once_add(astro_ctx *ctx, const int *d_list, const std::vector<int> &ptr, DevBuf &dBlk, DevBuf &dRu, double *K,
+                     double *d_loadInt);
 int hex81_run(astro_ctx *ctx, const int *d_list, const std::vector<int> &ptr, int build, double *K,
               const ElemDevState &st, const double *CItem, double gpc, double *d_loadInt, double *d_intLoad,
               double *d_intMat, double *d_ke, double *d_ru);                                       // elem_hex81.cu

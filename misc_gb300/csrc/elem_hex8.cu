@@ -316,6 +316,7 @@ struct Hex8DfArgs {
     const float2 *Cdf;     // (E,9) orthotropic C, double-float
     const double *orient;  // (E,9) column-major section orientation (used when ROT)
     double *K;             // BSR values or null
+    double *blkOut;        // instead of K: 64 blocks per listed element
     double *keOut;         // element matrices (E,24,24) column-major, element DOF order, or null
 };
 
@@ -468,13 +469,18 @@ template <bool ROT> __global__ void __launch_bounds__(32 * kDfW, 6) hex8_df_kern
         rotate_block<double>(Or, K1);
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the previous colour's blocks are complete
-    if (A.K) {
+    if (A.K || A.blkOut) {
 #pragma unroll
         for (int q = 0; q < 9; ++q) {
             sK[w][9 * lane + q] = K0[q];
             sK[w][9 * (lane + 32) + q] = K1[q];
         }
         __syncwarp();
+    }
+    if (A.blkOut)
+#pragma unroll
+        for (int q = 0; q < 18; ++q) A.blkOut[576 * (size_t)item + lane + 32 * q] = sK[w][lane + 32 * q];
+    if (A.K) {
 #pragma unroll
         for (int st = 0; st < kRmwSteps; ++st) {
             const int j = 3 * st + grp;
@@ -532,6 +538,8 @@ struct Hex8GenArgs {
     int dyn;
     double beta, delT;
     double *K;             // BSR values or null
+    double *blkOut;        // instead of K: 64 blocks per listed element
+    double *ruItem;        // instead of loadInt: (8 nodes, 3) residuals per listed element
     double *loadInt;       // internal-layout load, -= Ru (or null)
     double *keOut;         // element matrices (E,24,24) column-major, element DOF order, or null
     double *ruOut;         // (E,24) or null
@@ -800,6 +808,9 @@ __global__ void __launch_bounds__(32 * kGenW) hex8_gen_kernel(Hex8GenArgs A) {
 #pragma unroll
                 for (int v = 0; v < 3; ++v) A.loadInt[3 * (size_t)r + v] -= df_to_double(ru[k][v]);
             }
+            if (A.ruItem)
+#pragma unroll
+                for (int v = 0; v < 3; ++v) A.ruItem[24 * (size_t)item + 3 * a + v] = df_to_double(ru[k][v]);
             if (A.ruOut)
 #pragma unroll
                 for (int v = 0; v < 3; ++v) A.ruOut[24 * (size_t)e + 8 * v + a] = df_to_double(ru[k][v]);
@@ -896,6 +907,9 @@ __global__ void __launch_bounds__(32 * kGenW) hex8_gen_kernel(Hex8GenArgs A) {
             for (int j = 0; j < 3; ++j) dst[3 * i + j] = (a <= b) ? Kb[3 * i + j] : Kb[3 * j + i];
     }
     __syncwarp();
+    if (A.blkOut)
+#pragma unroll
+        for (int q = 0; q < 18; ++q) A.blkOut[576 * (size_t)item + lane + 32 * q] = S.o.K[lane + 32 * q];
     if (A.K) {
         const unsigned long long first = A.elFirst[e];
         const int grp = lane / 9, qq = lane - 9 * grp;
@@ -988,6 +1002,83 @@ static void colour_launch(Kern kernel, unsigned grid, unsigned block, cudaStream
     cudaLaunchKernelEx(&cfg, kernel, A);
 }
 
+// The blocks and residuals of one colour's elements, as their kernel would have added them: a thread per
+// block entry (three whole blocks and more a warp) and load entry.
+struct HexAddArgs {
+    const int *els;
+    int count, per;  // entries per element
+    const int *elBlk;
+    const unsigned long long *elFirst;
+    const int *elist, *rank;
+    const double *blk, *ru;
+    double *K, *loadInt;
+};
+__global__ void k_hex_add(HexAddArgs A) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    int q = t / A.per, k = t - q * A.per;
+    const bool in = q < A.count;
+    double v = 0.0;
+    double *dst = nullptr;
+    bool set = false;
+    if (in) {
+        const int e = A.els[q];
+        if (A.K && k < 576) {
+            const int j = k / 9;
+            v = A.blk[576 * (size_t)q + k];
+            dst = A.K + 9 * (size_t)A.elBlk[64 * (size_t)e + j] + k % 9;
+            set = (A.elFirst[e] >> j) & 1ull;
+        } else {
+            if (A.K) k -= 576;
+            v = -A.ru[24 * (size_t)q + k];
+            dst = A.loadInt + 3 * (size_t)(A.rank[A.elist[8 * (size_t)e + k / 3] - 1] - 1) + k % 3;
+        }
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the previous colour's entries are complete
+    if (in) *dst = set ? v : *dst + v;
+}
+
+// Meshes whose colours leave the SMs idle: all elements in one launch, their blocks and residuals into
+// scratch, then added colour by colour (the same sums).  A colour's launch takes the latency of one element
+// (17 .. 20 us in brick8) however few there are, an addition 2.3 us.  Whole calls, eight colours, brick8
+// undeformed and displaced, colour by colour -> at once: 819 elements 127 -> 61 and 233 -> 98 us; 4,096 150 -> 95 and 292 -> 208 us;
+// 12,288 209 -> 336 and 599 -> 635 us (the scratch leaves L2).  brickIM, whose elements take 40 times as
+// long, gains at any size by filling the SMs better, in groups of that many (4,125: 1.55 -> 1.01 ms; 16,384: 4.42 -> 3.74 ms).
+bool hex_at_once(int elements, size_t colours) { return colours > 2 && elements <= kHexAtOnce; }
+int hex_at_once_alloc(astro_ctx *ctx, int elements, bool blk, bool ru, DevBuf &dBlk, DevBuf &dRu) {
+    int rc;
+    if (blk && (rc = dev_alloc(ctx, dBlk, sizeof(double) * 576 * (size_t)elements))) return rc;
+    if (ru && (rc = dev_alloc(ctx, dRu, sizeof(double) * 24 * (size_t)elements))) {
+        dev_free(dBlk);
+        return rc;
+    }
+    return ASTRO_OK;
+}
+void hex_at_once_add(astro_ctx *ctx, const int *d_list, const std::vector<int> &ptr, DevBuf &dBlk, DevBuf &dRu, double *K,
+                     double *d_loadInt) {
+    HexAddArgs A;
+    A.elBlk = dptr<int>(ctx->d_elBlk);
+    A.elFirst = dptr<unsigned long long>(ctx->d_elFirst);
+    A.elist = dptr<int>(ctx->d_elist);
+    A.rank = dptr<int>(ctx->d_rank);
+    A.K = K;
+    A.loadInt = d_loadInt;
+    A.per = (K ? 576 : 0) + (d_loadInt ? 24 : 0);
+    bool chained = false;
+    for (size_t col = 0; col + 1 < ptr.size() && A.per; ++col) {
+        A.count = ptr[col + 1] - ptr[col];
+        if (!A.count) continue;
+        A.els = d_list + ptr[col];
+        A.blk = K ? dptr<double>(dBlk) + 576 * (size_t)(ptr[col] - ptr[0]) : nullptr;
+        A.ru = d_loadInt ? dptr<double>(dRu) + 24 * (size_t)(ptr[col] - ptr[0]) : nullptr;
+        colour_launch(k_hex_add, (unsigned)((A.count * A.per + 255) / 256), 256, ctx->stream, chained, A);
+        chained = true;
+    }
+    // (freed buffers stay with the context and its stream)
+    dev_free(dBlk);
+    dev_free(dRu);
+}
+
 template <class T, bool ROT, int FW> static void hex8_fast_launch(astro_ctx *ctx, const Hex8FastArgs<T> &A0) {
     Hex8FastArgs<T> A = A0;
     const std::vector<int> &ptr = ctx->c8Ptr;
@@ -1062,12 +1153,24 @@ static int hex8_gen_run(astro_ctx *ctx, const int *d_list, const std::vector<int
     A.gpcLo = g.lo;
     const bool rot = !ctx->orientIdentity;
     bool chained = false;
-    for (size_t col = 0; col + 1 < ptr.size(); ++col) {
-        const int cnt = ptr[col + 1] - ptr[col];
+    // all colours as one where the mesh is small
+    const bool once = hex_at_once(ptr.back() - ptr[0], ptr.size() - 1);
+    const std::vector<int> all = {ptr[0], ptr.back()}, &run = once ? all : ptr;
+    DevBuf dBlk, dRu;
+    A.blkOut = A.ruItem = nullptr;
+    if (once) {
+        const int rc = hex_at_once_alloc(ctx, ptr.back() - ptr[0], build && K, d_loadInt != nullptr, dBlk, dRu);
+        if (rc) return rc;
+        A.blkOut = dptr<double>(dBlk);
+        A.ruItem = dptr<double>(dRu);
+        A.K = A.loadInt = nullptr;
+    }
+    for (size_t col = 0; col + 1 < run.size(); ++col) {
+        const int cnt = run[col + 1] - run[col];
         if (!cnt) continue;
-        A.colorEls = d_list + ptr[col];
+        A.colorEls = d_list + run[col];
         A.count = cnt;
-        A.CdfItem = CdfItem ? CdfItem + 9 * (size_t)ptr[col] : nullptr;
+        A.CdfItem = CdfItem ? CdfItem + 9 * (size_t)run[col] : nullptr;
         const unsigned grid = (cnt + kGenW - 1) / kGenW;
         if (build) {
             if (rot)
@@ -1082,6 +1185,7 @@ static int hex8_gen_run(astro_ctx *ctx, const int *d_list, const std::vector<int
         }
         chained = true;
     }
+    if (once) hex_at_once_add(ctx, d_list, ptr, dBlk, dRu, build ? K : nullptr, d_loadInt);
     return cuda_check(ctx, cudaGetLastError(), "brick8 general-state kernel launch");
 }
 
@@ -1097,10 +1201,20 @@ static int hex8_df_run(astro_ctx *ctx, double *K, double *d_ke, const int *d_lis
     A.K = K;
     A.keOut = d_ke;
     bool chained = false;
-    for (size_t col = 0; col + 1 < ptr.size(); ++col) {
-        const int cnt = ptr[col + 1] - ptr[col];
+    const bool once = hex_at_once(ptr.back() - ptr[0], ptr.size() - 1);
+    const std::vector<int> all = {ptr[0], ptr.back()}, &run = once ? all : ptr;
+    DevBuf dBlk, dRu;
+    A.blkOut = nullptr;
+    if (once) {
+        const int rc = hex_at_once_alloc(ctx, ptr.back() - ptr[0], K != nullptr, false, dBlk, dRu);
+        if (rc) return rc;
+        A.blkOut = dptr<double>(dBlk);
+        A.K = nullptr;
+    }
+    for (size_t col = 0; col + 1 < run.size(); ++col) {
+        const int cnt = run[col + 1] - run[col];
         if (!cnt) continue;
-        A.colorEls = d_list + ptr[col];
+        A.colorEls = d_list + run[col];
         A.count = cnt;
         const unsigned grid = (cnt + kDfW - 1) / kDfW;
         if (ctx->orientIdentity)
@@ -1109,6 +1223,7 @@ static int hex8_df_run(astro_ctx *ctx, double *K, double *d_ke, const int *d_lis
             colour_launch(hex8_df_kernel<true>, grid, 32 * kDfW, ctx->stream, chained, A);
         chained = true;
     }
+    if (once) hex_at_once_add(ctx, d_list, ptr, dBlk, dRu, K, nullptr);
     return cuda_check(ctx, cudaGetLastError(), "brick8 FP64 zero-state kernel launch");
 }
 

@@ -47,6 +47,7 @@ struct Hex81Args {
     double gpc;                // Gauss point coordinate
     int build;                 // element matrix (1) or residual only (0)
     double *K, *loadInt, *intLoad, *intMat, *keOut, *ruOut;
+    double *blkOut, *ruItem;   // instead of K and loadInt: 64 blocks and (8 nodes, 3) residuals per listed element
     int nNodes, nEls, nBlocks;
     int *status;
 };
@@ -259,6 +260,8 @@ __global__ void __launch_bounds__(32) hex81_kernel(Hex81Args A) {
                 const int r = A.rank[A.elist[8 * (size_t)e + lane] - 1] - 1;
                 for (int v = 0; v < 3; ++v) A.loadInt[3 * (size_t)r + v] -= ru[v];
             }
+            if (A.ruItem)
+                for (int v = 0; v < 3; ++v) A.ruItem[24 * (size_t)item + 3 * lane + v] = ru[v];
             if (A.ruOut)
                 for (int v = 0; v < 3; ++v) A.ruOut[24 * (size_t)e + 8 * v + lane] = ru[v];
         } else if (A.intLoad) {
@@ -338,6 +341,11 @@ __global__ void __launch_bounds__(32) hex81_kernel(Hex81Args A) {
         double *ke = A.keOut + 576 * (size_t)e;
         for (int q = lane; q < 576; q += 32) ke[q] = S.K[33 * (q / 24) + q % 24];
     }
+    if (A.blkOut)
+        for (int q = lane; q < 576; q += 32) {
+            const int j = q / 9, qq = q - 9 * j;
+            A.blkOut[576 * (size_t)item + q] = S.K[33 * (8 * (qq % 3) + (j & 7)) + 8 * (qq / 3) + (j >> 3)];
+        }
     if (A.K) {
         const unsigned long long first = A.elFirst[e];
         const int grp = lane / 9, qq = lane - 9 * grp, bi = qq / 3, bj = qq % 3;
@@ -433,13 +441,31 @@ int hex81_run(astro_ctx *ctx, const int *d_list, const std::vector<int> &ptr, in
     A.nEls = ctx->P.E;
     A.nBlocks = ctx->P.nb;
     A.status = ASTRO_CHECKED ? dptr<int>(ctx->d_guard) : nullptr;
-    for (size_t col = 0; col + 1 < ptr.size(); ++col) {
-        const int cnt = ptr[col + 1] - ptr[col];
-        if (!cnt) continue;
-        A.els = d_list + ptr[col];
-        A.count = cnt;
-        A.CItem = CItem ? CItem + 9 * (size_t)ptr[col] : nullptr;
-        hex81_kernel<<<cnt, 32, 0, ctx->stream>>>(A);
+    // groups of elements across the colours (a colour alone is the whole of it in a mixed mesh's pass)
+    A.blkOut = A.ruItem = nullptr;
+    for (int lo = ptr[0]; lo < ptr.back();) {
+        const bool once = ptr.size() > 2;
+        const int hi = once ? std::min(ptr.back(), lo + kHexAtOnce) : ptr.back();
+        DevBuf dBlk, dRu;
+        if (once) {
+            const int rc = hex_at_once_alloc(ctx, hi - lo, build && K, d_loadInt != nullptr, dBlk, dRu);
+            if (rc) return rc;
+            A.blkOut = dptr<double>(dBlk);
+            A.ruItem = dptr<double>(dRu);
+            A.K = A.loadInt = nullptr;
+        }
+        A.els = d_list + lo;
+        A.count = hi - lo;
+        A.CItem = CItem ? CItem + 9 * (size_t)lo : nullptr;
+        hex81_kernel<<<A.count, 32, 0, ctx->stream>>>(A);
+        if (once) {
+            std::vector<int> part = {lo};
+            for (int p : ptr)
+                if (p > lo && p < hi) part.push_back(p);
+            part.push_back(hi);
+            hex_at_once_add(ctx, d_list, part, dBlk, dRu, build ? K : nullptr, d_loadInt);
+        }
+        lo = hi;
     }
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess && ASTRO_CHECKED) e = cudaStreamSynchronize(ctx->stream);
