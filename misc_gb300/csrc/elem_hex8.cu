@@ -481,13 +481,24 @@ template <bool ROT> __global__ void __launch_bounds__(32 * kDfW, 6) hex8_df_kern
 #pragma unroll
         for (int q = 0; q < 18; ++q) A.blkOut[576 * (size_t)item + lane + 32 * q] = sK[w][lane + 32 * q];
     if (A.K) {
+        // an element's blocks are distinct: the loads of a half before its stores
 #pragma unroll
-        for (int st = 0; st < kRmwSteps; ++st) {
-            const int j = 3 * st + grp;
-            if (grp < 3 && j < 64) {
-                double *dst = A.K + 9 * (size_t)sBlk[w][j] + qq;
-                const double v = sK[w][9 * j + qq];
-                *dst = ((first >> j) & 1ull) ? v : *dst + v;
+        for (int h = 0; h < 2; ++h) {
+            constexpr int H = kRmwSteps / 2;
+            double ov[H];
+#pragma unroll
+            for (int st = 0; st < H; ++st) {
+                const int j = 3 * (h * H + st) + grp;
+                ov[st] = 0.0;
+                if (grp < 3 && j < 64 && !((first >> j) & 1ull)) ov[st] = A.K[9 * (size_t)sBlk[w][j] + qq];
+            }
+#pragma unroll
+            for (int st = 0; st < H; ++st) {
+                const int j = 3 * (h * H + st) + grp;
+                if (grp < 3 && j < 64) {
+                    const double v = sK[w][9 * j + qq];
+                    A.K[9 * (size_t)sBlk[w][j] + qq] = ((first >> j) & 1ull) ? v : ov[st] + v;
+                }
             }
         }
     }
@@ -551,7 +562,9 @@ constexpr int kGenW = 2;  // warps per CTA
 struct GenSmem {
     union {
         struct {
-            float Ph[64][18], Pl[64][18], Qh[64][18], Ql[64][18];  // item gp*8 + a: 6x3 row-major
+            // item gp*8 + a: 6x3 row-major, and one more: phase 2's lanes read rows of their own, which
+            // at 18 words share banks four deep (at 19, two)
+            float Ph[64][19], Pl[64][19], Qh[64][19], Ql[64][19];
             float4 gh[64], gl[64], th[64], tl[64];
         } u;
         struct {
@@ -578,9 +591,19 @@ __global__ void __launch_bounds__(32 * kGenW) hex8_gen_kernel(Hex8GenArgs A) {
     GenSmem &S = sm[w];
     const int e = A.colorEls[item];
     asm volatile("griddepcontrol.launch_dependents;");  // chained colours, as in hex8_fast_kernel
+    unsigned long long first = 0;
     if (BUILD) {
-        S.blk[lane] = A.elBlk[64 * (size_t)e + lane];
-        S.blk[lane + 32] = A.elBlk[64 * (size_t)e + lane + 32];
+        first = A.elFirst[e];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int j = lane + 32 * h, k = A.elBlk[64 * (size_t)e + j];
+            S.blk[j] = k;
+            // the blocks to L2 for the additions at the end (72 bytes: both ends)
+            if (A.K && !((first >> j) & 1ull)) {
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(A.K + 9 * (size_t)k));
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(A.K + 9 * (size_t)k + 8));
+            }
+        }
     }
     const DF one{1.f, 0.f}, zero{0.f, 0.f};
     DF c[9];  // C11 C12 C13 C22 C23 C33 C44 C55 C66
@@ -911,15 +934,22 @@ __global__ void __launch_bounds__(32 * kGenW) hex8_gen_kernel(Hex8GenArgs A) {
 #pragma unroll
         for (int q = 0; q < 18; ++q) A.blkOut[576 * (size_t)item + lane + 32 * q] = S.o.K[lane + 32 * q];
     if (A.K) {
-        const unsigned long long first = A.elFirst[e];
+        // an element's blocks are distinct: all loads before the first store (one by one, each waited for
+        // its turn to L2)
         const int grp = lane / 9, qq = lane - 9 * grp;
+        double ov[kRmwSteps];
+#pragma unroll
+        for (int stp = 0; stp < kRmwSteps; ++stp) {
+            const int j = 3 * stp + grp;
+            ov[stp] = 0.0;
+            if (grp < 3 && j < 64 && !((first >> j) & 1ull)) ov[stp] = A.K[9 * (size_t)S.blk[j] + qq];
+        }
 #pragma unroll
         for (int stp = 0; stp < kRmwSteps; ++stp) {
             const int j = 3 * stp + grp;
             if (grp < 3 && j < 64) {
-                double *dst = A.K + 9 * (size_t)S.blk[j] + qq;
                 const double v = S.o.K[9 * j + qq];
-                *dst = ((first >> j) & 1ull) ? v : *dst + v;
+                A.K[9 * (size_t)S.blk[j] + qq] = ((first >> j) & 1ull) ? v : ov[stp] + v;
             }
         }
     }
