@@ -224,6 +224,7 @@ int ensure_K(astro_ctx *ctx, int which);          // device BSR value arrays (ct
 int ensure_io(astro_ctx *ctx, bool exportMat);    // host-vector staging buffers (ctx.cu)
 int panels_cases_solve(astro_ctx *ctx, double *d_vec, cudaStream_t s);      // panels.cu
 int panels_cases_columns(astro_ctx *ctx);
+int panels_cases_status(astro_ctx *ctx, cudaStream_t s);                      // panels.cu
 int panels_cases_launches(astro_ctx *ctx);                                   // panels.cu
 int panels_cases_would_twist(astro_ctx *ctx);                                // panels.cu
 int panels_factor_impl(astro_ctx *ctx, int32_t cluster_size, astro_panels_info *info, int factor);  // panels.cu

@@ -374,7 +374,7 @@ extern "C" int astro_newmark_cases(astro_ctx *ctx, const astro_newmark_cases_opt
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     if (rc) return rc;
-    if ((rc = cuda_check(ctx, es, "newmark cases steps"))) return rc;
+    if ((rc = cuda_check(ctx, es, "newmark cases steps")) || (rc = panels_cases_status(ctx, s))) return rc;
     // the last step's solve against its residual: max over cases of ||A du - r|| / ||r||
     double worst = 0.0;
     if (steps > 0) {

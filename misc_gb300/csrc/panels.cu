@@ -85,7 +85,8 @@ struct PanelPlan {
     // double-float copies for the many-column solve (k_band_solve_cases), built from factor
     // generation dfGen; the items and the right-hand-side block for casesCols columns
     int factorGen = 0, dfGen = -1, casesCols = 0, ring = 0;
-    DevBuf d_Lf, d_Lb, d_Wf, d_Wb, d_Dinv, d_items, d_X;
+    DevBuf d_Lf, d_Lb, d_Wf, d_Wb, d_Dinv, d_items, d_X, d_Mx;
+    int mGen = -1;  // factor generation of d_Mx
     // astro_panels_solve's work buffers (grow-only): right-hand sides in both orderings, the
     // refinement's residuals, the panel-layout block and the items
     DevBuf d_sRef, d_sVec, d_sRes, d_sBi, d_sX, d_sItems;
@@ -96,7 +97,7 @@ struct PanelPlan {
     double twFactorSeconds = 0.0;
     std::vector<PanelMeta> twMeta;
     DevBuf d_twMeta, d_twBand, d_twAw, d_twSched, d_twSchedPtr, d_twStatus, d_twLf, d_twLb, d_twWf, d_twWb, d_twDinv,
-        d_twItems, d_twX;
+        d_twItems, d_twX, d_twMx;
 };
 
 // lower-band entries of the BSR stiffness (dpn x dpn row-major blocks) into the tiles
@@ -1248,20 +1249,27 @@ __global__ void __launch_bounds__(kThreads, 2) k_band_solve_df(const PanelMeta *
 // single large band (a model's K_eff, factored once and solved at every time step) is instead a
 // chain of nbc dependent block rows per sweep, and FP64 runs at about 1/64 of the FP32 rate: one
 // CTA per column would spend tens of microseconds per block row.  So each (panel, column) gets a
-// cluster of CS CTAs (2, 4 or 8, autotuned) and the arithmetic runs in double-float on the FP32 pipe:
-//   * producer CTAs (ranks 1 .. CS-1), one warp per tile: for block row I they form
-//     sum_{d >= 2} L_{I,I-d} y_{I-d} from the solved rows in their shared-memory ring, reduce it
-//     across the CTA and store it into the leader's shared memory (distributed shared memory);
-//   * the leader (rank 0) forms L_{I,I-1} y_{I-1} from the row it solved last, waits at the
-//     cluster barrier, subtracts the partials from b_I and applies W_I = L_II^-1 (inverted once
-//     after the factorisation): y_I = W_I (b_I - ...), pushed into every CTA's ring;
-//   * one cluster barrier per block row (release / acquire orders the stores into distributed
-//     shared memory); the producers run one row ahead of the leader (their tiles need rows
-//     up to I - 2 only);
-//   * backward sweep the same with L^T (transposed copies of the tiles and of W) on D^-1 y.
+// cluster of CS CTAs (2, 4 or 8, autotuned) and the arithmetic runs in double-float on the FP32 pipe.
+// With W_I = L_II^-1 and M1_I = W_I L_{I,I-1}, M2_I = W_I L_{I,I-2} (formed once, in FP64),
+//   y_I = u_I - M1_I y_{I-1} - M2_I y_{I-2},   u_I = W_I (b_I - sum_{d >= 3} L_{I,I-d} y_{I-d}),
+// so that of a block row only the product with M1_I waits for the row before.  Three stages run side by side, each as
+// far ahead as the rows that it needs allow:
+//   * producer CTAs (ranks 1 .. CS-1), a warp per part of a tile: the sum over d >= 3 for row I + 3 from the
+//     solved rows up to I in their shared-memory ring, reduced across the CTA and sent to the leader;
+//   * the leader's warps 8 .. 15: u_I from those sums;
+//   * the leader's warps 0 .. 7: M1_I y_{I-1} and M2_I y_{I-2}, and y_I, sent to every CTA's ring;
+//   * backward sweep the same with L^T (transposed copies of the tiles and of W, M) on D^-1 y.
+// Rows and sums travel as asynchronous stores into the other CTA's shared memory that count on a barrier
+// there (mbarrier; four in turn: a stage is at most three rows ahead of another).  With a cluster barrier
+// per row its release alone took 1,000 clocks, and the sums by one warp as long (instruction fetch); now
+// all warps of a stage share a sum.  What bounds it: the way from a row to the sums three rows on, and the
+// tiles from L2.  25,350 DOF, 13 tiles, 17 cases in four CTAs each: half a sweep 445 us (with
+// one chain per row and a cluster barrier 665).
 // The band is copied once into double-float tiles in the forward (column-major) and backward
 // (row-major) layouts, so every tile load of a warp is 32 consecutive float2 per k.
-constexpr int kCW = 8;   // warps per CTA (the CTAs per cluster, CS, is a template parameter: 2, 4 or 8)
+constexpr int kCW = 8;   // warps of u's stage (the CTAs per cluster, CS, is a template parameter: 2, 4 or 8)
+constexpr int kCaseW = 2 * kCW;  // warps per CTA
+constexpr int kCaseWait = 1 << 20;  // polls of a barrier (about a second), then the status is set and waits skipped
 constexpr int kPrepW = 4;  // warps per CTA of the band copy
 
 struct CaseItem {
@@ -1361,182 +1369,390 @@ template <int K> __device__ __forceinline__ DF df_tree_sum(DF (&v)[K]) {
     return v[0];
 }
 
-// acc[r] += sum_{k in [k0, k1)} T[k * TB + r] v[k] (T a DF tile in global memory, v in shared)
-__device__ __forceinline__ void df_tile_rows(DF &acc, const float2 *__restrict__ T, const float2 *v, int r, int k0,
-                                             int k1) {
-    DF a2 = {0.f, 0.f};
-    int k = k0;
-    for (; k + 1 < k1; k += 2) {
-        const float2 l0 = __ldg(T + k * TB + r), l1 = __ldg(T + (k + 1) * TB + r);
-        const float2 y0 = v[k], y1 = v[k + 1];
-        df_acc(acc, l0.x, l0.y, y0.x, y0.y);
-        df_acc(a2, l1.x, l1.y, y1.x, y1.y);
+// M1_J, M2_J of k_band_solve_cases in FP64, rounded to double-float once: forward M[d-1] = W_J L_{J,J-d}, backward
+// M[2+d-1] = (L_{J+d,J} W_J)^T, column-major (entry (i, k) at k TB + i), stride mS between the four; zero where
+// the tile does not exist.  One warp per block column.
+__global__ void k_band_mprep(const PanelMeta *__restrict__ meta, int np, const double *__restrict__ band,
+                             float2 *__restrict__ Mx, size_t mS) {
+    __shared__ double sT[kPrepW][TB][TB + 1];
+    const int w = threadIdx.x / 32, lane = threadIdx.x % 32;
+    long long gJ = (long long)blockIdx.x * kPrepW + w;
+    int p = 0;
+    for (; p < np; ++p) {
+        if (gJ < meta[p].nbc) break;
+        gJ -= meta[p].nbc;
     }
-    if (k < k1) {
-        const float2 l0 = __ldg(T + k * TB + r);
-        const float2 y0 = v[k];
-        df_acc(acc, l0.x, l0.y, y0.x, y0.y);
+    if (p >= np) return;
+    const PanelMeta M = meta[p];
+    const int J = (int)gJ;
+    const bool fac = J < M.nfac;  // else W = I, and no column of L here
+    const size_t od = tile_off(M, J, 0), om = (size_t)M.xUnit * TB + (size_t)J * TT;
+    double x[TB];  // column `lane` of W
+    if (fac) {
+        for (int e = lane; e < TT; e += 32) sT[w][e % TB][e / TB] = band[od + e];
+        __syncwarp();
     }
-    acc = df_add(df_norm(acc), df_norm(a2));
+#pragma unroll
+    for (int i = 0; i < TB; ++i) {
+        double v = (i == lane) ? 1.0 : 0.0;
+        if (fac) {
+#pragma unroll
+            for (int k = 0; k < i; ++k) v -= sT[w][i][k] * x[k];
+        }
+        x[i] = v;
+    }
+    // backward: lane i has row i of M, sum_m W[m][i] L_{J+d,J}[k][m]
+    for (int d = 1; d <= 2; ++d) {
+        float2 *out = Mx + (1 + d) * mS + om;
+        const bool has = fac && d <= M.bt && J + d < M.nbc;
+        const double *T = band + (has ? tile_off(M, J, d) : 0);
+        for (int k = 0; k < TB; ++k) {
+            double v = 0.0;
+            if (has) {
+                double v1 = 0.0;
+#pragma unroll
+                for (int m = 0; m < TB; m += 2) {
+                    v = fma(x[m], __ldg(T + m * TB + k), v);
+                    v1 = fma(x[m + 1], __ldg(T + (m + 1) * TB + k), v1);
+                }
+                v += v1;
+            }
+            const DF f = df_from_double(v);
+            out[k * TB + lane] = make_float2(f.hi, f.lo);
+        }
+    }
+    // forward: lane i has row i of W, sum_m W[i][m] L_{J,J-d}[m][k]
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < TB; ++i) sT[w][i][lane] = x[i];
+    __syncwarp();
+#pragma unroll
+    for (int m = 0; m < TB; ++m) x[m] = sT[w][lane][m];
+    for (int d = 1; d <= 2; ++d) {
+        float2 *out = Mx + (d - 1) * mS + om;
+        const bool has = J - d >= 0 && d <= M.bt && J - d < M.nfac;
+        const double *T = band + (has ? tile_off(M, J - d, d) : 0);
+        for (int k = 0; k < TB; ++k) {
+            double v = 0.0;
+            if (has) {
+                double v1 = 0.0;
+#pragma unroll
+                for (int m = 0; m < TB; m += 2) {
+                    v = fma(x[m], __ldg(T + k * TB + m), v);
+                    v1 = fma(x[m + 1], __ldg(T + k * TB + m + 1), v1);
+                }
+                v += v1;
+            }
+            const DF f = df_from_double(v);
+            out[k * TB + lane] = make_float2(f.hi, f.lo);
+        }
+    }
+}
+
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ unsigned map_rank(unsigned a, int rank) {
+    unsigned d;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(rank));
+    return d;
+}
+// v into another CTA's shared memory, counted on its barrier
+__device__ __forceinline__ void send_df(unsigned addr, DF v, unsigned bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(addr), "f"(v.hi),
+                 "f"(v.lo), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void bar_init(unsigned bar, int count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(unsigned bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void bar_expect(unsigned bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity) {
+    for (int it = 0; it < kCaseWait; ++it) {
+        unsigned ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok)
+                     : "r"(bar), "r"(parity), "r"(1000)  // (a poll sleeps for a microsecond at most)
+                     : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+template <int WARPS> __device__ __forceinline__ void stage_barrier(int id) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(WARPS * 32) : "memory");
+}
+__device__ __forceinline__ DF df_xor(DF v, int m) {
+    return DF{__shfl_xor_sync(0xffffffffu, v.hi, m), __shfl_xor_sync(0xffffffffu, v.lo, m)};
+}
+
+constexpr int kRedLd = TB + 1;  // row stride of the partials: a warp reads them by column
+
+// Bytes of dynamic shared memory.
+static size_t cases_smem(int ring, int cs) {
+    return sizeof(float2) * ((size_t)TB * (ring + 4 * cs + 4) + 2 * kCaseW * kRedLd);
 }
 
 template <int CS>
-__global__ void __launch_bounds__(kCW * 32, 1) k_band_solve_cases(const PanelMeta *__restrict__ meta,
-                                                               const CaseItem *__restrict__ items,
-                                                               const float2 *__restrict__ Lf,
-                                                               const float2 *__restrict__ Lb,
-                                                               const float2 *__restrict__ Wf,
-                                                               const float2 *__restrict__ Wb,
-                                                               const float2 *__restrict__ Dinv, double *X, int nrhs,
-                                                               int ring) {
-    constexpr int kProdWarps = (CS - 1) * kCW;
+__global__ void __launch_bounds__(kCaseW * 32, 1) k_band_solve_cases(const PanelMeta *__restrict__ meta,
+                                                                     const CaseItem *__restrict__ items,
+                                                                     const float2 *__restrict__ Lf,
+                                                                     const float2 *__restrict__ Lb,
+                                                                     const float2 *__restrict__ Wf,
+                                                                     const float2 *__restrict__ Wb,
+                                                                     const float2 *__restrict__ Mx, size_t mS,
+                                                                     const float2 *__restrict__ Dinv, double *X, int nrhs,
+                                                                     int ring, int *status) {
+    // parts of a tile that the producers' warps take: with 13 tiles, 48 warps and more have a part at most
+    constexpr int NQ = CS == 2 ? 2 : 4;
+    constexpr int kProdWarps = (CS - 1) * kCaseW, H = TB / NQ, C = TB / 4;
+    constexpr unsigned kRow = TB * sizeof(float2);
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
     extern __shared__ float2 smf[];
-    float2 *sRing = smf;                           // [ring][TB]: solved rows
-    float2 *sRed = sRing + (size_t)ring * TB;      // [kCW][TB]: per-warp partials
-    float2 *sPart = sRed + kCW * TB;               // [2][CS][TB]: CTA partials (leader)
-    float2 *sV = sPart + 2 * CS * TB;             // [TB]
+    float2 *sRing = smf;                       // [ring][TB]: solved rows
+    float2 *sPart = sRing + (size_t)ring * TB; // [4][CS][TB]: the producers' sums (leader)
+    float2 *sU = sPart + 4 * CS * TB;          // [4][TB]
+    float2 *sRed = sU + 4 * TB;                // [2][kCaseW][kRedLd]: partials (leader: y's stage, then u's)
+    __shared__ __align__(8) unsigned long long sBar[8];  // rows (producers), sums (leader); u (leader)
+    __shared__ int sDead;                      // a wait was given up
     const CaseItem it = items[blockIdx.x / CS];
     const PanelMeta M = meta[it.panel];
     const int w = threadIdx.x / 32, r = threadIdx.x % 32;
     const int nbc = M.nbc, bt = M.bt;
     double *Xp = X + (size_t)M.xUnit * nrhs + (size_t)it.col * nbc * TB;
     const size_t wOff = (size_t)M.xUnit * TB;
-    float2 *leaderPart = cl.map_shared_rank(sPart, 0);
-    // step t = 0 .. 2 nbc - 1: forward rows I = t, then backward rows I = 2 nbc - 1 - t
-    auto rowOf = [&](int t) { return t < nbc ? t : 2 * nbc - 1 - t; };
-    // tiles below (forward) or right of (backward) the row that exist: min(bt, I) / min(bt, nbc - 1 - I)
-    auto dmaxOf = [&](int t) { return t < nbc ? min(bt, t) : min(bt, t - nbc); };
-    // tile d of step t: forward L_{I,I-d} = tile (I-d, d) of Lf; backward L_{I+d,I}^T = tile (I, d) of Lb
-    auto tileOf = [&](int t, int d) {
-        const int I = rowOf(t);
-        return t < nbc ? Lf + tile_off(M, I - d, d) : Lb + tile_off(M, I, d);
-    };
-    auto srcOf = [&](int t, int d) { return t < nbc ? rowOf(t) - d : rowOf(t) + d; };
-    // Each warp's next tile is loaded into registers one step ahead, so the loads are in flight
-    // during the cluster barrier and the leader's part of the step: producers the first tile of
-    // the warp (pf, the lane's row of it), the leader its four columns of L_{I,I+-1} (pl) and of
-    // W (pw), and warp 0 the right-hand side (pb) and D^-1 (pd).
-    const int d0 = 2 + (rank - 1) * kCW + w;
-    float2 pf[TB], pl[4], pw[4], pd = make_float2(0.f, 0.f);
-    double pb = 0.0;
-    const int t0 = it.t0, t1 = it.t1;
-    auto prefetch = [&](int t) {
-        if (t >= t1) return;
-        const int dm = dmaxOf(t), I = rowOf(t);
-        if (rank > 0) {
-            if (d0 <= dm) {
-                const float2 *T = tileOf(t, d0);
-#pragma unroll
-                for (int k = 0; k < TB; ++k) pf[k] = __ldg(T + k * TB + r);
-            }
-        } else {
-            if (dm >= 1) {
-                const float2 *T = tileOf(t, 1);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) pl[k] = __ldg(T + (4 * w + k) * TB + r);
-            }
-            const float2 *Wt = (t < nbc ? Wf : Wb) + wOff + (size_t)I * TT;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) pw[k] = __ldg(Wt + (4 * w + k) * TB + r);
-            if (w == 0) {
-                pb = Xp[(size_t)I * TB + r];
-                if (t >= nbc) pd = __ldg(Dinv + M.xUnit + (size_t)I * TB + r);
-            }
-        }
-    };
-    // a backward sweep that starts below the last row (the rows after it solved already, in X):
-    // those rows into every CTA's ring
-    if (t0 > nbc) {
-        const int I0 = 2 * nbc - 1 - t0;
-        for (int R = I0 + 1 + w; R <= min(nbc - 1, I0 + bt); R += kCW) {
-            const DF v = df_from_double(Xp[(size_t)R * TB + r]);
-            sRing[(size_t)(R % ring) * TB + r] = make_float2(v.hi, v.lo);
-        }
+    const unsigned bars = smem_u32(sBar), expect = rank > 0 ? kRow : (CS - 1) * kRow;
+    if (threadIdx.x == 0) {
+        sDead = 0;
+        for (int k = 0; k < 8; ++k) bar_init(bars + 8 * k, k < 4 ? 1 : kCW);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        for (int k = 0; k < 4; ++k) bar_expect(bars + 8 * k, expect);
     }
-    prefetch(t0);
-    for (int t = t0; t < t1; ++t) {
-        const int I = rowOf(t), dmax = dmaxOf(t), q = t < nbc ? t : t - nbc;
-        __syncthreads();  // the leader's last row is in its ring
+    // arrival number n of rows (sums), and the arming of number n + 4 by one thread
+    auto wait = [&](unsigned bar, int n) {
+        if (!sDead && !bar_wait(bar + 8 * (n & 3), (n >> 2) & 1)) {
+            sDead = 1;
+            atomicExch(status, -1);
+        }
+    };
+    auto arrived = [&](int n, bool arm) {
+        wait(bars, n);
+        if (arm) bar_expect(bars + 8 * (n & 3), expect);
+    };
+    // step t = 0 .. 2 nbc - 1: forward rows I = t, then backward rows I = 2 nbc - 1 - t.  Row k of a sweep
+    // (t = k or nbc + k) has tiles d <= min(bt, k): forward L_{I,I-d} = tile (I-d, d) of Lf, backward
+    // L_{I+d,I}^T = tile (I, d) of Lb.  Places advance by a constant from row to row (computed anew, with the
+    // ring's remainder, they took a third of a row's time).
+    int rowsIn = 0, sums = 0;  // rows taken from the leader (by it: sent), sums formed or taken
+    for (int seg = 0; seg < 2; ++seg) {  // forward and backward steps of the item
+        const int off = seg ? nbc : 0, k0 = max(it.t0, off) - off, k1 = min(it.t1, off + nbc) - off;
+        if (k0 >= k1) continue;
+        const int dir = seg ? -1 : 1, I0 = seg ? nbc - 1 - k0 : k0;  // the first row
+        // a backward sweep that starts below the last row (the rows after it solved already, in X):
+        // those rows into every CTA's ring
+        if (seg && k0 > 0) {
+            for (int R = I0 + 1 + w; R <= min(nbc - 1, I0 + bt); R += kCaseW) {
+                const DF v = df_from_double(Xp[(size_t)R * TB + r]);
+                sRing[(size_t)(R % ring) * TB + r] = make_float2(v.hi, v.lo);
+            }
+        }
+        cluster_barrier();
+        // the slot of the row d before I0, and the one after slot s
+        auto slotBefore = [&](int d) { return (I0 - dir * d + 2 * ring * nbc) % ring; };
+        auto nextSlot = [&](int s) { return dir > 0 ? (s + 1 < ring ? s + 1 : 0) : (s > 0 ? s - 1 : ring - 1); };
         if (rank > 0) {
-            DF acc = {0.f, 0.f}, a2 = {0.f, 0.f};
-            if (d0 <= dmax) {
-                const float2 *v = sRing + (size_t)(srcOf(t, d0) % ring) * TB;
+            // unit h of a row: part h % NQ of tile 3 + h / NQ, the first unit of a warp two rows ahead
+            const int h0 = (rank - 1) + (CS - 1) * w, d0 = 3 + h0 / NQ;
+            const long long rowStep = (long long)dir * (bt + 1) * TT;
+            auto unitOf = [&](int h) {
+                const int d = 3 + h / NQ;
+                return (seg ? Lb + tile_off(M, I0, d) : Lf + M.band + ((long long)(I0 - d) * (bt + 1) + d) * TT) +
+                       (h % NQ) * H * TB + r;
+            };
+            const float2 *T = unitOf(h0);
+            int slot = slotBefore(d0);
+            float2 pf[2][H];
+            auto prefetch = [&](int k, float2 (&q)[H]) {
+                if (k < k1 && d0 <= min(bt, k)) {
 #pragma unroll
-                for (int k = 0; k < TB; k += 2) {
-                    const float2 y0 = v[k], y1 = v[k + 1];
-                    df_acc(acc, pf[k].x, pf[k].y, y0.x, y0.y);
-                    df_acc(a2, pf[k + 1].x, pf[k + 1].y, y1.x, y1.y);
+                    for (int i = 0; i < H; ++i) q[i] = __ldg(T + i * TB);
+                }
+                T += rowStep;
+            };
+            const unsigned part = map_rank(smem_u32(sPart), 0), bar0 = map_rank(bars, 0);
+            auto row = [&](int k, float2 (&q)[H]) {
+                if (k - 3 >= k0) {
+                    arrived(rowsIn, threadIdx.x == 0);
+                    ++rowsIn;
+                }
+                const int dmax = min(bt, k);
+                DF acc = {0.f, 0.f}, a2 = {0.f, 0.f};
+                if (d0 <= dmax) {
+                    const float2 *v = sRing + slot * TB + (h0 % NQ) * H;
+#pragma unroll
+                    for (int i = 0; i < H; i += 2) {
+                        const float2 y0 = v[i], y1 = v[i + 1];
+                        df_acc(acc, q[i].x, q[i].y, y0.x, y0.y);
+                        df_acc(a2, q[i + 1].x, q[i + 1].y, y1.x, y1.y);
+                    }
+                }
+                prefetch(k + 2, q);
+                slot = nextSlot(slot);
+                for (int h = h0 + kProdWarps; 3 + h / NQ <= dmax; h += kProdWarps) {
+                    const float2 *L = unitOf(h) + (k - k0) * rowStep;
+                    const float2 *v = sRing + (size_t)((I0 + dir * (k - k0 - 3 - h / NQ)) % ring) * TB + (h % NQ) * H;
+                    acc = df_norm(acc);
+                    a2 = df_norm(a2);
+#pragma unroll
+                    for (int i = 0; i < H; i += 2) {
+                        const float2 l0 = __ldg(L + i * TB), l1 = __ldg(L + (i + 1) * TB), y0 = v[i], y1 = v[i + 1];
+                        df_acc(acc, l0.x, l0.y, y0.x, y0.y);
+                        df_acc(a2, l1.x, l1.y, y1.x, y1.y);
+                    }
                 }
                 acc = df_add(df_norm(acc), df_norm(a2));
-            }
-            for (int d = d0 + kProdWarps; d <= dmax; d += kProdWarps)
-                df_tile_rows(acc, tileOf(t, d), sRing + (size_t)(srcOf(t, d) % ring) * TB, r, 0, TB);
-            prefetch(t + 1);
-            sRed[w * TB + r] = make_float2(acc.hi, acc.lo);
-            __syncthreads();
-            if (w == 0) {
-                DF pv[kCW];
+                float2 *red = sRed + (sums & 1) * kCaseW * kRedLd;
+                red[w * kRedLd + r] = make_float2(acc.hi, acc.lo);
+                __syncthreads();
+                // two rows of the block a warp, a lane a partial
+                const int i = 2 * w + (r >> 4);
+                const float2 p = red[(r & 15) * kRedLd + i];
+                DF v = {p.x, p.y};
 #pragma unroll
-                for (int k = 0; k < kCW; ++k) pv[k] = DF{sRed[k * TB + r].x, sRed[k * TB + r].y};
-                const DF s = df_tree_sum(pv);
-                leaderPart[((q & 1) * CS + rank) * TB + r] = make_float2(s.hi, s.lo);
+                for (int m = 8; m; m >>= 1) v = df_add(v, df_xor(v, m));
+                if ((r & 15) == 0)
+                    send_df(part + (((sums & 3) * CS + rank) * TB + i) * (unsigned)sizeof(float2), v, bar0 + 8 * (sums & 3));
+                ++sums;
+            };
+            prefetch(k0, pf[0]);
+            prefetch(k0 + 1, pf[1]);
+            for (int k = k0; k < k1; k += 2) {
+                row(k, pf[0]);
+                if (k + 1 < k1) row(k + 1, pf[1]);
             }
-            cluster_barrier();
-        } else {
-            // L_{I,I+-1} times the row solved last, split over the warps by k
-            DF acc = {0.f, 0.f};
-            if (dmax >= 1) {
-                const float2 *v = sRing + (size_t)(srcOf(t, 1) % ring) * TB + 4 * w;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) df_acc(acc, pl[k].x, pl[k].y, v[k].x, v[k].y);
-                acc = df_norm(acc);
+            // the last rows
+            for (int n = max(0, k1 - k0 - 3); n < k1 - k0; ++n, ++rowsIn) {
+                arrived(rowsIn, false);
+                __syncthreads();
+                if (threadIdx.x == 0) bar_expect(bars + 8 * (rowsIn & 3), expect);
             }
-            sRed[w * TB + r] = make_float2(acc.hi, acc.lo);
-            cluster_barrier();
-            if (w == 0) {
-                DF v = df_from_double(pb);
-                if (t >= nbc) v = df_mul(v, DF{pd.x, pd.y});
-                DF pv[kCW + CS];  // the leader's warps' partials, then the producers' (slot CS: zero)
+        } else if (w >= kCW) {
+            const int uw = w - kCW;
+            struct Ops {
+                float2 w[4], d;
+                double b;
+            } op[2];
+            const float2 *Wt = (seg ? Wb : Wf) + wOff + (size_t)I0 * TT + 4 * uw * TB + r;
+            const float2 *dt = Dinv + M.xUnit + (size_t)I0 * TB + 4 * uw + (r & 3);
+            const double *bt_ = Xp + (size_t)I0 * TB + 4 * uw + (r & 3);
+            auto prefetch = [&](int k, Ops &q) {
+                if (k < k1) {
 #pragma unroll
-                for (int k = 0; k < kCW; ++k) pv[k] = DF{sRed[k * TB + r].x, sRed[k * TB + r].y};
-                pv[kCW] = DF{0.f, 0.f};
+                    for (int i = 0; i < 4; ++i) q.w[i] = __ldg(Wt + i * TB);
+                    q.b = *bt_;
+                    if (seg) q.d = __ldg(dt);
+                }
+                Wt += dir * TT;
+                dt += dir * TB;
+                bt_ += dir * TB;
+            };
+            auto row = [&](int k, Ops &q) {
+                DF v = df_from_double(q.b);
+                if (seg) v = df_mul(v, DF{q.d.x, q.d.y});
+                arrived(sums, threadIdx.x == kCW * 32);
+                DF pv[CS];
+                pv[0] = DF{0.f, 0.f};
 #pragma unroll
                 for (int c = 1; c < CS; ++c) {
-                    const float2 pc = sPart[((q & 1) * CS + c) * TB + r];
-                    pv[kCW + c] = DF{pc.x, pc.y};
+                    const float2 pc = sPart[((sums & 3) * CS + c) * TB + 4 * uw + (r & 3)];
+                    pv[c] = DF{pc.x, pc.y};
                 }
                 v = df_sub(v, df_tree_sum(pv));
-                sV[r] = make_float2(v.hi, v.lo);
-            }
-            __syncthreads();
-            // y_I = W v (forward) or x_I = W^T v (backward), split over the warps by k
-            DF a = {0.f, 0.f};
+                DF a = {0.f, 0.f};
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float2 vk = sV[4 * w + k];
-                df_acc(a, pw[k].x, pw[k].y, vk.x, vk.y);
-            }
-            a = df_norm(a);
-            sRed[w * TB + r] = make_float2(a.hi, a.lo);
-            __syncthreads();
-            if (w == 0) {
-                DF pv[kCW];
+                for (int i = 0; i < 4; ++i)
+                    df_acc(a, q.w[i].x, q.w[i].y, __shfl_sync(0xffffffffu, v.hi, i), __shfl_sync(0xffffffffu, v.lo, i));
+                a = df_norm(a);
+                float2 *red = sRed + (kCaseW + (sums & 1) * kCW) * kRedLd;
+                red[uw * kRedLd + r] = make_float2(a.hi, a.lo);
+                prefetch(k + 2, q);
+                stage_barrier<kCW>(2);
+                const int i = 4 * uw + (r >> 3);
+                const float2 p = red[(r & 7) * kRedLd + i];
+                a = DF{p.x, p.y};
 #pragma unroll
-                for (int k = 0; k < kCW; ++k) pv[k] = DF{sRed[k * TB + r].x, sRed[k * TB + r].y};
-                const DF y = df_tree_sum(pv);
-                const float2 yv = make_float2(y.hi, y.lo);
-                const size_t slot = (size_t)(I % ring) * TB + r;
-                for (int c = 0; c < CS; ++c) cl.map_shared_rank(sRing, c)[slot] = yv;
-                Xp[(size_t)I * TB + r] = df_to_double(y);
+                for (int m = 4; m; m >>= 1) a = df_add(a, df_xor(a, m));
+                if ((r & 7) == 0) sU[(sums & 3) * TB + i] = make_float2(a.hi, a.lo);
+                __syncwarp();
+                if (r == 0) bar_arrive(bars + 32 + 8 * (sums & 3));
+                ++sums;
+            };
+            prefetch(k0, op[0]);
+            prefetch(k0 + 1, op[1]);
+            for (int k = k0; k < k1; k += 2) {
+                row(k, op[0]);
+                if (k + 1 < k1) row(k + 1, op[1]);
             }
-            prefetch(t + 1);  // after the row's store: the first backward row reads it back
+        } else {
+            // warps 0 .. 3 the columns C w .. of M1, 4 .. 7 of M2
+            const int d = 1 + w / 4, c0 = C * (w & 3), lane8 = r & 7, i = 4 * w + (r >> 3);
+            const float2 *T = Mx + (size_t)(2 * seg + d - 1) * mS + wOff + (size_t)I0 * TT + c0 * TB + r;
+            float2 pm[2][C];
+            auto prefetch = [&](int k, float2 (&q)[C]) {
+                if (k < k1 && d <= min(bt, k)) {
+#pragma unroll
+                    for (int j = 0; j < C; ++j) q[j] = __ldg(T + j * TB);
+                }
+                T += dir * TT;
+            };
+            // a lane of an entry's eight sends it to a CTA
+            const unsigned ringTo = map_rank(smem_u32(sRing), lane8 < CS ? lane8 : 0) + i * (unsigned)sizeof(float2),
+                           barTo = map_rank(bars, lane8 < CS ? lane8 : 0);
+            int from = slotBefore(d), slot = slotBefore(0);
+            double *xp = Xp + (size_t)I0 * TB + i;
+            auto row = [&](int k, float2 (&q)[C]) {
+                DF acc = {0.f, 0.f}, a2 = {0.f, 0.f};
+                if (d <= min(bt, k)) {
+                    const float2 *v = sRing + from * TB + c0;
+#pragma unroll
+                    for (int j = 0; j < C; j += 2) {
+                        const float2 v0 = v[j], v1 = v[j + 1];
+                        df_acc(acc, q[j].x, q[j].y, v0.x, v0.y);
+                        df_acc(a2, q[j + 1].x, q[j + 1].y, v1.x, v1.y);
+                    }
+                    acc = df_add(df_norm(acc), df_norm(a2));
+                }
+                sRed[w * kRedLd + r] = make_float2(acc.hi, acc.lo);
+                stage_barrier<kCW>(1);
+                const float2 p = sRed[lane8 * kRedLd + i];
+                DF y = {p.x, p.y};
+#pragma unroll
+                for (int m = 4; m; m >>= 1) y = df_add(y, df_xor(y, m));
+                wait(bars + 32, sums);  // u of this row
+                const float2 u = sU[(sums & 3) * TB + i];
+                y = df_sub(DF{u.x, u.y}, y);
+                if (lane8 == 0) sRing[slot * TB + i] = make_float2(y.hi, y.lo);
+                else if (lane8 < CS) send_df(ringTo + slot * kRow, y, barTo + 8 * (rowsIn & 3));
+                stage_barrier<kCW>(1);
+                if (lane8 == 0) *xp = df_to_double(y);
+                xp += dir * TB;
+                prefetch(k + 2, q);
+                from = nextSlot(from);
+                slot = nextSlot(slot);
+                ++rowsIn;
+                ++sums;
+            };
+            prefetch(k0, pm[0]);
+            prefetch(k0 + 1, pm[1]);
+            for (int k = k0; k < k1; k += 2) {
+                row(k, pm[0]);
+                if (k + 1 < k1) row(k + 1, pm[1]);
+            }
         }
-        // the forward sweep's last rows are pushed before the backward sweep, and every row
-        // before any CTA exits
-        if (t == nbc - 1 || t == t1 - 1) cluster_barrier();
     }
+    if (sDead) __nanosleep(1000000);  // (stores of the others still on their way)
+    cluster_barrier();
 }
 
 // internal-layout columns (nrhs x n) <-> the padded panel layout
@@ -1837,7 +2053,7 @@ int plan_build(astro_ctx *ctx, PanelPlan &L, int cs) {
 void plan_free(PanelPlan *L) {
     DevBuf *b[] = {&L->d_meta,  &L->d_sched, &L->d_schedPtr, &L->d_panelOf, &L->d_pos,  &L->d_band,
                    &L->d_status, &L->d_penI, &L->d_penJ,     &L->d_penV,    &L->d_slices, &L->d_sexp,
-                   &L->d_Lf,    &L->d_Lb,    &L->d_Wf,       &L->d_Wb,      &L->d_Dinv,  &L->d_items,
+                   &L->d_Lf,    &L->d_Lb,    &L->d_Wf,       &L->d_Wb,      &L->d_Dinv,  &L->d_items, &L->d_Mx, &L->d_twMx,
                    &L->d_X,     &L->d_twMeta, &L->d_twBand, &L->d_twAw,  &L->d_twSched, &L->d_twSchedPtr,
                    &L->d_twStatus, &L->d_twLf, &L->d_twLb, &L->d_twWf, &L->d_twWb, &L->d_twDinv,
                    &L->d_twItems, &L->d_twX, &L->d_sRef, &L->d_sVec, &L->d_sRes, &L->d_sBi, &L->d_sX,
@@ -2151,7 +2367,7 @@ int panels_cases_prepare(astro_ctx *ctx, int ncols, size_t *bytes) {
     int rc;
     L->twist = twist_wanted(ctx, L);
     L->ring = L->maxBt + 2;
-    const size_t smem = sizeof(float2) * ((size_t)L->ring * TB + kCW * TB + 2 * 8 * TB + TB);
+    const size_t smem = cases_smem(L->ring, 8);
     if (L->twist) {
         if ((L->twGen != L->factorGen || L->twCols != ncols) && (rc = twist_prepare(ctx, L, ncols))) return rc;
         L->factorSeconds = L->twFactorSeconds;
@@ -2163,6 +2379,16 @@ int panels_cases_prepare(astro_ctx *ctx, int ncols, size_t *bytes) {
     }
     if (!L->factored) return set_err(ctx, ASTRO_ERR_STATE, "panels: no current factorisation (astro_panels_factor)");
     if ((rc = panels_df_copies(ctx, L))) return rc;
+    if (L->mGen != L->factorGen) {
+        const size_t mS = (size_t)L->xRows * TB;
+        long long cols = 0;
+        for (const PanelMeta &M : L->meta) cols += M.nbc;
+        if ((rc = grow(ctx, L->d_Mx, sizeof(float2) * 4 * mS))) return rc;
+        k_band_mprep<<<(unsigned)((cols + kPrepW - 1) / kPrepW), kPrepW * 32, 0, s>>>(
+            dptr<PanelMeta>(L->d_meta), L->np, dptr<double>(L->d_band), dptr<float2>(L->d_Mx), mS);
+        if ((rc = cuda_check(ctx, cudaGetLastError(), "panels cases prepare"))) return rc;
+        L->mGen = L->factorGen;
+    }
     if (L->casesCols != ncols) {
         std::vector<CaseItem> items;
         for (int p = 0; p < L->np; ++p)
@@ -2266,12 +2492,14 @@ static int twist_prepare(astro_ctx *ctx, PanelPlan *L, int ncols) {
         (rc = dev_alloc(ctx, L->d_twLb, sizeof(float2) * (size_t)band)) ||
         (rc = dev_alloc(ctx, L->d_twWf, sizeof(float2) * nd * TB)) ||
         (rc = dev_alloc(ctx, L->d_twWb, sizeof(float2) * nd * TB)) ||
+        (rc = dev_alloc(ctx, L->d_twMx, sizeof(float2) * 4 * nd * TB)) ||
         (rc = dev_alloc(ctx, L->d_twDinv, sizeof(float2) * nd)))
         return rc;
     const long long cols = (long long)nbcT + nbcB + m;
     k_band_dfprep<<<(unsigned)((cols + kPrepW - 1) / kPrepW), kPrepW * 32, 0, s>>>(
         dm, 3, db, dptr<float2>(L->d_twLf), dptr<float2>(L->d_twLb), dptr<float2>(L->d_twWf), dptr<float2>(L->d_twWb),
         dptr<float2>(L->d_twDinv));
+    k_band_mprep<<<(unsigned)((cols + kPrepW - 1) / kPrepW), kPrepW * 32, 0, s>>>(dm, 3, db, dptr<float2>(L->d_twMx), nd * TB);
     if ((rc = cuda_check(ctx, cudaGetLastError(), "twisted double-float copy"))) return rc;
     // items: forward T and B, the window, backward T and B (from the row before the window)
     std::vector<CaseItem> items;
@@ -2323,8 +2551,8 @@ int panels_cases_solve(astro_ctx *ctx, double *d_vec, cudaStream_t s) {
         auto sweep = [&](int first, int count) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3((unsigned)(count * cs));
-            cfg.blockDim = dim3(kCW * 32);
-            cfg.dynamicSmemBytes = sizeof(float2) * ((size_t)L->ring * TB + kCW * TB + 2 * cs * TB + TB);
+            cfg.blockDim = dim3(kCaseW * 32);
+            cfg.dynamicSmemBytes = cases_smem(L->ring, cs);
             cfg.stream = s;
             cudaLaunchAttribute at[1];
             at[0].id = cudaLaunchAttributeClusterDimension;
@@ -2337,7 +2565,8 @@ int panels_cases_solve(astro_ctx *ctx, double *d_vec, cudaStream_t s) {
             return cudaLaunchKernelEx(&cfg, kern, dm, (const CaseItem *)dptr<CaseItem>(L->d_twItems) + first,
                                       (const float2 *)dptr<float2>(L->d_twLf), (const float2 *)dptr<float2>(L->d_twLb),
                                       (const float2 *)dptr<float2>(L->d_twWf), (const float2 *)dptr<float2>(L->d_twWb),
-                                      (const float2 *)dptr<float2>(L->d_twDinv), X, nc, L->ring);
+                                      (const float2 *)dptr<float2>(L->d_twMx), (size_t)L->twRows * TB,
+                                      (const float2 *)dptr<float2>(L->d_twDinv), X, nc, L->ring, dptr<int>(L->d_status));
         };
         k_tw_move<<<mg, 256, 0, s>>>(nc, G, w, d_vec, dptr<int>(L->d_pos), dm, X, 0);
         CK(sweep(0, 2 * nc));
@@ -2352,8 +2581,8 @@ int panels_cases_solve(astro_ctx *ctx, double *d_vec, cudaStream_t s) {
                                     dptr<PanelMeta>(L->d_meta), dptr<double>(L->d_X), 1);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(L->np * nc * cs));
-    cfg.blockDim = dim3(kCW * 32);
-    cfg.dynamicSmemBytes = sizeof(float2) * ((size_t)L->ring * TB + kCW * TB + 2 * cs * TB + TB);
+    cfg.blockDim = dim3(kCaseW * 32);
+    cfg.dynamicSmemBytes = cases_smem(L->ring, cs);
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -2366,11 +2595,22 @@ int panels_cases_solve(astro_ctx *ctx, double *d_vec, cudaStream_t s) {
     CK(cudaLaunchKernelEx(&cfg, kern, (const PanelMeta *)dptr<PanelMeta>(L->d_meta),
                           (const CaseItem *)dptr<CaseItem>(L->d_items), (const float2 *)dptr<float2>(L->d_Lf),
                           (const float2 *)dptr<float2>(L->d_Lb), (const float2 *)dptr<float2>(L->d_Wf),
-                          (const float2 *)dptr<float2>(L->d_Wb), (const float2 *)dptr<float2>(L->d_Dinv),
-                          dptr<double>(L->d_X), nc, L->ring));
+                          (const float2 *)dptr<float2>(L->d_Wb), (const float2 *)dptr<float2>(L->d_Mx),
+                          (size_t)L->xRows * TB, (const float2 *)dptr<float2>(L->d_Dinv), dptr<double>(L->d_X), nc, L->ring, dptr<int>(L->d_status)));
     k_panel_move<<<mg, 256, 0, s>>>(P.n, P.dpn, nc, d_vec, dptr<int>(L->d_panelOf), dptr<int>(L->d_pos),
                                     dptr<PanelMeta>(L->d_meta), dptr<double>(L->d_X), 0);
     return cuda_check(ctx, cudaGetLastError(), "panels cases solve");
+}
+
+// Whether a wait of the solves since the last call was given up (waits for the stream).
+int panels_cases_status(astro_ctx *ctx, cudaStream_t s) {
+    PanelPlan *L = static_cast<PanelPlan *>(ctx->panels);
+    int st = 0;
+    CK(cudaMemcpyAsync(&st, L->d_status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    if (!st) return ASTRO_OK;
+    CK(cudaMemsetAsync(L->d_status.p, 0, sizeof(int), s));
+    return set_err(ctx, ASTRO_ERR_CUDA, "panels: a wait of the many-column solve was given up");
 }
 
 // Kernel launches of one panels_cases_solve (3, or 7 for the twisted solve).
