@@ -1254,22 +1254,22 @@ __global__ void __launch_bounds__(kThreads, 2) k_band_solve_df(const PanelMeta *
 //   y_I = u_I - M1_I y_{I-1} - M2_I y_{I-2},   u_I = W_I (b_I - sum_{d >= 3} L_{I,I-d} y_{I-d}),
 // so that of a block row only the product with M1_I waits for the row before.  Three stages run side by side, each as
 // far ahead as the rows that it needs allow:
-//   * producer CTAs (ranks 1 .. CS-1), a warp per part of a tile: the sum over d >= 3 for row I + 3 from the
-//     solved rows up to I in their shared-memory ring, reduced across the CTA and sent to the leader;
-//   * the leader's warps 8 .. 15: u_I from those sums;
-//   * the leader's warps 0 .. 7: M1_I y_{I-1} and M2_I y_{I-2}, and y_I, sent to every CTA's ring;
+//   * producer CTAs (ranks 1 .. CS-1), eight warps, half a tile each: the sum over d >= 3 for row I + 3 from
+//     the solved rows up to I in their shared-memory ring, reduced across the CTA and sent to the leader;
+//   * the leader's warp 12: b_I less those sums; warps 8 .. 11: u_I;
+//   * warps 4 .. 7: M2_I y_{I-2}, and rows to X; warps 0 .. 3: M1_I y_{I-1} and y_I, sent to every CTA's ring;
 //   * backward sweep the same with L^T (transposed copies of the tiles and of W, M) on D^-1 y.
 // Rows and sums travel as asynchronous stores into the other CTA's shared memory that count on a barrier
 // there (mbarrier; four in turn: a stage is at most three rows ahead of another).  With a cluster barrier
-// per row its release alone took 1,000 clocks, and the sums by one warp as long (instruction fetch); now
-// all warps of a stage share a sum.  What bounds it: the way from a row to the sums three rows on, and the
-// tiles from L2.  25,350 DOF, 13 tiles, 17 cases in four CTAs each: half a sweep 445 us (with
-// one chain per row and a cluster barrier 665).
+// per row its release alone took 1,000 clocks, and the sums by one warp as long (instruction fetch); with
+// sixteen warps to a stage the sums' instructions and the conversions (FP64 pipe) bound the row.  25,350
+// DOF, 13 tiles, 17 cases in four CTAs each: half a sweep 320 us (with one chain per row and a cluster
+// barrier 665, with sixteen warps 445).
 // The band is copied once into double-float tiles in the forward (column-major) and backward
 // (row-major) layouts, so every tile load of a warp is 32 consecutive float2 per k.
-constexpr int kCW = 8;   // warps of u's stage (the CTAs per cluster, CS, is a template parameter: 2, 4 or 8)
-constexpr int kCaseW = 2 * kCW;  // warps per CTA
-constexpr int kCaseWait = 1 << 20;  // polls of a barrier (about a second), then the status is set and waits skipped
+constexpr int kCW = 4;      // warps of a leader's product (the CTAs per cluster, CS, is a template parameter: 2, 4 or 8)
+constexpr int kCaseW = 16;  // warps per CTA
+constexpr int kCaseWait = 1 << 24;  // polls of a barrier (about a second or less), then the status is set and waits skipped
 constexpr int kPrepW = 4;  // warps per CTA of the band copy
 
 struct CaseItem {
@@ -1468,14 +1468,22 @@ __device__ __forceinline__ void bar_arrive(unsigned bar) { asm volatile("mbarrie
 __device__ __forceinline__ void bar_expect(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity) {
+// (test_wait: the threads that wait have nothing else to do, and try_wait's sleep costs 40 us of a half sweep)
+template <bool CLUSTER> __device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity, const int *dead) {
     for (int it = 0; it < kCaseWait; ++it) {
         unsigned ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok)
-                     : "r"(bar), "r"(parity), "r"(1000)  // (a poll sleeps for a microsecond at most)
-                     : "memory");
+        if constexpr (CLUSTER)
+            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                         : "=r"(ok)
+                         : "r"(bar), "r"(parity)
+                         : "memory");
+        else
+            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                         : "=r"(ok)
+                         : "r"(bar), "r"(parity)
+                         : "memory");
         if (ok) return true;
+        if ((it & 1023) == 1023 && *(volatile const int *)dead) return true;  // given up elsewhere: no more waits
     }
     return false;
 }
@@ -1488,9 +1496,13 @@ __device__ __forceinline__ DF df_xor(DF v, int m) {
 
 constexpr int kRedLd = TB + 1;  // row stride of the partials: a warp reads them by column
 
-// Bytes of dynamic shared memory.
+constexpr int kCasePW = 8;  // producers' warps of a CTA, half a tile each: with 13 tiles, 24 have one at most
+
+// Bytes of dynamic shared memory: a producer has the ring and its partials, the leader the last rows, sums, u, v
+// and its partials.
 static size_t cases_smem(int ring, int cs) {
-    return sizeof(float2) * ((size_t)TB * (ring + 4 * cs + 4) + 2 * kCaseW * kRedLd);
+    const size_t prod = (size_t)TB * ring + 2 * kCasePW * kRedLd, lead = (size_t)TB * (8 + 4 * cs + 8) + 7 * kCW * kRedLd;
+    return sizeof(float2) * std::max(prod, lead);
 }
 
 template <int CS>
@@ -1503,18 +1515,20 @@ __global__ void __launch_bounds__(kCaseW * 32, 1) k_band_solve_cases(const Panel
                                                                      const float2 *__restrict__ Mx, size_t mS,
                                                                      const float2 *__restrict__ Dinv, double *X, int nrhs,
                                                                      int ring, int *status) {
-    // parts of a tile that the producers' warps take: with 13 tiles, 48 warps and more have a part at most
-    constexpr int NQ = CS == 2 ? 2 : 4;
-    constexpr int kProdWarps = (CS - 1) * kCaseW, H = TB / NQ, C = TB / 4;
+    constexpr int PW = kCasePW;
+    constexpr int kProdWarps = (CS - 1) * PW, H = TB / 2, C = TB / kCW;
     constexpr unsigned kRow = TB * sizeof(float2);
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
     extern __shared__ float2 smf[];
-    float2 *sRing = smf;                       // [ring][TB]: solved rows
-    float2 *sPart = sRing + (size_t)ring * TB; // [4][CS][TB]: the producers' sums (leader)
-    float2 *sU = sPart + 4 * CS * TB;          // [4][TB]
-    float2 *sRed = sU + 4 * TB;                // [2][kCaseW][kRedLd]: partials (leader: y's stage, then u's)
-    __shared__ __align__(8) unsigned long long sBar[8];  // rows (producers), sums (leader); u (leader)
+    // producers: [ring][TB] solved rows, [2][PW][kRedLd] partials
+    float2 *sRing = smf, *sRed = sRing + (size_t)ring * TB;
+    // the leader: [8][TB] last rows, [4][CS][TB] sums, [4][TB] u, [4][TB] v, [kCW][kRedLd] partials of M1, [4][kCW] of
+    // M2, [2][kCW] of W
+    float2 *sPart = smf + 8 * TB, *sU = sPart + 4 * CS * TB, *sV = sU + 4 * TB;
+    if (rank == 0) sRed = sV + 4 * TB;
+    // four barriers in turn each: rows (producers) or sums (leader); u, v, M2's partials, rows in the leader
+    __shared__ __align__(8) unsigned long long sBar[20];
     __shared__ int sDead;                      // a wait was given up
     const CaseItem it = items[blockIdx.x / CS];
     const PanelMeta M = meta[it.panel];
@@ -1525,19 +1539,20 @@ __global__ void __launch_bounds__(kCaseW * 32, 1) k_band_solve_cases(const Panel
     const unsigned bars = smem_u32(sBar), expect = rank > 0 ? kRow : (CS - 1) * kRow;
     if (threadIdx.x == 0) {
         sDead = 0;
-        for (int k = 0; k < 8; ++k) bar_init(bars + 8 * k, k < 4 ? 1 : kCW);
+        for (int k = 0; k < 20; ++k) bar_init(bars + 8 * k, k < 4 || (k >= 8 && k < 12) ? 1 : kCW);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         for (int k = 0; k < 4; ++k) bar_expect(bars + 8 * k, expect);
     }
     // arrival number n of rows (sums), and the arming of number n + 4 by one thread
-    auto wait = [&](unsigned bar, int n) {
-        if (!sDead && !bar_wait(bar + 8 * (n & 3), (n >> 2) & 1)) {
-            sDead = 1;
-            atomicExch(status, -1);
-        }
+    auto gaveUp = [&] {
+        if (!sDead) atomicExch(status, -1);
+        sDead = 1;
+    };
+    auto wait = [&](unsigned bar, int n) {  // for a stage of this CTA
+        if (!bar_wait<false>(bar + 8 * (n & 3), (n >> 2) & 1, &sDead)) gaveUp();
     };
     auto arrived = [&](int n, bool arm) {
-        wait(bars, n);
+        if (!bar_wait<true>(bars + 8 * (n & 3), (n >> 2) & 1, &sDead)) gaveUp();
         if (arm) bar_expect(bars + 8 * (n & 3), expect);
     };
     // step t = 0 .. 2 nbc - 1: forward rows I = t, then backward rows I = 2 nbc - 1 - t.  Row k of a sweep
@@ -1552,36 +1567,39 @@ __global__ void __launch_bounds__(kCaseW * 32, 1) k_band_solve_cases(const Panel
         // a backward sweep that starts below the last row (the rows after it solved already, in X):
         // those rows into every CTA's ring
         if (seg && k0 > 0) {
-            for (int R = I0 + 1 + w; R <= min(nbc - 1, I0 + bt); R += kCaseW) {
+            for (int R = I0 + 1 + w; R <= min(nbc - 1, I0 + (rank ? bt : 2)); R += kCaseW) {
                 const DF v = df_from_double(Xp[(size_t)R * TB + r]);
-                sRing[(size_t)(R % ring) * TB + r] = make_float2(v.hi, v.lo);
+                sRing[(size_t)(rank ? R % ring : (k0 + I0 - R) & 7) * TB + r] = make_float2(v.hi, v.lo);
             }
         }
         cluster_barrier();
         // the slot of the row d before I0, and the one after slot s
         auto slotBefore = [&](int d) { return (I0 - dir * d + 2 * ring * nbc) % ring; };
         auto nextSlot = [&](int s) { return dir > 0 ? (s + 1 < ring ? s + 1 : 0) : (s > 0 ? s - 1 : ring - 1); };
-        if (rank > 0) {
-            // unit h of a row: part h % NQ of tile 3 + h / NQ, the first unit of a warp two rows ahead
-            const int h0 = (rank - 1) + (CS - 1) * w, d0 = 3 + h0 / NQ;
+        const unsigned barU = bars + 32, barV = bars + 64, barM = bars + 96, barY = bars + 128;
+        if (rank > 0 && w < PW) {
+            // unit h of a row: half h % 2 of tile 3 + h / 2, the first unit of a warp a row ahead
+            const int h0 = (rank - 1) + (CS - 1) * w, d0 = 3 + h0 / 2;
             const long long rowStep = (long long)dir * (bt + 1) * TT;
             auto unitOf = [&](int h) {
-                const int d = 3 + h / NQ;
+                const int d = 3 + h / 2;
                 return (seg ? Lb + tile_off(M, I0, d) : Lf + M.band + ((long long)(I0 - d) * (bt + 1) + d) * TT) +
-                       (h % NQ) * H * TB + r;
+                       (h % 2) * H * TB + r;
             };
             const float2 *T = unitOf(h0);
             int slot = slotBefore(d0);
-            float2 pf[2][H];
-            auto prefetch = [&](int k, float2 (&q)[H]) {
+            float2 pf[H];
+            auto prefetch = [&](int k) {
                 if (k < k1 && d0 <= min(bt, k)) {
 #pragma unroll
-                    for (int i = 0; i < H; ++i) q[i] = __ldg(T + i * TB);
+                    for (int i = 0; i < H; ++i) pf[i] = __ldg(T + i * TB);
                 }
                 T += rowStep;
             };
             const unsigned part = map_rank(smem_u32(sPart), 0), bar0 = map_rank(bars, 0);
-            auto row = [&](int k, float2 (&q)[H]) {
+            const int i = TB / PW * w + r / PW;  // the entry that the lane helps to sum
+            prefetch(k0);
+            for (int k = k0; k < k1; ++k, ++sums) {
                 if (k - 3 >= k0) {
                     arrived(rowsIn, threadIdx.x == 0);
                     ++rowsIn;
@@ -1589,165 +1607,174 @@ __global__ void __launch_bounds__(kCaseW * 32, 1) k_band_solve_cases(const Panel
                 const int dmax = min(bt, k);
                 DF acc = {0.f, 0.f}, a2 = {0.f, 0.f};
                 if (d0 <= dmax) {
-                    const float2 *v = sRing + slot * TB + (h0 % NQ) * H;
+                    const float2 *v = sRing + slot * TB + (h0 % 2) * H;
 #pragma unroll
-                    for (int i = 0; i < H; i += 2) {
-                        const float2 y0 = v[i], y1 = v[i + 1];
-                        df_acc(acc, q[i].x, q[i].y, y0.x, y0.y);
-                        df_acc(a2, q[i + 1].x, q[i + 1].y, y1.x, y1.y);
+                    for (int j = 0; j < H; j += 2) {
+                        const float2 y0 = v[j], y1 = v[j + 1];
+                        df_acc(acc, pf[j].x, pf[j].y, y0.x, y0.y);
+                        df_acc(a2, pf[j + 1].x, pf[j + 1].y, y1.x, y1.y);
                     }
                 }
-                prefetch(k + 2, q);
+                prefetch(k + 1);
                 slot = nextSlot(slot);
-                for (int h = h0 + kProdWarps; 3 + h / NQ <= dmax; h += kProdWarps) {
+                for (int h = h0 + kProdWarps; 3 + h / 2 <= dmax; h += kProdWarps) {
                     const float2 *L = unitOf(h) + (k - k0) * rowStep;
-                    const float2 *v = sRing + (size_t)((I0 + dir * (k - k0 - 3 - h / NQ)) % ring) * TB + (h % NQ) * H;
+                    const float2 *v = sRing + (size_t)((I0 + dir * (k - k0 - 3 - h / 2)) % ring) * TB + (h % 2) * H;
                     acc = df_norm(acc);
                     a2 = df_norm(a2);
-#pragma unroll
-                    for (int i = 0; i < H; i += 2) {
-                        const float2 l0 = __ldg(L + i * TB), l1 = __ldg(L + (i + 1) * TB), y0 = v[i], y1 = v[i + 1];
+#pragma unroll 4
+                    for (int j = 0; j < H; j += 2) {
+                        const float2 l0 = __ldg(L + j * TB), l1 = __ldg(L + (j + 1) * TB), y0 = v[j], y1 = v[j + 1];
                         df_acc(acc, l0.x, l0.y, y0.x, y0.y);
                         df_acc(a2, l1.x, l1.y, y1.x, y1.y);
                     }
                 }
                 acc = df_add(df_norm(acc), df_norm(a2));
-                float2 *red = sRed + (sums & 1) * kCaseW * kRedLd;
+                float2 *red = sRed + (sums & 1) * PW * kRedLd;
                 red[w * kRedLd + r] = make_float2(acc.hi, acc.lo);
-                __syncthreads();
-                // two rows of the block a warp, a lane a partial
-                const int i = 2 * w + (r >> 4);
-                const float2 p = red[(r & 15) * kRedLd + i];
+                stage_barrier<PW>(1);
+                const float2 p = red[(r % PW) * kRedLd + i];
                 DF v = {p.x, p.y};
 #pragma unroll
-                for (int m = 8; m; m >>= 1) v = df_add(v, df_xor(v, m));
-                if ((r & 15) == 0)
+                for (int m = PW / 2; m; m >>= 1) v = df_add(v, df_xor(v, m));
+                if (r % PW == 0)
                     send_df(part + (((sums & 3) * CS + rank) * TB + i) * (unsigned)sizeof(float2), v, bar0 + 8 * (sums & 3));
-                ++sums;
-            };
-            prefetch(k0, pf[0]);
-            prefetch(k0 + 1, pf[1]);
-            for (int k = k0; k < k1; k += 2) {
-                row(k, pf[0]);
-                if (k + 1 < k1) row(k + 1, pf[1]);
             }
             // the last rows
             for (int n = max(0, k1 - k0 - 3); n < k1 - k0; ++n, ++rowsIn) {
                 arrived(rowsIn, false);
-                __syncthreads();
+                stage_barrier<PW>(1);
                 if (threadIdx.x == 0) bar_expect(bars + 8 * (rowsIn & 3), expect);
             }
-        } else if (w >= kCW) {
-            const int uw = w - kCW;
-            struct Ops {
-                float2 w[4], d;
-                double b;
-            } op[2];
-            const float2 *Wt = (seg ? Wb : Wf) + wOff + (size_t)I0 * TT + 4 * uw * TB + r;
-            const float2 *dt = Dinv + M.xUnit + (size_t)I0 * TB + 4 * uw + (r & 3);
-            const double *bt_ = Xp + (size_t)I0 * TB + 4 * uw + (r & 3);
-            auto prefetch = [&](int k, Ops &q) {
+        } else if (rank == 0 && w == 3 * kCW) {
+            // v = b (D^-1 b backward) less the producers' sums
+            const float2 *dt = Dinv + M.xUnit + (size_t)I0 * TB + r;
+            const double *xb = Xp + (size_t)I0 * TB + r;
+            double b = 0.0;
+            float2 d = make_float2(0.f, 0.f);
+            auto prefetch = [&](int k) {
                 if (k < k1) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) q.w[i] = __ldg(Wt + i * TB);
-                    q.b = *bt_;
-                    if (seg) q.d = __ldg(dt);
+                    b = *xb;
+                    if (seg) d = __ldg(dt);
                 }
-                Wt += dir * TT;
                 dt += dir * TB;
-                bt_ += dir * TB;
+                xb += dir * TB;
             };
-            auto row = [&](int k, Ops &q) {
-                DF v = df_from_double(q.b);
-                if (seg) v = df_mul(v, DF{q.d.x, q.d.y});
-                arrived(sums, threadIdx.x == kCW * 32);
+            prefetch(k0);
+            for (int k = k0; k < k1; ++k, ++sums) {
+                DF v = df_from_double(b);
+                if (seg) v = df_mul(v, DF{d.x, d.y});
+                prefetch(k + 1);
+                arrived(sums, r == 0);
                 DF pv[CS];
                 pv[0] = DF{0.f, 0.f};
 #pragma unroll
                 for (int c = 1; c < CS; ++c) {
-                    const float2 pc = sPart[((sums & 3) * CS + c) * TB + 4 * uw + (r & 3)];
+                    const float2 pc = sPart[((sums & 3) * CS + c) * TB + r];
                     pv[c] = DF{pc.x, pc.y};
                 }
                 v = df_sub(v, df_tree_sum(pv));
-                DF a = {0.f, 0.f};
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    df_acc(a, q.w[i].x, q.w[i].y, __shfl_sync(0xffffffffu, v.hi, i), __shfl_sync(0xffffffffu, v.lo, i));
-                a = df_norm(a);
-                float2 *red = sRed + (kCaseW + (sums & 1) * kCW) * kRedLd;
-                red[uw * kRedLd + r] = make_float2(a.hi, a.lo);
-                prefetch(k + 2, q);
-                stage_barrier<kCW>(2);
-                const int i = 4 * uw + (r >> 3);
-                const float2 p = red[(r & 7) * kRedLd + i];
-                a = DF{p.x, p.y};
-#pragma unroll
-                for (int m = 4; m; m >>= 1) a = df_add(a, df_xor(a, m));
-                if ((r & 7) == 0) sU[(sums & 3) * TB + i] = make_float2(a.hi, a.lo);
+                sV[(sums & 3) * TB + r] = make_float2(v.hi, v.lo);
                 __syncwarp();
-                if (r == 0) bar_arrive(bars + 32 + 8 * (sums & 3));
-                ++sums;
-            };
-            prefetch(k0, op[0]);
-            prefetch(k0 + 1, op[1]);
-            for (int k = k0; k < k1; k += 2) {
-                row(k, op[0]);
-                if (k + 1 < k1) row(k + 1, op[1]);
+                if (r == 0) bar_arrive(barV + 8 * (sums & 3));
             }
-        } else {
-            // warps 0 .. 3 the columns C w .. of M1, 4 .. 7 of M2
-            const int d = 1 + w / 4, c0 = C * (w & 3), lane8 = r & 7, i = 4 * w + (r >> 3);
-            const float2 *T = Mx + (size_t)(2 * seg + d - 1) * mS + wOff + (size_t)I0 * TT + c0 * TB + r;
-            float2 pm[2][C];
-            auto prefetch = [&](int k, float2 (&q)[C]) {
-                if (k < k1 && d <= min(bt, k)) {
+        } else if (rank == 0 && w < 3 * kCW) {
+            // products: kind 0 M1 (then y), 1 M2 (and the rows to X), 2 W; columns c0 .. c0 + C - 1 of it
+            const int kind = w / kCW, c0 = C * (w % kCW), d = kind + 1, l = r & 3, i = C * (w % kCW) + r / 4;
+            const float2 *T = (kind < 2 ? Mx + (size_t)(2 * seg + kind) * mS : (seg ? Wb : Wf)) + wOff + (size_t)I0 * TT +
+                              c0 * TB + r;
+            float2 pm[C];
+            auto prefetch = [&](int k) {
+                if (k < k1 && (kind == 2 || d <= min(bt, k))) {
 #pragma unroll
-                    for (int j = 0; j < C; ++j) q[j] = __ldg(T + j * TB);
+                    for (int j = 0; j < C; ++j) pm[j] = __ldg(T + j * TB);
                 }
                 T += dir * TT;
             };
-            // a lane of an entry's eight sends it to a CTA
-            const unsigned ringTo = map_rank(smem_u32(sRing), lane8 < CS ? lane8 : 0) + i * (unsigned)sizeof(float2),
-                           barTo = map_rank(bars, lane8 < CS ? lane8 : 0);
-            int from = slotBefore(d), slot = slotBefore(0);
-            double *xp = Xp + (size_t)I0 * TB + i;
-            auto row = [&](int k, float2 (&q)[C]) {
+            // the warp's columns times v
+            auto product = [&](const float2 *v) {
                 DF acc = {0.f, 0.f}, a2 = {0.f, 0.f};
-                if (d <= min(bt, k)) {
-                    const float2 *v = sRing + from * TB + c0;
 #pragma unroll
-                    for (int j = 0; j < C; j += 2) {
-                        const float2 v0 = v[j], v1 = v[j + 1];
-                        df_acc(acc, q[j].x, q[j].y, v0.x, v0.y);
-                        df_acc(a2, q[j + 1].x, q[j + 1].y, v1.x, v1.y);
-                    }
-                    acc = df_add(df_norm(acc), df_norm(a2));
+                for (int j = 0; j < C; j += 2) {
+                    const float2 v0 = v[j], v1 = v[j + 1];
+                    df_acc(acc, pm[j].x, pm[j].y, v0.x, v0.y);
+                    df_acc(a2, pm[j + 1].x, pm[j + 1].y, v1.x, v1.y);
                 }
-                sRed[w * kRedLd + r] = make_float2(acc.hi, acc.lo);
-                stage_barrier<kCW>(1);
-                const float2 p = sRed[lane8 * kRedLd + i];
-                DF y = {p.x, p.y};
-#pragma unroll
-                for (int m = 4; m; m >>= 1) y = df_add(y, df_xor(y, m));
-                wait(bars + 32, sums);  // u of this row
-                const float2 u = sU[(sums & 3) * TB + i];
-                y = df_sub(DF{u.x, u.y}, y);
-                if (lane8 == 0) sRing[slot * TB + i] = make_float2(y.hi, y.lo);
-                else if (lane8 < CS) send_df(ringTo + slot * kRow, y, barTo + 8 * (rowsIn & 3));
-                stage_barrier<kCW>(1);
-                if (lane8 == 0) *xp = df_to_double(y);
-                xp += dir * TB;
-                prefetch(k + 2, q);
-                from = nextSlot(from);
-                slot = nextSlot(slot);
-                ++rowsIn;
-                ++sums;
+                return df_add(df_norm(acc), df_norm(a2));
             };
-            prefetch(k0, pm[0]);
-            prefetch(k0 + 1, pm[1]);
-            for (int k = k0; k < k1; k += 2) {
-                row(k, pm[0]);
-                if (k + 1 < k1) row(k + 1, pm[1]);
+            float2 *red1 = sRed, *red2 = red1 + kCW * kRedLd, *redU = red2 + 4 * kCW * kRedLd;
+            const int wr = w % kCW;
+            auto last = [&](int k) { return sRing + (k & 7) * TB; };  // row k in the leader
+            prefetch(k0);
+            if (kind == 0) {
+                const unsigned ringA = smem_u32(sRing) + i * (unsigned)sizeof(float2);
+                int slot = slotBefore(0);
+                for (int k = k0; k < k1; ++k, ++sums, ++rowsIn) {
+                    DF acc = {0.f, 0.f};
+                    if (d <= min(bt, k)) acc = product(last(k - d) + c0);
+                    red1[wr * kRedLd + r] = make_float2(acc.hi, acc.lo);
+                    prefetch(k + 1);
+                    wait(barM, sums);
+                    stage_barrier<kCW>(1);
+                    const float2 p = red1[l * kRedLd + i], q = red2[((sums & 3) * kCW + l) * kRedLd + i];
+                    DF y = df_add(DF{p.x, p.y}, DF{q.x, q.y});
+                    y = df_add(y, df_xor(y, 1));
+                    y = df_add(y, df_xor(y, 2));
+                    wait(barU, sums);
+                    const float2 u = sU[(sums & 3) * TB + i];
+                    y = df_sub(DF{u.x, u.y}, y);
+                    // the four lanes of an entry share the CTAs
+                    for (int c = l; c < CS; c += 4) {
+                        if (c == 0) last(k)[i] = make_float2(y.hi, y.lo);
+                        else send_df(map_rank(ringA, c) + slot * kRow, y, map_rank(bars, c) + 8 * (rowsIn & 3));
+                    }
+                    __syncwarp();
+                    if (r == 0) bar_arrive(barY + 8 * (rowsIn & 3));
+                    slot = nextSlot(slot);
+                    stage_barrier<kCW>(1);
+                }
+            } else if (kind == 1) {
+                double *xp = Xp + (size_t)I0 * TB + r;
+                auto store = [&](int k) {  // row k to X
+                    if (wr == 0) {
+                        const float2 y = last(k)[r];
+                        *xp = df_to_double(DF{y.x, y.y});
+                    }
+                    xp += dir * TB;
+                };
+                for (int k = k0; k < k1; ++k, ++sums) {
+                    if (k - 2 >= k0) {
+                        wait(barY, rowsIn);
+                        ++rowsIn;
+                    }
+                    DF acc = {0.f, 0.f};
+                    if (d <= min(bt, k)) acc = product(last(k - d) + c0);
+                    red2[((sums & 3) * kCW + wr) * kRedLd + r] = make_float2(acc.hi, acc.lo);
+                    __syncwarp();
+                    if (r == 0) bar_arrive(barM + 8 * (sums & 3));
+                    prefetch(k + 1);
+                    if (k - 2 >= k0) store(k - 2);
+                }
+                for (int n = max(k0, k1 - 2); n < k1; ++n, ++rowsIn) {
+                    wait(barY, rowsIn);
+                    store(n);
+                }
+            } else {
+                for (int k = k0; k < k1; ++k, ++sums) {
+                    wait(barV, sums);
+                    const DF acc = product(sV + (sums & 3) * TB + c0);
+                    float2 *red = redU + (sums & 1) * kCW * kRedLd;
+                    red[wr * kRedLd + r] = make_float2(acc.hi, acc.lo);
+                    prefetch(k + 1);
+                    stage_barrier<kCW>(2);
+                    const float2 p = red[l * kRedLd + i];
+                    DF u = {p.x, p.y};
+                    u = df_add(u, df_xor(u, 1));
+                    u = df_add(u, df_xor(u, 2));
+                    if (l == 0) sU[(sums & 3) * TB + i] = make_float2(u.hi, u.lo);
+                    __syncwarp();
+                    if (r == 0) bar_arrive(barU + 8 * (sums & 3));
+                }
             }
         }
     }
