@@ -8,7 +8,9 @@
 // the nodal DOF only, while the Gauss-point acceleration includes the bubbles' (the element's
 // gathered state has their displacements and previous displacements, no velocities).
 //
-// One warp per element, FP64 (brickIM is not on a benchmarked workload; the FP64 pipe bounds it):
+// One warp per element, FP64; the FP64 pipe (a warp instruction per 19 clocks and SM, whatever its lanes do)
+// bounds it, so what a few lanes do counts in full: a third round of two pairs and the LU of one lane were a fifth
+// of the kernel (4,125 elements: 885 -> 550 us):
 //   phase 1, lane gp < 8: Jacobian, its inverse, the eleven gradients, the displacement gradient
 //            over the eleven shape functions, Green-Lagrange strain, stress, G = Or + ux^T and the
 //            acceleration at the point;
@@ -16,7 +18,7 @@
 //            Q = w detJ C P, t = w detJ S g and the residual contribution P^T (w detJ stress);
 //   phase 3, the 66 shape-function pairs a <= b over the lanes: the 3x3 blocks of the 33x33
 //            element matrix (material + stress + Newmark mass) in shared memory;
-//   phase 4, condensation: the unpivoted LU of the internal 9x9 block (one lane), then the 24
+//   phase 4, condensation: the unpivoted LU of the internal 9x9 block over the lanes, then the 24
 //            nodal columns in parallel (each column's update reads only the unchanged internal
 //            rows and columns, so the order of the reference's column loop does not matter);
 //   outputs: the condensed 24x24 into the block-CSR matrix (colour-ordered, the first element to
@@ -270,33 +272,38 @@ __global__ void __launch_bounds__(32) hex81_kernel(Hex81Args A) {
     }
     if (!A.build) return;
     // ---- phase 3: pairs a <= b of the 11 shape functions (66) -----------------------------------------
-    double kt[3][10];  // up to three pairs per lane: 9 entries + the diagonal term
+    // two pairs per lane; the last two pairs, with a point per lane, in a tenth of a third round's time
+    double kt[3][10];  // 9 entries + the diagonal term
     int pa[3], pb[3];
+    auto point = [&](int a, int b, int gp, double *k) {
+        const int ia = 11 * gp + a, ib = 11 * gp + b;
+        for (int q = 0; q < 6; ++q)
+            for (int v = 0; v < 3; ++v)
+                for (int x = 0; x < 3; ++x) k[3 * v + x] += S.u.P[ia][3 * q + v] * S.u.Q[ib][3 * q + x];
+        double dg = S.g[gp][a][0] * S.u.t[ib][0] + S.g[gp][a][1] * S.u.t[ib][1] + S.g[gp][a][2] * S.u.t[ib][2];
+        if (a < 8 && b < 8) dg += S.N[gp][a] * S.u.mN[ib];
+        k[9] += dg;
+    };
     for (int k = 0; k < 3; ++k) {
         for (int q = 0; q < 10; ++q) kt[k][q] = 0.0;
-        int t = lane + 32 * k, a = 0;
-        pa[k] = pb[k] = -1;
-        if (t >= 66) continue;
+        int t = k < 2 ? lane + 32 * k : 64 + ((lane >> 3) & 1), a = 0;
         while (t >= 11 - a) {  // row-major upper triangle of the 11 x 11 pairs (t < 66: a stays < 11)
             t -= 11 - a;
             ++a;
         }
         pa[k] = a;
         pb[k] = a + t;
-        for (int gp = 0; gp < 8; ++gp) {
-            const int ia = 11 * gp + pa[k], ib = 11 * gp + pb[k];
-            for (int q = 0; q < 6; ++q)
-                for (int v = 0; v < 3; ++v)
-                    for (int x = 0; x < 3; ++x) kt[k][3 * v + x] += S.u.P[ia][3 * q + v] * S.u.Q[ib][3 * q + x];
-            double dg = S.g[gp][pa[k]][0] * S.u.t[ib][0] + S.g[gp][pa[k]][1] * S.u.t[ib][1] +
-                        S.g[gp][pa[k]][2] * S.u.t[ib][2];
-            if (pa[k] < 8 && pb[k] < 8) dg += S.N[gp][pa[k]] * S.u.mN[ib];
-            kt[k][9] += dg;
+        if (k < 2) {
+            for (int gp = 0; gp < 8; ++gp) point(pa[k], pb[k], gp, kt[k]);
+        } else {
+            point(pa[k], pb[k], lane & 7, kt[k]);
+            for (int q = 0; q < 10; ++q)
+                for (int m = 1; m < 8; m <<= 1) kt[k][q] += __shfl_xor_sync(0xffffffffu, kt[k][q], m);
         }
     }
     __syncwarp();
     for (int k = 0; k < 3; ++k) {
-        if (pa[k] < 0) continue;
+        if (k == 2 && (lane >= 16 || (lane & 7))) continue;
         const int a = pa[k], b = pb[k];
         for (int v = 0; v < 3; ++v)
             for (int x = 0; x < 3; ++x) {
@@ -307,21 +314,35 @@ __global__ void __launch_bounds__(32) hex81_kernel(Hex81Args A) {
     }
     __syncwarp();
     // ---- phase 4: condensation of the nine internal DOF -------------------------------------------
-    if (lane == 0) {
-        double L[9][9];
-        for (int r = 0; r < 9; ++r)
-            for (int cc = 0; cc < 9; ++cc) L[r][cc] = S.K[33 * (24 + cc) + 24 + r];
-        a_lu<double, 9>(&L[0][0], 9);
-        for (int r = 0; r < 9; ++r)
-            for (int cc = 0; cc < 9; ++cc) S.K[33 * (24 + cc) + 24 + r] = L[r][cc];
+    // a_lu's operations, column by column over the lanes; the reciprocals of the pivots kept for the solves
+    double *const L0 = &S.K[33 * 24 + 24];  // entry (r, c) at L0[33 c + r]
+    double f[9];
+    for (int k = 0; k < 9; ++k) {
+        f[k] = 1.0 / L0[33 * k + k];
+        if (lane > k && lane < 9) L0[33 * k + lane] = f[k] * L0[33 * k + lane];
+        __syncwarp();
+        const int m = 8 - k;
+        for (int q = lane; q < m * m; q += 32) {
+            const int r = k + 1 + q % m, c = k + 1 + q / m;
+            L0[33 * c + r] = L0[33 * c + r] - L0[33 * k + r] * L0[33 * c + k];
+        }
+        __syncwarp();
     }
-    __syncwarp();
     if (lane < 24) {
-        double L[9][9], bb[9], x[9];
+        double L[9][9], z[9], x[9];
         for (int r = 0; r < 9; ++r)
-            for (int cc = 0; cc < 9; ++cc) L[r][cc] = S.K[33 * (24 + cc) + 24 + r];
-        for (int k = 0; k < 9; ++k) bb[k] = S.K[33 * lane + 24 + k];
-        a_lu_solve<double, 9>(&L[0][0], bb, x, 9);
+            for (int cc = 0; cc < 9; ++cc) L[r][cc] = L0[33 * cc + r];
+        // a_lu_solve
+        for (int i = 0; i < 9; ++i) {
+            z[i] = S.K[33 * lane + 24 + i];
+            for (int k = 0; k < i; ++k) z[i] = z[i] - L[i][k] * z[k];
+        }
+        x[8] = z[8] / L[8][8];
+        for (int i = 7; i >= 0; --i) {
+            double dp = 0.0;
+            for (int k = i + 1; k < 9; ++k) dp = dp + L[i][k] * x[k];
+            x[i] = f[i] * (z[i] - dp);
+        }
         for (int i = 0; i < 24; ++i) {
             double s = S.K[33 * lane + i];
             for (int k = 0; k < 9; ++k) s -= S.K[33 * (24 + k) + i] * x[k];
@@ -441,11 +462,14 @@ int hex81_run(astro_ctx *ctx, const int *d_list, const std::vector<int> &ptr, in
     A.nEls = ctx->P.E;
     A.nBlocks = ctx->P.nb;
     A.status = ASTRO_CHECKED ? dptr<int>(ctx->d_guard) : nullptr;
-    // groups of elements across the colours (a colour alone is the whole of it in a mixed mesh's pass)
+    // groups of elements across the colours (a colour alone is the whole of it in a mixed mesh's pass), equal ones:
+    // a group of a few takes an element's latency too (95 us)
+    const int total = ptr.back() - ptr[0], groups = std::max(1, (total + kHexAtOnce / 2) / kHexAtOnce);
+    const int size = (total + groups - 1) / std::max(1, groups);
     A.blkOut = A.ruItem = nullptr;
     for (int lo = ptr[0]; lo < ptr.back();) {
         const bool once = ptr.size() > 2;
-        const int hi = once ? std::min(ptr.back(), lo + kHexAtOnce) : ptr.back();
+        const int hi = once ? std::min(ptr.back(), lo + size) : ptr.back();
         DevBuf dBlk, dRu;
         if (once) {
             const int rc = hex_at_once_alloc(ctx, hi - lo, build && K, d_loadInt != nullptr, dBlk, dRu);

@@ -9,8 +9,8 @@ from misc_gb300.astro import AstroGPU
 pytestmark = pytest.mark.gpu
 
 
-# 1 .. 4 colours of one element or more; 819; 4,096 | 4,352 elements (the bound, and a group of the rest); 8,448
-@pytest.mark.parametrize("dims", [(1, 1, 1), (2, 1, 1), (3, 2, 1), (13, 9, 7), (16, 16, 16), (16, 16, 17), (16, 16, 33)])
+# 1 .. 4 colours of one element or more; 819; 4,096 | 4,352 elements (the bound of bricks); 6,144 | 8,448 (two groups of brickIM)
+@pytest.mark.parametrize("dims", [(1, 1, 1), (2, 1, 1), (3, 2, 1), (13, 9, 7), (16, 16, 16), (16, 16, 17), (24, 16, 16), (16, 16, 33)])
 @pytest.mark.parametrize("displaced", [False, True])
 @pytest.mark.parametrize("im", [False, True])
 def test_assembly_is_the_sum_of_the_elements(dims, displaced, im):
