@@ -564,7 +564,8 @@ struct GenSmem {
         struct {
             // item gp*8 + a: 6x3 row-major, and one more: phase 2's lanes read rows of their own, which
             // at 18 words share banks four deep (at 19, two)
-            float Ph[64][19], Pl[64][19], Qh[64][19], Ql[64][19];
+            float Qh[64][19], Ql[64][19];
+            float2 G[8][9];  // G at the points
             float4 gh[64], gl[64], th[64], tl[64];
         } u;
         struct {
@@ -583,7 +584,7 @@ __device__ __forceinline__ DF df_shfl_xor(DF v, int m) {
 __device__ __forceinline__ DF df_fma(DF a, DF b, DF c) { return df_add(df_mul(a, b), c); }
 
 template <bool ROT, bool BUILD>
-__global__ void __launch_bounds__(32 * kGenW) hex8_gen_kernel(Hex8GenArgs A) {
+__global__ void __launch_bounds__(32 * kGenW, BUILD ? (ROT ? 6 : 7) : 1) hex8_gen_kernel(Hex8GenArgs A) {
     __shared__ GenSmem sm[kGenW];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int item = blockIdx.x * kGenW + w;
@@ -741,6 +742,9 @@ __global__ void __launch_bounds__(32 * kGenW) hex8_gen_kernel(Hex8GenArgs A) {
         for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int j = 0; j < 3; ++j) Gm[i][j] = df_add(Or[i][j], ux[j][i]);
+        if (BUILD && s == 0)
+#pragma unroll
+            for (int q = 0; q < 9; ++q) S.u.G[gp][q] = make_float2(Gm[q / 3][q % 3].hi, Gm[q / 3][q % 3].lo);
         // Newmark inertia: acceleration at the point, rho w detJ, and c1 c2 rho w detJ
         DF ag[3] = {zero, zero, zero}, rw = zero, mw = zero;
         if (A.dyn) {
@@ -779,13 +783,6 @@ __global__ void __launch_bounds__(32 * kGenW) hex8_gen_kernel(Hex8GenArgs A) {
             }
             if (BUILD) {
                 const int it = gp * 8 + a;
-#pragma unroll
-                for (int q = 0; q < 6; ++q)
-#pragma unroll
-                    for (int v = 0; v < 3; ++v) {
-                        S.u.Ph[it][3 * q + v] = P[q][v].hi;
-                        S.u.Pl[it][3 * q + v] = P[q][v].lo;
-                    }
 #pragma unroll
                 for (int v = 0; v < 3; ++v) {
                     DF Q[6];
@@ -863,22 +860,39 @@ __global__ void __launch_bounds__(32 * kGenW) hex8_gen_kernel(Hex8GenArgs A) {
         }
         const int unit = u0 + u, t = unit >> 3, p = unit & 7;
         const int ia = 8 * p + c_tileA[t], ib = 8 * p + c_tileB[t];
+        const float4 gh = S.u.gh[ia], gl = S.u.gl[ia], th = S.u.th[ib], tl = S.u.tl[ib];
+        // M = Bloc(g_a)^T Q_b, then G^T M: as many products as P_a^T Q_b, and P is neither stored nor read
+        DF m[9];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) m[q] = zero;
+        const float ah[3] = {gh.x, gh.y, gh.z}, al[3] = {gl.x, gl.y, gl.z};
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
-            float ph[3], pl[3], qh[3], ql[3];
+            // rows of M that Voigt row q enters, and with which component of g
+            const int r0 = q < 3 ? q : (q < 5 ? 0 : 1), c0 = q < 3 ? q : (q == 3 ? 1 : 2);
+            float qh[3], ql[3];
 #pragma unroll
             for (int v = 0; v < 3; ++v) {
-                ph[v] = S.u.Ph[ia][3 * q + v];
-                pl[v] = S.u.Pl[ia][3 * q + v];
                 qh[v] = S.u.Qh[ib][3 * q + v];
                 ql[v] = S.u.Ql[ib][3 * q + v];
             }
 #pragma unroll
-            for (int v = 0; v < 3; ++v)
-#pragma unroll
-                for (int x = 0; x < 3; ++x) df_acc(acc[3 * v + x], ph[v], pl[v], qh[x], ql[x]);
+            for (int x = 0; x < 3; ++x) {
+                df_acc(m[3 * r0 + x], ah[c0], al[c0], qh[x], ql[x]);
+                if (q >= 3) df_acc(m[3 * c0 + x], ah[r0], al[r0], qh[x], ql[x]);
+            }
         }
-        const float4 gh = S.u.gh[ia], gl = S.u.gl[ia], th = S.u.th[ib], tl = S.u.tl[ib];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+#pragma unroll
+            for (int x = 0; x < 3; ++x) m[3 * i + x] = df_norm(m[3 * i + x]);
+#pragma unroll
+            for (int v = 0; v < 3; ++v) {
+                const float2 G = S.u.G[p][3 * i + v];
+#pragma unroll
+                for (int x = 0; x < 3; ++x) df_acc(acc[3 * v + x], G.x, G.y, m[3 * i + x].hi, m[3 * i + x].lo);
+            }
+        }
         df_acc(geo, gh.x, gl.x, th.x, tl.x);
         df_acc(geo, gh.y, gl.y, th.y, tl.y);
         df_acc(geo, gh.z, gl.z, th.z, tl.z);
