@@ -978,18 +978,24 @@ static int resident_plan(astro_ctx *ctx, GmresWork &W, const Op<TM> &op, int m, 
 }
 
 // Enqueues one resident cycle.
+// (or, power > 0, as many power iterations of the hops' operator with the layout of degree deg)
 template <class TM, class TV, int DPN, bool POLY>
-static cudaError_t resident_cycle(GmresWork &W, const Op<TM> &op, TV *x, const double *b, int m, cudaStream_t s) {
+static cudaError_t resident_cycle(GmresWork &W, const Op<TM> &op, TV *x, const double *b, int m, cudaStream_t s, int power = 0,
+                                  int deg = 0) {
     GmresCtl *ctl = dptr<GmresCtl>(W.ctl);
     ResArgs<TM, TV> A{};
     A.op = op;
     if constexpr (POLY) {
         A.hop = W.hop;
-        A.deg = W.poly->deg;
-        A.theta = W.poly->theta;
-        A.delta = W.poly->delta;
         A.W = dptr<float>(W.polyW);
-        A.amod = W.poly->amod;
+        A.power = power;
+        A.deg = deg;
+        if (!power) {
+            A.deg = W.poly->deg;
+            A.theta = W.poly->theta;
+            A.delta = W.poly->delta;
+            A.amod = W.poly->amod;
+        }
     }
     A.y0s = W.y0s<TV>();
     A.x = x;
@@ -1433,6 +1439,9 @@ static int solve_static_dev(astro_ctx *ctx, const double *d_b, double *d_x, cons
             // the operator and its eigenvalue estimate depend only on the matrix: rebuilt when the
             // matrix (or its constraint scaling) changed, reused by repeated solves (time steps)
             const int opVer = k32_source_version(ctx) * 64 + (ctx->penVersion & 63);
+            if ((!W.polyW.p && (rc = dev_alloc(ctx, W.polyW, sizeof(ph.W)))) ||
+                (rc = resident_plan<float, float, DPN, true>(ctx, W, make_op<float>(ctx, K32p), m, pc->degree)))
+                return rc;
             if (W.hopVersion != opVer) {
                 k_sqrt_f<<<(n + 255) / 256, 256, 0, ctx->stream>>>(dptr<double>(W.dinv), dptr<float>(W.dsqT), n);
                 const long long tot = (long long)S * ld;
@@ -1447,9 +1456,25 @@ static int solve_static_dev(astro_ctx *ctx, const double *d_b, double *d_x, cons
                         dptr<double>(ctx->d_penVal), ctx->P.N, DPN, dptr<double>(W.dinv), dptr<double>(W.penS));
                     W.hop.penVal = dptr<double>(W.penS);
                 }
-                if ((rc = cuda_check(ctx, cudaGetLastError(), "preconditioner operator")) ||
-                    (rc = power_lambda<OpH, float, DPN>(ctx, W.hop, (const float *)nullptr, &W.lamEst)))
+                if ((rc = cuda_check(ctx, cudaGetLastError(), "preconditioner operator"))) return rc;
+                if (W.res.on) {
+                    // 50 iterations as in power_lambda
+                    CK((resident_cycle<float, float, DPN, true>(W, make_op<float>(ctx, K32p), nullptr, nullptr, m, ctx->stream, 50,
+                                                                pc->degree)));
+                    GmresCtl *ctl = dptr<GmresCtl>(W.ctl);
+                    int stuck = 0;
+                    CK(cudaMemcpyAsync(&W.lamEst, &ctl->y[0], sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+                    CK(cudaMemcpyAsync(&stuck, &ctl->stuck, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+                    CK(cudaStreamSynchronize(ctx->stream));
+                    if (stuck) {
+                        CK(cudaMemsetAsync(&ctl->stuck, 0, sizeof(int), ctx->stream));
+                        return set_err(ctx, ASTRO_ERR_CUDA, "a wait of the power iteration was given up");
+                    }
+                    if (!(std::isfinite(W.lamEst) && W.lamEst > 0.0))
+                        return set_err(ctx, ASTRO_ERR_NAN, "eigenvalue estimate is not positive");
+                } else if ((rc = power_lambda<OpH, float, DPN>(ctx, W.hop, (const float *)nullptr, &W.lamEst))) {
                     return rc;
+                }
                 W.hopVersion = opVer;
             }
             lam = W.lamEst * pc->lambda_scale;
@@ -1475,9 +1500,6 @@ static int solve_static_dev(astro_ctx *ctx, const double *d_b, double *d_x, cons
                 ph.amod = dptr<float>(W.amod);
             }
             W.poly = &ph;
-            if ((!W.polyW.p && (rc = dev_alloc(ctx, W.polyW, sizeof(ph.W)))) ||
-                (rc = resident_plan<float, float, DPN, true>(ctx, W, make_op<float>(ctx, K32p), m, ph.deg)))
-                return rc;
             // (the resident cycle keeps the operator in shared memory)
             if (!W.res.on) persistSet = persist_begin(ctx, W, &persistPrev);
             else W.apwOn = false;

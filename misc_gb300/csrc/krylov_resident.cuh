@@ -43,6 +43,7 @@ template <class TM, class TV> struct ResArgs {
     OpH hop;              // polynomial preconditioner (its values), or unused
     int deg;              // hops, 0 = Jacobi
     float theta, delta;   // the map of the recurrence
+    int power;            // power iterations of the hops' operator instead of a cycle; the norm to ctl->y[0]
     const float *W;       // hop weights, (deg + 1) x dpn x dpn, already divided by lambda
     const float *amod;    // per-node hop scales, or null
     const TV *y0s;        // scales a residual into the preconditioner's input
@@ -543,11 +544,73 @@ __global__ void __launch_bounds__(kResT, 1) k_gmres_resident(ResArgs<TM, TV> A) 
         }
         __syncwarp();
     };
+    // The product of the hops' operator with the gathered halo: eight rows a warp, four lanes a row (the lane's
+    // bits 3 and 4), each of which gets the row.
+    auto hopProduct = [&](TV (&a)[DPN]) {
+        constexpr int NL = 4;
+        const int sub = lane >> 3, r = wid * 8 + (lane & 7);
+        const bool own = r < rows;
+        const int p0 = pen && own ? pPtr[r] + NL - 1 - sub : 0, p1 = pen && own ? pPtr[r + 1] : 0;
+#pragma unroll
+        for (int q = 0; q < DPN; ++q) a[q] = TV(0);
+        if (own) {
+#pragma unroll 2
+            for (int s = sub; s < S; s += NL) {
+                const int at = s * Rp + r;
+                float kv[DD];
+#pragma unroll
+                for (int p = 0; p < BvShape<DPN>::NV; ++p) {
+                    const uint4 u = sKv[(s * BvShape<DPN>::NV + p) * Rp + r];
+                    const unsigned w4[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w4[e]));
+                        kv[8 * p + 2 * e] = f.x;
+                        kv[8 * p + 2 * e + 1] = f.y;
+                    }
+                }
+                TV xv[DPN];
+                if constexpr (DPN == 3) {
+                    const unsigned ch = sColH[at];
+                    kv[8] = h2f_bits((unsigned short)(ch >> 16));
+                    const float4 f = *reinterpret_cast<const float4 *>(sHalo + HS * (ch & 0xffff));
+                    xv[0] = f.x;
+                    xv[1] = f.y;
+                    xv[2] = f.z;
+                } else {
+                    const uint2 u = sKr[at];
+                    const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&u.x)),
+                                 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&u.y));
+                    kv[DD - 4] = f0.x;
+                    kv[DD - 3] = f0.y;
+                    kv[DD - 2] = f1.x;
+                    kv[DD - 1] = f1.y;
+#pragma unroll
+                    for (int jj = 0; jj < DPN; ++jj) xv[jj] = sHalo[HS * sCol[at] + jj];
+                }
+#pragma unroll
+                for (int i = 0; i < DPN; ++i)
+#pragma unroll
+                    for (int jj = 0; jj < DPN; ++jj) a[i] += (TV)kv[i * DPN + jj] * xv[jj];
+            }
+            for (int q = p0; q < p1; q += NL) {  // (from the last lane: 27 slots are one fewer there)
+                const float2 v = reinterpret_cast<const float2 *>(pVal)[q];
+                const float x = (float)sHalo[pInfo[q] & 0xffffff];
+                const TV pv = fmaf(v.x, x, v.y * x);
+#pragma unroll
+                for (int i = 0; i < DPN; ++i) a[i] += i == pInfo[q] >> 24 ? pv : TV(0);
+            }
+        }
+#pragma unroll
+        for (int o = 8; o < 32; o *= 2)
+#pragma unroll
+            for (int q = 0; q < DPN; ++q) a[q] += __shfl_xor_sync(0xffffffffu, a[q], o);
+    };
     // The hops of the preconditioner on y0 = S sw (exchange no); P v goes into the next exchange or, upd, is
-    // added to x.  False when a wait was given up.  Eight rows a warp, four lanes a row (the lane's bits 3 and
-    // 4), each with the row's recurrence; lane q < 3 of them collects components q, q + 3 of P v.
+    // added to x.  False when a wait was given up.  The four lanes of a row each
+    // have its recurrence; lane q < 3 of them collects components q, q + 3 of P v.
     auto hops = [&](const bool upd) -> bool {
-        constexpr int NL = 4, NZ = DPN / 3;
+        constexpr int NZ = DPN / 3;
         const int sub = lane >> 3, r = wid * 8 + (lane & 7), g = row0 + r;
         const bool own = r < rows;
         TV yc[DPN], yp[DPN], sc[DPN], za[NZ];
@@ -560,7 +623,6 @@ __global__ void __launch_bounds__(kResT, 1) k_gmres_resident(ResArgs<TM, TV> A) 
 #pragma unroll
         for (int z = 0; z < NZ; ++z) za[z] = TV(0);
         const TV dinvC = TV(1) / (TV)A.delta, theta = (TV)A.theta;
-        const int p0 = pen && own ? pPtr[r] + NL - 1 - sub : 0, p1 = pen && own ? pPtr[r + 1] : 0;
         // za += a_k W_k (s y)
         auto collect = [&](int k, const TV *y) {
             if (!own || sub > 2) return;
@@ -576,60 +638,7 @@ __global__ void __launch_bounds__(kResT, 1) k_gmres_resident(ResArgs<TM, TV> A) 
         for (int k = 0; k < A.deg; ++k) {
             if (!gather(no)) return false;
             TV a[DPN];
-#pragma unroll
-            for (int q = 0; q < DPN; ++q) a[q] = TV(0);
-            if (own) {
-#pragma unroll 2
-                for (int s = sub; s < S; s += NL) {
-                    const int at = s * Rp + r;
-                    float kv[DD];
-#pragma unroll
-                    for (int p = 0; p < BvShape<DPN>::NV; ++p) {
-                        const uint4 u = sKv[(s * BvShape<DPN>::NV + p) * Rp + r];
-                        const unsigned w4[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w4[e]));
-                            kv[8 * p + 2 * e] = f.x;
-                            kv[8 * p + 2 * e + 1] = f.y;
-                        }
-                    }
-                    TV xv[DPN];
-                    if constexpr (DPN == 3) {
-                        const unsigned ch = sColH[at];
-                        kv[8] = h2f_bits((unsigned short)(ch >> 16));
-                        const float4 f = *reinterpret_cast<const float4 *>(sHalo + HS * (ch & 0xffff));
-                        xv[0] = f.x;
-                        xv[1] = f.y;
-                        xv[2] = f.z;
-                    } else {
-                        const uint2 u = sKr[at];
-                        const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&u.x)),
-                                     f1 = __half22float2(*reinterpret_cast<const __half2 *>(&u.y));
-                        kv[DD - 4] = f0.x;
-                        kv[DD - 3] = f0.y;
-                        kv[DD - 2] = f1.x;
-                        kv[DD - 1] = f1.y;
-#pragma unroll
-                        for (int jj = 0; jj < DPN; ++jj) xv[jj] = sHalo[HS * sCol[at] + jj];
-                    }
-#pragma unroll
-                    for (int i = 0; i < DPN; ++i)
-#pragma unroll
-                        for (int jj = 0; jj < DPN; ++jj) a[i] += (TV)kv[i * DPN + jj] * xv[jj];
-                }
-                for (int q = p0; q < p1; q += NL) {  // (from the last lane: 27 slots are one fewer there)
-                    const float2 v = reinterpret_cast<const float2 *>(pVal)[q];
-                    const float x = (float)sHalo[pInfo[q] & 0xffffff];
-                    const TV pv = fmaf(v.x, x, v.y * x);
-#pragma unroll
-                    for (int i = 0; i < DPN; ++i) a[i] += i == pInfo[q] >> 24 ? pv : TV(0);
-                }
-            }
-#pragma unroll
-            for (int o = 8; o < 32; o *= 2)
-#pragma unroll
-                for (int q = 0; q < DPN; ++q) a[q] += __shfl_xor_sync(0xffffffffu, a[q], o);
+            hopProduct(a);
             const bool last = k + 1 == A.deg;
             const TV c = (k == 0 ? TV(1) : TV(2)) * dinvC;
 #pragma unroll
@@ -657,6 +666,65 @@ __global__ void __launch_bounds__(kResT, 1) k_gmres_resident(ResArgs<TM, TV> A) 
         }
         return true;
     };
+
+    // Power iterations y <- A^ y / ||y|| from a fixed pseudo-random vector (k_power_init's).  The norm of a vector
+    // is waited for behind the next product, which it scales.
+    if constexpr (POLY) {
+        if (A.power) {
+            const int sub = lane >> 3, r = wid * 8 + (lane & 7);
+            const bool own = r < rows;
+            auto start = [](unsigned i) {
+                unsigned h = i * 2654435761u + 0x9e3779b9u;
+                h ^= h >> 16;
+                h *= 0x85ebca6bu;
+                h ^= h >> 13;
+                h *= 0xc2b2ae35u;
+                h ^= h >> 16;
+                return (TV)((double)(h >> 8) * (2.0 / 16777216.0) - 1.0);
+            };
+            TV y[DPN];
+            ++no;
+            if (own && sub == 0) {
+#pragma unroll
+                for (int q = 0; q < DPN; ++q) y[q] = start((unsigned)((row0 + r) * DPN + q));
+                put_node(no, r, y);
+            }
+            for (int it = 0; it <= A.power; ++it) {
+                TV a[DPN];
+                const bool more = it < A.power;
+                if (more) {
+                    if (!gather(no)) break;
+                    hopProduct(a);
+                }
+                if (it) {  // the norm of the last vector
+                    totals(0, 1, it, sh1);
+                    if (t == 0) sInv = (TV)(sh1[0] > 0.0 ? rsqrt(sh1[0]) : 0.0);  // (of every thread: 20,000 clocks)
+                    wsync();
+                    if (sStuck) break;
+                }
+                if (!more) break;
+                const TV s = it ? sInv : TV(1);
+                ++no;
+                double yy = 0.0;
+#pragma unroll
+                for (int q = 0; q < DPN; ++q) {
+                    y[q] = s * a[q];
+                    if (own && q % 4 == sub) yy = fma(widen(y[q]), widen(y[q]), yy);
+                }
+                if (own && sub == 0) put_node(no, r, y);
+                yy = warp_sum(yy);
+                if (lane == 0) red[wid] = yy;
+                wsync();
+                if (wid == 0) {
+                    const double v = warp_sum(red[lane]);
+                    if (lane == 0) put_part(0, 0, v, it + 1);
+                }
+            }
+            if (t == 0 && sStuck) A.ctl->stuck = 1;
+            if (t == 0 && blockIdx.x == 0 && !sStuck) A.ctl->y[0] = sqrt(sh1[0]);
+            return;
+        }
+    }
 
     int j = 0;
     // The workers' part: r = b - A x (products in FP64, every row's sum in the order of the residual kernel: a
