@@ -202,7 +202,9 @@ typedef struct astro_solve_stats {
     double seconds;          /* device time of the solve, CUDA events */
     int32_t conditional_graph;  /* 1: the restart cycles ran as CUDA graphs whose Arnoldi steps sit
                                    behind conditional nodes (skipped after convergence); 0: the
-                                   unrolled graph (the driver refused conditional nodes) */
+                                   unrolled graph (the driver refused conditional nodes);
+                                   cycles resident on the SMs, where the operator fits their
+                                   shared memory, need neither and report as the graph would */
     int32_t fallback;        /* learned solver: 1 when it ended in a non-finite value, a breakdown or
                                 the iteration cap and the FP32 Jacobi solver finished the solve from
                                 the initial guess (the counts and seconds then cover both) */
@@ -245,7 +247,8 @@ int astro_get_dims(const astro_ctx *ctx, astro_dims *out);
 /* ASTRO_OPT_UNROLLED_CYCLES (default 0): when 1, the static solvers capture their restart cycles
  * as m unrolled Arnoldi steps (kernels that return at once after convergence) instead of
  * conditional graph nodes; the same kernels in the same order, so the results are identical.
- * For profilers that do not look inside conditional nodes, and for drivers without them. */
+ * For profilers that do not look inside conditional nodes, and for drivers without them.
+ * (Cycles that run resident on the SMs, one launch each, are the same under both values.) */
 #define ASTRO_OPT_UNROLLED_CYCLES 2
 /* ASTRO_OPT_BAND_FP64_UPDATE (default 1): the band LDL^T of astro_panels_factor (and of
  * astro_newmark_cases) runs its trailing tile updates in FP64 arithmetic; 0 selects the

@@ -19,6 +19,8 @@
 //     second update) and a restart
 //     cycle is captured once as a CUDA graph and replayed, the host reading one status word per
 //     cycle;
+//   * where the operator fits the SMs' shared memory the cycle (and the eigenvalue estimate of the polynomial
+//     preconditioner) is one cooperative launch instead: krylov_resident.cuh;
 //   * precision: the plain solver runs in FP64 throughout (the comparator).  The mixed solver
 //     runs the Krylov cycles in FP32 (FP32 matrix and basis) inside an FP64 iterative refinement
 //     whose residual b - A x is formed in FP64 arithmetic.
