@@ -117,6 +117,45 @@ __device__ void res_mark(const Op<TM> &op, int row0, int rows, unsigned *marks, 
     __syncthreads();
 }
 
+// The block columns of a CTA's rows, ascending, into list (kResT threads; marks: a byte per column of scratch);
+// their number, at most H of which are written.
+template <class TM>
+__device__ int res_list(const Op<TM> &op, int row0, int rows, int H, unsigned *marks, int *list) {
+    __shared__ int cnt[kResT + 1];
+    const int t = threadIdx.x, words = (op.N + 3) / 4;
+    if (rows > 0) res_mark(op, row0, rows, marks, words);
+    const int per = (words + kResT - 1) / kResT, w0 = min(words, t * per), w1 = min(words, w0 + per);
+    int c = 0;
+    if (rows > 0)
+        for (int i = w0; i < w1; ++i) c += __popc(marks[i]);
+    cnt[t + 1] = c;
+    if (t == 0) cnt[0] = 0;
+    __syncthreads();
+    for (int o = 1; o < kResT; o *= 2) {  // inclusive scan of cnt[1 ..]
+        const int v = t + 1 > o ? cnt[t + 1 - o] : 0;
+        __syncthreads();
+        cnt[t + 1] += v;
+        __syncthreads();
+    }
+    if (rows > 0 && cnt[kResT] <= H) {
+        int at = cnt[t];
+        for (int i = w0; i < w1; ++i)
+            for (unsigned b = marks[i]; b; b &= b - 1) list[at++] = 4 * i + (__ffs(b) - 1) / 8;
+    }
+    __syncthreads();
+    return cnt[kResT];
+}
+// Position of column c in the list.
+__device__ __forceinline__ int res_find(const int *list, int n, int c) {
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (list[mid] < c) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
 // Largest halo (most[0]) and number of penalty entries (most[1]) of a CTA.
 template <class TM> __global__ void k_res_halo(Op<TM> op, int R, int *most) {
     extern __shared__ unsigned marks[];
@@ -207,47 +246,17 @@ __global__ void __launch_bounds__(kResT, 1) k_gmres_resident(ResArgs<TM, TV> A) 
     // ---- the CTA's rows into shared memory: halo list, local columns, operator -----------------------
     {
         // marks of the halo in the (still unused) operator area
-        unsigned *marks = reinterpret_cast<unsigned *>(smem + L.k);
-        const int words = (A.N + 3) / 4;
-        if (rows > 0) res_mark(A.op, row0, rows, marks, words);
-        __shared__ int cnt[kResT + 1];
-        const int per = (words + kResT - 1) / kResT, w0 = min(words, t * per), w1 = min(words, w0 + per);
-        int c = 0;
-        if (rows > 0)
-            for (int i = w0; i < w1; ++i) c += __popc(marks[i]);
-        cnt[t + 1] = c;
-        if (t == 0) cnt[0] = 0;
-        __syncthreads();
-        for (int o = 1; o < kResT; o *= 2) {  // inclusive scan of cnt[1 ..]
-            const int v = t + 1 > o ? cnt[t + 1 - o] : 0;
-            __syncthreads();
-            cnt[t + 1] += v;
-            __syncthreads();
-        }
+        const int n = res_list(A.op, row0, rows, A.H, reinterpret_cast<unsigned *>(smem + L.k), sList);
         if (t == 0) {
-            sHaloN = cnt[kResT];
+            sHaloN = n;
             sStuck = 0;
         }
-        if (cnt[kResT] > A.H || nPen > A.P) {  // (the host sizes both by the same counts)
+        if (n > A.H || nPen > A.P) {  // (the host sizes both by the same counts)
             if (t == 0) A.ctl->stuck = 1;
             return;
         }
         __syncthreads();
-        if (rows > 0) {
-            int at = cnt[t];
-            for (int i = w0; i < w1; ++i)
-                for (unsigned b = marks[i]; b; b &= b - 1) sList[at++] = 4 * i + (__ffs(b) - 1) / 8;
-        }
-        __syncthreads();
-        auto find = [&](int c) {  // position of block column c in the (ascending) list
-            int lo = 0, hi = sHaloN - 1;
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (sList[mid] < c) lo = mid + 1;
-                else hi = mid;
-            }
-            return lo;
-        };
+        auto find = [&](int c) { return res_find(sList, sHaloN, c); };
         for (int i = t; i < S * Rp; i += kResT) {
             const int r = i % Rp, c = r < rows ? find(A.op.col[(size_t)(i / Rp) * A.op.ld + row0 + r]) : 0;
             if constexpr (POLY && DPN == 3) {

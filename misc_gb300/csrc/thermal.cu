@@ -22,7 +22,7 @@
 #include <vector>
 
 #include "astro_internal.h"
-#include "krylov_ops.cuh"
+#include "krylov_resident.cuh"
 #include "shell_props.cuh"
 
 namespace {
@@ -55,6 +55,7 @@ struct ThermPlan {
     DevBuf d_scr;  // bricks: the element stage's results of a chunk
     // the solve's slot-major copy of the matrix (entry s of row r at s * ld + r)
     DevBuf d_ell, d_ellCol;
+    DevBuf d_words;  // exchanged by the resident solve
     int slots = 0, ld = 0;
     // the solve's vectors and a batch of its iterations as a graph, with the pointers it was captured with
     DevBuf d_cg[8];  // x, r, z, p, Ap, 1 / diagonal, partials, scalars
@@ -689,6 +690,7 @@ constexpr int kCgBatch = 16;  // iterations between two looks at the residual (e
 struct CgScal {
     double rz[2];  // of even and odd iterations
     double rr, bb;
+    int its, stuck;  // resident: iterations done, and whether a wait was given up
 };
 
 // sum of n CTA partials, the same in every thread (warp 0 adds)
@@ -857,7 +859,261 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_dir(int n, int par, int wantR
     }
 }
 
+// The iterations resident on the SMs, for matrices that fit their shared memory (27 entries a row: 90,000 rows):
+// one cooperative launch, a CTA per SM with consecutive rows of the matrix and of all vectors, p's halo and the
+// dot products exchanged as numbered words (krylov_resident.cuh).  The same iteration, three launches of which
+// are 16.4 us on 70,785 nodes; here 13 us: the FP64 pipe (34 multiply-adds a row: 4.9 us) and two sums over
+// all CTAs, each of which waits for the other.
+struct CgRes {
+    astro_kry::Op<double> op;
+    double *x, *r, *p;
+    const double *dinv;
+    CgScal *sc;
+    ulonglong2 *words;  // all 0 at launch: cg_words()
+    double target;      // on |r|, looked at every kCgBatch iterations and after the last
+    int iters, N, R, G, H, P;
+};
+constexpr int kCgResIters = 1024;  // iterations of a launch
+struct CgResLayout {
+    size_t v, col, list, halo, own, pptr, pinfo, pval, total;
+};
+__host__ __device__ inline CgResLayout cg_res_layout(int N, int S, int R, int H, int P) {
+    const size_t rows = ((size_t)R + 3) / 4 * 4;
+    CgResLayout L;
+    size_t o = 0;
+    auto put = [&](size_t bytes) {
+        const size_t at = o;
+        o += (bytes + 15) / 16 * 16;
+        return at;
+    };
+    const size_t v = sizeof(double) * S * rows, marks = ((size_t)N + 3) / 4 * 4;
+    L.v = put(v > marks ? v : marks);
+    L.col = put(sizeof(unsigned short) * S * rows);
+    L.list = put(sizeof(int) * (size_t)H);
+    L.halo = put(sizeof(double) * (size_t)H);
+    L.own = put(sizeof(double) * 8 * rows);  // p, r, x, D^-1, A p (then z), three of partial products (then products)
+    L.pptr = put(P ? sizeof(int) * ((size_t)R + 1) : 0);
+    L.pinfo = put(sizeof(int) * (size_t)P);
+    L.pval = put(sizeof(double) * (size_t)P);
+    L.total = o;
+    return L;
+}
+// two exchanges of a vector, partials and every CTA's totals of three sums
+static size_t cg_words(int N, int G) { return 2 * (size_t)N + 6 * (size_t)G; }
+
+__global__ void __launch_bounds__(astro_kry::kResT, 1) k_cg_resident(CgRes A) {
+    using namespace astro_kry;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ double red[8], sTot[3], sRz, sCoef;
+    __shared__ int sStuck;
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    const int row0 = blockIdx.x * A.R, rows = max(0, min(A.R, A.N - row0)), Rp = (A.R + 3) / 4 * 4, S = A.op.S;
+    const CgResLayout L = cg_res_layout(A.N, S, A.R, A.H, A.P);
+    double *sv = reinterpret_cast<double *>(smem + L.v);
+    unsigned short *sCol = reinterpret_cast<unsigned short *>(smem + L.col);
+    int *sList = reinterpret_cast<int *>(smem + L.list);
+    double *sHalo = reinterpret_cast<double *>(smem + L.halo);
+    double *sp = reinterpret_cast<double *>(smem + L.own), *sr = sp + Rp, *sx = sr + Rp, *sd = sx + Rp, *sq = sd + Rp,
+           *sPart = sq + Rp;
+    int *pPtr = reinterpret_cast<int *>(smem + L.pptr), *pLoc = reinterpret_cast<int *>(smem + L.pinfo);
+    double *pVal = reinterpret_cast<double *>(smem + L.pval);
+    const bool pen = A.op.penPtr && A.P > 0 && rows > 0;
+    const int pen0 = pen ? A.op.penPtr[row0] : 0, nPen = pen ? A.op.penPtr[row0 + rows] - pen0 : 0;
+    const int halo = res_list(A.op, row0, rows, A.H, reinterpret_cast<unsigned *>(smem + L.v), sList);
+    if (halo > A.H || nPen > A.P) {  // (the host sizes both by the same counts)
+        if (t == 0) A.sc->stuck = 1;
+        return;
+    }
+    for (int i = t; i < S * Rp; i += kResT) {
+        const int r = i % Rp;
+        sCol[i] = r < rows ? (unsigned short)res_find(sList, halo, A.op.col[(size_t)(i / Rp) * A.op.ld + row0 + r]) : 0;
+    }
+    if (pen) {
+        for (int i = t; i <= rows; i += kResT) pPtr[i] = A.op.penPtr[row0 + i] - pen0;
+        for (int q = t; q < nPen; q += kResT) {
+            pLoc[q] = res_find(sList, halo, A.op.penCol[pen0 + q]);
+            pVal[q] = A.op.penVal[pen0 + q];
+        }
+    }
+    __syncthreads();  // (the marks are read)
+    for (int i = t; i < S * Rp; i += kResT) {
+        const int r = i % Rp;
+        sv[i] = r < rows ? __ldg(A.op.K + (size_t)(i / Rp) * A.op.ld + row0 + r) : 0.0;
+    }
+    ulonglong2 *const part = A.words + 2 * (size_t)A.N, *const total = part + 3 * (size_t)A.G;
+    unsigned no = 1;  // exchanges of p
+    for (int i = t; i < rows; i += kResT) {
+        sp[i] = A.p[row0 + i];
+        sr[i] = A.r[row0 + i];
+        sx[i] = A.x[row0 + i];
+        sd[i] = A.dinv[row0 + i];
+        word_put(A.words + (size_t)(no & 1) * A.N + row0 + i, sp[i], no);
+    }
+    if (t == 0) {
+        sRz = A.sc->rz[0];
+        sStuck = 0;
+    }
+    __syncthreads();
+    // a word of number e, polled
+    auto until = [&](ulonglong2 w, const ulonglong2 *p, unsigned e) {  // (w: the word's first load)
+        for (int it = 0; word_no(w) != e; w = word_get(p))
+            if (++it > kSpinLimit) {
+                sStuck = 1;
+                break;
+            }
+        return __longlong_as_double((long long)w.x);
+    };
+    auto poll = [&](const ulonglong2 *p, unsigned e) { return until(word_get(p), p, e); };
+    // sums k0 .. k0 + n - 1 over all CTAs of the rows' values at v, v + Rp, numbered e, to sTot: four warps add a
+    // CTA's, CTA k mod G adds sum k over the CTAs and hands it to all
+    auto sums = [&](const double *v, int k0, int n, unsigned e) {
+        __syncthreads();
+        if (wid < 4 * n) {
+            double a = 0.0;
+            for (int i = 32 * (wid & 3) + lane; i < rows; i += 128) a += v[(wid >> 2) * Rp + i];
+            a = warp_sum(a);
+            if (lane == 0) red[wid] = a;
+        }
+        __syncthreads();
+        if (t < n) word_put(part + (size_t)(k0 + t) * A.G + blockIdx.x, (red[4 * t] + red[4 * t + 1]) + (red[4 * t + 2] + red[4 * t + 3]), e);
+        const int mine = kResT / 32 - 1 - wid;  // sum that the warp adds up, if this CTA does
+        if (mine < n && (k0 + mine) % A.G == (int)blockIdx.x) {
+            constexpr int CN = kResMaxCtas / 32;  // all loads in flight
+            const ulonglong2 *p = part + (size_t)(k0 + mine) * A.G;
+            ulonglong2 w[CN];
+#pragma unroll
+            for (int u = 0; u < CN; ++u)
+                if (lane + 32 * u < A.G) w[u] = word_get(p + lane + 32 * u);
+            double a = 0.0;
+#pragma unroll
+            for (int u = 0; u < CN; ++u)
+                if (lane + 32 * u < A.G) a += until(w[u], p + lane + 32 * u, e);
+            a = warp_sum(a);
+            for (int q = lane; q < A.G; q += 32) word_put(total + 3 * (size_t)q + k0 + mine, a, e);
+        }
+        if (t < n) sTot[k0 + t] = poll(total + 3 * (size_t)blockIdx.x + k0 + t, e);
+    };
+    const int W = (Rp + 31) / 32 * 32, SG = 4 * W <= kResT ? 4 : (2 * W <= kResT ? 2 : 1), per = kResT / SG / 32 * 32;
+    const int grp = t / per, tt = t % per;
+    int it = 0;
+    double rr = 0.0;
+    for (bool done = false; it < A.iters && !done; ++it) {
+        // A p
+        const ulonglong2 *vec = A.words + (size_t)(no & 1) * A.N;
+        for (int i0 = t; i0 < halo; i0 += 4 * kResT) {  // four words in flight
+            ulonglong2 w[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (i0 + u * kResT < halo) w[u] = word_get(vec + sList[i0 + u * kResT]);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (i0 + u * kResT < halo) sHalo[i0 + u * kResT] = until(w[u], vec + sList[i0 + u * kResT], no);
+        }
+        __syncthreads();
+        if (sStuck) break;
+        for (int i0 = 0; i0 < Rp; i0 += per) {
+            const int i = i0 + tt;
+            const bool in = i < rows && grp < SG;
+            double a = 0.0;
+            if (in) {
+#pragma unroll 4
+                for (int s = grp; s < S; s += SG) a = fma(sv[s * Rp + i], sHalo[sCol[s * Rp + i]], a);
+                if (grp == 0 && pen)
+                    for (int q = pPtr[i]; q < pPtr[i + 1]; ++q) a += pVal[q] * sHalo[pLoc[q]];
+                if (grp) sPart[(grp - 1) * Rp + i] = a;
+            }
+            __syncthreads();
+            if (in && grp == 0) {
+                for (int g = 1; g < SG; ++g) a += sPart[(g - 1) * Rp + i];
+                sq[i] = a;
+                sPart[i] = sp[i] * a;  // (the entry's own partial product is read)
+            }
+            __syncthreads();
+        }
+        sums(sPart, 0, 1, 2 * no);
+        if (t == 0) sCoef = sRz / sTot[0];
+        __syncthreads();
+        if (sStuck) break;
+        const double alpha = sCoef;
+        for (int i = t; i < rows; i += kResT) {
+            sx[i] = sx[i] + alpha * sp[i];
+            const double ri = sr[i] - alpha * sq[i], zi = sd[i] * ri;
+            sr[i] = ri;
+            sq[i] = zi;
+            sPart[i] = ri * zi;
+            sPart[Rp + i] = ri * ri;
+        }
+        sums(sPart, 1, 2, 2 * no + 1);
+        if (t == 0) {
+            sCoef = sTot[1] / sRz;
+            sRz = sTot[1];
+        }
+        __syncthreads();
+        if (sStuck) break;
+        const double beta = sCoef;
+        rr = sTot[2];
+        ++no;
+        for (int i = t; i < rows; i += kResT) {
+            const double pi = sq[i] + beta * sp[i];
+            sp[i] = pi;
+            word_put(A.words + (size_t)(no & 1) * A.N + row0 + i, pi, no);
+        }
+        if ((it + 1) % kCgBatch == 0) done = !isfinite(rr) || sqrt(rr) <= A.target;
+    }
+    for (int i = t; i < rows; i += kResT) {
+        A.x[row0 + i] = sx[i];
+        A.r[row0 + i] = sr[i];
+        A.p[row0 + i] = sp[i];
+    }
+    if (t == 0 && sStuck) A.sc->stuck = 1;
+    if (t == 0 && blockIdx.x == 0) {
+        A.sc->rz[0] = sRz;
+        A.sc->rr = rr;
+        A.sc->its = it;
+    }
+}
+
 }  // namespace
+
+// Rows, halo and shared memory of the resident iterations; R = 0 when a CTA's part does not fit.
+static int cg_resident_plan(astro_ctx *ctx, ThermPlan *T, CgRes *A, size_t *smem) {
+    const int N = A->N;
+    int coop = 0, maxSm = 0, sms = 0, per = 0, rc;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device);
+    cudaDeviceGetAttribute(&maxSm, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    sms = std::max(1, std::min(sms, astro_kry::kResMaxCtas));
+    // (a CTA per SM, but 16 rows at least: every CTA is one more term of the sums)
+    const int R = std::max((N + sms - 1) / sms, 16), G = (N + R - 1) / R;
+    A->R = 0;
+    cudaFuncAttributes fa;
+    CK(cudaFuncGetAttributes(&fa, k_cg_resident));
+    const size_t room = (size_t)maxSm - fa.sharedSizeBytes;
+    if (!coop || cg_res_layout(N, A->op.S, R, R, 0).total > room) return ASTRO_OK;
+    int HP[2] = {0, 0};
+    int *d_HP = &A->sc->its;  // counted in the iterations' place
+    CK(cudaMemsetAsync(d_HP, 0, sizeof(HP), ctx->stream));
+    CK(cudaFuncSetAttribute(astro_kry::k_res_halo<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
+    astro_kry::k_res_halo<double><<<G, astro_kry::kThreads, (size_t)(N + 3) / 4 * 4, ctx->stream>>>(A->op, R, d_HP);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(HP, d_HP, sizeof(HP), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    CK(cudaMemsetAsync(d_HP, 0, sizeof(HP), ctx->stream));
+    *smem = cg_res_layout(N, A->op.S, R, HP[0], HP[1]).total;
+    if (HP[0] > 65535 || *smem > room) return ASTRO_OK;
+    CK(cudaFuncSetAttribute(k_cg_resident, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cg_resident, astro_kry::kResT, *smem) != cudaSuccess || per < 1) {
+        cudaGetLastError();
+        return ASTRO_OK;
+    }
+    if (!T->d_words.p && (rc = dev_alloc(ctx, T->d_words, sizeof(ulonglong2) * cg_words(N, G)))) return rc;
+    A->words = dptr<ulonglong2>(T->d_words);
+    A->R = R;
+    A->G = G;
+    A->H = HP[0];
+    A->P = HP[1];
+    return ASTRO_OK;
+}
 
 void thermal_release(astro_ctx *ctx) {
     ThermPlan *T = plan_of(ctx);
@@ -865,7 +1121,8 @@ void thermal_release(astro_ctx *ctx) {
     DevBuf *b[] = {&T->d_props,   &T->d_val,    &T->d_pos,    &T->d_rowStart, &T->d_elMatId, &T->d_matCond,
                    &T->d_matSH,   &T->d_layCond, &T->d_laySH, &T->d_mRange,   &T->d_mCol,    &T->d_sVal,
                    &T->d_sRhs,    &T->d_penPtr, &T->d_penCol, &T->d_penVal,   &T->d_mDef,    &T->d_gPtr,
-                   &T->d_gTerm,   &T->d_gRow,   &T->d_termRow, &T->d_ell,     &T->d_ellCol, &T->d_scr};
+                   &T->d_gTerm,   &T->d_gRow,   &T->d_termRow, &T->d_ell,     &T->d_ellCol, &T->d_scr,
+                   &T->d_words};
     for (DevBuf *x : b) dev_free(*x);
     for (DevBuf &x : T->d_cg) dev_free(x);
     if (T->cgExec) cudaGraphExecDestroy(T->cgExec);
@@ -1393,8 +1650,22 @@ extern "C" int astro_thermal_solve(astro_ctx *ctx, const double *rhs, double *dt
             k_cg_dir<<<rg, kCgThreads, 0, s>>>(N, par, want, S, pRz, pRr, dptr<double>(z), dptr<double>(p));
         }
     };
+    CgRes Q;
+    size_t smem = 0;
+    Q.op = {A.v, A.col, A.S, A.ld, A.pp, nullptr, A.pc, A.pv, N, 1};
+    Q.x = dptr<double>(x);
+    Q.r = dptr<double>(r);
+    Q.p = dptr<double>(p);
+    Q.dinv = dptr<double>(dinv);
+    Q.sc = S;
+    Q.N = N;
+    if ((rc = cg_resident_plan(ctx, T, &Q, &smem))) {
+        dev_free(b);
+        return rc;
+    }
     // a batch as a graph, kept while the matrix tables stay where they are
-    if (!T->cgExec || std::memcmp(&T->cgMat, &A, sizeof(A)) != 0) {
+    if (Q.R) {
+    } else if (!T->cgExec || std::memcmp(&T->cgMat, &A, sizeof(A)) != 0) {
         if (T->cgExec) cudaGraphExecDestroy(T->cgExec);
         T->cgExec = nullptr;
         cudaGraph_t g = nullptr;
@@ -1420,14 +1691,30 @@ extern "C" int astro_thermal_solve(astro_ctx *ctx, const double *rhs, double *dt
     const double bn = std::sqrt(hs.bb);
     if (bn == 0.0) status = ASTRO_OK;
     while (!rc && status == ASTRO_ERR_MAXIT && it < max_iters) {
-        const int chunk = std::min(kCgBatch, max_iters - it);
-        if (chunk == kCgBatch) cudaGraphLaunch(T->cgExec, s);
-        else iterate(it, chunk);
-        it += chunk;
-        cudaError_t e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&rr, &S->rr, sizeof(double), cudaMemcpyDeviceToHost, s);
+        cudaError_t e = cudaSuccess;
+        if (Q.R) {
+            Q.iters = std::min(kCgResIters, max_iters - it);
+            Q.target = rtol * bn;
+            void *args[] = {&Q};
+            e = cudaMemsetAsync(T->d_words.p, 0, T->d_words.bytes, s);
+            if (e == cudaSuccess)
+                e = cudaLaunchCooperativeKernel((const void *)k_cg_resident, dim3(Q.G), dim3(astro_kry::kResT), args, smem, s);
+        } else {
+            const int chunk = std::min(kCgBatch, max_iters - it);
+            if (chunk == kCgBatch) cudaGraphLaunch(T->cgExec, s);
+            else iterate(it, chunk);
+            it += chunk;
+            e = cudaGetLastError();
+        }
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&hs, S, sizeof(hs), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if ((rc = cuda_check(ctx, e, "thermal solve"))) break;
+        rr = hs.rr;
+        if (Q.R) it += hs.its;
+        if (hs.stuck) {
+            rc = set_err(ctx, ASTRO_ERR_CUDA, "thermal solve: a wait was given up");
+            break;
+        }
         if (!std::isfinite(rr)) {
             status = ASTRO_ERR_NAN;
             break;

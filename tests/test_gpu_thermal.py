@@ -6,6 +6,7 @@ conjugate-gradient solve against a direct solve.  1e-12 relative for element qua
 solutions."""
 import numpy as np
 import pytest
+import scipy.sparse as sp
 import scipy.sparse.linalg as spla
 
 from misc_gb300 import model as M
@@ -166,3 +167,36 @@ def test_brick_matrix_load_and_solve_over_sizes(dims, dynamic):
     x, stats = g.thermal_solve(b, rtol=1e-13)
     xd = d * np.linalg.solve(d[:, None] * K * d, d * b)
     assert stats.status == 0 and np.linalg.norm(x - xd) <= 1e-9 * np.linalg.norm(xd)
+
+
+# rows of a CTA of the resident iterations: 16 (a last CTA of 3), one to four threads a row; 100,878 nodes do not fit
+# the SMs' shared memory
+@pytest.mark.parametrize("dims", [(10, 10, 10), (24, 17, 13), (40, 30, 21), (50, 45, 42)])
+def test_solve_over_sizes(dims):
+    nx, ny, nz = dims
+    m = M.hex_block(nx, ny, nz, lx=nx * 0.1, ly=ny * 0.1, lz=nz * 0.1, seed=nx, jitter=0.2)
+    rng = np.random.default_rng(nx)
+    nm = len(m.material_density)
+    k = rng.uniform(20.0, 60.0, nm)
+    cond = np.concatenate([k[:, None] * np.ones((nm, 3)), np.zeros((nm, 3))], axis=1)
+    N = m.num_nodes
+    # one node fixed, two tied
+    mpc = (np.array([0, 1, 3]), np.array([1, N, N // 2]), np.array([1.0, 1.0, -1.0]), np.zeros(2))
+    g = AstroGPU(m)
+    g.thermal_setup(thermal_props(cond, np.full(nm, 400.0), mpc))
+    _, mat, cols = g.getThermalSolnLoad(1)
+    mm, _ = g.scaleThermalMPC()
+    rank = g.current_rank - 1
+    el = rank[np.asarray(m.element_list)[:, :8] - 1]
+    # a row's entries: the nodes of its elements
+    pairs = np.unique(np.repeat(el, 8, axis=1).ravel() * np.int64(N) + np.tile(el, (1, 8)).ravel())
+    rows = np.concatenate([[0], np.cumsum(np.bincount(pairs // N, minlength=N))])
+    A = sp.csr_matrix((mat, cols - 1, rows), shape=(N, N))
+    C = sp.csr_matrix((mm, (np.array([0, 1, 1]), rank[mpc[1] - 1])), shape=(2, N))
+    b = rng.standard_normal(N)
+    x, stats = g.thermal_solve(b, rtol=1e-10)
+    assert stats.status == 0 and stats.rel_residual <= 1e-10
+    r = np.linalg.norm(b - (A @ x + C.T @ (C @ x)))
+    # the recurrence's residual drifts from the true one by roundings of A x (the penalty is 100 max|A|)
+    noise = 27 * 1.1e-16 * stats.iterations * np.linalg.norm(abs(A) @ abs(x) + abs(C).T @ (abs(C) @ abs(x)))
+    assert r <= 1.01e-10 * np.linalg.norm(b) + noise
