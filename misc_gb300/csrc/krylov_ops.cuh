@@ -132,9 +132,10 @@ __device__ __forceinline__ TA ell_row_comp(const Op<TM> &op, int r, int i, const
 // xor-shuffles (result in all of them); the products accumulate in TA, thread sub == 0 adds the penalty.
 template <class TA, class TM, class TX, int DPN, int RT>
 __device__ __forceinline__ void ell_row_part(const Op<TM> &op, int r, int sub, const TX *__restrict__ x, TA y[DPN]) {
-    // U slots at a time, every load of them in flight before the first product (one slot at a time waits
-    // for its column, then for x: two trips to L2 a slot)
-    constexpr int U = DPN == 3 ? 4 : 2;
+    // Eight lanes (few rows): U slots at a time, every load of them in flight before the first product (one slot
+    // at a time waits for its column, then for x: two trips to L2 a slot).  With rows enough to hide that the
+    // registers cost more than they give (70,785 rows: a step 165 us so, 144 us a slot at a time).
+    constexpr int U = RT == 8 ? (DPN == 3 ? 4 : 2) : 1;
 #pragma unroll
     for (int i = 0; i < DPN; ++i) y[i] = TA(0);
     const size_t ld = (size_t)op.ld;

@@ -1254,7 +1254,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_band_solve_df(const PanelMeta *
 //   y_I = u_I - M1_I y_{I-1} - M2_I y_{I-2},   u_I = W_I (b_I - sum_{d >= 3} L_{I,I-d} y_{I-d}),
 // so that of a block row only the product with M1_I waits for the row before.  Three stages run side by side, each as
 // far ahead as the rows that it needs allow:
-//   * producer CTAs (ranks 1 .. CS-1), eight warps, half a tile each: the sum over d >= 3 for row I + 3 from
+//   * producer CTAs (ranks 1 .. CS-1), eight warps (sixteen for bands with more tiles), half a tile each: the sum over d >= 3 for row I + 3 from
 //     the solved rows up to I in their shared-memory ring, reduced across the CTA and sent to the leader;
 //   * the leader's warp 12: b_I less those sums; warps 8 .. 11: u_I;
 //   * warps 4 .. 7: M2_I y_{I-2}, and rows to X; warps 0 .. 3: M1_I y_{I-1} and y_I, sent to every CTA's ring;
@@ -1496,16 +1496,15 @@ __device__ __forceinline__ DF df_xor(DF v, int m) {
 
 constexpr int kRedLd = TB + 1;  // row stride of the partials: a warp reads them by column
 
-constexpr int kCasePW = 8;  // producers' warps of a CTA, half a tile each: with 13 tiles, 24 have one at most
-
-// Bytes of dynamic shared memory: a producer has the ring and its partials, the leader the last rows, sums, u, v
-// and its partials.
-static size_t cases_smem(int ring, int cs) {
-    const size_t prod = (size_t)TB * ring + 2 * kCasePW * kRedLd, lead = (size_t)TB * (8 + 4 * cs + 8) + 7 * kCW * kRedLd;
+// Bytes of dynamic shared memory with pw producers' warps: a producer has the ring and its partials, the leader
+// the last rows, sums, u, v and its partials.
+static size_t cases_smem(int ring, int cs, int pw) {
+    const size_t prod = (size_t)TB * ring + 2 * pw * kRedLd, lead = (size_t)TB * (8 + 4 * cs + 8) + 7 * kCW * kRedLd;
     return sizeof(float2) * std::max(prod, lead);
 }
 
-template <int CS>
+// PW: producers' warps of a CTA, half a tile each.
+template <int CS, int PW>
 __global__ void __launch_bounds__(kCaseW * 32, 1) k_band_solve_cases(const PanelMeta *__restrict__ meta,
                                                                      const CaseItem *__restrict__ items,
                                                                      const float2 *__restrict__ Lf,
@@ -1515,7 +1514,6 @@ __global__ void __launch_bounds__(kCaseW * 32, 1) k_band_solve_cases(const Panel
                                                                      const float2 *__restrict__ Mx, size_t mS,
                                                                      const float2 *__restrict__ Dinv, double *X, int nrhs,
                                                                      int ring, int *status) {
-    constexpr int PW = kCasePW;
     constexpr int kProdWarps = (CS - 1) * PW, H = TB / 2, C = TB / kCW;
     constexpr unsigned kRow = TB * sizeof(float2);
     cg::cluster_group cl = cg::this_cluster();
@@ -1622,11 +1620,17 @@ __global__ void __launch_bounds__(kCaseW * 32, 1) k_band_solve_cases(const Panel
                     const float2 *v = sRing + (size_t)((I0 + dir * (k - k0 - 3 - h / 2)) % ring) * TB + (h % 2) * H;
                     acc = df_norm(acc);
                     a2 = df_norm(a2);
-#pragma unroll 4
-                    for (int j = 0; j < H; j += 2) {
-                        const float2 l0 = __ldg(L + j * TB), l1 = __ldg(L + (j + 1) * TB), y0 = v[j], y1 = v[j + 1];
-                        df_acc(acc, l0.x, l0.y, y0.x, y0.y);
-                        df_acc(a2, l1.x, l1.y, y1.x, y1.y);
+#pragma unroll
+                    for (int q = 0; q < H; q += 8) {  // eight loads in flight
+                        float2 l[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) l[j] = __ldg(L + (q + j) * TB);
+#pragma unroll
+                        for (int j = 0; j < 8; j += 2) {
+                            const float2 y0 = v[q + j], y1 = v[q + j + 1];
+                            df_acc(acc, l[j].x, l[j].y, y0.x, y0.y);
+                            df_acc(a2, l[j + 1].x, l[j + 1].y, y1.x, y1.y);
+                        }
                     }
                 }
                 acc = df_add(df_norm(acc), df_norm(a2));
@@ -2385,6 +2389,16 @@ static bool twist_wanted(const astro_ctx *ctx, const PanelPlan *L) {
 
 int panels_cases_would_twist(astro_ctx *ctx) { return twist_wanted(ctx, static_cast<PanelPlan *>(ctx->panels)); }
 
+// Producers' warps of a CTA: sixteen where eight would leave a warp more than the half tile that it loads ahead
+// (25 tiles: 4.1 against 7.8 ms for 17 columns), and a ring that large leaves room for their partials.
+static int cases_pw(const PanelPlan *L, int cs) {
+    return 2 * (L->maxBt - 2) > (cs - 1) * 8 && L->ring <= 850 ? 16 : 8;
+}
+static auto cases_kernel(int cs, int pw) {
+    if (pw == 16) return cs == 2 ? k_band_solve_cases<2, 16> : (cs == 8 ? k_band_solve_cases<8, 16> : k_band_solve_cases<4, 16>);
+    return cs == 2 ? k_band_solve_cases<2, 8> : (cs == 8 ? k_band_solve_cases<8, 8> : k_band_solve_cases<4, 8>);
+}
+
 int panels_cases_prepare(astro_ctx *ctx, int ncols, size_t *bytes) {
     PanelPlan *L = static_cast<PanelPlan *>(ctx->panels);
     if (ncols < 1) return set_err(ctx, ASTRO_ERR_ARG, "panels: no right-hand sides");
@@ -2394,13 +2408,12 @@ int panels_cases_prepare(astro_ctx *ctx, int ncols, size_t *bytes) {
     int rc;
     L->twist = twist_wanted(ctx, L);
     L->ring = L->maxBt + 2;
-    const size_t smem = cases_smem(L->ring, 8);
+    for (int cs : {2, 4, 8})
+        CK(cudaFuncSetAttribute(cases_kernel(cs, cases_pw(L, cs)), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)cases_smem(L->ring, cs, cases_pw(L, cs))));
     if (L->twist) {
         if ((L->twGen != L->factorGen || L->twCols != ncols) && (rc = twist_prepare(ctx, L, ncols))) return rc;
         L->factorSeconds = L->twFactorSeconds;
-        CK(cudaFuncSetAttribute(k_band_solve_cases<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        CK(cudaFuncSetAttribute(k_band_solve_cases<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        CK(cudaFuncSetAttribute(k_band_solve_cases<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         if (bytes) *bytes = 2 * sizeof(float2) * (size_t)L->twBandDoubles;
         return cuda_check(ctx, cudaStreamSynchronize(s), "panels cases prepare");
     }
@@ -2428,9 +2441,6 @@ int panels_cases_prepare(astro_ctx *ctx, int ncols, size_t *bytes) {
         CK(cudaMemsetAsync(L->d_X.p, 0, sizeof(double) * (size_t)L->xRows * ncols, s));
         L->casesCols = ncols;
     }
-    CK(cudaFuncSetAttribute(k_band_solve_cases<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CK(cudaFuncSetAttribute(k_band_solve_cases<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CK(cudaFuncSetAttribute(k_band_solve_cases<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if (bytes) *bytes = 2 * sizeof(float2) * (size_t)L->bandDoubles;
     return cuda_check(ctx, cudaStreamSynchronize(s), "panels cases prepare");
 }
@@ -2579,7 +2589,7 @@ int panels_cases_solve(astro_ctx *ctx, double *d_vec, cudaStream_t s) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3((unsigned)(count * cs));
             cfg.blockDim = dim3(kCaseW * 32);
-            cfg.dynamicSmemBytes = cases_smem(L->ring, cs);
+            cfg.dynamicSmemBytes = cases_smem(L->ring, cs, cases_pw(L, cs));
             cfg.stream = s;
             cudaLaunchAttribute at[1];
             at[0].id = cudaLaunchAttributeClusterDimension;
@@ -2588,7 +2598,7 @@ int panels_cases_solve(astro_ctx *ctx, double *d_vec, cudaStream_t s) {
             at[0].val.clusterDim.z = 1;
             cfg.attrs = at;
             cfg.numAttrs = 1;
-            auto kern = cs == 2 ? k_band_solve_cases<2> : (cs == 8 ? k_band_solve_cases<8> : k_band_solve_cases<4>);
+            auto kern = cases_kernel(cs, cases_pw(L, cs));
             return cudaLaunchKernelEx(&cfg, kern, dm, (const CaseItem *)dptr<CaseItem>(L->d_twItems) + first,
                                       (const float2 *)dptr<float2>(L->d_twLf), (const float2 *)dptr<float2>(L->d_twLb),
                                       (const float2 *)dptr<float2>(L->d_twWf), (const float2 *)dptr<float2>(L->d_twWb),
@@ -2609,7 +2619,7 @@ int panels_cases_solve(astro_ctx *ctx, double *d_vec, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(L->np * nc * cs));
     cfg.blockDim = dim3(kCaseW * 32);
-    cfg.dynamicSmemBytes = cases_smem(L->ring, cs);
+    cfg.dynamicSmemBytes = cases_smem(L->ring, cs, cases_pw(L, cs));
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -2618,7 +2628,7 @@ int panels_cases_solve(astro_ctx *ctx, double *d_vec, cudaStream_t s) {
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    auto kern = cs == 2 ? k_band_solve_cases<2> : (cs == 8 ? k_band_solve_cases<8> : k_band_solve_cases<4>);
+    auto kern = cases_kernel(cs, cases_pw(L, cs));
     CK(cudaLaunchKernelEx(&cfg, kern, (const PanelMeta *)dptr<PanelMeta>(L->d_meta),
                           (const CaseItem *)dptr<CaseItem>(L->d_items), (const float2 *)dptr<float2>(L->d_Lf),
                           (const float2 *)dptr<float2>(L->d_Lb), (const float2 *)dptr<float2>(L->d_Wf),
