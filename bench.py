@@ -734,8 +734,8 @@ def _newmark_cases_eval(a, nm):
                                 "seconds per solve of all cases"},
            "solve_chain": {"block_rows_per_sweep": nbc, "us_per_block_row": 1e3 * ms / (2 * nbc),
                            "note": "each step solves every case by forward and backward sweeps over the band's "
-                                   "32-row block rows; a row waits for the previous one (one cluster barrier per "
-                                   "row), so the step time is the chain of 2 x block rows, not HBM traffic"},
+                                   "32-row block rows; a row waits for a product with the previous one, "
+                                   "so the step time is the chain of 2 x block rows, not HBM traffic"},
            "method": "K_eff + C^T C factored once (FP64 band LDL^T), linearised residual through the assembled "
                      "K and K_eff, cluster band solve of all cases per step (double-float), CUDA graph per step"}
     g2 = g
@@ -949,7 +949,7 @@ def _widened_eval(a):
         "ldl_fact_s": best(lambda: g1.getSparseLDLFact(lt, g1.lt_range)),
         "ldl_fact_resident_s": min(resident() for _ in range(3)),
         "ldl_solve_s": best(lambda: g1.solveSparseLDLFact(rhs, fac, g1.lt_range)),
-        "path": "one 512-thread CTA sweeping the profile's rows, as the reference's row-sequential algorithm; "
+        "path": "the profile's independent parts as 32 x 32 band tiles, side by side; "
                 "host clock, host buffers copied in and out"}
     del g1
     gc.collect()
