@@ -2149,6 +2149,9 @@ int panels_factor_impl(astro_ctx *ctx, int32_t cluster_size, astro_panels_info *
              (rc = upload(ctx, L->d_penV, ctx->penV.data(), sizeof(double) * L->penCount))))
             return rc;
     }
+    // the status word of this plan's factorisation and many-column solves, whichever of them runs: a new plan's
+    // is a recycled buffer's, an older one's may be that of a factorisation that failed
+    CK(cudaMemsetAsync(L->d_status.p, 0, sizeof(int), s));
     if (!factor) {
         L->kVersion = ctx->k64Version;
         L->penVersion = ctx->penVersion;
@@ -2159,7 +2162,6 @@ int panels_factor_impl(astro_ctx *ctx, int32_t cluster_size, astro_panels_info *
     }
     if (!L->d_band.p && (rc = dev_alloc(ctx, L->d_band, sizeof(double) * (size_t)L->bandDoubles))) return rc;
     CK(cudaMemsetAsync(L->d_band.p, 0, sizeof(double) * (size_t)L->bandDoubles, s));
-    CK(cudaMemsetAsync(L->d_status.p, 0, sizeof(int), s));
     const long long fillN = (long long)P.nb * P.dpn * P.dpn;
     k_band_fill<<<(unsigned)((fillN + 255) / 256), 256, 0, s>>>(
         P.nb, P.dpn, dptr<int>(ctx->d_bRow), dptr<int>(ctx->d_bCol), dptr<double>(ctx->d_K64),
