@@ -278,6 +278,11 @@ int astro_get_dims(const astro_ctx *ctx, astro_dims *out);
  * double-float solve added to x.  1: the sweeps in FP64 from the factor itself (no copies, half
  * the device memory); 2: the double-float sweeps without the refinement pass. */
 #define ASTRO_OPT_PANELS_SOLVE 8
+/* ASTRO_OPT_RESIDENT (default 1): the iterations of the static and thermal solvers run resident on the SMs, one
+ * launch a restart cycle, where the operator fits their shared memory.  0: as captured graphs at every size (the
+ * same arithmetic but for the order of sums), for profilers that want the single kernels and for tests of the
+ * graphs on small models. */
+#define ASTRO_OPT_RESIDENT 9
 int astro_set_option(astro_ctx *ctx, int32_t option, int32_t value);
 
 /* The CUDA stream (cudaStream_t) the context launches on, for callers that order their own work

@@ -1321,6 +1321,10 @@ extern "C" int astro_set_option(astro_ctx *ctx, int32_t option, int32_t value) {
         krylov_release(ctx);  // recapture the cycles in the chosen form
         return ASTRO_OK;
     }
+    if (option == ASTRO_OPT_RESIDENT) {
+        ctx->resident = value ? 1 : 0;
+        return ASTRO_OK;
+    }
     if (option == ASTRO_OPT_CASES_TWIST) {
         if (value < 0 || value > 2) return set_err(ctx, ASTRO_ERR_ARG, "ASTRO_OPT_CASES_TWIST: 0, 1 or 2");
         ctx->casesTwist = value;

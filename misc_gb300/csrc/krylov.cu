@@ -942,7 +942,7 @@ static int resident_plan(astro_ctx *ctx, GmresWork &W, const Op<TM> &op, int m, 
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device);
     cudaDeviceGetAttribute(&maxSm, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
     const int R = std::max((N + std::min(sms, kResMaxCtas) - 1) / std::min(sms, kResMaxCtas), (int)std::ceil(std::sqrt(N / 10.0))), G = (N + R - 1) / R;
-    if (!coop || (POLY && R > kResMaxRows)) return ASTRO_OK;
+    if (!ctx->resident || !coop || (POLY && R > kResMaxRows)) return ASTRO_OK;
     const void *f = (const void *)k_gmres_resident<TM, TV, DPN, POLY>;
     cudaFuncAttributes fa;
     CK(cudaFuncGetAttributes(&fa, f));

@@ -1089,7 +1089,7 @@ static int cg_resident_plan(astro_ctx *ctx, ThermPlan *T, CgRes *A, size_t *smem
     cudaFuncAttributes fa;
     CK(cudaFuncGetAttributes(&fa, k_cg_resident));
     const size_t room = (size_t)maxSm - fa.sharedSizeBytes;
-    if (!coop || cg_res_layout(N, A->op.S, R, R, 0).total > room) return ASTRO_OK;
+    if (!ctx->resident || !coop || cg_res_layout(N, A->op.S, R, R, 0).total > room) return ASTRO_OK;
     int HP[2] = {0, 0};
     int *d_HP = &A->sc->its;  // counted in the iterations' place
     CK(cudaMemsetAsync(d_HP, 0, sizeof(HP), ctx->stream));
