@@ -283,6 +283,10 @@ int astro_get_dims(const astro_ctx *ctx, astro_dims *out);
  * same arithmetic but for the order of sums), for profilers that want the single kernels and for tests of the
  * graphs on small models. */
 #define ASTRO_OPT_RESIDENT 9
+/* ASTRO_OPT_POLL_LIMIT (default 0: about a second): how often a CTA of a kernel whose CTAs exchange data looks
+ * for a word of another before it gives up.  A solve whose wait was given up goes on in the form that has no such
+ * waits.  For tests of that path; too small a limit costs time, not results. */
+#define ASTRO_OPT_POLL_LIMIT 10
 int astro_set_option(astro_ctx *ctx, int32_t option, int32_t value);
 
 /* The CUDA stream (cudaStream_t) the context launches on, for callers that order their own work

@@ -29,6 +29,7 @@ OPT_BRICK_WARPS, OPT_PANEL_CLUSTER, OPT_CASES_CLUSTER = 4, 5, 6
 OPT_CASES_TWIST = 7
 OPT_PANELS_SOLVE = 8
 OPT_RESIDENT = 9
+OPT_POLL_LIMIT = 10
 
 _LIB = None
 

@@ -80,6 +80,7 @@ struct astro_ctx {
     void *solveWork[3] = {nullptr, nullptr, nullptr};
     int unrolledCycles = 0;  // ASTRO_OPT_UNROLLED_CYCLES
     int resident = 1;        // ASTRO_OPT_RESIDENT
+    int pollLimit = 0;       // ASTRO_OPT_POLL_LIMIT
     cudaStream_t stream = nullptr;
     cudaStream_t stream2 = nullptr;  // copies that overlap the element kernels
     // the FP32 assembly pass (one launch per colour) captured once as a graph and replayed

@@ -1321,6 +1321,11 @@ extern "C" int astro_set_option(astro_ctx *ctx, int32_t option, int32_t value) {
         krylov_release(ctx);  // recapture the cycles in the chosen form
         return ASTRO_OK;
     }
+    if (option == ASTRO_OPT_POLL_LIMIT) {
+        if (value < 0) return set_err(ctx, ASTRO_ERR_ARG, "ASTRO_OPT_POLL_LIMIT: 0 or a number of polls");
+        ctx->pollLimit = value;
+        return ASTRO_OK;
+    }
     if (option == ASTRO_OPT_RESIDENT) {
         ctx->resident = value ? 1 : 0;
         return ASTRO_OK;

@@ -742,6 +742,7 @@ struct GmresWork {
         bool on = false;
         int R = 0, G = 0, H = 0, P = 0, vShared = 0;
         size_t smem = 0;
+        int polls = kSpinLimit;
     } res;
     DevBuf polyW, resWords;  // its hop weights and exchanged words
     // vector that scales a residual into the preconditioner's input: D^-1 (Jacobi) or S (poly)
@@ -930,6 +931,12 @@ static double sum_parts(astro_ctx *ctx, GmresWork &W, int which, int *rc) {
     return s;
 }
 
+// A code of gmres_solve that is not about the iteration (a CUDA error, no memory): the solve ends with it and x is
+// not updated.
+static bool solver_failed(int rc) {
+    return rc != ASTRO_OK && rc != ASTRO_ERR_MAXIT && rc != ASTRO_ERR_NAN && rc != ASTRO_ERR_BREAKDOWN;
+}
+
 // Rows and shared memory of the resident cycle, or off when a CTA's part does not fit.  A CTA per SM, but
 // no fewer than sqrt(N / 10) rows: every CTA adds the partial sums of all of them, which in FP64 costs
 // it a tenth of a row's products per CTA.  The halo of the rows is counted on the device (the penalty
@@ -975,6 +982,7 @@ static int resident_plan(astro_ctx *ctx, GmresWork &W, const Op<TM> &op, int m, 
     W.res.H = H;
     W.res.P = P;
     W.res.vShared = vs;
+    W.res.polls = ctx->pollLimit ? ctx->pollLimit : kSpinLimit;
     W.res.on = true;
     return ASTRO_OK;
 }
@@ -1014,6 +1022,7 @@ static cudaError_t resident_cycle(GmresWork &W, const Op<TM> &op, TV *x, const d
     A.H = W.res.H;
     A.P = W.res.P;
     A.vShared = W.res.vShared;
+    A.polls = W.res.polls;
     const void *f = (const void *)k_gmres_resident<TM, TV, DPN, POLY>;
     cudaError_t e = cudaMemsetAsync(W.resWords.p, 0, W.resWords.bytes, s);
     void *args[] = {&A};
@@ -1142,14 +1151,20 @@ static int gmres_solve(astro_ctx *ctx, GmresWork &W, const TM *K, TV *x, const d
         int j, done, breakdown, nonfinite, stuck;
     } hc;
     for (int cyc = 0; cyc < maxCycles; ++cyc) {
+        cudaError_t launched = cudaSuccess;
         if (!W.res.on) CK(cudaGraphLaunch(exec, s));
-        else if (!W.poly) CK((resident_cycle<TM, TV, DPN, false>(W, op, x, b, m, s)));
-        else if constexpr (sizeof(TV) == 4) CK((resident_cycle<TM, TV, DPN, true>(W, op, x, b, m, s)));
-        CK(cudaMemcpyAsync(&hc, &ctl->resest, sizeof(hc), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        if (hc.stuck) {
+        else if (!W.poly) launched = resident_cycle<TM, TV, DPN, false>(W, op, x, b, m, s);
+        else if constexpr (sizeof(TV) == 4) launched = resident_cycle<TM, TV, DPN, true>(W, op, x, b, m, s);
+        if (launched == cudaSuccess) {
+            CK(cudaMemcpyAsync(&hc, &ctl->resest, sizeof(hc), cudaMemcpyDeviceToHost, s));
+            CK(cudaStreamSynchronize(s));
+        }
+        if (launched != cudaSuccess || hc.stuck) {
+            // the GPU does not hold the whole grid now (other work on it): the rest of the solve as graphs
+            cudaGetLastError();
+            W.res.on = false;
             CK(cudaMemsetAsync(&ctl->stuck, 0, sizeof(int), s));
-            return set_err(ctx, ASTRO_ERR_CUDA, "a wait of the solver's cycle was given up");
+            return gmres_solve<TM, TV, DPN>(ctx, W, K, x, b, tgtAbs, maxCycles - cyc, m, iters, cycles, finalRes);
         }
         *iters += hc.j;
         *cycles += 1;
@@ -1396,6 +1411,10 @@ static int solve_static_dev(astro_ctx *ctx, const double *d_b, double *d_x, cons
         while (rc == ASTRO_OK) {
             int grc = gmres_solve<double, double, DPN>(ctx, W, K64p, x, bb, tgt, maxCycles - cycles, m,
                                                        &iters, &cycles, &est);
+            if (solver_failed(grc)) {
+                rc = grc;
+                break;
+            }
             if ((rc = true_residual<DPN>(ctx, W, 64, x, bb, &rel, r))) break;
             if (rel <= o->rtol) break;
             if (grc == ASTRO_ERR_NAN) {
@@ -1407,7 +1426,7 @@ static int solve_static_dev(astro_ctx *ctx, const double *d_b, double *d_x, cons
                 break;
             }
         }
-        CK(cudaMemcpyAsync(d_x, W.x64.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
+        if (!solver_failed(rc)) CK(cudaMemcpyAsync(d_x, W.x64.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
     } else {
         const float *K32p = ell_of<float>(ctx, &rc);
         if (rc) return rc;
@@ -1461,22 +1480,24 @@ static int solve_static_dev(astro_ctx *ctx, const double *d_b, double *d_x, cons
                 if ((rc = cuda_check(ctx, cudaGetLastError(), "preconditioner operator"))) return rc;
                 if (W.res.on) {
                     // 50 iterations as in power_lambda
-                    CK((resident_cycle<float, float, DPN, true>(W, make_op<float>(ctx, K32p), nullptr, nullptr, m, ctx->stream, 50,
-                                                                pc->degree)));
                     GmresCtl *ctl = dptr<GmresCtl>(W.ctl);
                     int stuck = 0;
-                    CK(cudaMemcpyAsync(&W.lamEst, &ctl->y[0], sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-                    CK(cudaMemcpyAsync(&stuck, &ctl->stuck, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-                    CK(cudaStreamSynchronize(ctx->stream));
-                    if (stuck) {
-                        CK(cudaMemsetAsync(&ctl->stuck, 0, sizeof(int), ctx->stream));
-                        return set_err(ctx, ASTRO_ERR_CUDA, "a wait of the power iteration was given up");
+                    const cudaError_t launched = resident_cycle<float, float, DPN, true>(
+                        W, make_op<float>(ctx, K32p), nullptr, nullptr, m, ctx->stream, 50, pc->degree);
+                    if (launched == cudaSuccess) {
+                        CK(cudaMemcpyAsync(&W.lamEst, &ctl->y[0], sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+                        CK(cudaMemcpyAsync(&stuck, &ctl->stuck, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+                        CK(cudaStreamSynchronize(ctx->stream));
                     }
-                    if (!(std::isfinite(W.lamEst) && W.lamEst > 0.0))
+                    if (launched != cudaSuccess || stuck) {  // as a given-up cycle: the rest of the solve as graphs
+                        cudaGetLastError();
+                        W.res.on = false;
+                        CK(cudaMemsetAsync(&ctl->stuck, 0, sizeof(int), ctx->stream));
+                    } else if (!(std::isfinite(W.lamEst) && W.lamEst > 0.0)) {
                         return set_err(ctx, ASTRO_ERR_NAN, "eigenvalue estimate is not positive");
-                } else if ((rc = power_lambda<OpH, float, DPN>(ctx, W.hop, (const float *)nullptr, &W.lamEst))) {
-                    return rc;
+                    }
                 }
+                if (!W.res.on && (rc = power_lambda<OpH, float, DPN>(ctx, W.hop, (const float *)nullptr, &W.lamEst))) return rc;
                 W.hopVersion = opVer;
             }
             lam = W.lamEst * pc->lambda_scale;
@@ -1534,6 +1555,10 @@ static int solve_static_dev(astro_ctx *ctx, const double *d_b, double *d_x, cons
                                                      m, &iters, &cycles, &est);
             if (rci == ASTRO_ERR_NAN) {
                 rc = set_err(ctx, ASTRO_ERR_NAN, "non-finite value in the FP32 inner solve");
+                break;
+            }
+            if (solver_failed(rci)) {
+                rc = rci;
                 break;
             }
             k_axpy_f2d<<<(n + 255) / 256, 256, 0, ctx->stream>>>(d_x, d32, n);
@@ -1874,6 +1899,10 @@ static int krylov_newmark_dpn(astro_ctx *ctx, const astro_newmark_opts *o, const
                                                      m, &iters, &cycles, &est);
             if (grc == ASTRO_ERR_NAN) {
                 rc = set_err(ctx, ASTRO_ERR_NAN, "non-finite value in the Newmark step solve");
+                break;
+            }
+            if (solver_failed(grc)) {
+                rc = grc;
                 break;
             }
             if (grc != ASTRO_OK) worst = grc;

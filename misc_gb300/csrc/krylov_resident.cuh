@@ -27,14 +27,14 @@
 // has read x from the owners of its halo, who wrote x after they had read x - 1.  The owners of a CTA's halo
 // are also those who read its rows: the pattern is symmetric.  The launch is cooperative, so all CTAs are
 // resident, and every poll is bounded: past the limit the CTA sets ctl->stuck and returns, as the others
-// then do.
+// then do; the host takes the solve on in the graph's form (x is then a part of the way, which a cycle may start from).
 #pragma once
 #include "krylov_ops.cuh"
 
 namespace astro_kry {
 
 constexpr int kResT = 1024, kResW = kResT / 32;
-constexpr int kSpinLimit = 1 << 21;  // polls of a word (more than a second)
+constexpr int kSpinLimit = 1 << 21;  // polls of a word (more than a second), unless ASTRO_OPT_POLL_LIMIT says else
 constexpr int kResMaxRows = 256;     // rows of a CTA in the hops: a warp takes eight, four lanes each
 constexpr int kResMaxCtas = 160;
 
@@ -56,6 +56,7 @@ template <class TM, class TV> struct ResArgs {
     const double *target;
     int m, N, R, G, H, P; // H, P: capacity of the halo and of a CTA's penalty entries
     int vShared;
+    int polls;            // limit of a wait
 };
 
 struct ResLayout {
@@ -331,7 +332,7 @@ __global__ void __launch_bounds__(kResT, 1) k_gmres_resident(ResArgs<TM, TV> A) 
                 w[u] = word_get(p[u]);
             }
             for (int it = 0; word_no(w[0]) != e || word_no(w[1]) != e;) {
-                if (++it > kSpinLimit) {
+                if (++it > A.polls) {
                     sStuck = 1;
                     break;
                 }
@@ -368,7 +369,7 @@ __global__ void __launch_bounds__(kResT, 1) k_gmres_resident(ResArgs<TM, TV> A) 
             const ulonglong2 *p = part + ((size_t)pass * (kMaxM + 2) + k) * A.G;
             ulonglong2 w[CN];
             bool all = false;
-            for (int it = 0; !all && it < kSpinLimit; ++it) {
+            for (int it = 0; !all && it < A.polls; ++it) {
                 all = true;
 #pragma unroll
                 for (int u = 0; u < CN; ++u) w[u] = lane + 32 * u < A.G ? word_get(p + lane + 32 * u) : make_ulonglong2(0, (unsigned long long)e << 32);
@@ -388,7 +389,7 @@ __global__ void __launch_bounds__(kResT, 1) k_gmres_resident(ResArgs<TM, TV> A) 
             const ulonglong2 *p = total + ((size_t)pass * A.G + blockIdx.x) * (kMaxM + 2) + k;
             ulonglong2 w = word_get(p);
             for (int it = 0; word_no(w) != e; w = word_get(p))
-                if (++it > kSpinLimit) {
+                if (++it > A.polls) {
                     sStuck = 1;
                     break;
                 }

@@ -5,7 +5,8 @@ import numpy as np
 import pytest
 
 from misc_gb300 import model as M
-from misc_gb300.astro import AstroError, AstroGPU
+from misc_gb300.astro import (OPT_POLL_LIMIT, OPT_RESIDENT, SOLVER_FGMRES_LEARNED, SOLVER_FGMRES_MIXED,
+                              SOLVER_GMRES_JACOBI_FP64, AstroError, AstroGPU, precond_init)
 
 pytestmark = pytest.mark.gpu
 
@@ -36,3 +37,68 @@ def test_time_stepping_after_a_failed_factorisation():
         g.panels_factor(0)
     assert e.value.code == 4
     assert np.array_equal(g.newmark_cases(1e-5, pattern, amp)[0], ref)
+
+
+def _block(resident=1, polls=0):
+    g = AstroGPU(M.hex_block(7, 6, 5, lx=0.7, ly=0.6, lz=0.5, jitter=0.1, seed=4))
+    g.set_option(OPT_RESIDENT, resident)
+    g.set_option(OPT_POLL_LIMIT, polls)
+    g.getElasticSolnLoad(1, export=False)
+    g.assemble_fp32()
+    g.scaleElasticMPC()
+    return g, g.static_rhs()
+
+
+@pytest.mark.parametrize("method", [SOLVER_GMRES_JACOBI_FP64, SOLVER_FGMRES_MIXED, SOLVER_FGMRES_LEARNED])
+def test_solve_goes_on_when_a_wait_is_given_up(method):
+    """A limit of one poll runs out in the first exchange of the resident cycle (and of the power iteration before
+    it): the solve goes on as graphs, from the same x, so with their bits; with the limit back the next one is
+    resident again."""
+    graph, b = _block(resident=0)
+    ug, sg = graph.solve_static(b, method=method, rtol=1e-10)
+    g, _ = _block()
+    u, s = g.solve_static(b, method=method, rtol=1e-10)
+    few, _ = _block(polls=1)
+    uf, sf = few.solve_static(b, method=method, rtol=1e-10)
+    assert sf.status == 0 and sf.fallback == 0 and sf.rel_residual <= 1e-10
+    assert np.array_equal(uf, ug) and sf.iterations == sg.iterations
+    few.set_option(OPT_POLL_LIMIT, 0)
+    ua, sa = few.solve_static(b, method=method, rtol=1e-10)
+    assert sa.status == 0 and sa.rel_residual <= 1e-10
+    if method != SOLVER_FGMRES_LEARNED:  # (which keeps its eigenvalue estimate, here that of the graph's iteration)
+        assert np.array_equal(ua, u) and sa.iterations == s.iterations
+
+
+def test_resident_six_dof_goes_on_when_a_wait_is_given_up():
+    g = AstroGPU(M.plate_shell(nx=9, ny=7, lx=0.9, ly=0.7, t=0.05, E=7.0e10, nu=0.33, rho=2700.0, pressure=1.0e3))
+    g.getElasticSolnLoad(1, export=False)
+    g.scaleElasticMPC()
+    b = g.static_rhs()
+    p = precond_init(16, 1000.0, 6)
+    for polls in (0, 1, 0):
+        g.set_option(OPT_POLL_LIMIT, polls)
+        u, st = g.solve_static(b, method=SOLVER_FGMRES_LEARNED, rtol=1e-8, precond=p)
+        assert st.status == 0 and st.fallback == 0 and st.rel_residual <= 1e-8
+
+
+def test_three_contexts_solve_at_once():
+    """Resident launches of three contexts, each as wide as the GPU, from three threads."""
+    import threading
+    made = [_block() for _ in range(3)]
+    ref = made[0][0].solve_static(made[0][1], rtol=1e-10)[0]
+    out = [None] * 3
+    gate = threading.Barrier(3)
+
+    def run(i):
+        g, b = made[i]
+        gate.wait()
+        out[i] = [g.solve_static(b, method=m, rtol=1e-10) for _ in range(4) for m in (SOLVER_GMRES_JACOBI_FP64, SOLVER_FGMRES_LEARNED)]
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for res in out:
+        for u, st in res:
+            assert st.status == 0 and st.rel_residual <= 1e-10
+            assert np.linalg.norm(u - ref) <= 1e-6 * np.linalg.norm(ref)
