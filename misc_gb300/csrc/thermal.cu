@@ -872,6 +872,7 @@ struct CgRes {
     ulonglong2 *words;  // all 0 at launch: cg_words()
     double target;      // on |r|, looked at every kCgBatch iterations and after the last
     int iters, N, R, G, H, P;
+    int polls;          // limit of a wait
 };
 constexpr int kCgResIters = 1024;  // iterations of a launch
 struct CgResLayout {
@@ -957,7 +958,7 @@ __global__ void __launch_bounds__(astro_kry::kResT, 1) k_cg_resident(CgRes A) {
     // a word of number e, polled
     auto until = [&](ulonglong2 w, const ulonglong2 *p, unsigned e) {  // (w: the word's first load)
         for (int it = 0; word_no(w) != e; w = word_get(p))
-            if (++it > kSpinLimit) {
+            if (++it > A.polls) {
                 sStuck = 1;
                 break;
             }
@@ -1112,6 +1113,7 @@ static int cg_resident_plan(astro_ctx *ctx, ThermPlan *T, CgRes *A, size_t *smem
     A->G = G;
     A->H = HP[0];
     A->P = HP[1];
+    A->polls = ctx->pollLimit ? ctx->pollLimit : astro_kry::kSpinLimit;
     return ASTRO_OK;
 }
 
@@ -1638,9 +1640,12 @@ extern "C" int astro_thermal_solve(astro_ctx *ctx, const double *rhs, double *dt
                                                            dptr<double>(T->d_ell),
                                                            newCols ? dptr<int>(T->d_ellCol) : nullptr);
     double *pPap = dptr<double>(part), *pRz = pPap + rg, *pRr = pRz + rg;
-    k_cg_init<<<rg, kCgThreads, 0, s>>>(A, dptr<double>(b), dptr<double>(x), dptr<double>(dinv), dptr<double>(r),
-                                        dptr<double>(p), pRz, pRr);
-    k_cg_init_sum<<<1, kCgThreads, 0, s>>>((int)rg, pRz, pRr, S);
+    auto start = [&] {
+        k_cg_init<<<rg, kCgThreads, 0, s>>>(A, dptr<double>(b), dptr<double>(x), dptr<double>(dinv), dptr<double>(r),
+                                            dptr<double>(p), pRz, pRr);
+        k_cg_init_sum<<<1, kCgThreads, 0, s>>>((int)rg, pRz, pRr, S);
+    };
+    start();
     auto iterate = [&](int it0, int count) {
         for (int k = 0; k < count; ++k) {
             const int par = (it0 + k) & 1, want = k == count - 1;
@@ -1664,8 +1669,8 @@ extern "C" int astro_thermal_solve(astro_ctx *ctx, const double *rhs, double *dt
         return rc;
     }
     // a batch as a graph, kept while the matrix tables stay where they are
-    if (Q.R) {
-    } else if (!T->cgExec || std::memcmp(&T->cgMat, &A, sizeof(A)) != 0) {
+    auto batch = [&]() -> int {
+        if (T->cgExec && std::memcmp(&T->cgMat, &A, sizeof(A)) == 0) return ASTRO_OK;
         if (T->cgExec) cudaGraphExecDestroy(T->cgExec);
         T->cgExec = nullptr;
         cudaGraph_t g = nullptr;
@@ -1676,12 +1681,14 @@ extern "C" int astro_thermal_solve(astro_ctx *ctx, const double *rhs, double *dt
         }
         if (e == cudaSuccess) e = cudaGraphInstantiate(&T->cgExec, g, 0);
         if (g) cudaGraphDestroy(g);
-        if ((rc = cuda_check(ctx, e, "thermal solve graph"))) {
-            T->cgExec = nullptr;
-            dev_free(b);
-            return rc;
-        }
-        std::memcpy(&T->cgMat, &A, sizeof(A));
+        const int grc = cuda_check(ctx, e, "thermal solve graph");
+        if (grc) T->cgExec = nullptr;
+        else std::memcpy(&T->cgMat, &A, sizeof(A));
+        return grc;
+    };
+    if (!Q.R && (rc = batch())) {
+        dev_free(b);
+        return rc;
     }
     double rr = 0.0;
     CgScal hs{};
@@ -1692,6 +1699,7 @@ extern "C" int astro_thermal_solve(astro_ctx *ctx, const double *rhs, double *dt
     if (bn == 0.0) status = ASTRO_OK;
     while (!rc && status == ASTRO_ERR_MAXIT && it < max_iters) {
         cudaError_t e = cudaSuccess;
+        bool refused = false;
         if (Q.R) {
             Q.iters = std::min(kCgResIters, max_iters - it);
             Q.target = rtol * bn;
@@ -1699,22 +1707,29 @@ extern "C" int astro_thermal_solve(astro_ctx *ctx, const double *rhs, double *dt
             e = cudaMemsetAsync(T->d_words.p, 0, T->d_words.bytes, s);
             if (e == cudaSuccess)
                 e = cudaLaunchCooperativeKernel((const void *)k_cg_resident, dim3(Q.G), dim3(astro_kry::kResT), args, smem, s);
+            refused = e != cudaSuccess;
         } else {
             const int chunk = std::min(kCgBatch, max_iters - it);
             if (chunk == kCgBatch) cudaGraphLaunch(T->cgExec, s);
-            else iterate(it, chunk);
+            else iterate(0, chunk);  // (after whole batches: even)
             it += chunk;
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(&hs, S, sizeof(hs), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (refused || (e == cudaSuccess && hs.stuck)) {
+            // the GPU does not hold the whole grid now (other work on it): on from this x in batches (the CTAs
+            // may have stopped at different iterations, so r and p are formed anew)
+            cudaGetLastError();
+            if (!refused) it += hs.its;
+            Q.R = 0;
+            if ((rc = cuda_check(ctx, cudaMemsetAsync(sc.p, 0, sizeof(CgScal), s), "thermal solve")) || (rc = batch())) break;
+            start();
+            continue;
+        }
         if ((rc = cuda_check(ctx, e, "thermal solve"))) break;
         rr = hs.rr;
         if (Q.R) it += hs.its;
-        if (hs.stuck) {
-            rc = set_err(ctx, ASTRO_ERR_CUDA, "thermal solve: a wait was given up");
-            break;
-        }
         if (!std::isfinite(rr)) {
             status = ASTRO_ERR_NAN;
             break;

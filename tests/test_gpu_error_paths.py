@@ -6,7 +6,7 @@ import pytest
 
 from misc_gb300 import model as M
 from misc_gb300.astro import (OPT_POLL_LIMIT, OPT_RESIDENT, SOLVER_FGMRES_LEARNED, SOLVER_FGMRES_MIXED,
-                              SOLVER_GMRES_JACOBI_FP64, AstroError, AstroGPU, precond_init)
+                              SOLVER_GMRES_JACOBI_FP64, AstroError, AstroGPU, precond_init, thermal_props)
 
 pytestmark = pytest.mark.gpu
 
@@ -102,3 +102,34 @@ def test_three_contexts_solve_at_once():
         for u, st in res:
             assert st.status == 0 and st.rel_residual <= 1e-10
             assert np.linalg.norm(u - ref) <= 1e-6 * np.linalg.norm(ref)
+
+
+def _thermal(resident=1, polls=0):
+    m = M.hex_block(7, 6, 5, jitter=0.1, seed=4)
+    g = AstroGPU(m)
+    g.set_option(OPT_RESIDENT, resident)
+    g.set_option(OPT_POLL_LIMIT, polls)
+    hot = np.nonzero(m.node_list[:, 0] < 1e-9)[0] + 1
+    k, nm = len(hot), len(m.material_density)
+    g.thermal_setup(thermal_props(np.tile([50.0, 50.0, 50.0, 0.0, 0.0, 0.0], (nm, 1)), np.full(nm, 400.0),
+                                  mpc=(np.arange(k + 1), hot, np.ones(k), np.full(k, 3.0))))
+    load = g.getThermalSolnLoad(1, export=False)[0]
+    g.scaleThermalMPC()
+    return g, g.thermal_heat_gen(1.0e4, thermal_load=g.getThermalConstraintLoad(None, load))
+
+
+def test_thermal_solve_goes_on_when_a_wait_is_given_up():
+    """The resident conjugate gradients give up in their first exchange, before x moves: the batches that follow
+    start where the graph's do.  The cap on the iterations and the next solve are as ever."""
+    graph, b = _thermal(resident=0)
+    xg, sg = graph.thermal_solve(b, rtol=1e-12)
+    x, s = _thermal()[0].thermal_solve(b, rtol=1e-12)
+    g, _ = _thermal(polls=1)
+    xf, sf = g.thermal_solve(b, rtol=1e-12)
+    assert sf.status == 0 and np.array_equal(xf, xg) and sf.iterations == sg.iterations
+    with pytest.raises(AstroError) as e:
+        g.thermal_solve(b, rtol=1e-12, max_iters=21)
+    assert e.value.code == 7
+    g.set_option(OPT_POLL_LIMIT, 0)
+    xa, sa = g.thermal_solve(b, rtol=1e-12)
+    assert sa.status == 0 and np.array_equal(xa, x) and sa.iterations == s.iterations
