@@ -1269,7 +1269,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_band_solve_df(const PanelMeta *
 // (row-major) layouts, so every tile load of a warp is 32 consecutive float2 per k.
 constexpr int kCW = 4;      // warps of a leader's product (the CTAs per cluster, CS, is a template parameter: 2, 4 or 8)
 constexpr int kCaseW = 16;  // warps per CTA
-constexpr int kCaseWait = 1 << 24;  // polls of a barrier (about a second or less), then the status is set and waits skipped
+constexpr int kCaseWait = 1 << 24;  // polls of a barrier (about a second or less), unless ASTRO_OPT_POLL_LIMIT says else
 constexpr int kPrepW = 4;  // warps per CTA of the band copy
 
 struct CaseItem {
@@ -1469,23 +1469,24 @@ __device__ __forceinline__ void bar_expect(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 // (test_wait: the threads that wait have nothing else to do, and try_wait's sleep costs 40 us of a half sweep)
-template <bool CLUSTER> __device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity, const int *dead) {
-    for (int it = 0; it < kCaseWait; ++it) {
-        unsigned ok;
-        if constexpr (CLUSTER)
-            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                         : "=r"(ok)
-                         : "r"(bar), "r"(parity)
-                         : "memory");
-        else
-            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                         : "=r"(ok)
-                         : "r"(bar), "r"(parity)
-                         : "memory");
-        if (ok) return true;
-        if ((it & 1023) == 1023 && *(volatile const int *)dead) return true;  // given up elsewhere: no more waits
-    }
-    return false;
+template <bool CLUSTER> __device__ __forceinline__ bool bar_test(unsigned bar, unsigned parity) {
+    unsigned ok;
+    if constexpr (CLUSTER)
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok)
+                     : "r"(bar), "r"(parity)
+                     : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok)
+                     : "r"(bar), "r"(parity)
+                     : "memory");
+    return ok;
+}
+template <bool CLUSTER> __device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity, const int *dead, int polls) {
+    for (int left = polls; !bar_test<CLUSTER>(bar, parity);)
+        if (--left <= 0 || ((left & 1023) == 0 && *(volatile const int *)dead)) return false;  // (or given up elsewhere)
+    return true;
 }
 template <int WARPS> __device__ __forceinline__ void stage_barrier(int id) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(WARPS * 32) : "memory");
@@ -1513,7 +1514,7 @@ __global__ void __launch_bounds__(kCaseW * 32, 1) k_band_solve_cases(const Panel
                                                                      const float2 *__restrict__ Wb,
                                                                      const float2 *__restrict__ Mx, size_t mS,
                                                                      const float2 *__restrict__ Dinv, double *X, int nrhs,
-                                                                     int ring, int *status) {
+                                                                     int ring, int *status, int polls) {
     constexpr int kProdWarps = (CS - 1) * PW, H = TB / 2, C = TB / kCW;
     constexpr unsigned kRow = TB * sizeof(float2);
     cg::cluster_group cl = cg::this_cluster();
@@ -1541,17 +1542,27 @@ __global__ void __launch_bounds__(kCaseW * 32, 1) k_band_solve_cases(const Panel
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         for (int k = 0; k < 4; ++k) bar_expect(bars + 8 * k, expect);
     }
-    // arrival number n of rows (sums), and the arming of number n + 4 by one thread
+    // A thread whose wait was given up goes through the rest of its rows without arriving, arming or sending, so
+    // that no barrier counts a phase too many: the stages that need its rows give up in turn within three rows.
+    bool alive = true;
     auto gaveUp = [&] {
         if (!sDead) atomicExch(status, -1);
         sDead = 1;
+        alive = false;
     };
     auto wait = [&](unsigned bar, int n) {  // for a stage of this CTA
-        if (!bar_wait<false>(bar + 8 * (n & 3), (n >> 2) & 1, &sDead)) gaveUp();
+        if (!bar_wait<false>(bar + 8 * (n & 3), (n >> 2) & 1, &sDead, polls)) gaveUp();
     };
+    auto arrive = [&](unsigned bar, int n) {
+        if (alive) bar_arrive(bar + 8 * (n & 3));
+    };
+    auto expectNext = [&](int n) {
+        if (alive) bar_expect(bars + 8 * (n & 3), expect);
+    };
+    // arrival number n of rows (sums), and the arming of number n + 4 by one thread
     auto arrived = [&](int n, bool arm) {
-        if (!bar_wait<true>(bars + 8 * (n & 3), (n >> 2) & 1, &sDead)) gaveUp();
-        if (arm) bar_expect(bars + 8 * (n & 3), expect);
+        if (!bar_wait<true>(bars + 8 * (n & 3), (n >> 2) & 1, &sDead, polls)) gaveUp();
+        if (arm) expectNext(n);
     };
     // step t = 0 .. 2 nbc - 1: forward rows I = t, then backward rows I = 2 nbc - 1 - t.  Row k of a sweep
     // (t = k or nbc + k) has tiles d <= min(bt, k): forward L_{I,I-d} = tile (I-d, d) of Lf, backward
@@ -1641,14 +1652,14 @@ __global__ void __launch_bounds__(kCaseW * 32, 1) k_band_solve_cases(const Panel
                 DF v = {p.x, p.y};
 #pragma unroll
                 for (int m = PW / 2; m; m >>= 1) v = df_add(v, df_xor(v, m));
-                if (r % PW == 0)
+                if (r % PW == 0 && alive)
                     send_df(part + (((sums & 3) * CS + rank) * TB + i) * (unsigned)sizeof(float2), v, bar0 + 8 * (sums & 3));
             }
             // the last rows
             for (int n = max(0, k1 - k0 - 3); n < k1 - k0; ++n, ++rowsIn) {
                 arrived(rowsIn, false);
                 stage_barrier<PW>(1);
-                if (threadIdx.x == 0) bar_expect(bars + 8 * (rowsIn & 3), expect);
+                if (threadIdx.x == 0) expectNext(rowsIn);
             }
         } else if (rank == 0 && w == 3 * kCW) {
             // v = b (D^-1 b backward) less the producers' sums
@@ -1680,7 +1691,7 @@ __global__ void __launch_bounds__(kCaseW * 32, 1) k_band_solve_cases(const Panel
                 v = df_sub(v, df_tree_sum(pv));
                 sV[(sums & 3) * TB + r] = make_float2(v.hi, v.lo);
                 __syncwarp();
-                if (r == 0) bar_arrive(barV + 8 * (sums & 3));
+                if (r == 0) arrive(barV, sums);
             }
         } else if (rank == 0 && w < 3 * kCW) {
             // products: kind 0 M1 (then y), 1 M2 (and the rows to X), 2 W; columns c0 .. c0 + C - 1 of it
@@ -1730,10 +1741,10 @@ __global__ void __launch_bounds__(kCaseW * 32, 1) k_band_solve_cases(const Panel
                     // the four lanes of an entry share the CTAs
                     for (int c = l; c < CS; c += 4) {
                         if (c == 0) last(k)[i] = make_float2(y.hi, y.lo);
-                        else send_df(map_rank(ringA, c) + slot * kRow, y, map_rank(bars, c) + 8 * (rowsIn & 3));
+                        else if (alive) send_df(map_rank(ringA, c) + slot * kRow, y, map_rank(bars, c) + 8 * (rowsIn & 3));
                     }
                     __syncwarp();
-                    if (r == 0) bar_arrive(barY + 8 * (rowsIn & 3));
+                    if (r == 0) arrive(barY, rowsIn);
                     slot = nextSlot(slot);
                     stage_barrier<kCW>(1);
                 }
@@ -1755,7 +1766,7 @@ __global__ void __launch_bounds__(kCaseW * 32, 1) k_band_solve_cases(const Panel
                     if (d <= min(bt, k)) acc = product(last(k - d) + c0);
                     red2[((sums & 3) * kCW + wr) * kRedLd + r] = make_float2(acc.hi, acc.lo);
                     __syncwarp();
-                    if (r == 0) bar_arrive(barM + 8 * (sums & 3));
+                    if (r == 0) arrive(barM, sums);
                     prefetch(k + 1);
                     if (k - 2 >= k0) store(k - 2);
                 }
@@ -1777,13 +1788,17 @@ __global__ void __launch_bounds__(kCaseW * 32, 1) k_band_solve_cases(const Panel
                     u = df_add(u, df_xor(u, 2));
                     if (l == 0) sU[(sums & 3) * TB + i] = make_float2(u.hi, u.lo);
                     __syncwarp();
-                    if (r == 0) bar_arrive(barU + 8 * (sums & 3));
+                    if (r == 0) arrive(barU, sums);
                 }
             }
         }
     }
-    if (sDead) __nanosleep(1000000);  // (stores of the others still on their way)
     cluster_barrier();
+    // (all have issued their stores; what a CTA waited for has arrived, but into one that gave up some may be on
+    // their way yet, and its shared memory has to be there)
+    if (sDead)
+        for (const long long t = clock64(); clock64() - t < 1000000;) {
+        }
 }
 
 // internal-layout columns (nrhs x n) <-> the padded panel layout
@@ -2440,9 +2455,11 @@ int panels_cases_prepare(astro_ctx *ctx, int ncols, size_t *bytes) {
         if ((rc = upload(ctx, L->d_items, items.data(), sizeof(CaseItem) * items.size())) ||
             (rc = dev_alloc(ctx, L->d_X, sizeof(double) * (size_t)L->xRows * ncols)))
             return rc;
-        CK(cudaMemsetAsync(L->d_X.p, 0, sizeof(double) * (size_t)L->xRows * ncols, s));
         L->casesCols = ncols;
     }
+    // (the rows that pad a panel are never written but by the solve, which keeps zeros there and values that are not
+    // numbers too: those of an earlier run that failed)
+    CK(cudaMemsetAsync(L->d_X.p, 0, sizeof(double) * (size_t)L->xRows * ncols, s));
     if (bytes) *bytes = 2 * sizeof(float2) * (size_t)L->bandDoubles;
     return cuda_check(ctx, cudaStreamSynchronize(s), "panels cases prepare");
 }
@@ -2605,7 +2622,8 @@ int panels_cases_solve(astro_ctx *ctx, double *d_vec, cudaStream_t s) {
                                       (const float2 *)dptr<float2>(L->d_twLf), (const float2 *)dptr<float2>(L->d_twLb),
                                       (const float2 *)dptr<float2>(L->d_twWf), (const float2 *)dptr<float2>(L->d_twWb),
                                       (const float2 *)dptr<float2>(L->d_twMx), (size_t)L->twRows * TB,
-                                      (const float2 *)dptr<float2>(L->d_twDinv), X, nc, L->ring, dptr<int>(L->d_status));
+                                      (const float2 *)dptr<float2>(L->d_twDinv), X, nc, L->ring, dptr<int>(L->d_status),
+                                      ctx->pollLimit ? ctx->pollLimit : kCaseWait);
         };
         k_tw_move<<<mg, 256, 0, s>>>(nc, G, w, d_vec, dptr<int>(L->d_pos), dm, X, 0);
         CK(sweep(0, 2 * nc));
@@ -2635,7 +2653,8 @@ int panels_cases_solve(astro_ctx *ctx, double *d_vec, cudaStream_t s) {
                           (const CaseItem *)dptr<CaseItem>(L->d_items), (const float2 *)dptr<float2>(L->d_Lf),
                           (const float2 *)dptr<float2>(L->d_Lb), (const float2 *)dptr<float2>(L->d_Wf),
                           (const float2 *)dptr<float2>(L->d_Wb), (const float2 *)dptr<float2>(L->d_Mx),
-                          (size_t)L->xRows * TB, (const float2 *)dptr<float2>(L->d_Dinv), dptr<double>(L->d_X), nc, L->ring, dptr<int>(L->d_status)));
+                          (size_t)L->xRows * TB, (const float2 *)dptr<float2>(L->d_Dinv), dptr<double>(L->d_X), nc, L->ring, dptr<int>(L->d_status),
+                          ctx->pollLimit ? ctx->pollLimit : kCaseWait));
     k_panel_move<<<mg, 256, 0, s>>>(P.n, P.dpn, nc, d_vec, dptr<int>(L->d_panelOf), dptr<int>(L->d_pos),
                                     dptr<PanelMeta>(L->d_meta), dptr<double>(L->d_X), 0);
     return cuda_check(ctx, cudaGetLastError(), "panels cases solve");

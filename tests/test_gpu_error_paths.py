@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from misc_gb300 import model as M
-from misc_gb300.astro import (OPT_POLL_LIMIT, OPT_RESIDENT, SOLVER_FGMRES_LEARNED, SOLVER_FGMRES_MIXED,
+from misc_gb300.astro import (OPT_CASES_CLUSTER, OPT_POLL_LIMIT, OPT_RESIDENT, SOLVER_FGMRES_LEARNED, SOLVER_FGMRES_MIXED,
                               SOLVER_GMRES_JACOBI_FP64, AstroError, AstroGPU, precond_init, thermal_props)
 
 pytestmark = pytest.mark.gpu
@@ -133,3 +133,23 @@ def test_thermal_solve_goes_on_when_a_wait_is_given_up():
     g.set_option(OPT_POLL_LIMIT, 0)
     xa, sa = g.thermal_solve(b, rtol=1e-12)
     assert sa.status == 0 and np.array_equal(xa, x) and sa.iterations == s.iterations
+
+
+@pytest.mark.parametrize("twist", [0, 2])
+@pytest.mark.parametrize("cluster", [2, 4, 8])
+def test_time_stepping_reports_a_wait_that_is_given_up(twist, cluster):
+    """A limit of one poll runs out in every stage of the many-column solve: each launch ends by itself, the call
+    returns the error, and with the limit back the next call on the context is a fresh context's bit for bit."""
+    g, h = AstroGPU(_plate()), AstroGPU(_plate())
+    for c in (g, h):
+        c.set_option(7, twist)
+        c.set_option(OPT_CASES_CLUSTER, cluster)
+    pattern, amp = _cases(g)
+    ref = h.newmark_cases(1e-5, pattern, amp)[0]
+    for graph in (True, False):
+        g.set_option(OPT_POLL_LIMIT, 1)
+        with pytest.raises(AstroError) as e:
+            g.newmark_cases(1e-5, pattern, amp, graph=graph)
+        assert e.value.code == 2 and "given up" in str(e.value)
+        g.set_option(OPT_POLL_LIMIT, 0)
+        assert np.array_equal(g.newmark_cases(1e-5, pattern, amp, graph=graph)[0], ref)
