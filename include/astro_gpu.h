@@ -287,6 +287,9 @@ int astro_get_dims(const astro_ctx *ctx, astro_dims *out);
  * for a word of another before it gives up.  A solve whose wait was given up goes on in the form that has no such
  * waits.  For tests of that path; too small a limit costs time, not results. */
 #define ASTRO_OPT_POLL_LIMIT 10
+/* ASTRO_OPT_FAIL_ALLOC (default 0: none): that one of the context's device allocations to come, counted from 1, is
+ * refused with ASTRO_ERR_NOMEM.  For tests of what a call leaves behind and of the paths that need less memory. */
+#define ASTRO_OPT_FAIL_ALLOC 11
 int astro_set_option(astro_ctx *ctx, int32_t option, int32_t value);
 
 /* The CUDA stream (cudaStream_t) the context launches on, for callers that order their own work

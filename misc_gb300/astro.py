@@ -30,6 +30,7 @@ OPT_CASES_TWIST = 7
 OPT_PANELS_SOLVE = 8
 OPT_RESIDENT = 9
 OPT_POLL_LIMIT = 10
+OPT_FAIL_ALLOC = 11
 
 _LIB = None
 

@@ -81,6 +81,7 @@ struct astro_ctx {
     int unrolledCycles = 0;  // ASTRO_OPT_UNROLLED_CYCLES
     int resident = 1;        // ASTRO_OPT_RESIDENT
     int pollLimit = 0;       // ASTRO_OPT_POLL_LIMIT
+    int failAlloc = 0;       // ASTRO_OPT_FAIL_ALLOC: allocations until one is refused
     cudaStream_t stream = nullptr;
     cudaStream_t stream2 = nullptr;  // copies that overlap the element kernels
     // the FP32 assembly pass (one launch per colour) captured once as a graph and replayed

@@ -66,6 +66,8 @@ int dev_alloc(astro_ctx *c, DevBuf &b, size_t bytes) {
         return ASTRO_OK;
     }
     dev_free(b);
+    if (c->failAlloc && --c->failAlloc == 0)
+        return set_err(c, ASTRO_ERR_NOMEM, "allocation refused (ASTRO_OPT_FAIL_ALLOC)");
     auto it = cap <= kPoolOne ? c->pool.find(cap) : c->pool.end();
     if (it != c->pool.end()) {
         b.p = it->second;
@@ -1319,6 +1321,11 @@ extern "C" int astro_set_option(astro_ctx *ctx, int32_t option, int32_t value) {
     if (option == ASTRO_OPT_UNROLLED_CYCLES) {
         ctx->unrolledCycles = value ? 1 : 0;
         krylov_release(ctx);  // recapture the cycles in the chosen form
+        return ASTRO_OK;
+    }
+    if (option == ASTRO_OPT_FAIL_ALLOC) {
+        if (value < 0) return set_err(ctx, ASTRO_ERR_ARG, "ASTRO_OPT_FAIL_ALLOC: 0 or a number of allocations");
+        ctx->failAlloc = value;
         return ASTRO_OK;
     }
     if (option == ASTRO_OPT_POLL_LIMIT) {

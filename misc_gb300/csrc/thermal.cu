@@ -56,7 +56,7 @@ struct ThermPlan {
     // the solve's slot-major copy of the matrix (entry s of row r at s * ld + r)
     DevBuf d_ell, d_ellCol;
     DevBuf d_words;  // exchanged by the resident solve
-    int slots = 0, ld = 0;
+    int slots = 0, ld = 0, haveCols = 0;  // haveCols: d_ellCol is filled
     // the solve's vectors and a batch of its iterations as a graph, with the pointers it was captured with
     DevBuf d_cg[8];  // x, r, z, p, Ap, 1 / diagonal, partials, scalars
     cudaGraphExec_t cgExec = nullptr;
@@ -1599,7 +1599,6 @@ extern "C" int astro_thermal_solve(astro_ctx *ctx, const double *rhs, double *dt
     DevBuf b, &x = T->d_cg[0], &r = T->d_cg[1], &z = T->d_cg[2], &p = T->d_cg[3], &Ap = T->d_cg[4], &dinv = T->d_cg[5],
               &part = T->d_cg[6], &sc = T->d_cg[7];
     int rc;
-    bool newCols = false;
     if (!T->slots) {
         for (int i = 0; i < N; ++i) T->slots = std::max(T->slots, P.bRowPtr[i + 1] - P.bRowPtr[i]);
         T->ld = (N + 31) / 32 * 32;
@@ -1612,16 +1611,23 @@ extern "C" int astro_thermal_solve(astro_ctx *ctx, const double *rhs, double *dt
             (rc = dev_alloc(ctx, Ap, sizeof(double) * N)) || (rc = dev_alloc(ctx, dinv, sizeof(double) * N)) ||
             (rc = dev_alloc(ctx, part, sizeof(double) * 3 * rg)) || (rc = dev_alloc(ctx, sc, sizeof(CgScal))))
             return rc;
-        newCols = true;
     }
     if ((rc = upload(ctx, b, rhs, sizeof(double) * N)) ||
         (rc = cuda_check(ctx, cudaMemcpyAsync(x.p, dtemp, sizeof(double) * N, cudaMemcpyHostToDevice, s), "upload"))) {
         dev_free(b);
         return rc;
     }
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
+    struct Events {
+        cudaEvent_t e0 = nullptr, e1 = nullptr;
+        Events() {
+            cudaEventCreate(&e0);
+            cudaEventCreate(&e1);
+        }
+        ~Events() {
+            cudaEventDestroy(e0);
+            cudaEventDestroy(e1);
+        }
+    } ev;
     CgMat A;
     std::memset(&A, 0, sizeof(A));  // compared bytewise as the graph's key
     A.N = N;
@@ -1634,11 +1640,16 @@ extern "C" int astro_thermal_solve(astro_ctx *ctx, const double *rhs, double *dt
     A.pv = dptr<double>(T->d_penVal);
     CgScal *S = dptr<CgScal>(sc);
     cudaMemsetAsync(sc.p, 0, sizeof(CgScal), s);
-    cudaEventRecord(e0, s);
+    cudaEventRecord(ev.e0, s);
     k_cg_ell<<<(unsigned)((ellN + 255) / 256), 256, 0, s>>>(N, T->slots, T->ld, dptr<int>(ctx->d_bRowPtr),
                                                            dptr<int>(ctx->d_bCol), dptr<double>(T->d_val),
                                                            dptr<double>(T->d_ell),
-                                                           newCols ? dptr<int>(T->d_ellCol) : nullptr);
+                                                           T->haveCols ? nullptr : dptr<int>(T->d_ellCol));
+    if ((rc = cuda_check(ctx, cudaGetLastError(), "thermal solve"))) {
+        dev_free(b);
+        return rc;
+    }
+    T->haveCols = 1;
     double *pPap = dptr<double>(part), *pRz = pPap + rg, *pRr = pRz + rg;
     auto start = [&] {
         k_cg_init<<<rg, kCgThreads, 0, s>>>(A, dptr<double>(b), dptr<double>(x), dptr<double>(dinv), dptr<double>(r),
@@ -1736,7 +1747,7 @@ extern "C" int astro_thermal_solve(astro_ctx *ctx, const double *rhs, double *dt
         }
         if (std::sqrt(rr) <= rtol * bn) status = ASTRO_OK;
     }
-    cudaEventRecord(e1, s);
+    cudaEventRecord(ev.e1, s);
     if (!rc) {
         cudaError_t e = cudaMemcpyAsync(dtemp, x.p, sizeof(double) * N, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -1749,11 +1760,9 @@ extern "C" int astro_thermal_solve(astro_ctx *ctx, const double *rhs, double *dt
         stats->rel_residual = bn > 0.0 ? std::sqrt(rr) / bn : 0.0;
         stats->residual_kind = 64;
         float ms = 0.0f;
-        cudaEventElapsedTime(&ms, e0, e1);
+        cudaEventElapsedTime(&ms, ev.e0, ev.e1);
         stats->seconds = ms * 1e-3;
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     dev_free(b);
     if (rc) return rc;
     if (status == ASTRO_ERR_MAXIT) return set_err(ctx, ASTRO_ERR_MAXIT, "thermal solve: iteration limit");

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from misc_gb300 import model as M
-from misc_gb300.astro import (OPT_CASES_CLUSTER, OPT_POLL_LIMIT, OPT_RESIDENT, SOLVER_FGMRES_LEARNED, SOLVER_FGMRES_MIXED,
+from misc_gb300.astro import (OPT_CASES_CLUSTER, OPT_FAIL_ALLOC, OPT_POLL_LIMIT, OPT_RESIDENT, SOLVER_FGMRES_LEARNED, SOLVER_FGMRES_MIXED,
                               SOLVER_GMRES_JACOBI_FP64, AstroError, AstroGPU, precond_init, thermal_props)
 
 pytestmark = pytest.mark.gpu
@@ -153,3 +153,23 @@ def test_time_stepping_reports_a_wait_that_is_given_up(twist, cluster):
         assert e.value.code == 2 and "given up" in str(e.value)
         g.set_option(OPT_POLL_LIMIT, 0)
         assert np.array_equal(g.newmark_cases(1e-5, pattern, amp, graph=graph)[0], ref)
+
+
+def test_thermal_solve_after_a_refused_allocation():
+    """Whichever of the first solve's allocations is refused, the next solve builds what is missing (the table of
+    columns among it, which only the first call fills)."""
+    x, s = _thermal()[0].thermal_solve(_thermal()[1], rtol=1e-12)
+    refused = 0
+    for k in range(1, 40):
+        g, b = _thermal()
+        g.set_option(OPT_FAIL_ALLOC, k)
+        try:
+            xk = g.thermal_solve(b, rtol=1e-12)[0]
+        except AstroError as e:
+            assert e.code == 9
+            refused += 1
+            xk = g.thermal_solve(b, rtol=1e-12)[0]
+        assert np.array_equal(xk, x), k
+        if refused < k:
+            break
+    assert refused >= 10
