@@ -1197,14 +1197,13 @@ static int hex8_gen_run(astro_ctx *ctx, const int *d_list, const std::vector<int
     A.gpcLo = g.lo;
     const bool rot = !ctx->orientIdentity;
     bool chained = false;
-    // all colours as one where the mesh is small
-    const bool once = hex_at_once(ptr.back() - ptr[0], ptr.size() - 1);
-    const std::vector<int> all = {ptr[0], ptr.back()}, &run = once ? all : ptr;
+    // all colours as one where the mesh is small (and there is room for the scratch)
     DevBuf dBlk, dRu;
+    const bool once = hex_at_once(ptr.back() - ptr[0], ptr.size() - 1) &&
+                      hex_at_once_alloc(ctx, ptr.back() - ptr[0], build && K, d_loadInt != nullptr, dBlk, dRu) == ASTRO_OK;
+    const std::vector<int> all = {ptr[0], ptr.back()}, &run = once ? all : ptr;
     A.blkOut = A.ruItem = nullptr;
     if (once) {
-        const int rc = hex_at_once_alloc(ctx, ptr.back() - ptr[0], build && K, d_loadInt != nullptr, dBlk, dRu);
-        if (rc) return rc;
         A.blkOut = dptr<double>(dBlk);
         A.ruItem = dptr<double>(dRu);
         A.K = A.loadInt = nullptr;
@@ -1245,13 +1244,12 @@ static int hex8_df_run(astro_ctx *ctx, double *K, double *d_ke, const int *d_lis
     A.K = K;
     A.keOut = d_ke;
     bool chained = false;
-    const bool once = hex_at_once(ptr.back() - ptr[0], ptr.size() - 1);
-    const std::vector<int> all = {ptr[0], ptr.back()}, &run = once ? all : ptr;
     DevBuf dBlk, dRu;
+    const bool once = hex_at_once(ptr.back() - ptr[0], ptr.size() - 1) &&
+                      hex_at_once_alloc(ctx, ptr.back() - ptr[0], K != nullptr, false, dBlk, dRu) == ASTRO_OK;
+    const std::vector<int> all = {ptr[0], ptr.back()}, &run = once ? all : ptr;
     A.blkOut = nullptr;
     if (once) {
-        const int rc = hex_at_once_alloc(ctx, ptr.back() - ptr[0], K != nullptr, false, dBlk, dRu);
-        if (rc) return rc;
         A.blkOut = dptr<double>(dBlk);
         A.K = nullptr;
     }

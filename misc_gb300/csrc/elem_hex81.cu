@@ -466,18 +466,18 @@ int hex81_run(astro_ctx *ctx, const int *d_list, const std::vector<int> &ptr, in
     // a group of a few takes an element's latency too (95 us)
     const int total = ptr.back() - ptr[0], groups = std::max(1, (total + kHexAtOnce / 2) / kHexAtOnce);
     const int size = (total + groups - 1) / std::max(1, groups);
-    A.blkOut = A.ruItem = nullptr;
+    bool once = ptr.size() > 2;
+    size_t col = 0;  // colour by colour where there is no room for the scratch
     for (int lo = ptr[0]; lo < ptr.back();) {
-        const bool once = ptr.size() > 2;
-        const int hi = once ? std::min(ptr.back(), lo + size) : ptr.back();
+        while (ptr[col + 1] <= lo) ++col;
+        int hi = std::min(ptr.back(), lo + size);
         DevBuf dBlk, dRu;
-        if (once) {
-            const int rc = hex_at_once_alloc(ctx, hi - lo, build && K, d_loadInt != nullptr, dBlk, dRu);
-            if (rc) return rc;
-            A.blkOut = dptr<double>(dBlk);
-            A.ruItem = dptr<double>(dRu);
-            A.K = A.loadInt = nullptr;
-        }
+        once = once && hex_at_once_alloc(ctx, hi - lo, build && K, d_loadInt != nullptr, dBlk, dRu) == ASTRO_OK;
+        if (!once) hi = ptr[col + 1];
+        A.blkOut = once ? dptr<double>(dBlk) : nullptr;
+        A.ruItem = once ? dptr<double>(dRu) : nullptr;
+        A.K = once ? nullptr : K;
+        A.loadInt = once ? nullptr : d_loadInt;
         A.els = d_list + lo;
         A.count = hi - lo;
         A.CItem = CItem ? CItem + 9 * (size_t)lo : nullptr;

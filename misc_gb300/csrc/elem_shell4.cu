@@ -102,7 +102,7 @@ int shell_sections_prepare(astro_ctx *ctx, const astro_model *m) {
 // may cover several colours and a colour several chunks, the updates keep the order of the list.
 // byItem (complex step): element k of the list has its own properties, props[k], and with slot adds to
 // load vector slot[k] (of lengths n and intVecSize).
-constexpr int kShellChunk = 32768;
+constexpr int kShellChunk = 32768, kShellChunkMin = 256;
 
 static int shell_pipeline(astro_ctx *ctx, const ElemDevState &st, const int *d_els, const std::vector<int> &ptr,
                           const ShellProps *props, double gpc, double *d_loadInt, double *d_intLoad, int buildMat,
@@ -113,14 +113,18 @@ static int shell_pipeline(astro_ctx *ctx, const ElemDevState &st, const int *d_e
     // per-element scratch of the pipeline, kept in the context (grown on demand)
     DevBuf &fr = ctx->d_shFr, &gp = ctx->d_shGp, &de = ctx->d_shDe, &kf = ctx->d_shKf;
     int rc;
-    const int cap = std::min(kShellChunk, last - first);
-    if (cap > ctx->shScratchEls) {
+    int cap = std::min(kShellChunk, last - first);
+    while (cap > ctx->shScratchEls) {
         ctx->shScratchEls = 0;
-        if ((rc = dev_alloc(ctx, fr, sizeof(ShellFrame) * (size_t)cap))) return rc;
-        if ((rc = dev_alloc(ctx, gp, sizeof(ShellGP) * 4 * (size_t)cap))) return rc;
-        if ((rc = dev_alloc(ctx, de, sizeof(double) * 4 * 32 * 9 * (size_t)cap))) return rc;
-        if ((rc = dev_alloc(ctx, kf, sizeof(double) * 32 * 33 * (size_t)cap))) return rc;
-        ctx->shScratchEls = cap;
+        if (!(rc = dev_alloc(ctx, fr, sizeof(ShellFrame) * (size_t)cap)) &&
+            !(rc = dev_alloc(ctx, gp, sizeof(ShellGP) * 4 * (size_t)cap)) &&
+            !(rc = dev_alloc(ctx, de, sizeof(double) * 4 * 32 * 9 * (size_t)cap)) &&
+            !(rc = dev_alloc(ctx, kf, sizeof(double) * 32 * 33 * (size_t)cap)))
+            ctx->shScratchEls = cap;
+        else if (rc != ASTRO_ERR_NOMEM || cap <= kShellChunkMin)
+            return rc;
+        else
+            cap = (cap + 1) / 2;  // smaller chunks give the same
     }
     ShellPipe A = {};
     A.nodes = dptr<double>(ctx->d_nodes);

@@ -333,13 +333,14 @@ static SolidCsArgs solid_cs_args(astro_ctx *ctx, int dvar, double h, const ElemD
 
 // The listed elements (colour by colour: colour c's from start[c]), at most kCsChunk at once.
 static int solid_cs_run(astro_ctx *ctx, const SolidCsArgs &B, const std::vector<int> &start) {
-    constexpr int kCsChunk = 1 << 17;  // 35 MB of residuals
+    constexpr int kCsChunk = 1 << 17, kCsMin = 256;  // 35 MB of residuals; no fewer where there is no room for those
     const int total = start.back();
+    int cap = std::min(total, kCsChunk);
     DevBuf ru;
-    int rc;
-    if ((rc = dev_alloc(ctx, ru, sizeof(double) * 33 * (size_t)std::min(total, kCsChunk)))) return rc;
-    for (int k0 = 0; k0 < total; k0 += kCsChunk) {
-        const int k1 = std::min(total, k0 + kCsChunk);
+    for (int rc; (rc = dev_alloc(ctx, ru, sizeof(double) * 33 * (size_t)cap)) != ASTRO_OK; cap = (cap + 1) / 2)
+        if (rc != ASTRO_ERR_NOMEM || cap <= kCsMin) return rc;
+    for (int k0 = 0; k0 < total; k0 += cap) {
+        const int k1 = std::min(total, k0 + cap);
         auto part = [&](int lo, int hi) {
             SolidCsArgs A = B;
             A.els = B.els + lo;

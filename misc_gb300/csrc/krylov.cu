@@ -794,7 +794,10 @@ template <class TM> static const TM *ell_of(astro_ctx *ctx, int *rc) {
         if ((*rc = dev_alloc(ctx, ctx->d_ellCol, sizeof(int) * (size_t)S * ld))) return nullptr;
         needCol = true;
     }
-    if (!dst.p && (*rc = dev_alloc(ctx, dst, sizeof(TM) * (size_t)S * dd * ld))) return nullptr;
+    if (!dst.p && (*rc = dev_alloc(ctx, dst, sizeof(TM) * (size_t)S * dd * ld))) {
+        if (needCol) dev_free(ctx->d_ellCol);  // not filled: the next call's
+        return nullptr;
+    }
     if (ver != cur || needCol) {
         const long long tot = (long long)S * ld;
         const unsigned g = (unsigned)((tot + 255) / 256);
@@ -957,7 +960,8 @@ static int resident_plan(astro_ctx *ctx, GmresWork &W, const Op<TM> &op, int m, 
     auto need = [&](int H, int P, int vShared) { return res_layout<TM, TV, DPN>(N, op.S, R, H, P, m, deg, vShared).total; };
     if (need(R, 0, 0) > room) return ASTRO_OK;
     int HP[2] = {0, 0}, rc;
-    if (!W.resWords.p && (rc = dev_alloc(ctx, W.resWords, sizeof(ulonglong2) * res_words<TV, DPN>(N, G)))) return rc;
+    if (!W.resWords.p && (rc = dev_alloc(ctx, W.resWords, sizeof(ulonglong2) * res_words<TV, DPN>(N, G))))
+        return rc == ASTRO_ERR_NOMEM ? ASTRO_OK : rc;
     int *d_HP = reinterpret_cast<int *>(W.tgt.p);
     static_assert(sizeof(HP) <= sizeof(double), "counted in the target's place");
     CK(cudaMemsetAsync(d_HP, 0, sizeof(HP), ctx->stream));

@@ -623,9 +623,13 @@ static int ldl_fact_dev(astro_ctx *ctx, double *d_A, const int *d_R, const int *
     constexpr int kNone = 0x7f7f7f7f;
     int rc, hs = 0;
     SkyPlan L;
-    if (sky_plan(h_R, n, L)) {
-        SkyPanels S;
-        if ((rc = sky_upload(ctx, L, d_R, false, S))) return rc;
+    SkyPanels S;
+    bool tiled = sky_plan(h_R, n, L);
+    if (tiled && (rc = sky_upload(ctx, L, d_R, false, S))) {
+        if (rc != ASTRO_ERR_NOMEM) return rc;
+        tiled = false;  // no room for the tiles: the row sweep needs none
+    }
+    if (tiled) {
         CK(cudaMemsetAsync(st, 0x7f, sizeof(int), ctx->stream));
         CK(cudaMemsetAsync(st + 1, 0, sizeof(int), ctx->stream));
         // as many CTAs a panel as its update has tiles, and as the GPU holds for all panels
@@ -696,11 +700,14 @@ extern "C" int astro_ldl_solve(astro_ctx *ctx, double *soln, const double *rhs, 
     CK(cudaMemcpyAsync(dR.p, l_range, sizeof(int) * (size_t)(l_dim + 1), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(db.p, rhs, sizeof(double) * (size_t)l_dim, cudaMemcpyHostToDevice, ctx->stream));
     SkyPlan P;
-    if (sky_plan(l_range, l_dim, P)) {
-        SkyPanels S;
-        if ((rc = sky_upload(ctx, P, dptr<int>(dR), true, S)) ||
-            (rc = sky_scratch(ctx, ctx->d_sky[8], sizeof(double) * (size_t)P.rows)))
-            return rc;
+    SkyPanels S;
+    bool tiled = sky_plan(l_range, l_dim, P);
+    if (tiled && ((rc = sky_upload(ctx, P, dptr<int>(dR), true, S)) ||
+                  (rc = sky_scratch(ctx, ctx->d_sky[8], sizeof(double) * (size_t)P.rows)))) {
+        if (rc != ASTRO_ERR_NOMEM) return rc;
+        tiled = false;  // as in the factor
+    }
+    if (tiled) {
         double *tf = dptr<double>(ctx->d_sky[6]), *tb = dptr<double>(ctx->d_sky[7]);
         k_sky_tiles<<<(unsigned)P.tiles, kSkyThreads, 0, ctx->stream>>>(S, dptr<double>(dL), tf, tb);
         const int nring = P.maxBt + 2;

@@ -1107,7 +1107,8 @@ static int cg_resident_plan(astro_ctx *ctx, ThermPlan *T, CgRes *A, size_t *smem
         cudaGetLastError();
         return ASTRO_OK;
     }
-    if (!T->d_words.p && (rc = dev_alloc(ctx, T->d_words, sizeof(ulonglong2) * cg_words(N, G)))) return rc;
+    if (!T->d_words.p && (rc = dev_alloc(ctx, T->d_words, sizeof(ulonglong2) * cg_words(N, G))))
+        return rc == ASTRO_ERR_NOMEM ? ASTRO_OK : rc;
     A->words = dptr<ulonglong2>(T->d_words);
     A->R = R;
     A->G = G;
@@ -1264,16 +1265,18 @@ static int up_opt(astro_ctx *ctx, DevBuf &b, const double *h, int n) {
 // The bricks of a colour-grouped list (device els, colour c covering ptr[c] .. ptr[c+1]): the element
 // stage for a chunk of up to 256 k elements of any colours (90 MB of scratch), then the updates colour
 // by colour in the order of the list.
-constexpr int kThChunk = 1 << 18;
+constexpr int kThChunk = 1 << 18, kChunkMin = 256;
 
 template <class F>
 static int th_bricks(astro_ctx *ctx, ThermPlan *T, ThArgs A, const int *els, const std::vector<int> &ptr,
                      const double *mult, F stage) {
-    const int total = ptr.back(), cap = std::min(kThChunk, total);
+    const int total = ptr.back();
+    int cap = std::min(kThChunk, total);
     if (!total) return ASTRO_OK;
-    if (T->d_scr.bytes < sizeof(double) * kThScr * (size_t)cap) {
+    while (T->d_scr.bytes < sizeof(double) * kThScr * (size_t)cap) {
         const int rc = dev_alloc(ctx, T->d_scr, sizeof(double) * kThScr * (size_t)cap);
-        if (rc) return rc;
+        if (rc && (rc != ASTRO_ERR_NOMEM || cap <= kChunkMin)) return rc;
+        if (rc) cap = (cap + 1) / 2;  // smaller chunks give the same
     }
     A.scr = dptr<double>(T->d_scr);
     for (int c0 = 0; c0 < total; c0 += cap) {
