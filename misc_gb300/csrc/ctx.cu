@@ -43,9 +43,10 @@ int cuda_check(astro_ctx *c, cudaError_t e, const char *what) {
 // The entry points allocate their temporaries per call, and cudaMalloc and cudaFree cost tens to
 // hundreds of microseconds each (cudaFree waits for the device): assembly at a displaced state and one
 // product with the operator on the 64x32x32 block 5.18 -> 4.40 ms without them.  So freed buffers stay with their context and the
-// next request of about the size takes one.  All work on a context's buffers is issued on its one
-// stream by its one host thread, so a buffer is reused in the order of that stream (the staged host
-// copies synchronise it first).  Bounded: buffers above kPoolOne and what exceeds kPoolAll go back to
+// next request of about the size takes one.  Work on a context's buffers is issued on its stream by its
+// one host thread, so a buffer is reused in the order of that stream.  What runs on other streams waits
+// for it first: the staged host copies each time, the export's column numbers (stream2) when their
+// buffer is new, which it then keeps (ensure_io).  Bounded: buffers above kPoolOne and what exceeds kPoolAll go back to
 // the driver at once, everything when an allocation fails and with the context.
 constexpr size_t kPoolOne = 32u << 20, kPoolAll = 256u << 20;
 
@@ -494,7 +495,11 @@ int ensure_io(astro_ctx *ctx, bool exportMat) {
     if (!ctx->d_ioInt.p && (rc = dev_alloc(ctx, ctx->d_ioInt, sizeof(double) * P.n))) return rc;
     if (exportMat) {
         if (!ctx->d_exMat.p && (rc = dev_alloc(ctx, ctx->d_exMat, sizeof(double) * (size_t)P.elMatSize))) return rc;
-        if (!ctx->d_exCols.p && (rc = dev_alloc(ctx, ctx->d_exCols, sizeof(int) * (size_t)P.elMatSize))) return rc;
+        if (!ctx->d_exCols.p) {
+            if ((rc = dev_alloc(ctx, ctx->d_exCols, sizeof(int) * (size_t)P.elMatSize))) return rc;
+            // written on stream2: queued work may still use the block that the buffer was before
+            CK(cudaStreamSynchronize(ctx->stream));
+        }
     }
     if (!ctx->stream2) CK(cudaStreamCreateWithFlags(&ctx->stream2, cudaStreamNonBlocking));
     return ASTRO_OK;

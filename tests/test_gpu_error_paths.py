@@ -268,3 +268,18 @@ def test_calls_with_a_refused_allocation(name):
         if not refused:
             break
     assert not refused and routes >= 1, (k, routes)
+
+
+def test_first_export_after_a_failed_call():
+    """A call that fails leaves work queued on buffers that it has given back; the column numbers of the first export
+    are formed on another stream, in a buffer that may be one of them."""
+    m = _bricks()
+    values, cols = AstroGPU(m).getElasticSolnLoad(1)[2:4]
+    g = AstroGPU(m)
+    u = np.random.default_rng(1).normal(0.0, 1e-3, g.n)
+    for _ in range(3):
+        with pytest.raises(AstroError) as e:  # no time step
+            g.getElasticSolnLoad(1, state=M.make_state(g.n, disp=u, prev_disp=u, prev_vel=u, prev_acc=u, dynamic=1), export=False)
+        assert e.value.code == 1
+    v, c = g.getElasticSolnLoad(1)[2:4]
+    assert np.array_equal(c, cols) and np.array_equal(v, values)
