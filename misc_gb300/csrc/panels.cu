@@ -502,25 +502,13 @@ __global__ void __launch_bounds__(kThreads, MODE == 2 ? 1 : 2) k_band_ldl(const 
     }
 }
 
-// 1 / d by one third-order (Halley) step on the hardware's approximate reciprocal: with
-// y (1 - e) d = 1, y (1 + e + e^2) leaves a relative error of e^3 (below 2^-57 for the 20 bits of
-// the approximation), then one rounding.  Subnormal and huge arguments, for which the approximation
-// flushes or overflows, take the division.
-__device__ __forceinline__ double recip64(double d) {
-    const unsigned ex = ((unsigned)__double2hiint(d) >> 20) & 0x7ffu;
-    if (ex < 4u || ex > 2040u) return 1.0 / d;
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    const double e = fma(-d, y, 1.0);
-    return fma(y, fma(e, e, e), y);
-}
-
 // LDL^T of the lower triangle of a 32 x 32 tile in shared memory (L below the diagonal, D on it),
 // the whole CTA.  GB300's FP64 pipe takes one warp instruction per 19 clocks from an SM and one
 // per 64 from a warp (measured), so the chain is kept to one warp and short: it factors four
 // columns at a time in registers (lane = row), the next four columns are brought up to date by
-// four warps, and the remaining columns within the bandwidth by warps 1 .. 7 while warp 0 factors on
-// (20.7 k clocks for a full tile).
+// four warps, and the remaining columns within the bandwidth by warps 1 .. 7 while warp 0 factors on.
+// (The pivots' reciprocals are the division's: one from the hardware's approximation and a step of third
+// order was a last place off in 1 of 4,000, for 3 to 5 % of a skyline factor and solve.)
 __device__ void tile_ldl(double (*S)[TB + 1], double (*sU)[4][TB], int t, int bw) {
     const int lane = t & 31, w = t >> 5;
     for (int b = 0; b < 8; ++b) {
@@ -532,7 +520,7 @@ __device__ void tile_ldl(double (*S)[TB + 1], double (*sU)[4][TB], int t, int bw
             for (int k = 0; k < 4; ++k) v[k] = S[lane][c0 + k];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const double inv = recip64(__shfl_sync(0xffffffffu, v[k], c0 + k));
+                const double inv = 1.0 / __shfl_sync(0xffffffffu, v[k], c0 + k);
                 const double l = v[k] * inv;
 #pragma unroll
                 for (int m = k + 1; m < 4; ++m) v[m] = fma(-l, __shfl_sync(0xffffffffu, v[k], c0 + m), v[m]);
