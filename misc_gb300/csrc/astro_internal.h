@@ -92,6 +92,7 @@ struct astro_ctx {
     // host model copy
     std::vector<double> nodes;  // (N,3)
     std::vector<int> elist;     // (E,8)
+    int repeats = 0;            // a brick names a node twice (a collapsed hexahedron)
     std::vector<int> etype, esec;
     std::vector<double> elMat;  // per element materialElastic(9) (solids)
     std::vector<double> elDensity;  // per element materialDensity (solids)

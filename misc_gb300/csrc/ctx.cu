@@ -187,6 +187,9 @@ extern "C" int astro_ctx_create(const astro_model *m, astro_ctx **out) {
     // host model copies
     ctx->nodes.assign(m->node_list, m->node_list + 3 * (size_t)P.N);
     ctx->elist.assign(m->element_list, m->element_list + 8 * (size_t)P.E);
+    for (int e = 0; e < P.E && !ctx->repeats; ++e)
+        for (int a = 1; a < 8 && m->element_type[e] != 41; ++a)
+            for (int b = 0; b < a; ++b) ctx->repeats |= ctx->elist[8 * (size_t)e + a] == ctx->elist[8 * (size_t)e + b];
     ctx->etype.assign(m->element_type, m->element_type + P.E);
     ctx->esec.assign(m->element_section, m->element_section + P.E);
     const int S = m->num_sections;

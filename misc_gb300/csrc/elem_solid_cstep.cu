@@ -27,6 +27,7 @@ namespace {
 struct SolidCsArgs {
     const int *els;  // listed elements (0-based)
     int count;
+    int repeats;     // elements may name a node twice
     double *ru;      // their Im(Ru): 33 values each, shape function by shape function
     const int *etype, *elist, *rank, *esec;
     const double *nodes;      // (N,3), real design values applied
@@ -254,10 +255,9 @@ __global__ void __launch_bounds__(8 * kCsItems) k_solid_cstep(SolidCsArgs A) {
         }
 }
 
-// Subtracts the Im(Ru) of one colour's elements, a thread per element and shape function.
-__global__ void k_solid_cs_add(SolidCsArgs A) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x, q = t / 11, a = t % 11;
-    if (q >= A.count) return;
+// Subtracts the Im(Ru) of one colour's elements, a thread per element and shape function (where an element may
+// name a node twice, its first thread takes them all in turn).
+__device__ __forceinline__ void cs_add(const SolidCsArgs &A, int q, int a) {
     const int e = A.els[q], et = A.etype[e];
     const double *ru = A.ru + 33 * (size_t)q + 3 * a;
     if (a < 8) {
@@ -268,6 +268,13 @@ __global__ void k_solid_cs_add(SolidCsArgs A) {
         double *intAcc = A.dvars ? A.intAcc + (size_t)(A.dvars[q] - A.dvarBase) * A.intAccStride : A.intAcc;
         for (int v = 0; v < 3; ++v) intAcc[A.intVecOff[e] + 3 * v + a - 8] -= ru[v];
     }
+}
+__global__ void k_solid_cs_add(SolidCsArgs A) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, q = t / 11, a = t % 11;
+    if (q >= A.count) return;
+    if (!A.repeats) cs_add(A, q, a);
+    else if (a == 0)
+        for (int k = 0; k < 11; ++k) cs_add(A, q, k);
 }
 
 }  // namespace
@@ -301,6 +308,7 @@ static void solid_dvar_elements(const astro_ctx *ctx, int dvar, std::vector<int>
 static SolidCsArgs solid_cs_args(astro_ctx *ctx, int dvar, double h, const ElemDevState &s, double *d_acc,
                                  double *d_intAcc) {
     SolidCsArgs A;
+    A.repeats = ctx->repeats;
     A.etype = dptr<int>(ctx->d_etype);
     A.elist = dptr<int>(ctx->d_elist);
     A.rank = dptr<int>(ctx->d_rank);

@@ -256,6 +256,7 @@ struct ThArgs {
     double *load, *val;
     double *scr;  // bricks: per listed element kThScr doubles (the element stage's results)
     int q0;       // bricks, scatter: the colour's first element in the list
+    int repeats;  // bricks, scatter: elements may name a node twice
 };
 
 template <int NPE>
@@ -527,20 +528,26 @@ __global__ void __launch_bounds__(kThThreads) k_th_brick_heat(ThArgs A, double q
 }
 
 // One colour's bricks from the scratch: 64 threads an element for the matrix entries (buildMat), then 8
-// for the load: -Rt, or with mult + mult[element] times the heat generation
+// for the load: -Rt, or with mult + mult[element] times the heat generation.  Where an element may name a
+// node twice, its entries for that node are one: a thread an element then, its entries in turn.
 __global__ void k_th_brick_add(ThArgs A, const double *__restrict__ mult) {
     const int per = A.buildMat ? 72 : 8;
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= (long long)per * A.count) return;
-    const int q = A.q0 + (int)(t / per), i = (int)(t % per) - (per - 8);
-    const int e = A.els[q];
-    const double *scr = A.scr + (size_t)q * kThScr;
-    if (i < 0) {
-        const int ab = i + 64, a = ab >> 3, b = ab & 7;
-        A.val[A.elBlk[64 * (size_t)e + ab]] += scr[a <= b ? th_sym(a, b) : th_sym(b, a)];
-    } else if (A.load) {
-        const int r = A.rank[A.elist[8 * (size_t)e + i] - 1] - 1;
-        A.load[r] += mult ? mult[q] * scr[36 + i] : -scr[36 + i];
+    auto add = [&](int q, int i) {
+        const int e = A.els[q];
+        const double *scr = A.scr + (size_t)q * kThScr;
+        if (i < 0) {
+            const int ab = i + 64, a = ab >> 3, b = ab & 7;
+            A.val[A.elBlk[64 * (size_t)e + ab]] += scr[a <= b ? th_sym(a, b) : th_sym(b, a)];
+        } else if (A.load) {
+            const int r = A.rank[A.elist[8 * (size_t)e + i] - 1] - 1;
+            A.load[r] += mult ? mult[q] * scr[36 + i] : -scr[36 + i];
+        }
+    };
+    if (!A.repeats) {
+        if (t < (long long)per * A.count) add(A.q0 + (int)(t / per), (int)(t % per) - (per - 8));
+    } else if (t < A.count) {
+        for (int i = 8 - per; i < 8; ++i) add(A.q0 + (int)t, i);
     }
 }
 
@@ -1253,6 +1260,7 @@ static ThArgs th_args(astro_ctx *ctx, ThermPlan *T) {
     A.elBlk = dptr<int>(ctx->d_elBlk);
     A.props = dptr<double>(T->d_props);
     A.shell = ctx->hasShell;
+    A.repeats = ctx->repeats;
     return A;
 }
 
