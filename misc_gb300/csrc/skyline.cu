@@ -559,9 +559,9 @@ struct SkyPlan {
 constexpr size_t kSkyRingMax = 128 * 1024;  // shared memory for the solve's ring of solved rows
 
 // Splits the profile at the rows that no later row reaches across (panels of at least 64 rows and
-// n / 128, so that a profile of many tiny blocks does not become as many padded tiles).  False where
-// band tiles do not suit the profile: the band of its longest row is so much larger than the profile
-// itself (over 8 times, and over 256 MB) or so wide that the row sweeps of one CTA are the better way.
+// n / 128, so that a profile of many tiny blocks does not become as many padded tiles).  False where the
+// tiles take too much memory (the band of the longest row over 8 times the profile, and over 256 MB) or the
+// ring of solved rows more shared memory than there is.
 static bool sky_plan(const int *R, int n, SkyPlan &L) {
     std::vector<int> reach(n + 1);  // first column of any row >= i
     reach[n] = n;
@@ -598,6 +598,27 @@ static bool sky_plan(const int *R, int n, SkyPlan &L) {
     return true;
 }
 
+// CTAs a panel of the factor: as many as its update has tiles, and as the GPU holds for all panels.
+static int sky_ctas(const SkyPlan &L, int sms) {
+    int cs = 1;
+    while (cs < 16 && cs < L.maxBt * (L.maxBt + 1) / 2 && 2 * cs * (int)L.meta.size() <= sms) cs *= 2;
+    return cs;
+}
+
+// Whether the factor is shorter in tiles than by the row sweep.  Tiles: the widest panel's block columns at
+// 15 us and its tile updates at 10.4 us a CTA (4,000 rows of 900 entries 31 ms, 12,000 of 2 5.8 ms).  Rows: 1.35 us
+// each, 4.35 in a CTA wider than a warp, and 0.07 us an entry (20 ms where the last of 4,000 rows of 2 spans
+// the profile; that row's band takes 218 ms in tiles; with a last row of 500 entries 18.9 and 10.5 ms).  The solves
+// gain in tiles wherever those fit (the same two profiles 31 -> 8.8 and 30 -> 1.8 ms).
+static bool sky_tiles_pay(const SkyPlan &L, const int *R, int n, int maxBW, int sms) {
+    double tiles = 0.0;
+    for (const PanelMeta &M : L.meta) {
+        const double b = M.bt, updates = (M.nbc - b) * b * (b + 1) / 2 + (b - 1) * b * (b + 1) / 6;
+        tiles = std::max(tiles, 15.0 * M.nbc + 10.4 * updates / sky_ctas(L, sms));
+    }
+    return tiles <= (sky_threads(maxBW) > 32 ? 4.35 : 1.35) * n + 0.07 * R[n];
+}
+
 // The plan's tables to the device (d_sky[5]) and the tile buffers (d_sky[6], and d_sky[7] for the
 // solves' row-major copy); the profile's row ranges are d_R.
 static int sky_upload(astro_ctx *ctx, const SkyPlan &L, const int *d_R, bool both, SkyPanels &S) {
@@ -621,10 +642,12 @@ static int sky_upload(astro_ctx *ctx, const SkyPlan &L, const int *d_R, bool bot
 static int ldl_fact_dev(astro_ctx *ctx, double *d_A, const int *d_R, const int *h_R, int n) {
     int *st = dptr<int>(ctx->d_status);
     constexpr int kNone = 0x7f7f7f7f;
-    int rc, hs = 0;
+    int rc, hs = 0, sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    const int maxBW = skyline_maxbw(h_R, n);
     SkyPlan L;
     SkyPanels S;
-    bool tiled = sky_plan(h_R, n, L);
+    bool tiled = sky_plan(h_R, n, L) && sky_tiles_pay(L, h_R, n, maxBW, sms);
     if (tiled && (rc = sky_upload(ctx, L, d_R, false, S))) {
         if (rc != ASTRO_ERR_NOMEM) return rc;
         tiled = false;  // no room for the tiles: the row sweep needs none
@@ -632,17 +655,12 @@ static int ldl_fact_dev(astro_ctx *ctx, double *d_A, const int *d_R, const int *
     if (tiled) {
         CK(cudaMemsetAsync(st, 0x7f, sizeof(int), ctx->stream));
         CK(cudaMemsetAsync(st + 1, 0, sizeof(int), ctx->stream));
-        // as many CTAs a panel as its update has tiles, and as the GPU holds for all panels
-        int sms = 0, cs = 1;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-        while (cs < 16 && cs < L.maxBt * (L.maxBt + 1) / 2 && 2 * cs * S.np <= sms) cs *= 2;
         double *tiles = dptr<double>(ctx->d_sky[6]);
         k_sky_tiles<<<(unsigned)L.tiles, kSkyThreads, 0, ctx->stream>>>(S, d_A, tiles, nullptr);
         const int *sched = S.row0 + S.np + 1;
-        CK(band_ldl64(S.meta, sched, sched + S.np, S.np, cs, tiles, st + 1, ctx->stream));
+        CK(band_ldl64(S.meta, sched, sched + S.np, S.np, sky_ctas(L, sms), tiles, st + 1, ctx->stream));
         k_sky_untile<<<(unsigned)L.tiles, kSkyThreads, 0, ctx->stream>>>(S, tiles, d_A, st);
     } else {
-        const int maxBW = skyline_maxbw(h_R, n);
         DevBuf &diag = ctx->d_sky[3], &dl = ctx->d_sky[4];
         if ((rc = sky_scratch(ctx, diag, sizeof(double) * (size_t)(n + 1))) ||
             (rc = sky_scratch(ctx, dl, sizeof(double) * (size_t)(maxBW + 2))))
