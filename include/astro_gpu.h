@@ -609,9 +609,13 @@ int astro_newmark_run_states(astro_ctx *ctx, const astro_newmark_opts *opts, con
  * and keeps the fastest for the context:
  *   ASTRO_TUNE_BRICK_WARPS    the zero-state brick kernel's warps per CTA (1, 2, 4): FP32 assembly
  *                             passes (brick8 meshes; leaves the FP32 assembly resident);
- *   ASTRO_TUNE_PANEL_CLUSTER  the band factorisation's CTAs per cluster (2, 4, 8): one
- *                             astro_panels_factor each (needs the FP64 assembly and the scaled
- *                             constraints); astro_panels_factor with cluster_size 0 then uses it;
+ *   ASTRO_TUNE_PANEL_CLUSTER  the band factorisation's CTAs per cluster (2, 4, 8; 0 where the
+ *                             untuned choice, 16, is the fastest): one astro_panels_factor each
+ *                             (needs the FP64 assembly and the scaled constraints);
+ *                             astro_panels_factor with cluster_size 0 then uses it.  With FP64
+ *                             updates (ASTRO_OPT_BAND_FP64_UPDATE 1) also for the double-float
+ *                             factorisation, whose choice the other kinds of update take; else
+ *                             for the context's kind;
  *   ASTRO_TUNE_CASES_CLUSTER  the many-column band solve's CTAs per cluster (2, 4, 8): solves of
  *                             the factorisation prepared by the last astro_newmark_cases.
  * cache_path (may be NULL): a text file of lines "<key> <choice> <seconds>", the key naming the

@@ -173,7 +173,8 @@ struct astro_ctx {
     int tuneCasesCluster = 0;  // many-column band solve: CTAs per cluster (2, 4, 8)
     int casesTwist = 1;        // ASTRO_OPT_CASES_TWIST
     int panelsSolve = 0;       // ASTRO_OPT_PANELS_SOLVE
-    int tunePanelCluster = 0;  // band factorisation: CTAs per cluster (2, 4, 8)
+    // band factorisation: CTAs per cluster (2, 4, 8), of the FP64 updates and of the other kinds
+    int tunePanelCluster = 0, tunePanelClusterOther = 0;
 };
 
 // error helpers

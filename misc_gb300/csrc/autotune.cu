@@ -109,21 +109,43 @@ extern "C" int astro_autotune(astro_ctx *ctx, int32_t what, const char *cache_pa
         ctx->asmGraph = nullptr;
     }
     if (what & ASTRO_TUNE_PANEL_CLUSTER) {
-        const std::string key = gpu + "/panel_cluster/N" + std::to_string(P.N) + "/nb" + std::to_string(P.nb);
-        int best = 0;
-        if (!cache_find(cache_path, key, &best)) {
-            double bestS = 1e30;
-            for (int cs : {2, 4, 8}) {
-                astro_panels_info info{};
-                if ((rc = astro_panels_factor(ctx, cs, &info))) return rc;
-                if (info.factor_seconds < bestS) {
-                    bestS = info.factor_seconds;
-                    best = cs;
+        // The kinds of update want different clusters (512 panels: FP64 8, double-float and mma.sync 4, 0.52 against
+        // 0.65 s and 1.83 against 2.77 s with 8), and the three that are not FP64, which divide a panel alike,
+        // about the same ones: FP64 and double-float are timed, or the context's own kind when that is not FP64.
+        const int own = ctx->bandFp64Update;
+        auto tune = [&](int kind, int &choice) -> int {
+            const std::string key = gpu + (kind == 1 ? "/panel_cluster_fp64/N" : "/panel_cluster_kind" + std::to_string(kind) + "/N") +
+                                    std::to_string(P.N) + "/nb" + std::to_string(P.nb);
+            int best = 0;
+            if (!cache_find(cache_path, key, &best)) {
+                ctx->bandFp64Update = kind;
+                choice = 0;
+                double bestS = 1e30;
+                int rule = 0, err = ASTRO_OK;
+                for (int cs : {0, 2, 4, 8}) {  // 0: the choice of the rule, 16 perhaps
+                    if (cs && cs == rule) continue;
+                    astro_panels_info info{};
+                    if ((err = astro_panels_factor(ctx, cs, &info))) break;
+                    if (!cs) rule = info.cluster_size;
+                    if (info.factor_seconds < bestS) {
+                        bestS = info.factor_seconds;
+                        best = cs || rule > 8 ? cs : rule;
+                    }
                 }
+                ctx->bandFp64Update = own;
+                if (err) return err;
+                cache_add(cache_path, key, best, bestS);
             }
-            cache_add(cache_path, key, best, bestS);
+            choice = best;
+            return ASTRO_OK;
+        };
+        if (own == 1) {
+            // (a matrix that only FP64 factors: no choice for the others)
+            if (tune(3, ctx->tunePanelClusterOther)) ctx->tunePanelClusterOther = 0;
+            if ((rc = tune(1, ctx->tunePanelCluster))) return rc;
+        } else if ((rc = tune(own, ctx->tunePanelClusterOther))) {
+            return rc;
         }
-        ctx->tunePanelCluster = best;
     }
     if (what & ASTRO_TUNE_CASES_CLUSTER) {
         int np = 0, bw = 0;
@@ -159,7 +181,7 @@ extern "C" int astro_autotune(astro_ctx *ctx, int32_t what, const char *cache_pa
     }
     if (choices) {
         choices[0] = ctx->tuneHex8Warps;
-        choices[1] = ctx->tunePanelCluster;
+        choices[1] = ctx->bandFp64Update == 1 ? ctx->tunePanelCluster : ctx->tunePanelClusterOther;
         choices[2] = ctx->tuneCasesCluster;
     }
     return ASTRO_OK;

@@ -1371,7 +1371,7 @@ extern "C" int astro_set_option(astro_ctx *ctx, int32_t option, int32_t value) {
             ctx->asmExec = nullptr;
             ctx->asmGraph = nullptr;
         } else if (option == ASTRO_OPT_PANEL_CLUSTER) {
-            ctx->tunePanelCluster = value;
+            ctx->tunePanelCluster = ctx->tunePanelClusterOther = value;
         } else {
             ctx->tuneCasesCluster = value;
         }

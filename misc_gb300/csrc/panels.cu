@@ -68,7 +68,7 @@ struct SolveItem {
 struct PanelPlan {
     int np = 0;
     int cs = 0, workers = 0;
-    int csAsked = 0;  // the cluster size the plan was asked for (0: plan_build's choice)
+    int csAsked = 0;  // the cluster size the plan was asked for (0: cluster_rule)
     int factored = 0, kVersion = -1, penVersion = -1;
     int maxBw = 0;
     long long bandDoubles = 0, xRows = 0;
@@ -1917,6 +1917,16 @@ __global__ void k_tw_move(int nc, TwistGeom G, int w, double *__restrict__ vec, 
 constexpr size_t kSolveSmem = sizeof(double) * (kGroups * TB * (TB + 1) + kGroups * TB * (kSolveCols + 1));
 
 // connected components, orderings, bandwidths, storage and the cluster schedule
+// CTAs a panel when none were asked for: 16 (the largest cluster of the hardware) for the FP64 factorisation
+// of few panels, when the GPU holds them all at a CTA per SM and a block column has more tile updates than
+// 8 CTAs (the updates are bound by the FP64 pipes of the panel's own SMs: 64 x 64 plate in two halves,
+// bandwidth 401, 50.8 ms with 8, 26.5 ms with 16); else 8, as for the variants with portable clusters.
+int cluster_rule(const astro_ctx *ctx, const PanelPlan &L) {
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    return ctx->bandFp64Update == 1 && 16 * std::max(L.np, 2) <= sms && L.maxBt >= 4 ? 16 : 8;
+}
+
 int plan_build(astro_ctx *ctx, PanelPlan &L, int cs) {
     const AstroPrep &P = ctx->P;
     const int N = P.N, dpn = P.dpn;
@@ -2018,12 +2028,7 @@ int plan_build(astro_ctx *ctx, PanelPlan &L, int cs) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
     L.csAsked = cs;
-    if (cs == 0)
-        // 16 CTAs a panel (the largest cluster of the hardware) for the FP64 factorisation of few
-        // panels, when the GPU holds them all at a CTA per SM and a block column has more tile
-        // updates than 8 CTAs: the updates are bound by the FP64 pipes of the panel's own SMs.
-        // 64 x 64 plate in two halves, bandwidth 401: 50.8 ms with 8, 26.5 ms with 16.
-        cs = ctx->bandFp64Update == 1 && 16 * std::max(np, 2) <= sms && L.maxBt >= 4 ? 16 : 8;
+    if (cs == 0) cs = cluster_rule(ctx, L);
     // clusters: as many as fit at once, panels by longest processing time first
     L.cs = cs;
     int maxClusters = 0;
@@ -2120,15 +2125,15 @@ void panels_release(astro_ctx *ctx) {
 // (the twisted many-column solve).
 int panels_factor_impl(astro_ctx *ctx, int32_t cluster_size, astro_panels_info *info, int factor) {
     if (!ctx) return ASTRO_ERR_ARG;
-    if (cluster_size == 0) cluster_size = ctx->tunePanelCluster;  // autotuned, or 0: plan_build's choice
+    // autotuned for this kind of update, or 0: cluster_rule
+    if (cluster_size == 0) cluster_size = ctx->bandFp64Update == 1 ? ctx->tunePanelCluster : ctx->tunePanelClusterOther;
     if (cluster_size != 0 && cluster_size != 1 && cluster_size != 2 && cluster_size != 4 && cluster_size != 8)
         return set_err(ctx, ASTRO_ERR_ARG, "panels: cluster_size must be 1, 2, 4 or 8");
     if (!ctx->haveK64) return set_err(ctx, ASTRO_ERR_STATE, "panels: FP64 stiffness not assembled");
     if (ctx->P.mpcDim > 0 && !ctx->mpcScaled)
         return set_err(ctx, ASTRO_ERR_STATE, "panels: constraints not scaled (astro_scale_mpc)");
     PanelPlan *L = static_cast<PanelPlan *>(ctx->panels);
-    // (16 CTAs are for the FP64 updates: the other variants' clusters are of the portable sizes)
-    if (L && ((L->csAsked != cluster_size && L->cs != cluster_size) || (L->cs == 16 && ctx->bandFp64Update != 1))) {
+    if (L && L->cs != (cluster_size ? cluster_size : cluster_rule(ctx, *L))) {
         panels_release(ctx);
         L = nullptr;
     }
