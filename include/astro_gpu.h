@@ -248,7 +248,8 @@ int astro_get_dims(const astro_ctx *ctx, astro_dims *out);
  * as m unrolled Arnoldi steps (kernels that return at once after convergence) instead of
  * conditional graph nodes; the same kernels in the same order, so the results are identical.
  * For profilers that do not look inside conditional nodes, and for drivers without them.
- * (Cycles that run resident on the SMs, one launch each, are the same under both values.) */
+ * (Cycles that run resident on the SMs, one launch each, are the same under both values:
+ * ASTRO_OPT_RESIDENT.) */
 #define ASTRO_OPT_UNROLLED_CYCLES 2
 /* ASTRO_OPT_BAND_FP64_UPDATE (default 1): the band LDL^T of astro_panels_factor (and of
  * astro_newmark_cases) runs its trailing tile updates in FP64 arithmetic; 0 selects the
@@ -284,8 +285,8 @@ int astro_get_dims(const astro_ctx *ctx, astro_dims *out);
  * graphs on small models. */
 #define ASTRO_OPT_RESIDENT 9
 /* ASTRO_OPT_POLL_LIMIT (default 0: about a second): how often a CTA of a kernel whose CTAs exchange data looks
- * for a word of another before it gives up.  A solve whose wait was given up goes on in the form that has no such
- * waits.  For tests of that path; too small a limit costs time, not results. */
+ * for a word of another before it gives up.  A static or thermal solve whose wait was given up goes on in the form
+ * that has no such waits; astro_newmark_cases ends with ASTRO_ERR_CUDA.  For tests of those paths. */
 #define ASTRO_OPT_POLL_LIMIT 10
 /* ASTRO_OPT_FAIL_ALLOC (default 0: none): that one of the context's device allocations to come, counted from 1, is
  * refused with ASTRO_ERR_NOMEM.  For tests of what a call leaves behind and of the paths that need less memory. */
@@ -789,7 +790,8 @@ int astro_read_step_file(const char *path, int32_t num_nodes, int32_t el_mat_dim
 
 /* Measurement hook: the average device time (CUDA events, reps launches after five warm-up
  * launches) of one preconditioner hop on the operator of the last learned solve of this context,
- * and the bytes one hop moves (FP16 block planes, columns, and the hop's vector loads and stores).
+ * by the kernel of the captured graphs (solves that run resident do not launch it), and the bytes one
+ * hop moves (FP16 block planes, columns, and the hop's vector loads and stores).
  * No counterpart in the reference. */
 int astro_precond_time_hop(astro_ctx *ctx, int32_t reps, double *us_per_hop, double *bytes_per_hop);
 

@@ -588,7 +588,7 @@ __device__ void tile_rows(double (*A)[TB + 1], const double (*sL)[TB + 1], int t
 //             thread loads the next item's operands during the current one.
 // One cluster barrier after each.  Bound: the FP64 pipe in the updates (9.5 us a tile and SM), and
 // for a narrow band the chain rows -> first update -> diagonal tile.  32 panels of 8 .. 36 elements a
-// side: 12.1 ms, against 26.1 ms with every CTA factoring the diagonal tile for itself (a division
+// side: 12.5 ms, against 26.1 ms with every CTA factoring the diagonal tile for itself (a division
 // per thread and pivot) and the rows below on consecutive threads of the first CTA; the 64 x 64
 // plate's two halves at 8 CTAs: 50.8 against 70.8 ms.
 __global__ void __launch_bounds__(kThreads, 2) k_band_ldl64(const PanelMeta *__restrict__ meta,
@@ -1919,8 +1919,8 @@ constexpr size_t kSolveSmem = sizeof(double) * (kGroups * TB * (TB + 1) + kGroup
 // connected components, orderings, bandwidths, storage and the cluster schedule
 // CTAs a panel when none were asked for: 16 (the largest cluster of the hardware) for the FP64 factorisation
 // of few panels, when the GPU holds them all at a CTA per SM and a block column has more tile updates than
-// 8 CTAs (the updates are bound by the FP64 pipes of the panel's own SMs: 64 x 64 plate in two halves,
-// bandwidth 401, 50.8 ms with 8, 26.5 ms with 16); else 8, as for the variants with portable clusters.
+// 8 CTAs (the updates are bound by the FP64 pipes of the panel's own SMs: 64 x 64 plate, bandwidth 401,
+// 94 ms with 8, 48 ms with 16); else 8, as for the variants with portable clusters.
 int cluster_rule(const astro_ctx *ctx, const PanelPlan &L) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
@@ -2400,7 +2400,7 @@ static bool twist_wanted(const astro_ctx *ctx, const PanelPlan *L) {
 int panels_cases_would_twist(astro_ctx *ctx) { return twist_wanted(ctx, static_cast<PanelPlan *>(ctx->panels)); }
 
 // Producers' warps of a CTA: sixteen where eight would leave a warp more than the half tile that it loads ahead
-// (25 tiles: 4.1 against 7.8 ms for 17 columns), and a ring that large leaves room for their partials.
+// (25 tiles and four CTAs: 4.1 against 7.8 ms for 17 columns), and a ring that large leaves room for their partials.
 static int cases_pw(const PanelPlan *L, int cs) {
     return 2 * (L->maxBt - 2) > (cs - 1) * 8 && L->ring <= 850 ? 16 : 8;
 }

@@ -136,8 +136,8 @@ __global__ void __launch_bounds__(kT) k_ldl_solve(double *soln, const double *rh
 // panels at the rows it does not cross, each panel is laid out in 32 x 32 band tiles, and the panels
 // run side by side: the factor by the FP64 band LDL^T of the panels (band_ldl64), the solves by one
 // CTA per panel.  What lies outside the profile is zero in the tiles and stays zero.  Factor and solve
-// through the host-buffer entry points: 2,214 rows of at most 11 entries 8.2 -> 0.45 ms, 6,750 rows
-// of 101 55.0 -> 2.9 ms (factor 0.23 and 1.94 ms, solve 0.08 and 0.52 ms on the GPU).
+// through the host-buffer entry points: 2,214 rows of at most 11 entries 8.2 -> 0.46 ms, 6,750 rows
+// of 101 55.0 -> 3.0 ms (factor 0.25 and 2.1 ms, solve 0.08 and 0.52 ms on the GPU).
 constexpr int kSkyThreads = 256;
 
 struct SkyPanels {
