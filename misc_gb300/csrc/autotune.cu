@@ -154,7 +154,8 @@ extern "C" int astro_autotune(astro_ctx *ctx, int32_t what, const char *cache_pa
         panels_shape(ctx, &np, &bw, &bandBytes, &fs);
         const int cols = panels_cases_columns(ctx);
         if (!cols) return set_err(ctx, ASTRO_ERR_STATE, "autotune: no prepared many-column solve (astro_newmark_cases)");
-        const std::string key = gpu + "/cases_cluster/n" + std::to_string(P.n) + "/bw" + std::to_string(bw) + "/cols" +
+        // (a key of the present kernel: choices cached for the one with a cluster barrier a row are not applied)
+        const std::string key = gpu + "/cases_cluster_staged/n" + std::to_string(P.n) + "/bw" + std::to_string(bw) + "/cols" +
                                 std::to_string(cols) + (panels_cases_launches(ctx) == 7 ? "/twisted" : "");
         int best = 0;
         if (!cache_find(cache_path, key, &best)) {

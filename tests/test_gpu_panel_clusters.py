@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from misc_gb300 import model as M
-from misc_gb300.astro import OPT_BAND_FP64_UPDATE, TUNE_PANEL_CLUSTER, AstroGPU
+from misc_gb300.astro import OPT_BAND_FP64_UPDATE, TUNE_CASES_CLUSTER, TUNE_PANEL_CLUSTER, AstroGPU
 
 pytestmark = pytest.mark.gpu
 
@@ -58,3 +58,17 @@ def test_plan_is_kept_when_the_rule_picks_its_cluster():
     assert np.array_equal(g.panels_solve(b)[0], x8)
     assert g.panels_factor(4).cluster_size == 4
     assert np.linalg.norm(g.panels_solve(b)[0] - x8) <= 1e-10 * np.linalg.norm(x8)
+
+
+def test_choices_cached_for_earlier_kernels_are_not_applied(tmp_path):
+    m = M.plate_shell(nx=8, ny=8, lx=1.0, ly=1.0, t=0.01, E=7e10, nu=0.33, rho=2700.0, pressure=0.0, clamp="ss", y0=0.0)
+    cache = tmp_path / "t.txt"
+    for what, then, now in ((TUNE_PANEL_CLUSTER, "/panel_cluster/", "/panel_cluster_fp64/"),
+                            (TUNE_CASES_CLUSTER, "/cases_cluster/", "/cases_cluster_staged/")):
+        g = AstroGPU(m)
+        g.newmark_cases(1e-5, np.eye(g.n)[[200, 230]], np.ones((2, 2)))
+        g.autotune(what, cache)
+        line = [x for x in cache.read_text().splitlines() if now in x][0]
+        cache.write_text(" ".join([line.split()[0].replace(now, then), "4", "0.0"]) + "\n")
+        g.autotune(what, cache)
+        assert any(now in x for x in cache.read_text().splitlines())
