@@ -540,7 +540,7 @@ __device__ __forceinline__ double lane_sum(const double *part, int nparts, size_
 }
 
 // Least squares H y = g (upper triangular j x j), one warp: lane = row (two rows a lane), the columns from
-// the last; a quotient by the reciprocal with one correction, so that the chain per column is four
+// the last; a quotient by the reciprocal with one correction (Markstein), so that the chain per column is four
 // multiply-adds instead of a division (one thread: 128 us a cycle of 50 steps).
 __global__ void k_lsq(GmresCtl *ctl) {
     static_assert(kMaxM <= 64, "two rows a lane");

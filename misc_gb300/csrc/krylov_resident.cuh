@@ -272,7 +272,8 @@ __global__ void __launch_bounds__(kResT, 1) k_gmres_resident(ResArgs<TM, TV> A) 
             for (int q = t; q < nPen; q += kResT) {
                 const int c = A.op.penCol[pen0 + q];
                 pInfo[q] = (HS * find(c / DPN) + c % DPN) | A.op.penRow[pen0 + q] << 24;
-                // hops: as two floats, whose products with a float are added with one rounding to speak of
+                // hops: as two floats, whose products with a float are added with one rounding to speak of (the
+                // FP64 product rounded to a float in all but one of 60 million random pairs)
                 const double v = POLY ? A.hop.penVal[pen0 + q] : A.op.penVal[pen0 + q];
                 if constexpr (POLY) {
                     reinterpret_cast<float2 *>(pVal)[q] = make_float2((float)v, (float)(v - (double)(float)v));
@@ -834,7 +835,7 @@ __global__ void __launch_bounds__(kResT, 1) k_gmres_resident(ResArgs<TM, TV> A) 
         }
         if (sStuck) return;  // (the workers met this barrier on their way out)
     }
-    // ---- least squares and the update of x --------------------------------------------------------------
+    // ---- least squares (as k_lsq) and the update of x ---------------------------------------------------
     if (wid == 0) {
         double g[2], d[2], rc[2];
 #pragma unroll
